@@ -245,8 +245,8 @@ def measured_fma_peaks(lib):
 def binding_roofline(kernels, peaks, peak_kind, fma, precision, mhz):
     """Roofline of the step's dominant kernel against the unit that binds it:
     the tensor pipe (split-precision contraction: bf16 MMA flops over the
-    measured cuBLAS bf16 peak), the FP32 pipe (double-float ring DFTs: FP32
-    instructions of the work model over the measured FP32 FMA instruction
+    measured cuBLAS bf16 peak), the integer multiply-add rate (ring DFTs: the
+    work model's multiply-adds over half the measured FP32 FMA instruction
     rate), the FP64 pipe (FP64 kernels: flops over the measured FP64 FMA
     peak), else HBM (algorithmic bytes over the measured copy bandwidth)."""
     dom = max(kernels, key=lambda c: kernels[c]["ms"])
@@ -259,13 +259,13 @@ def binding_roofline(kernels, peaks, peak_kind, fma, precision, mhz):
         roof = {"bound": "tensor", "unit": "TFLOP/s", "achieved": ach, "peak": peaks.get("bf16_tflops"),
                 "peak_source": f"{peak_kind} (MEASURED_PEAKS.json bf16 burst)",
                 "work": f"{DIGIT_PRODUCTS} bf16 products per FP64-equivalent multiply-add"}
-    elif dom == "ring_dft" and precision == "mixed":
-        ach = kd["flops"] / sec / 1e12  # the timing record carries the model FP32 instruction count
-        roof = {"bound": "fp32", "unit": "Tinst/s", "achieved": ach, "peak": fma["fp32_tflops"] / 2,
-                "peak_source": "measured in this run: FP32 FMA chains on every SM (s2let_gpu_fma_rate), "
-                               "one instruction per FMA",
-                "work": "double-float FP32 instructions of the Bluestein work model (csrc/kernels.cu ring_work)"}
-    elif dom in ("fp64_contraction", "ring_dft"):
+    elif dom == "ring_dft":
+        ach = kd["flops"] / sec / 1e12  # the timing record carries the model multiply-add count
+        roof = {"bound": "int32", "unit": "Tinst/s", "achieved": ach, "peak": fma["fp32_tflops"] / 4,
+                "peak_source": "half the FP32 FMA instruction rate measured in this run (s2let_gpu_fma_rate): the "
+                               "issue rate of a 32 x 32 + 64 multiply-add",
+                "work": "integer multiply-adds of the Bluestein work model (csrc/ring.cu ring_work)"}
+    elif dom == "fp64_contraction":
         ach = kd["flops"] / sec / 1e12
         roof = {"bound": "fp64", "unit": "TFLOP/s", "achieved": ach, "peak": fma["fp64_tflops"],
                 "peak_source": "measured in this run: FP64 FMA chains on every SM (s2let_gpu_fma_rate)"}
@@ -648,7 +648,7 @@ def run_host_call_workload(a, world, rank):
         out.update({
             "metric": "lm2wav+wav2lm maps/s at L=1024, N=4 (drop-in host calls, split precision)",
             "value": 1.0 / res[1][0], "ms_per_step": 1e3 * res[1][0],
-            "dtype": "f64 in/out; double-float contractions and ring DFTs on the FP32 pipe (split precision)",
+            "dtype": "f64 in/out; double-float contractions on the FP32 pipe, 64-bit fixed-point ring DFTs (split precision)",
             "config": {"workload": "one real map's flm, L=1024, N=4, B=2, J_min=2, upsample=0; "
                                    "s2let_analysis_lm2wav_real + s2let_synthesis_wav2lm_real"},
             "fp64_path": {"value": 1.0 / res[0][0], "ms_per_step": 1e3 * res[0][0]},
@@ -839,7 +839,7 @@ def run_recompute_workload(a, world, rank, local):
                       "FP32 storage, split precision, autotuned launch shapes)",
             "value": whole_job_rate(n, world, ms_cfg4 * 1e-3), "ms_per_step": ms_cfg4,
             "per_kernel_ms_per_step": bd_cfg4,
-            "dtype": "f32 storage; double-float recomputed-table contractions and ring DFTs (split precision)",
+            "dtype": "f32 storage; double-float recomputed-table contractions, 64-bit fixed-point ring DFTs (split precision)",
             "config": {"workload": "256 maps, L log-uniform on [64, 512] rounded to even, N in {1,3,5}, "
                                    "spin in {0,2} (spin 0 real, spin 2 complex), B=2, J_min=1, MW, "
                                    "power-law flm; recomputed Wigner tables",
@@ -907,7 +907,7 @@ def run_recompute_workload(a, world, rank, local):
             "metric": "px2wav+wav2px maps/s at L=2048, N=4 (recomputed Wigner tables, split precision)",
             "per_kernel_ms_per_step": bd,
             "value": whole_job_rate(1, world, ms * 1e-3), "ms_per_step": ms,
-            "dtype": "double-float recomputed-table contractions and ring DFTs, FP64 quadrature",
+            "dtype": "double-float recomputed-table contractions, 64-bit fixed-point ring DFTs, FP64 quadrature",
             "fp64_path": {"value": whole_job_rate(1, world, ms64 * 1e-3), "ms_per_step": ms64,
                           "max_rel_err_round_trip": err64, "per_kernel_ms_per_step": bd64},
             "max_rel_err_f_wav_vs_fp64": float(((w - w64).abs().max() / w64.abs().max()).item()),

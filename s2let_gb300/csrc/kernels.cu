@@ -1,16 +1,10 @@
 // Transform kernels, FP64 path.
 //
-//  k_ring      batched Bluestein DFT of rings (length 2bl-1 on MW, 2bl on MWSS
-//              sampling) in shared memory: chirp premultiply, radix-2 DIT FFT of the padded length,
-//              pointwise multiply by the chirp-kernel spectrum, DIF inverse FFT,
-//              chirp postmultiply.  Two real rings share one complex FFT.
 //  k_contract  per-m Legendre/Wigner contraction against the cached d-tables,
 //              tiled through shared memory (table tiles loaded coalesced along
 //              their contiguous axis, coefficient tiles broadcast).
 //  k_gamma_*   DFT over the 2N-1 gamma samples of the rotation group.
 //  k_merge     harmonic tiling merge (lmn -> lm) fused over scales/directions.
-#include <cooperative_groups.h>
-
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -37,516 +31,10 @@ namespace {
 __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
-__device__ __forceinline__ double2 cmulc(double2 a, double2 b) {  // a * conj(b)
-  return make_double2(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y);
-}
 __device__ __forceinline__ double2 conj2(double2 a) { return make_double2(a.x, -a.y); }
 __device__ __forceinline__ double2 add2(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ double2 sub2(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
 __device__ __forceinline__ double2 scl2(double2 a, double s) { return make_double2(a.x * s, a.y * s); }
-__device__ __forceinline__ int brev(int k, int logP) {
-  return logP == 0 ? 0 : (int)(__brev((unsigned)k) >> (32 - logP));
-}
-
-// ---------------------------------------------------------------------------
-// Ring DFT (Bluestein)
-// ---------------------------------------------------------------------------
-
-struct RingArgs {
-  const void *rings;
-  double2 *rings_out;  // inverse: output rings (as double2 or double)
-  int64_t ring_stride;  // between rings of one map
-  int64_t map_stride;   // between maps
-  int rpm;              // rings per map
-  const double2 *spec_in;
-  double2 *spec_out;
-  int64_t spec_stride;      // between spectra of one map
-  int64_t spec_map_stride;  // between maps (spectra of ring r at spec_base(r))
-  int spec_rpm;             // spectra per map
-  int herm;                 // complex inverse: m < 0 taken as conj of m > 0 (real-valued ring)
-  int sw, mlo;
-  int nrings, bl, K, P, logP;
-  const double2 *chirp, *bhat, *tw;
-  const float4 *chirp_df, *bhat_df, *tw_df;
-};
-
-namespace cg = cooperative_groups;
-
-// One launch of ring DFTs fused with the gamma DFT (k_ring_inverse_gamma_df,
-// k_gamma_ring_forward_df): NN <= kFuseMaxNN n-components per ring.
-constexpr int kFuseMaxNN = 8;
-constexpr int kFuseMaxTw = 128;
-struct GammaFuse {
-  const double2 *G;  // synthesis input: spectrum of component k of ring (b, t) at G + b gms + k gks + t W
-  double2 *Gout;     // analysis output, the same addressing (all m from -(bl-1))
-  int64_t gms, gks;
-  int W, nt;
-  int herm_k;  // real signals: the component with n = 0 (m >= 0 stored, at offset bl-1), else -1
-  void *fw;    // gamma slice g of ring (b, t) at fw + b fms + g npx + t K (double, or double2 unless real)
-  int64_t fms, npx;
-  int ng, real;
-  float4 tw[kFuseMaxTw];  // [g NN + k] double-float twiddles with their normalisation
-};
-
-// element offset of ring r (rings of a map are ring_stride apart, maps map_stride)
-__device__ __forceinline__ int64_t ring_base(const RingArgs &a, int r) {
-  return (int64_t)(r / a.rpm) * a.map_stride + (int64_t)(r % a.rpm) * a.ring_stride;
-}
-__device__ __forceinline__ int64_t spec_base(const RingArgs &a, int r) {
-  return (int64_t)(r / a.spec_rpm) * a.spec_map_stride + (int64_t)(r % a.spec_rpm) * a.spec_stride;
-}
-
-// In-place transforms on the shared buffer.
-__device__ void fft_dit(double2 *buf, const double2 *__restrict__ tw, int P, int logP) {
-  for (int s = 1; s <= logP; ++s) {
-    const int half = 1 << (s - 1);
-    for (int i = threadIdx.x; i < P / 2; i += blockDim.x) {
-      const int j = i & (half - 1);
-      const int i0 = ((i >> (s - 1)) << s) + j, i1 = i0 + half;
-      const double2 w = __ldg(&tw[j << (logP - s)]);
-      const double2 u = buf[i0], v = cmul(buf[i1], w);
-      buf[i0] = add2(u, v);
-      buf[i1] = sub2(u, v);
-    }
-    __syncthreads();
-  }
-}
-__device__ void ifft_dif(double2 *buf, const double2 *__restrict__ tw, int P, int logP) {
-  for (int s = logP; s >= 1; --s) {
-    const int half = 1 << (s - 1);
-    for (int i = threadIdx.x; i < P / 2; i += blockDim.x) {
-      const int j = i & (half - 1);
-      const int i0 = ((i >> (s - 1)) << s) + j, i1 = i0 + half;
-      const double2 w = conj2(__ldg(&tw[j << (logP - s)]));
-      const double2 u = buf[i0], v = buf[i1];
-      buf[i0] = add2(u, v);
-      buf[i1] = cmul(sub2(u, v), w);
-    }
-    __syncthreads();
-  }
-}
-
-// Bluestein core: buf holds a_j (bit-reversed positions) on entry; on exit
-// buf[brev(k)] holds P * y_k where y = a (*) chirp-kernel.
-__device__ void bluestein_core(double2 *buf, const RingArgs &a) {
-  __syncthreads();
-  fft_dit(buf, a.tw, a.P, a.logP);
-  for (int k = threadIdx.x; k < a.P; k += blockDim.x) buf[k] = cmul(buf[k], __ldg(&a.bhat[k]));
-  __syncthreads();
-  ifft_dif(buf, a.tw, a.P, a.logP);
-}
-
-template <bool REAL>
-__global__ void __launch_bounds__(512) k_ring_forward(RingArgs a) {
-  extern __shared__ double2 buf[];
-  const int K = a.K, P = a.P, logP = a.logP;
-  const int r0 = REAL ? 2 * blockIdx.x : blockIdx.x;
-  const bool has1 = REAL && (r0 + 1 < a.nrings);
-  for (int j = threadIdx.x; j < P; j += blockDim.x) {
-    double2 z = make_double2(0.0, 0.0);
-    if (j < K) {
-      if (REAL) {
-        z.x = ((const double *)a.rings)[ring_base(a, r0) + j];
-        if (has1) z.y = ((const double *)a.rings)[ring_base(a, r0 + 1) + j];
-      } else {
-        z = ((const double2 *)a.rings)[ring_base(a, r0) + j];
-      }
-      z = cmulc(z, __ldg(&a.chirp[j]));  // x_j conj(c_j)
-    }
-    buf[brev(j, logP)] = z;
-  }
-  bluestein_core(buf, a);
-  const double inv = 1.0 / (double)P;
-  if (!REAL) {
-    double2 *out = a.spec_out + spec_base(a, r0);
-    for (int c = threadIdx.x; c < a.sw; c += blockDim.x) {
-      const int m = a.mlo + c;
-      const int k = ((m % K) + K) % K;
-      out[c] = scl2(cmulc(buf[brev(k, logP)], __ldg(&a.chirp[k])), inv);
-    }
-  } else {
-    double2 *out0 = a.spec_out + spec_base(a, r0);
-    for (int m = threadIdx.x; m < a.sw; m += blockDim.x) {
-      const int km = (K - m) % K;
-      const double2 zm = scl2(cmulc(buf[brev(m, logP)], __ldg(&a.chirp[m])), inv);
-      const double2 zk = scl2(cmulc(buf[brev(km, logP)], __ldg(&a.chirp[km])), inv);
-      const double2 zc = conj2(zk);
-      // A = (Z_m + conj Z_{-m})/2,  B = (Z_m - conj Z_{-m})/(2i)
-      out0[m] = make_double2(0.5 * (zm.x + zc.x), 0.5 * (zm.y + zc.y));
-      if (has1) {
-        const double2 d = sub2(zm, zc);
-        out0[a.spec_stride + m] = make_double2(0.5 * d.y, -0.5 * d.x);
-      }
-    }
-  }
-}
-
-template <bool REAL>
-__global__ void __launch_bounds__(512) k_ring_inverse(RingArgs a) {
-  extern __shared__ double2 buf[];
-  const int K = a.K, P = a.P, logP = a.logP, bl = a.bl;
-  const int r0 = REAL ? 2 * blockIdx.x : blockIdx.x;
-  const bool has1 = REAL && (r0 + 1 < a.nrings);
-  const double2 *s0 = a.spec_in + spec_base(a, r0);
-  for (int j = threadIdx.x; j < P; j += blockDim.x) {
-    double2 z = make_double2(0.0, 0.0);
-    if (j < K) {
-      const int m = (j < bl) ? j : j - K;  // frequency of DFT bin j
-      if (REAL) {
-        const int am = m < 0 ? -m : m;
-        if (am < a.sw) {
-          double2 A = s0[am];
-          double2 B = has1 ? s0[a.spec_stride + am] : make_double2(0.0, 0.0);
-          if (m < 0) {
-            A = conj2(A);
-            B = conj2(B);
-          }
-          z = make_double2(A.x - B.y, A.y + B.x);  // A + i B
-        }
-      } else {
-        const int c = m - a.mlo;
-        if (c >= 0 && c < a.sw)
-          z = s0[c];
-        else if (a.herm && m < 0 && -m - a.mlo < a.sw)
-          z = conj2(s0[-m - a.mlo]);
-      }
-      // inverse DFT = conj(forward(conj z)):  a_j = conj(z_j) conj(c_j)
-      z = conj2(cmul(z, __ldg(&a.chirp[j])));
-    }
-    buf[brev(j, logP)] = z;
-  }
-  bluestein_core(buf, a);
-  const double inv = 1.0 / (double)P;
-  for (int p = threadIdx.x; p < K; p += blockDim.x) {
-    // f_p = conj(conj(c_p) y_p) = c_p conj(y_p)
-    const double2 y = scl2(buf[brev(p, logP)], inv);
-    const double2 f = cmul(__ldg(&a.chirp[p]), conj2(y));
-    if (REAL) {
-      ((double *)a.rings_out)[ring_base(a, r0) + p] = f.x;
-      if (has1) ((double *)a.rings_out)[ring_base(a, r0 + 1) + p] = f.y;
-    } else {
-      a.rings_out[ring_base(a, r0) + p] = f;
-    }
-  }
-}
-
-// ---------------------------------------------------------------------------
-// Ring DFT in double-float arithmetic (split-precision path)
-//
-// Values are unevaluated sums hi + lo of two floats (48-bit significand, unit
-// roundoff 2^-48, error-free transformations of Dekker/Knuth: two-sum,
-// two-product by FMA).  Every operation is an explicit round-to-nearest
-// intrinsic so that no multiply-add is contracted.  The same Bluestein steps
-// as the FP64 kernels run on the FP32 pipe; each ring (pair) is scaled by a
-// power of two first so that the float exponent range never limits accuracy.
-//
-// Sums and products are left unnormalised (no fast-two-sum after the error
-// term is accumulated): hi + lo still equals the value to within the rounding
-// of lo, and |lo| grows by at most ulp(hi)/2 plus the inputs' lo per
-// operation, so after k operations it stays below k 2^-24 of the block's
-// magnitude and its own rounding below k 2^-48.  Normwise this costs about a
-// factor 2 in the error of a 4096-point transform (6.6e-15 -> 1.4e-14, l2,
-// emulated on the CPU) for 22 % fewer FP32 instructions per butterfly; the
-// FP64 widening at the end accepts any hi/lo split.
-// ---------------------------------------------------------------------------
-
-// Stages are paired (radix 2^2): one pass over shared memory and one barrier
-// per two radix-2 stages; a leftover single stage when log2 P is odd.
-//
-// Shared-memory layout: element i of the P = 2^lg point buffer (16-byte
-// complex double-float values, no padding) lives at swz(i) = i ^ X(i), where
-// X(i) XORs bits 3-4 of i into bits 1-2, bits 3-5 into bits 0-2 and bits
-// lg-3..lg-1 into bits 0-2 (the last term only for lg > 6).  X depends only on
-// bits >= 3 and sets only bits 0-2, so swz is a bijection and its own inverse,
-// and it is linear over GF(2): swz(a ^ b) = swz(a) ^ swz(b).  Every access
-// pattern below (bit-reversed scatter and gather, the radix-2^2 passes at every
-// span, stride-4 and linear sweeps) then touches 8 distinct 16-byte bank groups
-// per quarter warp for P >= 256 (checked by enumerating the patterns on the
-// CPU), without the 1/8 padding a skewed layout needs: a 4096-point buffer
-// takes 64 KB, which leaves room in L1 for the twiddle table.
-struct Swz {
-  int top;  // lg - 3 when lg > 6, else 31 (the term vanishes for non-negative i)
-};
-__device__ __forceinline__ Swz swz_of(int logP) { return Swz{logP > 6 ? logP - 3 : 31}; }
-__device__ __forceinline__ int swz(int i, Swz z) {
-  return i ^ ((i >> 2) & 6) ^ ((i >> 3) & 7) ^ ((i >> z.top) & 7);
-}
-__device__ __forceinline__ float4 dc_mul_mi(float4 a) { return make_float4(a.z, a.w, -a.x, -a.y); }  // a * (-i)
-__device__ __forceinline__ float4 dc_mul_pi(float4 a) { return make_float4(-a.z, -a.w, a.x, a.y); }  // a * (+i)
-
-// Read-only table loads with an L1 eviction priority: the twiddle table is
-// read by every pass of every ring on the SM (kept: evict_last); the chirp and
-// the chirp-kernel spectrum are read once per ring (evict_first).
-__device__ __forceinline__ float4 ld_keep(const float4 *p) {
-  float4 v;
-  asm("ld.global.nc.L1::evict_last.v4.f32 {%0, %1, %2, %3}, [%4];"
-      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-      : "l"(p));
-  return v;
-}
-__device__ __forceinline__ float4 ld_once(const float4 *p) {
-  float4 v;
-  asm("ld.global.nc.L1::evict_first.v4.f32 {%0, %1, %2, %3}, [%4];"
-      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-      : "l"(p));
-  return v;
-}
-
-// bit-reversed input, natural output, forward transform (w = e^{-2 pi i k / P}).
-// The input is zero-padded past P/2 (the Bluestein sequences have K <= P/2
-// values), i.e. zero at every odd bit-reversed position, and the first two
-// stages have unit twiddles: that pass is a 4-point DFT of (a0, 0, a2, 0).
-// In every pass the four points p0 + c h (c < 4) differ from p0 only in bits
-// that are zero in p0, so their buffer slots are swz(p0) ^ swz(c h).
-__device__ void fft_dit_df(float4 *buf, const float4 *__restrict__ tw, int P, int logP) {
-  const Swz z = swz_of(logP);
-  for (int i = threadIdx.x; i < P / 4; i += blockDim.x) {
-    const int b = swz(4 * i, z);
-    const float4 a0 = buf[b], a2 = buf[b ^ 2], a2m = dc_mul_mi(a2);
-    buf[b] = dc_add(a0, a2);
-    buf[b ^ 2] = dc_sub(a0, a2);
-    buf[b ^ 1] = dc_add(a0, a2m);
-    buf[b ^ 3] = dc_sub(a0, a2m);
-  }
-  __syncthreads();
-  int s = 3;
-  for (; s + 1 <= logP; s += 2) {
-    const int h = 1 << (s - 1);
-    const int q1 = swz(h, z), q2 = swz(2 * h, z), q3 = swz(3 * h, z);
-    for (int i = threadIdx.x; i < P / 4; i += blockDim.x) {
-      const int jp = i & (h - 1);
-      const int b = swz(((i >> (s - 1)) << (s + 1)) + jp, z);
-      const float4 w1 = ld_keep(&tw[jp << (logP - s)]);
-      const float4 w2 = ld_keep(&tw[jp << (logP - s - 1)]);
-      const float4 a0 = buf[b], a1 = buf[b ^ q1], a2 = buf[b ^ q2], a3 = buf[b ^ q3];
-      const float4 t1 = dc_mul(a1, w1), t3 = dc_mul(a3, w1);
-      const float4 b0 = dc_add(a0, t1), b1 = dc_sub(a0, t1), b2 = dc_add(a2, t3), b3 = dc_sub(a2, t3);
-      const float4 u2 = dc_mul(b2, w2), u3 = dc_mul_mi(dc_mul(b3, w2));
-      buf[b] = dc_add(b0, u2);
-      buf[b ^ q2] = dc_sub(b0, u2);
-      buf[b ^ q1] = dc_add(b1, u3);
-      buf[b ^ q3] = dc_sub(b1, u3);
-    }
-    __syncthreads();
-  }
-  if (s == logP) {
-    const int half = 1 << (s - 1);
-    const int qh = swz(half, z);
-    for (int i = threadIdx.x; i < P / 2; i += blockDim.x) {
-      const int j = i & (half - 1);
-      const int b = swz(((i >> (s - 1)) << s) + j, z);
-      const float4 w = ld_keep(&tw[j << (logP - s)]);
-      const float4 u = buf[b], v = dc_mul(buf[b ^ qh], w);
-      buf[b] = dc_add(u, v);
-      buf[b ^ qh] = dc_sub(u, v);
-    }
-    __syncthreads();
-  }
-}
-// natural input, bit-reversed output, unnormalised inverse transform.  Only
-// the outputs at even bit-reversed positions (natural index < P/2) are
-// produced: the Bluestein result needs K <= P/2 of them.  The last pass has
-// unit twiddles.
-__device__ void ifft_dif_df(float4 *buf, const float4 *__restrict__ tw, int P, int logP) {
-  const Swz z = swz_of(logP);
-  int s = logP;
-  for (; s >= 3; s -= 2) {
-    const int h = 1 << (s - 2);
-    const int q1 = swz(h, z), q2 = swz(2 * h, z), q3 = swz(3 * h, z);
-    for (int i = threadIdx.x; i < P / 4; i += blockDim.x) {
-      const int jp = i & (h - 1);
-      const int b = swz(((i >> (s - 2)) << s) + jp, z);
-      const float4 c2 = ld_keep(&tw[jp << (logP - s)]);
-      const float4 c1 = ld_keep(&tw[jp << (logP - s + 1)]);
-      const float4 a0 = buf[b], a1 = buf[b ^ q1], a2 = buf[b ^ q2], a3 = buf[b ^ q3];
-      const float4 b0 = dc_add(a0, a2), b1 = dc_add(a1, a3);
-      const float4 b2 = dc_mulc(dc_sub(a0, a2), c2), b3 = dc_mul_pi(dc_mulc(dc_sub(a1, a3), c2));
-      buf[b] = dc_add(b0, b1);
-      buf[b ^ q1] = dc_mulc(dc_sub(b0, b1), c1);
-      buf[b ^ q2] = dc_add(b2, b3);
-      buf[b ^ q3] = dc_mulc(dc_sub(b2, b3), c1);
-    }
-    __syncthreads();
-  }
-  if (s == 2) {  // stages 2 and 1, unit twiddles, even outputs only
-    for (int i = threadIdx.x; i < P / 4; i += blockDim.x) {
-      const int b = swz(4 * i, z);
-      const float4 a0 = buf[b], a1 = buf[b ^ 1], a2 = buf[b ^ 2], a3 = buf[b ^ 3];
-      buf[b] = dc_add(dc_add(a0, a2), dc_add(a1, a3));
-      buf[b ^ 2] = dc_add(dc_sub(a0, a2), dc_mul_pi(dc_sub(a1, a3)));
-    }
-    __syncthreads();
-  } else if (s == 1) {
-    for (int i = threadIdx.x; i < P / 2; i += blockDim.x) {
-      const int b = swz(2 * i, z);
-      buf[b] = dc_add(buf[b], buf[b ^ 1]);
-    }
-    __syncthreads();
-  }
-}
-// pointwise product with the chirp-kernel spectrum (every slot, any order)
-__device__ __forceinline__ void kernel_multiply_df(float4 *buf, const float4 *__restrict__ bhat, int P, int logP) {
-  const Swz z = swz_of(logP);
-  for (int k = threadIdx.x; k < P; k += blockDim.x) {
-    const int b = swz(k, z);
-    buf[b] = dc_mul(buf[b], ld_once(&bhat[k]));
-  }
-  __syncthreads();
-}
-// buffer slot of bit-reversed position k
-__device__ __forceinline__ int slot_brev(int k, int logP) { return swz(brev(k, logP), swz_of(logP)); }
-
-// block-wide max of an int (blockDim.x <= 1024)
-__device__ int block_max_int(int v) {
-  __shared__ int redi[32];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) redi[threadIdx.x >> 5] = v;
-  __syncthreads();
-  int m = 0;
-  for (int i = 0; i < (int)((blockDim.x + 31) >> 5); ++i) m = max(m, redi[i]);
-  return m;
-}
-__device__ __forceinline__ int emax2(int m, double2 z) { return max(m, max(exp_field(z.x), exp_field(z.y))); }
-
-template <bool REAL>
-__global__ void __launch_bounds__(512, 3) k_ring_forward_df(RingArgs a) {
-  extern __shared__ float4 bufd[];
-  const int K = a.K, P = a.P, logP = a.logP;
-  const int r0 = REAL ? 2 * blockIdx.x : blockIdx.x;
-  const bool has1 = REAL && (r0 + 1 < a.nrings);
-  int em = 0;
-  for (int j = threadIdx.x; j < K; j += blockDim.x) {
-    if (REAL) {
-      em = max(em, exp_field(((const double *)a.rings)[ring_base(a, r0) + j]));
-      if (has1) em = max(em, exp_field(((const double *)a.rings)[ring_base(a, r0 + 1) + j]));
-    } else {
-      em = emax2(em, ((const double2 *)a.rings)[ring_base(a, r0) + j]);
-    }
-  }
-  const int e = block_scale(block_max_int(em));
-  for (int j = threadIdx.x; j < P; j += blockDim.x) {
-    float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (j < K) {
-      double2 v;
-      if (REAL) {
-        v.x = ((const double *)a.rings)[ring_base(a, r0) + j];
-        v.y = has1 ? ((const double *)a.rings)[ring_base(a, r0 + 1) + j] : 0.0;
-      } else {
-        v = ((const double2 *)a.rings)[ring_base(a, r0) + j];
-      }
-      z = dc_mulc(dc_split(v, e), ld_once(&a.chirp_df[j]));
-    }
-    bufd[slot_brev(j, logP)] = z;
-  }
-  __syncthreads();
-  fft_dit_df(bufd, a.tw_df, P, logP);
-  kernel_multiply_df(bufd, a.bhat_df, P, logP);
-  ifft_dif_df(bufd, a.tw_df, P, logP);
-  const int eo = e - logP;  // undo the ring scaling and the 1/P of the unnormalised transforms
-  if (!REAL) {
-    double2 *out = a.spec_out + spec_base(a, r0);
-    for (int c = threadIdx.x; c < a.sw; c += blockDim.x) {
-      const int m = a.mlo + c;
-      const int k = ((m % K) + K) % K;
-      out[c] = dc_to(dc_mulc(bufd[slot_brev(k, logP)], ld_once(&a.chirp_df[k])), eo);
-    }
-  } else {
-    double2 *out0 = a.spec_out + spec_base(a, r0);
-    for (int m = threadIdx.x; m < a.sw; m += blockDim.x) {
-      const int km = (K - m) % K;
-      const float4 zm = dc_mulc(bufd[slot_brev(m, logP)], ld_once(&a.chirp_df[m]));
-      const float4 zc = dc_conj(dc_mulc(bufd[slot_brev(km, logP)], ld_once(&a.chirp_df[km])));
-      // A = (Z_m + conj Z_{-m})/2,  B = (Z_m - conj Z_{-m})/(2i)
-      const double2 s = dc_to(dc_add(zm, zc), eo - 1);
-      out0[m] = s;
-      if (has1) {
-        const double2 d = dc_to(dc_sub(zm, zc), eo - 1);
-        out0[a.spec_stride + m] = make_double2(d.y, -d.x);
-      }
-    }
-  }
-}
-
-template <bool REAL>
-__global__ void __launch_bounds__(512, 3) k_ring_inverse_df(RingArgs a) {
-  extern __shared__ float4 bufd[];
-  const int K = a.K, P = a.P, logP = a.logP, bl = a.bl;
-  const int r0 = REAL ? 2 * blockIdx.x : blockIdx.x;
-  const bool has1 = REAL && (r0 + 1 < a.nrings);
-  const double2 *s0 = a.spec_in + spec_base(a, r0);
-  int em = 0;
-  for (int c = threadIdx.x; c < a.sw; c += blockDim.x) {
-    em = emax2(em, s0[c]);
-    if (has1) em = emax2(em, s0[a.spec_stride + c]);
-  }
-  const int e = block_scale(block_max_int(em));
-  for (int j = threadIdx.x; j < P; j += blockDim.x) {
-    float4 zz = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (j < K) {
-      const int m = (j < bl) ? j : j - K;
-      if (REAL) {
-        const int am = m < 0 ? -m : m;
-        if (am < a.sw) {
-          float4 A = dc_split(s0[am], e);
-          float4 B = has1 ? dc_split(s0[a.spec_stride + am], e) : make_float4(0.f, 0.f, 0.f, 0.f);
-          if (m < 0) {
-            A = dc_conj(A);
-            B = dc_conj(B);
-          }
-          // A + i B
-          zz = dmk(df_add(dre(A), df_neg(dim_(B))), df_add(dim_(A), dre(B)));
-        }
-      } else {
-        const int c = m - a.mlo;
-        if (c >= 0 && c < a.sw)
-          zz = dc_split(s0[c], e);
-        else if (a.herm && m < 0 && -m - a.mlo < a.sw)
-          zz = dc_conj(dc_split(s0[-m - a.mlo], e));
-      }
-    }
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    // inverse DFT = conj(forward(conj z)):  a_j = conj(z_j) conj(c_j)
-    if (j < K) v = dc_conj(dc_mul(zz, ld_once(&a.chirp_df[j])));
-    bufd[slot_brev(j, logP)] = v;
-  }
-  __syncthreads();
-  fft_dit_df(bufd, a.tw_df, P, logP);
-  kernel_multiply_df(bufd, a.bhat_df, P, logP);
-  ifft_dif_df(bufd, a.tw_df, P, logP);
-  const int eo = e - logP;
-  for (int p = threadIdx.x; p < K; p += blockDim.x) {
-    // f_p = c_p conj(y_p)
-    const double2 f = dc_to(dc_mul(ld_once(&a.chirp_df[p]), dc_conj(bufd[slot_brev(p, logP)])), eo);
-    if (REAL) {
-      ((double *)a.rings_out)[ring_base(a, r0) + p] = f.x;
-      if (has1) ((double *)a.rings_out)[ring_base(a, r0 + 1) + p] = f.y;
-    } else {
-      a.rings_out[ring_base(a, r0) + p] = f;
-    }
-  }
-}
-
-RingArgs ring_args(const RingFFT &rf, int bl, int nrings) {
-  RingArgs a{};
-  a.spec_rpm = 1 << 30;  // single-level spectrum addressing unless set
-  a.spec_map_stride = 0;
-  a.K = rf.K;
-  a.P = rf.P;
-  a.logP = rf.logP;
-  a.bl = bl;
-  a.nrings = nrings;
-  a.chirp = rf.chirp;
-  a.bhat = rf.bhat;
-  a.tw = rf.tw;
-  a.chirp_df = rf.chirp_df;
-  a.bhat_df = rf.bhat_df;
-  a.tw_df = rf.tw_df;
-  return a;
-}
-
-int ring_threads(int P) { return P / 2 >= 512 ? 512 : (P / 2 >= 32 ? P / 2 : 32); }
 
 // ---------------------------------------------------------------------------
 // Contractions
@@ -1480,205 +968,6 @@ __global__ void k_gamma_px_anal_df(const void *__restrict__ in, int64_t in_ms, d
 }
 
 // ---------------------------------------------------------------------------
-// Ring DFTs and gamma DFT in one launch (split-precision path)
-//
-// The n-components F_k(t, p) (k < NN) of one theta-ring are transformed by a
-// thread-block cluster of NN CTAs, one per component, each with the padded
-// Bluestein buffer of the single-ring kernels (3 CTAs per SM, as there).  The
-// gamma DFT exchanges values between the components of a pixel through
-// distributed shared memory, so the n-components never go to HBM:
-//   synthesis: each CTA runs the inverse ring DFT of its component and leaves
-//              F_k(p) (double-float) in its buffer; after a cluster barrier
-//              each CTA computes the gamma slices f_g(p) of its share of the
-//              pixels from all NN buffers and writes them to f_wav.
-//   analysis:  each CTA reads the gamma slices of its share of the pixels,
-//              forms every component F_k(p), premultiplies by the chirp and
-//              stores it into CTA k's buffer; after a cluster barrier each CTA
-//              runs the forward ring DFT of its component and writes its
-//              spectrum.
-// One power-of-two scale per ring, the largest over the cluster (exchanged
-// through shared memory before the transforms), so the components combine
-// without rescaling.
-// ---------------------------------------------------------------------------
-
-__device__ __forceinline__ int cluster_max_int(cg::cluster_group &cl, int *slot, int v, int nn) {
-  const int m = block_max_int(v);
-  if (threadIdx.x == 0) *slot = m;
-  cl.sync();
-  int r = 0;
-  for (int j = 0; j < nn; ++j) r = max(r, *cl.map_shared_rank(slot, j));
-  return r;
-}
-
-template <int NN, bool REAL>
-__global__ void __launch_bounds__(512, 3) k_ring_inverse_gamma_df(RingArgs a, GammaFuse gf) {
-  extern __shared__ float4 bufd[];
-  __shared__ int s_em, s_e;
-  cg::cluster_group cl = cg::this_cluster();
-  const int k = (int)cl.block_rank();
-  const int r = blockIdx.x / NN;
-  const int b = r / gf.nt, t = r - b * gf.nt;
-  const int K = a.K, P = a.P, logP = a.logP, bl = a.bl;
-  const bool herm = (k == gf.herm_k);
-  const int sw = herm ? bl : gf.W, mlo = herm ? 0 : -(bl - 1);
-  const double2 *s0 = gf.G + (int64_t)b * gf.gms + (int64_t)k * gf.gks + (int64_t)t * gf.W + (herm ? bl - 1 : 0);
-  int em = 0;
-  for (int c = threadIdx.x; c < sw; c += blockDim.x) em = emax2(em, s0[c]);
-  const int e = block_scale(cluster_max_int(cl, &s_em, em, NN));
-  if (threadIdx.x == 0) s_e = e;  // read back after the transforms: fewer live registers in them
-  for (int j = threadIdx.x; j < P; j += blockDim.x) {
-    float4 zz = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (j < K) {
-      const int m = (j < bl) ? j : j - K;
-      const int c = m - mlo;
-      if (c >= 0 && c < sw)
-        zz = dc_split(s0[c], e);
-      else if (herm && m < 0 && -m < sw)
-        zz = dc_conj(dc_split(s0[-m], e));
-      zz = dc_conj(dc_mul(zz, ld_once(&a.chirp_df[j])));
-    }
-    bufd[slot_brev(j, logP)] = zz;
-  }
-  __syncthreads();
-  fft_dit_df(bufd, a.tw_df, P, logP);
-  kernel_multiply_df(bufd, a.bhat_df, P, logP);
-  ifft_dif_df(bufd, a.tw_df, P, logP);
-  // F_k(p) = c_p conj(y_p), in place (p -> brev(p) is one-to-one)
-  for (int p = threadIdx.x; p < K; p += blockDim.x) {
-    const int i = slot_brev(p, logP);
-    bufd[i] = dc_mul(ld_once(&a.chirp_df[p]), dc_conj(bufd[i]));
-  }
-  cl.sync();
-  // gamma slices of this CTA's share of the pixels
-  const int eo = s_e - logP;
-  const int kk = (int)cl.block_rank(), rr = blockIdx.x / NN;
-  const int bb = rr / gf.nt, tt = rr - bb * gf.nt;
-  const int chunk = (K + NN - 1) / NN;
-  const int p1 = min(K, (kk + 1) * chunk);
-  const int64_t obase = (int64_t)bb * gf.fms + (int64_t)tt * K;
-  // gamma_g and gamma_{ng-g} have conjugate twiddles: with w = C + i S,
-  //   real:    f_g = A - B, f_{ng-g} = A + B, A = sum_k C Re z_k, B = sum_k S Im z_k
-  //   complex: f_g = U + i V, f_{ng-g} = U - i V, U = sum_k C z_k, V = sum_k S z_k
-  for (int p = kk * chunk + threadIdx.x; p < p1; p += blockDim.x) {
-    const int i = slot_brev(p, logP);
-    float4 z[NN];
-#pragma unroll
-    for (int j = 0; j < NN; ++j) z[j] = *cl.map_shared_rank(bufd + i, j);
-    for (int g = 0; 2 * g <= gf.ng; ++g) {
-      const int g2 = gf.ng - g;  // the conjugate partner (g = 0 and g2 == g have none)
-      const int64_t o = obase + (int64_t)g * gf.npx + p, o2 = obase + (int64_t)g2 * gf.npx + p;
-      const bool pair = g > 0 && g2 != g;
-      if (REAL) {
-        float2 A = make_float2(0.f, 0.f), B = make_float2(0.f, 0.f);
-#pragma unroll
-        for (int j = 0; j < NN; ++j) {
-          const float4 w = gf.tw[g * NN + j];
-          A = df_add(A, df_mul(dre(w), dre(z[j])));
-          B = df_add(B, df_mul(dim_(w), dim_(z[j])));
-        }
-        const float2 f1 = df_add(A, df_neg(B));
-        ((double *)gf.fw)[o] = join_scaled(f1.x, f1.y, eo);
-        if (pair) {
-          const float2 f2 = df_add(A, B);
-          ((double *)gf.fw)[o2] = join_scaled(f2.x, f2.y, eo);
-        }
-      } else {
-        float4 U = make_float4(0.f, 0.f, 0.f, 0.f), V = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int j = 0; j < NN; ++j) {
-          const float4 w = gf.tw[g * NN + j];
-          U = dmk(df_add(dre(U), df_mul(dre(w), dre(z[j]))), df_add(dim_(U), df_mul(dre(w), dim_(z[j]))));
-          V = dmk(df_add(dre(V), df_mul(dim_(w), dre(z[j]))), df_add(dim_(V), df_mul(dim_(w), dim_(z[j]))));
-        }
-        const float4 iV = dc_mul_pi(V);
-        const float4 f1 = dc_add(U, iV);
-        ((double2 *)gf.fw)[o] = dc_to(f1, eo);
-        if (pair) ((double2 *)gf.fw)[o2] = dc_to(dc_sub(U, iV), eo);
-      }
-    }
-  }
-  cl.sync();  // peers read this buffer until here
-}
-
-template <int NN, bool REAL>
-__global__ void __launch_bounds__(512, 3) k_gamma_ring_forward_df(RingArgs a, GammaFuse gf) {
-  extern __shared__ float4 bufd[];
-  __shared__ int s_em, s_e;
-  cg::cluster_group cl = cg::this_cluster();
-  const int k = (int)cl.block_rank();
-  const int r = blockIdx.x / NN;
-  const int b = r / gf.nt, t = r - b * gf.nt;
-  const int K = a.K, P = a.P, logP = a.logP;
-  const int chunk = (K + NN - 1) / NN;
-  const int p0 = k * chunk, p1 = min(K, p0 + chunk);
-  const int64_t ibase = (int64_t)b * gf.fms + (int64_t)t * K;
-  int em = 0;
-  for (int p = p0 + threadIdx.x; p < p1; p += blockDim.x)
-    for (int g = 0; g < gf.ng; ++g) {
-      const int64_t o = ibase + (int64_t)g * gf.npx + p;
-      if (REAL)
-        em = max(em, exp_field(((const double *)gf.fw)[o]));
-      else
-        em = emax2(em, ((const double2 *)gf.fw)[o]);
-    }
-  const int e = block_scale(cluster_max_int(cl, &s_em, em, NN));
-  if (threadIdx.x == 0) s_e = e;  // read back after the transforms: fewer live registers in them
-  // the zero padding of this CTA's own buffer
-  for (int j = K + threadIdx.x; j < P; j += blockDim.x) bufd[slot_brev(j, logP)] = make_float4(0.f, 0.f, 0.f, 0.f);
-  // gamma_g and gamma_{ng-g} have conjugate twiddles w = C + i S and C - i S:
-  // each pair contributes C (f_g + f_{ng-g}) + i S (f_g - f_{ng-g})
-  for (int p = p0 + threadIdx.x; p < p1; p += blockDim.x) {
-    float4 acc[NN];
-#pragma unroll
-    for (int j = 0; j < NN; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int g = 0; 2 * g <= gf.ng; ++g) {
-      const int g2 = gf.ng - g;
-      const bool pair = g > 0 && g2 != g;
-      const int64_t o = ibase + (int64_t)g * gf.npx + p, o2 = ibase + (int64_t)g2 * gf.npx + p;
-      if (REAL) {
-        const float2 fa = df_split(((const double *)gf.fw)[o], e);
-        const float2 fb = pair ? df_split(((const double *)gf.fw)[o2], e) : make_float2(0.f, 0.f);
-        const float2 Pp = df_add(fa, fb), Q = df_add(fa, df_neg(fb));
-#pragma unroll
-        for (int j = 0; j < NN; ++j) {
-          const float4 w = gf.tw[g * NN + j];
-          acc[j] = dmk(df_add(dre(acc[j]), df_mul(dre(w), Pp)), df_add(dim_(acc[j]), df_mul(dim_(w), Q)));
-        }
-      } else {
-        const float4 fa = dc_split(((const double2 *)gf.fw)[o], e);
-        const float4 fb = pair ? dc_split(((const double2 *)gf.fw)[o2], e) : make_float4(0.f, 0.f, 0.f, 0.f);
-        const float4 Pp = dc_add(fa, fb), Q = dc_sub(fa, fb);
-#pragma unroll
-        for (int j = 0; j < NN; ++j) {
-          const float4 w = gf.tw[g * NN + j];
-          // C P + i S Q
-          const float2 re = df_add(df_mul(dre(w), dre(Pp)), df_neg(df_mul(dim_(w), dim_(Q))));
-          const float2 im = df_add(df_mul(dre(w), dim_(Pp)), df_mul(dim_(w), dre(Q)));
-          acc[j] = dc_add(acc[j], dmk(re, im));
-        }
-      }
-    }
-    const float4 ch = ld_once(&a.chirp_df[p]);
-    const int i = slot_brev(p, logP);
-#pragma unroll
-    for (int j = 0; j < NN; ++j) *cl.map_shared_rank(bufd + i, j) = dc_mulc(acc[j], ch);
-  }
-  cl.sync();  // every component's buffer is complete
-  fft_dit_df(bufd, a.tw_df, P, logP);
-  kernel_multiply_df(bufd, a.bhat_df, P, logP);
-  ifft_dif_df(bufd, a.tw_df, P, logP);
-  const int eo = s_e - logP;
-  const int kk = (int)cl.block_rank(), rr = blockIdx.x / NN;
-  const int bb = rr / gf.nt, tt = rr - bb * gf.nt;
-  double2 *out = gf.Gout + (int64_t)bb * gf.gms + (int64_t)kk * gf.gks + (int64_t)tt * gf.W;
-  for (int c = threadIdx.x; c < gf.W; c += blockDim.x) {
-    const int m = c - (a.bl - 1);
-    const int q = ((m % K) + K) % K;
-    out[c] = dc_to(dc_mulc(bufd[slot_brev(q, logP)], ld_once(&a.chirp_df[q])), eo);
-  }
-}
-
-// ---------------------------------------------------------------------------
 // lmn -> lm merge
 // ---------------------------------------------------------------------------
 
@@ -1769,312 +1058,6 @@ __global__ void k_axpby(const double *x, int64_t xs, double *y, int64_t ys, int6
 // ===========================================================================
 // wrappers
 // ===========================================================================
-
-namespace {
-
-// Shared memory of the ring kernels: one P-point buffer of 16-byte values.
-// The double-float kernels (3 CTAs per SM) ask for a carveout just large
-// enough for three buffers, so that the rest of the SM's L1 keeps the twiddle
-// table (32 KB at P = 4096).
-void ring_smem_attrs(const void *kernel, size_t smem, bool df) {
-  if (smem > 48 * 1024) S2G_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  if (df) {
-    constexpr double kMaxSmemPerSm = 228.0 * 1024.0;
-    const int pct = std::min(100, (int)std::ceil(100.0 * 3.0 * (double)(smem + 2048) / kMaxSmemPerSm) + 1);
-    S2G_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, pct));
-  }
-}
-
-template <class KF>
-void launch_ring(KF kernel, const RingArgs &a, int nblk, int P, cudaStream_t st, bool df = false) {
-  const size_t smem = sizeof(double2) * (size_t)P;
-  ring_smem_attrs((const void *)kernel, smem, df);
-  kernel<<<nblk, ring_threads(P), smem, st>>>(a);
-  S2G_LAUNCHED();
-}
-
-// Work model of one Bluestein transform of padded length P (for the timing
-// report): the split path counts double-float FP32 instructions (32 per
-// element per radix-2 stage and FFT with unnormalised adds of 8 and complex
-// multiplies of 32 instructions, less the pruned first and last passes; 32
-// for the kernel-spectrum multiply and 64 K / P for the two chirps); the FP64
-// path counts 5 P log2 P flop per FFT.
-double ring_work(const RingArgs &a, int nblk) {
-  const double P = a.P, lg = a.logP;
-  if (t_precision == 1) return (double)nblk * P * (64.0 * lg - 56.0 + 64.0 * a.K / P);
-  return (double)nblk * (10.0 * P * lg + 6.0 * P + 12.0 * a.K);
-}
-
-void run_ring_forward(const RingArgs &a, int nrings, bool real, cudaStream_t st) {
-  const int nblk = real ? (nrings + 1) / 2 : nrings;
-  KTimer kt(KC_RING, st, timing_enabled() ? ring_work(a, nblk) : 0.0,
-            (double)nrings * a.K * (real ? 8.0 : 16.0) + (double)nrings * a.sw * 16.0);
-  if (t_precision == 1) {
-    if (real)
-      launch_ring(k_ring_forward_df<true>, a, nblk, a.P, st, true);
-    else
-      launch_ring(k_ring_forward_df<false>, a, nblk, a.P, st, true);
-  } else if (real) {
-    launch_ring(k_ring_forward<true>, a, nblk, a.P, st);
-  } else {
-    launch_ring(k_ring_forward<false>, a, nblk, a.P, st);
-  }
-}
-
-void run_ring_inverse(const RingArgs &a, int nrings, bool real, cudaStream_t st) {
-  const int nblk = real ? (nrings + 1) / 2 : nrings;
-  KTimer kt(KC_RING, st, timing_enabled() ? ring_work(a, nblk) : 0.0,
-            (double)nrings * a.K * (real ? 8.0 : 16.0) + (double)nrings * a.sw * 16.0);
-  if (t_precision == 1) {
-    if (real)
-      launch_ring(k_ring_inverse_df<true>, a, nblk, a.P, st, true);
-    else
-      launch_ring(k_ring_inverse_df<false>, a, nblk, a.P, st, true);
-  } else if (real) {
-    launch_ring(k_ring_inverse<true>, a, nblk, a.P, st);
-  } else {
-    launch_ring(k_ring_inverse<false>, a, nblk, a.P, st);
-  }
-}
-
-// Twiddles of the fused gamma DFT: synthesis c e^{i n_k gamma_g} (x2 for
-// n_k != 0 on real signals, which stand for the +-n pair), analysis
-// c e^{-i n_k gamma_g}; gamma_g = 2 pi g / ng, as double-float pairs.
-void fuse_twiddles(GammaFuse &gf, const std::vector<int> &ns, int ng, bool real, double c, bool synth) {
-  const int nn = (int)ns.size();
-  for (int g = 0; g < ng; ++g)
-    for (int k = 0; k < nn; ++k) {
-      const long double x = 2.0L * (long double)((ns[k] * g) % ng) / (long double)ng;  // angle / pi
-      const long double pi = 3.141592653589793238462643383279502884L;
-      const double f = synth ? ((real && ns[k] != 0) ? 2.0 * c : c) : c;
-      const double re = (double)(f * cosl(pi * x)), im = (double)((synth ? f : -f) * sinl(pi * x));
-      const float rh = (float)re, ih = (float)im;
-      gf.tw[g * nn + k] = make_float4(rh, (float)(re - (double)rh), ih, (float)(im - (double)ih));
-    }
-}
-
-template <class KF>
-void launch_fused(KF kernel, const RingArgs &a, const GammaFuse &gf, int nrings, int nn, cudaStream_t st) {
-  const size_t smem = sizeof(float4) * (size_t)a.P;
-  ring_smem_attrs((const void *)kernel, smem, true);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(nrings * nn));
-  cfg.blockDim = dim3(ring_threads(a.P));
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = (unsigned)nn;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  S2G_CUDA(cudaLaunchKernelEx(&cfg, kernel, a, gf));
-  S2G_LAUNCHED();
-}
-
-}  // namespace
-
-namespace {
-// Whether a cluster of nn CTAs of the fused kernels (P-point buffers) can be
-// resident on this GPU: asked once per (nn, P) of the device in use.
-bool cluster_fits(int nn, int P) {
-  static std::mutex mu;
-  static std::map<std::pair<int, int>, bool> known;
-  std::lock_guard<std::mutex> lk(mu);
-  const auto key = std::make_pair(nn, P);
-  auto it = known.find(key);
-  if (it != known.end()) return it->second;
-  const void *kern = nullptr;
-  switch (nn) {
-    case 2: kern = (const void *)k_ring_inverse_gamma_df<2, false>; break;
-    case 3: kern = (const void *)k_ring_inverse_gamma_df<3, false>; break;
-    case 4: kern = (const void *)k_ring_inverse_gamma_df<4, false>; break;
-    case 5: kern = (const void *)k_ring_inverse_gamma_df<5, false>; break;
-    case 6: kern = (const void *)k_ring_inverse_gamma_df<6, false>; break;
-    case 7: kern = (const void *)k_ring_inverse_gamma_df<7, false>; break;
-    default: kern = (const void *)k_ring_inverse_gamma_df<8, false>; break;
-  }
-  const size_t smem = sizeof(float4) * (size_t)P;
-  ring_smem_attrs(kern, smem, true);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)nn);
-  cfg.blockDim = dim3(ring_threads(P));
-  cfg.dynamicSmemBytes = smem;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = (unsigned)nn;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  int nclusters = 0;
-  const cudaError_t e = cudaOccupancyMaxActiveClusters(&nclusters, kern, &cfg);
-  if (e != cudaSuccess) cudaGetLastError();  // a refusal only means: not fusable here
-  const bool ok = e == cudaSuccess && nclusters > 0;
-  known[key] = ok;
-  return ok;
-}
-}  // namespace
-
-bool ring_gamma_fusable(int nn, int ng, int bl, int ss) {
-  if (t_precision != 1 || nn < 2 || nn > kFuseMaxNN || ng * nn > kFuseMaxTw) return false;
-  return cluster_fits(nn, ring_fft(grid_ring_len(bl, ss)).P);
-}
-
-void ring_inverse_gamma(const double2 *G, int64_t gms, int64_t gks, const std::vector<int> &ns, int ng, bool real,
-                        double c, void *fw, int64_t fms, int nb, int bl, int ss, cudaStream_t st) {
-  const int nn = (int)ns.size();
-  S2G_REQUIRE(ring_gamma_fusable(nn, ng, bl, ss), ERR_UNSUPPORTED, "fused ring/gamma DFT: unsupported shape");
-  const int nt = grid_rings(bl, ss), nrings = nb * nt;
-  if (nrings <= 0) return;
-  const RingFFT &rf = ring_fft(grid_ring_len(bl, ss));
-  RingArgs a = ring_args(rf, bl, nrings);
-  GammaFuse gf{};
-  gf.G = G;
-  gf.gms = gms;
-  gf.gks = gks;
-  gf.W = 2 * bl - 1;
-  gf.nt = nt;
-  gf.herm_k = -1;
-  for (int k = 0; k < nn; ++k)
-    if (real && ns[k] == 0) gf.herm_k = k;
-  gf.fw = fw;
-  gf.fms = fms;
-  gf.npx = (int64_t)nt * a.K;
-  gf.ng = ng;
-  gf.real = real ? 1 : 0;
-  fuse_twiddles(gf, ns, ng, real, c, true);
-  const double px = (double)nrings * a.K;
-  KTimer kt(KC_RING, st, timing_enabled() ? ring_work(a, nrings * nn) + px * ng * nn * (real ? 24.0 : 48.0) : 0.0,
-            (double)nrings * nn * gf.W * 16.0 + px * ng * (real ? 8.0 : 16.0));
-  switch (nn) {
-#define S2G_FUSE(N)                                                              \
-  case N:                                                                        \
-    if (real)                                                                    \
-      launch_fused(k_ring_inverse_gamma_df<N, true>, a, gf, nrings, N, st);     \
-    else                                                                         \
-      launch_fused(k_ring_inverse_gamma_df<N, false>, a, gf, nrings, N, st);    \
-    break;
-    S2G_FUSE(2) S2G_FUSE(3) S2G_FUSE(4) S2G_FUSE(5) S2G_FUSE(6) S2G_FUSE(7) S2G_FUSE(8)
-#undef S2G_FUSE
-    default: break;
-  }
-}
-
-void gamma_ring_forward(const void *fw, int64_t fms, const std::vector<int> &ns, int ng, bool real, double c,
-                        double2 *Gout, int64_t gms, int64_t gks, int nb, int bl, int ss, cudaStream_t st) {
-  const int nn = (int)ns.size();
-  S2G_REQUIRE(ring_gamma_fusable(nn, ng, bl, ss), ERR_UNSUPPORTED, "fused ring/gamma DFT: unsupported shape");
-  const int nt = grid_rings(bl, ss), nrings = nb * nt;
-  if (nrings <= 0) return;
-  const RingFFT &rf = ring_fft(grid_ring_len(bl, ss));
-  RingArgs a = ring_args(rf, bl, nrings);
-  GammaFuse gf{};
-  gf.Gout = Gout;
-  gf.gms = gms;
-  gf.gks = gks;
-  gf.W = 2 * bl - 1;
-  gf.nt = nt;
-  gf.herm_k = -1;
-  gf.fw = const_cast<void *>(fw);
-  gf.fms = fms;
-  gf.npx = (int64_t)nt * a.K;
-  gf.ng = ng;
-  gf.real = real ? 1 : 0;
-  fuse_twiddles(gf, ns, ng, real, c, false);
-  const double px = (double)nrings * a.K;
-  KTimer kt(KC_RING, st, timing_enabled() ? ring_work(a, nrings * nn) + px * ng * nn * (real ? 24.0 : 48.0) : 0.0,
-            (double)nrings * nn * gf.W * 16.0 + px * ng * (real ? 8.0 : 16.0));
-  switch (nn) {
-#define S2G_FUSE(N)                                                              \
-  case N:                                                                        \
-    if (real)                                                                    \
-      launch_fused(k_gamma_ring_forward_df<N, true>, a, gf, nrings, N, st);     \
-    else                                                                         \
-      launch_fused(k_gamma_ring_forward_df<N, false>, a, gf, nrings, N, st);    \
-    break;
-    S2G_FUSE(2) S2G_FUSE(3) S2G_FUSE(4) S2G_FUSE(5) S2G_FUSE(6) S2G_FUSE(7) S2G_FUSE(8)
-#undef S2G_FUSE
-    default: break;
-  }
-}
-
-namespace {
-
-}  // namespace
-
-void ring_forward(const void *rings, int64_t ring_stride, int64_t map_stride, int rpm, double2 *spec,
-                  int64_t spec_stride, int sw, int mlo, int nrings, int bl, int ss, bool real, cudaStream_t st) {
-  if (nrings <= 0) return;
-  const RingFFT &rf = ring_fft(grid_ring_len(bl, ss));
-  RingArgs a = ring_args(rf, bl, nrings);
-  a.rings = rings;
-  a.ring_stride = ring_stride;
-  a.map_stride = map_stride;
-  a.rpm = rpm;
-  a.spec_out = spec;
-  a.spec_stride = spec_stride;
-  a.sw = sw;
-  a.mlo = mlo;
-  run_ring_forward(a, nrings, real, st);
-}
-
-void ring_inverse(const double2 *spec, int64_t spec_stride, int sw, int mlo, void *rings,
-                  int64_t ring_stride, int64_t map_stride, int rpm, int nrings, int bl, int ss, bool real,
-                  cudaStream_t st) {
-  if (nrings <= 0) return;
-  const RingFFT &rf = ring_fft(grid_ring_len(bl, ss));
-  RingArgs a = ring_args(rf, bl, nrings);
-  a.spec_in = spec;
-  a.spec_stride = spec_stride;
-  a.sw = sw;
-  a.mlo = mlo;
-  a.rings_out = (double2 *)rings;
-  a.ring_stride = ring_stride;
-  a.map_stride = map_stride;
-  a.rpm = rpm;
-  run_ring_inverse(a, nrings, real, st);
-}
-
-void ring_forward_c(const double2 *rings, int64_t ring_stride, int64_t map_stride, int rpm, double2 *spec,
-                    int64_t spec_stride, int64_t spec_map_stride, int spec_rpm, int sw, int mlo, int nrings, int bl,
-                    int ss, cudaStream_t st) {
-  if (nrings <= 0) return;
-  const RingFFT &rf = ring_fft(grid_ring_len(bl, ss));
-  RingArgs a = ring_args(rf, bl, nrings);
-  a.rings = rings;
-  a.ring_stride = ring_stride;
-  a.map_stride = map_stride;
-  a.rpm = rpm;
-  a.spec_out = spec;
-  a.spec_stride = spec_stride;
-  a.spec_map_stride = spec_map_stride;
-  a.spec_rpm = spec_rpm;
-  a.sw = sw;
-  a.mlo = mlo;
-  run_ring_forward(a, nrings, false, st);
-}
-
-void ring_inverse_c(const double2 *spec, int64_t spec_stride, int64_t spec_map_stride, int spec_rpm, int sw,
-                    int mlo, bool herm, double2 *rings, int64_t ring_stride, int64_t map_stride, int rpm, int nrings,
-                    int bl, int ss, cudaStream_t st) {
-  if (nrings <= 0) return;
-  const RingFFT &rf = ring_fft(grid_ring_len(bl, ss));
-  RingArgs a = ring_args(rf, bl, nrings);
-  a.spec_in = spec;
-  a.spec_stride = spec_stride;
-  a.spec_map_stride = spec_map_stride;
-  a.spec_rpm = spec_rpm;
-  a.herm = herm ? 1 : 0;
-  a.sw = sw;
-  a.mlo = mlo;
-  a.rings_out = rings;
-  a.ring_stride = ring_stride;
-  a.map_stride = map_stride;
-  a.rpm = rpm;
-  run_ring_inverse(a, nrings, false, st);
-}
 
 void release_df_tables() {
   std::lock_guard<std::mutex> lk(g_dft_mu);

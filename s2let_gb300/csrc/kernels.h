@@ -124,10 +124,9 @@ void gamma_px_synthesis(const double2 *F, void *out, int64_t out_ms, const int *
 void gamma_px_analysis(const void *in, int64_t in_ms, double2 *F, const int *ns, int nn, int ng, int bl, int ss,
                        int nb, bool real, double c, cudaStream_t st);
 
-// Ring DFTs fused with the gamma DFT in one launch (split precision; a
-// thread-block cluster per ring, one CTA per n-component), usable when
-// ring_gamma_fusable(nn, ng, bl, ss): the split-precision path, 2 <= nn <= 8,
-// nn ng <= 128, and a cluster of nn CTAs fits on this GPU (asked once per
+// Ring DFTs fused with the gamma DFT in one launch (a thread-block cluster per
+// ring, one CTA per n-component), usable when ring_gamma_fusable(nn, ng, bl,
+// ss): 2 <= nn <= 8, nn ng <= 128, and a cluster of nn CTAs fits on this GPU (asked once per
 // shape; otherwise the ring and gamma DFTs run as separate launches).
 // Component k of ring (b, t), t < nt, has its
 // spectrum at G + b gms + k gks + t W (W = 2bl-1, m from -(bl-1); on real

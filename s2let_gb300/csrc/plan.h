@@ -60,16 +60,20 @@ struct WignerTable {
 inline int grid_rings(int bl, int ss) { return ss ? bl + 1 : bl; }
 inline int grid_ring_len(int bl, int ss) { return ss ? 2 * bl : 2 * bl - 1; }
 
-// Bluestein data for ring length K (odd or even), padded FFT size P = 2^logP >= 2K-1.
+// Bluestein data for ring length K (odd or even), padded FFT size P = 2^logP >=
+// max(2K-1, 8), as 62-bit fixed-point constants (fxarith.h)
 struct RingFFT {
   int K = 0, P = 0, logP = 0;
-  double2 *chirp = nullptr;  // K entries, exp(i pi k^2 / K)
-  double2 *bhat = nullptr;   // P entries, FFT_P of the wrapped chirp
-  double2 *tw = nullptr;     // P/2 entries, exp(-2 pi i k / P)
-  // the same three arrays as double-float pairs (re.hi, re.lo, im.hi, im.lo)
-  // for the FP32-pipe transform of the split-precision path
-  float4 *chirp_df = nullptr, *bhat_df = nullptr, *tw_df = nullptr;
+  int eb = 0;             // the kernel spectrum is bhat 2^eb
+  int4 *chirp = nullptr;  // K entries, exp(i pi k^2 / K)
+  int4 *bhat = nullptr;   // P entries, FFT_P of the wrapped chirp over 2^eb
+  // twiddles w = exp(-2 pi i / P) of the radix-4 passes, level by level: the
+  // pass of span h (P/4, P/16, ... down to h0 = 4, or 2 for odd logP) has
+  // w^j, w^2j, w^3j (j = k P / (4h), k < h) at h - h0, + h, + 2h: P - h0 entries
+  int4 *tw = nullptr;
 };
+// re + i im (magnitude at most 1) as (re.h, re.l, im.h, im.l), v = (h 2^32 + l) 2^-62, |l| < 2^31
+int4 fixed62(long double re, long double im);
 
 // rc: recomputed (checkpointed) table instead of stored D and Q
 const WignerTable &wigner_table(int bl, int an, int ss = 0, bool rc = false);

@@ -1,0 +1,925 @@
+// Ring DFTs: batched Bluestein transforms of the theta rings (length 2bl-1 on
+// MW, 2bl on MWSS sampling) in shared memory, and the same fused with the
+// gamma DFT across a thread-block cluster.
+//
+// Arithmetic.  Block fixed point on 64-bit integers (fxarith.h): each ring (or
+// pair of real rings, or ring of all n-components) is scaled by one power of
+// two from its largest exponent field, transformed in integers, and widened
+// to FP64 once per output.  Forward and inverse transform are radix-4 with a
+// factor 1/4 per stage, which keeps every magnitude bounded (|sum of four / 4|
+// <= max) without a data-dependent branch; between the two transforms the
+// block is shifted up by the headroom measured on the block itself.  A
+// rounding error of about one unit per stage against a root-mean-square
+// level that halves per stage leaves about 2^-51 of a noise-like ring's level
+// at P = 4096 (and less at smaller P) on both transforms together: the
+// accuracy of an FP64 transform of the ring, which both precision modes use.
+// Bounds (K <= P/2 samples; components, not magnitudes):
+//   after the chirp            < 2^59.5   (2^61 input / 4; |re + i im| adds half a bit)
+//   forward stages             < 2^61     (the first, unscaled stage pair doubles at most)
+//   shifted                    < 2^61     (the next two stages do not raise a magnitude)
+//   times the kernel spectrum  < 2^59.5
+//   inverse stages             < 2^61.5   (sums of four before their 1/4; last pair unscaled)
+// A ring that holds an infinity or a NaN comes out as NaN.
+//
+// What bounds it: the wide multiply-adds (half rate) and the integer adds of
+// the butterflies; a 4-point, two-stage butterfly takes 36 multiply-adds and
+// 45 adds and shifts, against 256 FP32 instructions in double-float and 32
+// FP64 instructions at 1/64 rate.  Measured, px2wav + wav2px at L = 1024, N = 4
+// (real maps), rings and gamma DFTs: 2 maps in FP64 19.2 ms with FP64
+// butterflies, 3.8 ms so; 32 maps at split precision 60.6 ms in double-float.
+//
+// Table data comes as 62-bit fixed point (RingFFT, plan.h): chirp exp(i pi k^2
+// / K), the passes' twiddles level by level (the passes below the first read
+// 16 KB of them at P = 4096, contiguously, so they stay in L1), and the
+// spectrum of the wrapped chirp over 2^eb.
+#include <cooperative_groups.h>
+
+#include <algorithm>
+#include <climits>
+#include <cmath>
+#include <map>
+#include <mutex>
+#include <vector>
+
+#include "common.h"
+#include "fxarith.h"
+#include "kernels.h"
+#include "timing.h"
+
+namespace s2g {
+
+namespace {
+
+namespace cg = cooperative_groups;
+
+struct RingArgs {
+  const void *rings;
+  double2 *rings_out;  // inverse: output rings (as double2 or double)
+  int64_t ring_stride;  // between rings of one map
+  int64_t map_stride;   // between maps
+  int rpm;              // rings per map
+  const double2 *spec_in;
+  double2 *spec_out;
+  int64_t spec_stride;      // between spectra of one map
+  int64_t spec_map_stride;  // between maps (spectra of ring r at spec_base(r))
+  int spec_rpm;             // spectra per map
+  int herm;                 // complex inverse: m < 0 taken as conj of m > 0 (real-valued ring)
+  int sw, mlo;
+  int nrings, bl, K, P, logP;
+  int eb;  // the kernel spectrum is bhat 2^eb
+  const int4 *chirp, *bhat, *tw;
+};
+
+// One launch of ring DFTs fused with the gamma DFT (k_ring_inverse_gamma,
+// k_gamma_ring_forward): NN <= kFuseMaxNN n-components per ring.
+constexpr int kFuseMaxNN = 8;
+constexpr int kFuseMaxTw = 128;
+struct GammaFuse {
+  const double2 *G;  // synthesis input: spectrum of component k of ring (b, t) at G + b gms + k gks + t W
+  double2 *Gout;     // analysis output, the same addressing (all m from -(bl-1))
+  int64_t gms, gks;
+  int W, nt;
+  int herm_k;  // real signals: the component with n = 0 (m >= 0 stored, at offset bl-1), else -1
+  void *fw;    // gamma slice g of ring (b, t) at fw + b fms + g npx + t K (double, or double2 unless real)
+  int64_t fms, npx;
+  int ng, real;
+  int et;                // the twiddles below are over 2^et
+  int4 tw[kFuseMaxTw];  // [g NN + k] twiddles with their normalisation
+};
+
+// element offset of ring r (rings of a map are ring_stride apart, maps map_stride)
+__device__ __forceinline__ int64_t ring_base(const RingArgs &a, int r) {
+  return (int64_t)(r / a.rpm) * a.map_stride + (int64_t)(r % a.rpm) * a.ring_stride;
+}
+__device__ __forceinline__ int64_t spec_base(const RingArgs &a, int r) {
+  return (int64_t)(r / a.spec_rpm) * a.spec_map_stride + (int64_t)(r % a.spec_rpm) * a.spec_stride;
+}
+
+// Shared-memory layout: element i of the P = 2^lg point buffer (16-byte
+// complex values, no padding) lives at swz(i) = i ^ X(i), where X(i) XORs bits
+// 3-4 of i into bits 1-2, bits 3-5 into bits 0-2 and bits lg-3..lg-1 into bits
+// 0-2 (the last term only for lg > 6).  X depends only on bits >= 3 and sets
+// only bits 0-2, so swz is a bijection and its own inverse, and it is linear
+// over GF(2): swz(a ^ b) = swz(a) ^ swz(b).  Every access pattern below (bit-
+// reversed scatter and gather, the radix-4 passes at every span, stride-4 and
+// linear sweeps) then touches 8 distinct 16-byte bank groups per quarter warp
+// for P >= 256 (checked by enumerating the patterns on the CPU), without the
+// 1/8 padding a skewed layout needs.
+struct Swz {
+  int top;  // lg - 3 when lg > 6, else 31 (the term vanishes for non-negative i)
+};
+__device__ __forceinline__ Swz swz_of(int logP) { return Swz{logP > 6 ? logP - 3 : 31}; }
+__device__ __forceinline__ int swz(int i, Swz z) {
+  return i ^ ((i >> 2) & 6) ^ ((i >> 3) & 7) ^ ((i >> z.top) & 7);
+}
+__device__ __forceinline__ int brev(int k, int logP) { return (int)(__brev((unsigned)k) >> (32 - logP)); }
+// buffer slot of bit-reversed position k
+__device__ __forceinline__ int slot_brev(int k, int logP) { return swz(brev(k, logP), swz_of(logP)); }
+
+// Read-only table loads with an L1 eviction priority: the twiddle table is
+// read by every pass of every ring on the SM (kept: evict_last); the chirp and
+// the chirp-kernel spectrum are read once per ring (evict_first).
+__device__ __forceinline__ int4 ld_keep(const int4 *p) {
+  int4 v;
+  asm("ld.global.nc.L1::evict_last.v4.s32 {%0, %1, %2, %3}, [%4];"
+      : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+      : "l"(p));
+  return v;
+}
+__device__ __forceinline__ int4 ld_once(const int4 *p) {
+  int4 v;
+  asm("ld.global.nc.L1::evict_first.v4.s32 {%0, %1, %2, %3}, [%4];"
+      : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+      : "l"(p));
+  return v;
+}
+
+// bits of the high word's magnitude (headroom tracking)
+__device__ __forceinline__ int high_bits(longlong2 v) {
+  const int x = (int)(v.x >> 32), y = (int)(v.y >> 32);
+  return (x ^ (x >> 31)) | (y ^ (y >> 31));
+}
+
+// forward butterfly on bit-reversed data: stages s and s + 1 with
+// w1 = w^2j (elements 1), w2 = w^j (elements 2), w3 = w^3j (elements 3), over 4
+__device__ __forceinline__ void dit4(longlong2 &a0, longlong2 &a1, longlong2 &a2, longlong2 &a3, int4 w1, int4 w2,
+                                     int4 w3) {
+  const longlong2 t0 = fx_sar(a0, 2), t1 = fx_mul4(a1, w1), t2 = fx_mul4(a2, w2), t3 = fx_mul4(a3, w3);
+  const longlong2 b0 = fx_add(t0, t1), b1 = fx_sub(t0, t1), b2 = fx_add(t2, t3), b3 = fx_mul_i(fx_sub(t2, t3));
+  a0 = fx_add(b0, b2);
+  a2 = fx_sub(b0, b2);
+  a1 = fx_sub(b1, b3);
+  a3 = fx_add(b1, b3);
+}
+// inverse butterfly, natural to bit-reversed order, over 4
+__device__ __forceinline__ void dif4(longlong2 &a0, longlong2 &a1, longlong2 &a2, longlong2 &a3, int4 w1, int4 w2,
+                                     int4 w3) {
+  const longlong2 b0 = fx_add(a0, a2), b1 = fx_add(a1, a3), b2 = fx_sub(a0, a2), b3 = fx_mul_i(fx_sub(a1, a3));
+  a0 = fx_sar(fx_add(b0, b1), 2);
+  a1 = fx_mulc4(fx_sub(b0, b1), w1);
+  a2 = fx_mulc4(fx_add(b2, b3), w2);
+  a3 = fx_mulc4(fx_sub(b2, b3), w3);
+}
+
+// Bluestein core.  On entry (barrier not yet passed) the even bit-reversed
+// positions hold a_j (slot_brev(j), j < P/2; the second half of the sequence
+// is zero and is not read); on exit, after a barrier, slot_brev(k) holds y_k 2^S
+// for k < P/2, y the convolution times P, S the sum of the scalings.  Returns
+// the shift applied between the transforms.  P >= 8.
+//   stages: even log2 P: a 4-point pass of (a0, 0, a2, 0) with unit twiddles,
+//   odd: a copy (stage 1 of (a0, 0)); then radix-4 passes; the last of them,
+//   the kernel-spectrum product and the first inverse pass work on the same
+//   four elements and stay in registers; inverse radix-4 passes; a last pass
+//   with unit twiddles, even outputs only.
+__device__ int bluestein(longlong2 *buf, const RingArgs &a, int *s_mx) {
+  const int P = a.P, logP = a.logP;
+  const int4 *__restrict__ tw = a.tw;
+  const Swz z = swz_of(logP);
+  const int h0 = logP & 1 ? 2 : 4;
+  int mx = 0;
+  if (threadIdx.x == 0) *s_mx = 0;
+  __syncthreads();
+  int s;
+  if (logP & 1) {
+    for (int i = threadIdx.x; i < P / 2; i += blockDim.x) {
+      const int b = swz(2 * i, z);
+      const longlong2 v = buf[b];
+      buf[b ^ 1] = v;
+      if (logP == 3) mx |= high_bits(v);
+    }
+    s = 2;
+  } else {
+    for (int i = threadIdx.x; i < P / 4; i += blockDim.x) {
+      const int b = swz(4 * i, z);
+      const longlong2 a0 = buf[b], a2 = buf[b ^ 2];
+      const longlong2 v0 = fx_add(a0, a2), v2 = fx_sub(a0, a2);
+      const longlong2 ia = fx_mul_i(a2), v1 = fx_sub(a0, ia), v3 = fx_add(a0, ia);
+      buf[b] = v0;
+      buf[b ^ 2] = v2;
+      buf[b ^ 1] = v1;
+      buf[b ^ 3] = v3;
+      if (logP == 4) mx |= high_bits(v0) | high_bits(v1) | high_bits(v2) | high_bits(v3);
+    }
+    s = 3;
+  }
+  if (logP > 4) __syncthreads();
+  for (; s + 1 < logP; s += 2) {
+    const int h = 1 << (s - 1);
+    const int q1 = swz(h, z), q2 = swz(2 * h, z), q3 = swz(3 * h, z);
+    const bool track = s + 3 == logP;
+    for (int i = threadIdx.x; i < P / 4; i += blockDim.x) {
+      const int jp = i & (h - 1);
+      const int b = swz(((i >> (s - 1)) << (s + 1)) + jp, z);
+      const int4 *w = tw + (h - h0) + jp;
+      const int4 w2 = ld_keep(w), w1 = ld_keep(w + h), w3 = ld_keep(w + 2 * h);
+      longlong2 a0 = buf[b], a1 = buf[b ^ q1], a2 = buf[b ^ q2], a3 = buf[b ^ q3];
+      dit4(a0, a1, a2, a3, w1, w2, w3);
+      buf[b] = a0;
+      buf[b ^ q1] = a1;
+      buf[b ^ q2] = a2;
+      buf[b ^ q3] = a3;
+      if (track) mx |= high_bits(a0) | high_bits(a1) | high_bits(a2) | high_bits(a3);
+    }
+    if (!track) __syncthreads();
+  }
+  mx = __reduce_or_sync(0xffffffffu, mx);
+  if ((threadIdx.x & 31) == 0) atomicOr(s_mx, mx);
+  __syncthreads();
+  const int sh = max(0, __clz(*s_mx) - 3);  // components < 2^61 afterwards
+  {  // last forward pass, kernel spectrum, first inverse pass
+    const int h = P / 4;
+    const int q1 = swz(h, z), q2 = swz(2 * h, z), q3 = swz(3 * h, z);
+    for (int i = threadIdx.x; i < h; i += blockDim.x) {
+      const int b = swz(i, z);
+      longlong2 a0 = fx_shl(buf[b], sh), a1 = fx_shl(buf[b ^ q1], sh), a2 = fx_shl(buf[b ^ q2], sh),
+                a3 = fx_shl(buf[b ^ q3], sh);
+      const int4 *w = tw + (h - h0) + i;
+      const int4 w2 = ld_once(w), w1 = ld_once(w + h), w3 = ld_once(w + 2 * h);
+      dit4(a0, a1, a2, a3, w1, w2, w3);
+      a0 = fx_mul4(a0, ld_once(&a.bhat[i]));
+      a1 = fx_mul4(a1, ld_once(&a.bhat[i + h]));
+      a2 = fx_mul4(a2, ld_once(&a.bhat[i + 2 * h]));
+      a3 = fx_mul4(a3, ld_once(&a.bhat[i + 3 * h]));
+      dif4(a0, a1, a2, a3, w1, w2, w3);
+      buf[b] = a0;
+      buf[b ^ q1] = a1;
+      buf[b ^ q2] = a2;
+      buf[b ^ q3] = a3;
+    }
+    __syncthreads();
+  }
+  for (s = logP - 2; s >= 3; s -= 2) {
+    const int h = 1 << (s - 2);
+    const int q1 = swz(h, z), q2 = swz(2 * h, z), q3 = swz(3 * h, z);
+    for (int i = threadIdx.x; i < P / 4; i += blockDim.x) {
+      const int jp = i & (h - 1);
+      const int b = swz(((i >> (s - 2)) << s) + jp, z);
+      const int4 *w = tw + (h - h0) + jp;
+      const int4 w2 = ld_keep(w), w1 = ld_keep(w + h), w3 = ld_keep(w + 2 * h);
+      longlong2 a0 = buf[b], a1 = buf[b ^ q1], a2 = buf[b ^ q2], a3 = buf[b ^ q3];
+      dif4(a0, a1, a2, a3, w1, w2, w3);
+      buf[b] = a0;
+      buf[b ^ q1] = a1;
+      buf[b ^ q2] = a2;
+      buf[b ^ q3] = a3;
+    }
+    __syncthreads();
+  }
+  if (s == 2) {  // stages 2 and 1, unit twiddles, even outputs only
+    for (int i = threadIdx.x; i < P / 4; i += blockDim.x) {
+      const int b = swz(4 * i, z);
+      const longlong2 a0 = buf[b], a1 = buf[b ^ 1], a2 = buf[b ^ 2], a3 = buf[b ^ 3];
+      buf[b] = fx_add(fx_add(a0, a2), fx_add(a1, a3));
+      buf[b ^ 2] = fx_add(fx_sub(a0, a2), fx_mul_i(fx_sub(a1, a3)));
+    }
+  } else {
+    for (int i = threadIdx.x; i < P / 2; i += blockDim.x) {
+      const int b = swz(2 * i, z);
+      buf[b] = fx_add(buf[b], buf[b ^ 1]);
+    }
+  }
+  __syncthreads();
+  return sh;
+}
+// a value q in the buffer of a block with exponent e, split to `bits` bits, is
+// q 2^k after the chirp (over 4) and the core: 2 per radix-4 pass and product,
+// the shift, the kernel spectrum's exponent, and the 1/P of the transforms
+__device__ __forceinline__ int core_exponent(const RingArgs &a, int e, int bits, int sh) {
+  const int passes = (a.logP - 1) >> 1;  // radix-4 passes of one direction
+  return e - bits + 2 + 4 * passes + 2 + a.eb - sh - a.logP;
+}
+
+// block-wide max of an int (blockDim.x <= 1024)
+__device__ int block_max_int(int v) {
+  __shared__ int redi[32];
+  v = __reduce_max_sync(0xffffffffu, v);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) redi[threadIdx.x >> 5] = v;
+  __syncthreads();
+  int m = 0;
+  for (int i = 0; i < (int)((blockDim.x + 31) >> 5); ++i) m = max(m, redi[i]);
+  return m;
+}
+__device__ __forceinline__ int emax2(int m, double2 z) { return max(m, max(exp_field(z.x), exp_field(z.y))); }
+
+__device__ __forceinline__ double2 nan2() {
+  const double n = double_of(0x7FF8000000000000ull);
+  return make_double2(n, n);
+}
+
+constexpr int kRingThreads = 256;
+
+template <bool REAL>
+__global__ void __launch_bounds__(kRingThreads, 3) k_ring_forward(RingArgs a) {
+  extern __shared__ longlong2 buf[];
+  __shared__ int s_mx;
+  const int K = a.K, P = a.P, logP = a.logP;
+  const int r0 = REAL ? 2 * blockIdx.x : blockIdx.x;
+  const bool has1 = REAL && (r0 + 1 < a.nrings);
+  int em = 0;
+  for (int j = threadIdx.x; j < K; j += blockDim.x) {
+    if (REAL) {
+      em = max(em, exp_field(((const double *)a.rings)[ring_base(a, r0) + j]));
+      if (has1) em = max(em, exp_field(((const double *)a.rings)[ring_base(a, r0 + 1) + j]));
+    } else {
+      em = emax2(em, ((const double2 *)a.rings)[ring_base(a, r0) + j]);
+    }
+  }
+  em = block_max_int(em);
+  const int e = fx_exp(em);
+  for (int j = threadIdx.x; j < P / 2; j += blockDim.x) {
+    longlong2 v = make_longlong2(0, 0);
+    if (j < K) {
+      double2 x;
+      if (REAL) {
+        x.x = ((const double *)a.rings)[ring_base(a, r0) + j];
+        x.y = has1 ? ((const double *)a.rings)[ring_base(a, r0 + 1) + j] : 0.0;
+      } else {
+        x = ((const double2 *)a.rings)[ring_base(a, r0) + j];
+      }
+      v = fx_mulc4(fx_split2<61>(x, e), ld_once(&a.chirp[j]));  // x_j conj(c_j)
+    }
+    buf[slot_brev(j, logP)] = v;
+  }
+  const int sh = bluestein(buf, a, &s_mx);
+  const int k0 = core_exponent(a, e, 61, sh);
+  if (!REAL) {
+    double2 *out = a.spec_out + spec_base(a, r0);
+    for (int c = threadIdx.x; c < a.sw; c += blockDim.x) {
+      const int m = a.mlo + c;
+      const int k = m < 0 ? m + K : m;
+      const longlong2 y = fx_mulc(buf[slot_brev(k, logP)], ld_once(&a.chirp[k]));
+      out[c] = em == kExpNonFinite ? nan2() : fx_join2(y, k0);
+    }
+  } else {
+    double2 *out0 = a.spec_out + spec_base(a, r0);
+    for (int m = threadIdx.x; m < a.sw; m += blockDim.x) {
+      const int km = m ? K - m : 0;
+      const longlong2 zm = fx_mulc(buf[slot_brev(m, logP)], ld_once(&a.chirp[m]));
+      const longlong2 zc = fx_conj(fx_mulc(buf[slot_brev(km, logP)], ld_once(&a.chirp[km])));
+      // A = (Z_m + conj Z_{-m})/2,  B = (Z_m - conj Z_{-m})/(2i)
+      out0[m] = em == kExpNonFinite ? nan2() : fx_join2(fx_add(zm, zc), k0 - 1);
+      if (has1) {
+        const longlong2 d = fx_sub(zm, zc);
+        out0[a.spec_stride + m] = em == kExpNonFinite ? nan2() : fx_join2(make_longlong2(d.y, -d.x), k0 - 1);
+      }
+    }
+  }
+}
+
+template <bool REAL>
+__global__ void __launch_bounds__(kRingThreads, 3) k_ring_inverse(RingArgs a) {
+  extern __shared__ longlong2 buf[];
+  __shared__ int s_mx;
+  constexpr int BITS = REAL ? 60 : 61;  // A + i B of two rings
+  const int K = a.K, P = a.P, logP = a.logP, bl = a.bl;
+  const int r0 = REAL ? 2 * blockIdx.x : blockIdx.x;
+  const bool has1 = REAL && (r0 + 1 < a.nrings);
+  const double2 *s0 = a.spec_in + spec_base(a, r0);
+  int em = 0;
+  for (int c = threadIdx.x; c < a.sw; c += blockDim.x) {
+    em = emax2(em, s0[c]);
+    if (has1) em = emax2(em, s0[a.spec_stride + c]);
+  }
+  em = block_max_int(em);
+  const int e = fx_exp(em);
+  for (int j = threadIdx.x; j < P / 2; j += blockDim.x) {
+    longlong2 v = make_longlong2(0, 0);
+    if (j < K) {
+      const int m = (j < bl) ? j : j - K;  // frequency of DFT bin j
+      if (REAL) {
+        const int am = m < 0 ? -m : m;
+        if (am < a.sw) {
+          longlong2 A = fx_split2<BITS>(s0[am], e);
+          longlong2 B = has1 ? fx_split2<BITS>(s0[a.spec_stride + am], e) : make_longlong2(0, 0);
+          if (m < 0) {
+            A = fx_conj(A);
+            B = fx_conj(B);
+          }
+          v = fx_add(A, fx_mul_i(B));
+        }
+      } else {
+        const int c = m - a.mlo;
+        if (c >= 0 && c < a.sw)
+          v = fx_split2<BITS>(s0[c], e);
+        else if (a.herm && m < 0 && -m - a.mlo < a.sw)
+          v = fx_conj(fx_split2<BITS>(s0[-m - a.mlo], e));
+      }
+      // inverse DFT = conj(forward(conj z)):  a_j = conj(z_j) conj(c_j)
+      v = fx_conj(fx_mul4(v, ld_once(&a.chirp[j])));
+    }
+    buf[slot_brev(j, logP)] = v;
+  }
+  const int sh = bluestein(buf, a, &s_mx);
+  const int k0 = core_exponent(a, e, BITS, sh);
+  for (int p = threadIdx.x; p < K; p += blockDim.x) {
+    // f_p = c_p conj(y_p)
+    const longlong2 y = fx_mul(fx_conj(buf[slot_brev(p, logP)]), ld_once(&a.chirp[p]));
+    const double2 f = em == kExpNonFinite ? nan2() : fx_join2(y, k0);
+    if (REAL) {
+      ((double *)a.rings_out)[ring_base(a, r0) + p] = f.x;
+      if (has1) ((double *)a.rings_out)[ring_base(a, r0 + 1) + p] = f.y;
+    } else {
+      a.rings_out[ring_base(a, r0) + p] = f;
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Ring DFTs and gamma DFT in one launch
+//
+// The n-components F_k(t, p) (k < NN) of one theta-ring are transformed by a
+// thread-block cluster of NN CTAs, one per component, each with the padded
+// Bluestein buffer of the single-ring kernels.  The gamma DFT exchanges values
+// between the components of a pixel through distributed shared memory, so the
+// n-components never go to HBM:
+//   synthesis: each CTA runs the inverse ring DFT of its component and leaves
+//              F_k(p) in its buffer; after a cluster barrier each CTA computes
+//              the gamma slices f_g(p) of its share of the pixels from all NN
+//              buffers and writes them to f_wav.
+//   analysis:  each CTA reads the gamma slices of its share of the pixels,
+//              forms every component F_k(p), premultiplies by the chirp and
+//              stores it into CTA k's buffer; after a cluster barrier each CTA
+//              runs the forward ring DFT of its component and writes its
+//              spectrum.
+// One power-of-two scale per ring, the largest over the cluster; after the
+// synthesis transforms the components are aligned to the largest exponent.
+// gamma_g and gamma_{ng-g} have conjugate twiddles, so each pair of slices
+// shares its products.
+// ---------------------------------------------------------------------------
+
+__device__ __forceinline__ int cluster_max_int(cg::cluster_group &cl, int *slot, int v, int nn) {
+  const int m = block_max_int(v);
+  if (threadIdx.x == 0) *slot = m;
+  cl.sync();
+  int r = 0;
+  for (int j = 0; j < nn; ++j) r = max(r, *cl.map_shared_rank(slot, j));
+  return r;
+}
+
+template <int NN, bool REAL>
+__global__ void __launch_bounds__(kRingThreads, 3) k_ring_inverse_gamma(RingArgs a, const __grid_constant__ GammaFuse gf) {
+  extern __shared__ longlong2 buf[];
+  __shared__ int s_mx, s_em, s_k;
+  cg::cluster_group cl = cg::this_cluster();
+  const int k = (int)cl.block_rank();
+  const int r = blockIdx.x / NN;
+  const int b = r / gf.nt, t = r - b * gf.nt;
+  const int K = a.K, P = a.P, logP = a.logP, bl = a.bl;
+  const bool herm = (k == gf.herm_k);
+  const int sw = herm ? bl : gf.W, mlo = herm ? 0 : -(bl - 1);
+  const double2 *s0 = gf.G + (int64_t)b * gf.gms + (int64_t)k * gf.gks + (int64_t)t * gf.W + (herm ? bl - 1 : 0);
+  int em = 0;
+  for (int c = threadIdx.x; c < sw; c += blockDim.x) em = emax2(em, s0[c]);
+  em = cluster_max_int(cl, &s_em, em, NN);
+  const int e = fx_exp(em);
+  for (int j = threadIdx.x; j < P / 2; j += blockDim.x) {
+    longlong2 v = make_longlong2(0, 0);
+    if (j < K) {
+      const int m = (j < bl) ? j : j - K;
+      const int c = m - mlo;
+      if (c >= 0 && c < sw)
+        v = fx_split2<61>(s0[c], e);
+      else if (herm && m < 0 && -m < sw)
+        v = fx_conj(fx_split2<61>(s0[-m], e));
+      v = fx_conj(fx_mul4(v, ld_once(&a.chirp[j])));
+    }
+    buf[slot_brev(j, logP)] = v;
+  }
+  const int sh = bluestein(buf, a, &s_mx);
+  // F_k(p) = c_p conj(y_p), in place (p -> brev(p) is one-to-one); components < 2^61.5
+  for (int p = threadIdx.x; p < K; p += blockDim.x) {
+    const int i = slot_brev(p, logP);
+    buf[i] = fx_mul(fx_conj(buf[i]), ld_once(&a.chirp[p]));
+  }
+  if (threadIdx.x == 0) s_k = core_exponent(a, e, 61, sh);
+  cl.sync();
+  // gamma slices of this CTA's share of the pixels
+  int kj[NN], km = INT_MIN;
+#pragma unroll
+  for (int j = 0; j < NN; ++j) {
+    kj[j] = *cl.map_shared_rank(&s_k, j);
+    km = max(km, kj[j]);
+  }
+  const int ko = km + 2 + gf.et;
+  const bool bad = em == kExpNonFinite;
+  const int chunk = (K + NN - 1) / NN;
+  const int p1 = min(K, (k + 1) * chunk);
+  const int64_t obase = (int64_t)b * gf.fms + (int64_t)t * K;
+  // with w = C + i S (each product over 4: sums of 8 stay below 2^62.5):
+  //   real:    f_g = A - B, f_{ng-g} = A + B, A = sum_k C Re z_k, B = sum_k S Im z_k
+  //   complex: f_g = U + i V, f_{ng-g} = U - i V, U = sum_k C z_k, V = sum_k S z_k
+  for (int p = k * chunk + threadIdx.x; p < p1; p += blockDim.x) {
+    const int i = slot_brev(p, logP);
+    longlong2 z[NN];
+#pragma unroll
+    for (int j = 0; j < NN; ++j) z[j] = fx_sar(*cl.map_shared_rank(buf + i, j), min(63, km - kj[j]));
+    for (int g = 0; 2 * g <= gf.ng; ++g) {
+      const int g2 = gf.ng - g;  // the conjugate partner (g = 0 and g2 == g have none)
+      const int64_t o = obase + (int64_t)g * gf.npx + p, o2 = obase + (int64_t)g2 * gf.npx + p;
+      const bool pair = g > 0 && g2 != g;
+      if (REAL) {
+        long long A = 0, B = 0;
+#pragma unroll
+        for (int j = 0; j < NN; ++j) {
+          const int4 w = gf.tw[g * NN + j];
+          A = fx_mac4(A, z[j].x, w.x, w.y);
+          B = fx_mac4(B, z[j].y, w.z, w.w);
+        }
+        ((double *)gf.fw)[o] = bad ? nan2().x : fx_join(A - B, ko);
+        if (pair) ((double *)gf.fw)[o2] = bad ? nan2().x : fx_join(A + B, ko);
+      } else {
+        longlong2 U = make_longlong2(0, 0), V = make_longlong2(0, 0);
+#pragma unroll
+        for (int j = 0; j < NN; ++j) {
+          const int4 w = gf.tw[g * NN + j];
+          U = make_longlong2(fx_mac4(U.x, z[j].x, w.x, w.y), fx_mac4(U.y, z[j].y, w.x, w.y));
+          V = make_longlong2(fx_mac4(V.x, z[j].x, w.z, w.w), fx_mac4(V.y, z[j].y, w.z, w.w));
+        }
+        const longlong2 iV = fx_mul_i(V);
+        ((double2 *)gf.fw)[o] = bad ? nan2() : fx_join2(fx_add(U, iV), ko);
+        if (pair) ((double2 *)gf.fw)[o2] = bad ? nan2() : fx_join2(fx_sub(U, iV), ko);
+      }
+    }
+  }
+  cl.sync();  // peers read this buffer until here
+}
+
+template <int NN, bool REAL>
+__global__ void __launch_bounds__(kRingThreads, 3) k_gamma_ring_forward(RingArgs a, const __grid_constant__ GammaFuse gf) {
+  extern __shared__ longlong2 buf[];
+  __shared__ int s_mx, s_em;
+  cg::cluster_group cl = cg::this_cluster();
+  const int k = (int)cl.block_rank();
+  const int r = blockIdx.x / NN;
+  const int b = r / gf.nt, t = r - b * gf.nt;
+  const int K = a.K, P = a.P, logP = a.logP;
+  const int chunk = (K + NN - 1) / NN;
+  const int p0 = k * chunk, p1 = min(K, p0 + chunk);
+  const int64_t ibase = (int64_t)b * gf.fms + (int64_t)t * K;
+  int em = 0;
+  for (int p = p0 + threadIdx.x; p < p1; p += blockDim.x)
+    for (int g = 0; g < gf.ng; ++g) {
+      const int64_t o = ibase + (int64_t)g * gf.npx + p;
+      if (REAL)
+        em = max(em, exp_field(((const double *)gf.fw)[o]));
+      else
+        em = emax2(em, ((const double2 *)gf.fw)[o]);
+    }
+  em = cluster_max_int(cl, &s_em, em, NN);
+  const int e = fx_exp(em);
+  // the zero padding of this CTA's own buffer
+  for (int j = K + threadIdx.x; j < P / 2; j += blockDim.x) buf[slot_brev(j, logP)] = make_longlong2(0, 0);
+  // gamma_g and gamma_{ng-g} have conjugate twiddles w = C + i S and C - i S:
+  // each pair contributes C (f_g + f_{ng-g}) + i S (f_g - f_{ng-g}).  The
+  // twiddles' magnitudes sum to at most 1 over g (et), so F_k / 4 stays below
+  // 2^59.5 and the chirp is applied at full scale.
+  for (int p = p0 + threadIdx.x; p < p1; p += blockDim.x) {
+    longlong2 acc[NN];
+#pragma unroll
+    for (int j = 0; j < NN; ++j) acc[j] = make_longlong2(0, 0);
+    for (int g = 0; 2 * g <= gf.ng; ++g) {
+      const int g2 = gf.ng - g;
+      const bool pair = g > 0 && g2 != g;
+      const int64_t o = ibase + (int64_t)g * gf.npx + p, o2 = ibase + (int64_t)g2 * gf.npx + p;
+      if (REAL) {
+        const long long fa = fx_split<61>(((const double *)gf.fw)[o], e);
+        const long long fb = pair ? fx_split<61>(((const double *)gf.fw)[o2], e) : 0;
+        const long long Pp = fa + fb, Q = fa - fb;
+#pragma unroll
+        for (int j = 0; j < NN; ++j) {
+          const int4 w = gf.tw[g * NN + j];
+          acc[j] = make_longlong2(fx_mac4(acc[j].x, Pp, w.x, w.y), fx_mac4(acc[j].y, Q, w.z, w.w));
+        }
+      } else {
+        const longlong2 fa = fx_split2<61>(((const double2 *)gf.fw)[o], e);
+        const longlong2 fb = pair ? fx_split2<61>(((const double2 *)gf.fw)[o2], e) : make_longlong2(0, 0);
+        const longlong2 Pp = fx_add(fa, fb), Q = fx_sub(fa, fb);
+#pragma unroll
+        for (int j = 0; j < NN; ++j) {
+          const int4 w = gf.tw[g * NN + j];
+          // C P + i S Q
+          acc[j] = make_longlong2(fx_mac4(fx_mac4(acc[j].x, Pp.x, w.x, w.y), -Q.y, w.z, w.w),
+                                  fx_mac4(fx_mac4(acc[j].y, Pp.y, w.x, w.y), Q.x, w.z, w.w));
+        }
+      }
+    }
+    const int4 ch = ld_once(&a.chirp[p]);
+    const int i = slot_brev(p, logP);
+#pragma unroll
+    for (int j = 0; j < NN; ++j) *cl.map_shared_rank(buf + i, j) = fx_mulc(acc[j], ch);
+  }
+  cl.sync();  // every component's buffer is complete
+  const int sh = bluestein(buf, a, &s_mx);
+  // split to 61 bits, over 4 in the gamma sums as after a scaled chirp, times 2^et
+  const int k0 = core_exponent(a, e, 61, sh) + gf.et;
+  double2 *out = gf.Gout + (int64_t)b * gf.gms + (int64_t)k * gf.gks + (int64_t)t * gf.W;
+  for (int c = threadIdx.x; c < gf.W; c += blockDim.x) {
+    const int m = c - (a.bl - 1);
+    const int q = m < 0 ? m + K : m;
+    const longlong2 y = fx_mulc(buf[slot_brev(q, logP)], ld_once(&a.chirp[q]));
+    out[c] = em == kExpNonFinite ? nan2() : fx_join2(y, k0);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// launches
+// ---------------------------------------------------------------------------
+
+RingArgs ring_args(const RingFFT &rf, int bl, int nrings) {
+  RingArgs a{};
+  a.spec_rpm = 1 << 30;  // single-level spectrum addressing unless set
+  a.spec_map_stride = 0;
+  a.K = rf.K;
+  a.P = rf.P;
+  a.logP = rf.logP;
+  a.eb = rf.eb;
+  a.bl = bl;
+  a.nrings = nrings;
+  a.chirp = rf.chirp;
+  a.bhat = rf.bhat;
+  a.tw = rf.tw;
+  return a;
+}
+
+int ring_threads(int P) { return std::min(kRingThreads, std::max(32, P / 4)); }
+size_t ring_smem(int P) { return sizeof(longlong2) * (size_t)P; }
+
+// Shared memory of the ring kernels: one P-point buffer of 16-byte values,
+// with a carveout just large enough for the resident buffers (three at P =
+// 4096), so that the rest of the SM's L1 keeps the twiddle table (48 KB there).
+void ring_smem_attrs(const void *kernel, size_t smem) {
+  if (smem > 48 * 1024) S2G_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  constexpr double kMaxSmemPerSm = 228.0 * 1024.0;
+  const int pct = std::min(100, (int)std::ceil(100.0 * 3.0 * (double)(smem + 2048) / kMaxSmemPerSm) + 1);
+  S2G_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, pct));
+}
+
+template <class KF>
+void launch_ring(KF kernel, const RingArgs &a, int nblk, cudaStream_t st) {
+  ring_smem_attrs((const void *)kernel, ring_smem(a.P));
+  kernel<<<nblk, ring_threads(a.P), ring_smem(a.P), st>>>(a);
+  S2G_LAUNCHED();
+}
+
+// Work model of one Bluestein transform of padded length P (for the timing
+// report), in 32 x 32 + 64 multiply-adds: 12 per complex product; 3 products
+// per 4 points and radix-4 pass ((log2 P - 1)/2 passes each way), one per
+// point for the kernel spectrum and two per sample for the chirps.
+double ring_work(const RingArgs &a, int nblk) {
+  const double P = a.P, passes = (a.logP - 1) / 2;
+  return (double)nblk * 12.0 * (2.0 * passes * 0.75 * P + P + 2.0 * a.K);
+}
+
+void run_ring_forward(const RingArgs &a, int nrings, bool real, cudaStream_t st) {
+  const int nblk = real ? (nrings + 1) / 2 : nrings;
+  KTimer kt(KC_RING, st, timing_enabled() ? ring_work(a, nblk) : 0.0,
+            (double)nrings * a.K * (real ? 8.0 : 16.0) + (double)nrings * a.sw * 16.0);
+  if (real)
+    launch_ring(k_ring_forward<true>, a, nblk, st);
+  else
+    launch_ring(k_ring_forward<false>, a, nblk, st);
+}
+
+void run_ring_inverse(const RingArgs &a, int nrings, bool real, cudaStream_t st) {
+  const int nblk = real ? (nrings + 1) / 2 : nrings;
+  KTimer kt(KC_RING, st, timing_enabled() ? ring_work(a, nblk) : 0.0,
+            (double)nrings * a.K * (real ? 8.0 : 16.0) + (double)nrings * a.sw * 16.0);
+  if (real)
+    launch_ring(k_ring_inverse<true>, a, nblk, st);
+  else
+    launch_ring(k_ring_inverse<false>, a, nblk, st);
+}
+
+// Twiddles of the fused gamma DFT: synthesis c e^{i n_k gamma_g} (x2 for
+// n_k != 0 on real signals, which stand for the +-n pair), analysis
+// c e^{-i n_k gamma_g}; gamma_g = 2 pi g / ng.  Stored over 2^et: synthesis
+// |w| <= 1, analysis sum_g |w| <= 1.
+void fuse_twiddles(GammaFuse &gf, const std::vector<int> &ns, int ng, bool real, double c, bool synth) {
+  const int nn = (int)ns.size();
+  const double top = synth ? (real ? 2.0 * c : c) : ng * c;
+  gf.et = 0;
+  while (std::ldexp(1.0, gf.et) < top) ++gf.et;
+  while (std::ldexp(1.0, gf.et - 1) >= top) --gf.et;
+  for (int g = 0; g < ng; ++g)
+    for (int k = 0; k < nn; ++k) {
+      const long double x = 2.0L * (long double)((ns[k] * g) % ng) / (long double)ng;  // angle / pi
+      const long double pi = 3.141592653589793238462643383279502884L;
+      const long double f = ldexpl(synth && real && ns[k] != 0 ? 2.0L * c : (long double)c, -gf.et);
+      gf.tw[g * nn + k] = fixed62(f * cosl(pi * x), (synth ? f : -f) * sinl(pi * x));
+    }
+}
+
+cudaLaunchConfig_t fused_config(int nctas, int nn, int P, cudaLaunchAttribute *at, cudaStream_t st) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)nctas);
+  cfg.blockDim = dim3(ring_threads(P));
+  cfg.dynamicSmemBytes = ring_smem(P);
+  cfg.stream = st;
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)nn;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+
+template <class KF>
+void launch_fused(KF kernel, const RingArgs &a, const GammaFuse &gf, int nrings, int nn, cudaStream_t st) {
+  ring_smem_attrs((const void *)kernel, ring_smem(a.P));
+  cudaLaunchAttribute at[1];
+  const cudaLaunchConfig_t cfg = fused_config(nrings * nn, nn, a.P, at, st);
+  S2G_CUDA(cudaLaunchKernelEx(&cfg, kernel, a, gf));
+  S2G_LAUNCHED();
+}
+
+// Whether a cluster of nn CTAs of the fused kernels (P-point buffers) can be
+// resident on this GPU: asked once per (nn, P) of the device in use.
+bool cluster_fits(int nn, int P) {
+  static std::mutex mu;
+  static std::map<std::pair<int, int>, bool> known;
+  std::lock_guard<std::mutex> lk(mu);
+  const auto key = std::make_pair(nn, P);
+  auto it = known.find(key);
+  if (it != known.end()) return it->second;
+  const void *kern = nullptr;
+  switch (nn) {
+    case 2: kern = (const void *)k_ring_inverse_gamma<2, false>; break;
+    case 3: kern = (const void *)k_ring_inverse_gamma<3, false>; break;
+    case 4: kern = (const void *)k_ring_inverse_gamma<4, false>; break;
+    case 5: kern = (const void *)k_ring_inverse_gamma<5, false>; break;
+    case 6: kern = (const void *)k_ring_inverse_gamma<6, false>; break;
+    case 7: kern = (const void *)k_ring_inverse_gamma<7, false>; break;
+    default: kern = (const void *)k_ring_inverse_gamma<8, false>; break;
+  }
+  bool ok = ring_smem(P) <= 227 * 1024;
+  if (ok) {
+    ring_smem_attrs(kern, ring_smem(P));
+    cudaLaunchAttribute at[1];
+    const cudaLaunchConfig_t cfg = fused_config(nn, nn, P, at, nullptr);
+    int nclusters = 0;
+    const cudaError_t e = cudaOccupancyMaxActiveClusters(&nclusters, kern, &cfg);
+    if (e != cudaSuccess) cudaGetLastError();  // a refusal only means: not fusable here
+    ok = e == cudaSuccess && nclusters > 0;
+  }
+  known[key] = ok;
+  return ok;
+}
+
+}  // namespace
+
+bool ring_gamma_fusable(int nn, int ng, int bl, int ss) {
+  if (nn < 2 || nn > kFuseMaxNN || ng * nn > kFuseMaxTw) return false;
+  return cluster_fits(nn, ring_fft(grid_ring_len(bl, ss)).P);
+}
+
+namespace {
+// the parts of a fused launch that both directions share
+GammaFuse gamma_fuse(const RingArgs &a, int64_t gms, int64_t gks, const std::vector<int> &ns, int ng, bool real,
+                     double c, void *fw, int64_t fms, int nt, bool synth) {
+  GammaFuse gf{};
+  gf.gms = gms;
+  gf.gks = gks;
+  gf.W = 2 * a.bl - 1;
+  gf.nt = nt;
+  gf.herm_k = -1;
+  gf.fw = fw;
+  gf.fms = fms;
+  gf.npx = (int64_t)nt * a.K;
+  gf.ng = ng;
+  gf.real = real ? 1 : 0;
+  fuse_twiddles(gf, ns, ng, real, c, synth);
+  return gf;
+}
+// multiply-adds of the gamma products: 3 per real product, (ng + 1)/2 slice pairs
+double gamma_work(double px, int ng, int nn, bool real) { return px * ((ng + 1) / 2) * nn * (real ? 6.0 : 12.0); }
+}  // namespace
+
+void ring_inverse_gamma(const double2 *G, int64_t gms, int64_t gks, const std::vector<int> &ns, int ng, bool real,
+                        double c, void *fw, int64_t fms, int nb, int bl, int ss, cudaStream_t st) {
+  const int nn = (int)ns.size();
+  S2G_REQUIRE(ring_gamma_fusable(nn, ng, bl, ss), ERR_UNSUPPORTED, "fused ring/gamma DFT: unsupported shape");
+  const int nt = grid_rings(bl, ss), nrings = nb * nt;
+  if (nrings <= 0) return;
+  const RingArgs a = ring_args(ring_fft(grid_ring_len(bl, ss)), bl, nrings);
+  GammaFuse gf = gamma_fuse(a, gms, gks, ns, ng, real, c, fw, fms, nt, true);
+  gf.G = G;
+  for (int k = 0; k < nn; ++k)
+    if (real && ns[k] == 0) gf.herm_k = k;
+  const double px = (double)nrings * a.K;
+  KTimer kt(KC_RING, st, timing_enabled() ? ring_work(a, nrings * nn) + gamma_work(px, ng, nn, real) : 0.0,
+            (double)nrings * nn * gf.W * 16.0 + px * ng * (real ? 8.0 : 16.0));
+  switch (nn) {
+#define S2G_FUSE(N)                                                          \
+  case N:                                                                    \
+    if (real)                                                                \
+      launch_fused(k_ring_inverse_gamma<N, true>, a, gf, nrings, N, st);    \
+    else                                                                     \
+      launch_fused(k_ring_inverse_gamma<N, false>, a, gf, nrings, N, st);   \
+    break;
+    S2G_FUSE(2) S2G_FUSE(3) S2G_FUSE(4) S2G_FUSE(5) S2G_FUSE(6) S2G_FUSE(7) S2G_FUSE(8)
+#undef S2G_FUSE
+    default: break;
+  }
+}
+
+void gamma_ring_forward(const void *fw, int64_t fms, const std::vector<int> &ns, int ng, bool real, double c,
+                        double2 *Gout, int64_t gms, int64_t gks, int nb, int bl, int ss, cudaStream_t st) {
+  const int nn = (int)ns.size();
+  S2G_REQUIRE(ring_gamma_fusable(nn, ng, bl, ss), ERR_UNSUPPORTED, "fused ring/gamma DFT: unsupported shape");
+  const int nt = grid_rings(bl, ss), nrings = nb * nt;
+  if (nrings <= 0) return;
+  const RingArgs a = ring_args(ring_fft(grid_ring_len(bl, ss)), bl, nrings);
+  GammaFuse gf = gamma_fuse(a, gms, gks, ns, ng, real, c, const_cast<void *>(fw), fms, nt, false);
+  gf.Gout = Gout;
+  const double px = (double)nrings * a.K;
+  KTimer kt(KC_RING, st, timing_enabled() ? ring_work(a, nrings * nn) + gamma_work(px, ng, nn, real) : 0.0,
+            (double)nrings * nn * gf.W * 16.0 + px * ng * (real ? 8.0 : 16.0));
+  switch (nn) {
+#define S2G_FUSE(N)                                                          \
+  case N:                                                                    \
+    if (real)                                                                \
+      launch_fused(k_gamma_ring_forward<N, true>, a, gf, nrings, N, st);    \
+    else                                                                     \
+      launch_fused(k_gamma_ring_forward<N, false>, a, gf, nrings, N, st);   \
+    break;
+    S2G_FUSE(2) S2G_FUSE(3) S2G_FUSE(4) S2G_FUSE(5) S2G_FUSE(6) S2G_FUSE(7) S2G_FUSE(8)
+#undef S2G_FUSE
+    default: break;
+  }
+}
+
+void ring_forward(const void *rings, int64_t ring_stride, int64_t map_stride, int rpm, double2 *spec,
+                  int64_t spec_stride, int sw, int mlo, int nrings, int bl, int ss, bool real, cudaStream_t st) {
+  if (nrings <= 0) return;
+  const RingFFT &rf = ring_fft(grid_ring_len(bl, ss));
+  RingArgs a = ring_args(rf, bl, nrings);
+  a.rings = rings;
+  a.ring_stride = ring_stride;
+  a.map_stride = map_stride;
+  a.rpm = rpm;
+  a.spec_out = spec;
+  a.spec_stride = spec_stride;
+  a.sw = sw;
+  a.mlo = mlo;
+  run_ring_forward(a, nrings, real, st);
+}
+
+void ring_inverse(const double2 *spec, int64_t spec_stride, int sw, int mlo, void *rings,
+                  int64_t ring_stride, int64_t map_stride, int rpm, int nrings, int bl, int ss, bool real,
+                  cudaStream_t st) {
+  if (nrings <= 0) return;
+  const RingFFT &rf = ring_fft(grid_ring_len(bl, ss));
+  RingArgs a = ring_args(rf, bl, nrings);
+  a.spec_in = spec;
+  a.spec_stride = spec_stride;
+  a.sw = sw;
+  a.mlo = mlo;
+  a.rings_out = (double2 *)rings;
+  a.ring_stride = ring_stride;
+  a.map_stride = map_stride;
+  a.rpm = rpm;
+  run_ring_inverse(a, nrings, real, st);
+}
+
+void ring_forward_c(const double2 *rings, int64_t ring_stride, int64_t map_stride, int rpm, double2 *spec,
+                    int64_t spec_stride, int64_t spec_map_stride, int spec_rpm, int sw, int mlo, int nrings, int bl,
+                    int ss, cudaStream_t st) {
+  if (nrings <= 0) return;
+  const RingFFT &rf = ring_fft(grid_ring_len(bl, ss));
+  RingArgs a = ring_args(rf, bl, nrings);
+  a.rings = rings;
+  a.ring_stride = ring_stride;
+  a.map_stride = map_stride;
+  a.rpm = rpm;
+  a.spec_out = spec;
+  a.spec_stride = spec_stride;
+  a.spec_map_stride = spec_map_stride;
+  a.spec_rpm = spec_rpm;
+  a.sw = sw;
+  a.mlo = mlo;
+  run_ring_forward(a, nrings, false, st);
+}
+
+void ring_inverse_c(const double2 *spec, int64_t spec_stride, int64_t spec_map_stride, int spec_rpm, int sw,
+                    int mlo, bool herm, double2 *rings, int64_t ring_stride, int64_t map_stride, int rpm, int nrings,
+                    int bl, int ss, cudaStream_t st) {
+  if (nrings <= 0) return;
+  const RingFFT &rf = ring_fft(grid_ring_len(bl, ss));
+  RingArgs a = ring_args(rf, bl, nrings);
+  a.spec_in = spec;
+  a.spec_stride = spec_stride;
+  a.spec_map_stride = spec_map_stride;
+  a.spec_rpm = spec_rpm;
+  a.herm = herm ? 1 : 0;
+  a.sw = sw;
+  a.mlo = mlo;
+  a.rings_out = rings;
+  a.ring_stride = ring_stride;
+  a.map_stride = map_stride;
+  a.rpm = rpm;
+  run_ring_inverse(a, nrings, false, st);
+}
+
+}  // namespace s2g
