@@ -414,23 +414,31 @@ int s2let_gpu_last_error(void);
 const char *s2let_gpu_last_error_string(void);
 
 /* Arithmetic used by subsequent calls of this thread.
- *   0 = FP64 throughout (default);
+ *   0 = FP64 (default): FP64 inputs, outputs and rounding error throughout.
+ *       On stored Wigner tables from band-limit 128 the contractions run on
+ *       the tensor cores in eight bf16 digit slices (55-bit operands, products
+ *       summed exactly but for terms below 2^-56 of the operands' scales), as
+ *       long as a third of the device memory stays free beside the sliced
+ *       tables; else, and at smaller band-limits, on the FP64 pipe.  Ring and
+ *       gamma DFTs run in 64-bit block fixed point.
  *   1 = split precision (within 1e-10 of the FP64 path): on stored Wigner
  *       tables the Legendre/Wigner contraction of batches of two maps or
- *       more runs on the tensor cores (bf16 digit slices, FP32 accumulation,
- *       FP64 combination); one-map calls (s2let_gpu_set_df_max_maps) and
- *       band-limits below 128 contract in double-float arithmetic on the FP32
- *       pipe; recomputed tables regenerate and contract in double-float; ring
- *       and gamma DFTs in double-float. */
+ *       more runs on the tensor cores (seven bf16 digit slices; eight for the
+ *       adjoints); one-map calls (s2let_gpu_set_df_max_maps) and band-limits
+ *       below 128 contract in double-float arithmetic on the FP32 pipe;
+ *       recomputed tables regenerate and contract in double-float; ring and
+ *       gamma DFTs as in the FP64 mode. */
 int s2let_gpu_set_precision(int mode);
 int s2let_gpu_get_precision(void);
 
-/* Double-float copies of the stored Wigner tables for the double-float
- * contractions of the split-precision path (1 = default): built on first use,
- * the same size as the FP64 tables, skipped when they would leave less than
- * 4 GiB of device memory free; 0 = split the FP64 values as they are read
- * (slower, no extra memory).  Process-wide; copies are freed by
- * s2let_gpu_release_plans.  Returns the status. */
+/* Optional copies of the stored Wigner tables (1 = default), built on first use
+ * and freed by s2let_gpu_release_plans: the double-float copies of the split-
+ * precision one-map contractions (the size of the FP64 tables; skipped when
+ * they would leave less than 4 GiB of device memory free), and the eight-slice
+ * digit panels of the FP64 mode's contractions and of the adjoints (16 bytes
+ * per table entry; skipped when less than a third of the device memory would
+ * stay free).  0 = no such copies: the FP64 values are read as they are
+ * (slower, no extra memory).  Process-wide.  Returns the status. */
 int s2let_gpu_set_split_tables(int on);
 int s2let_gpu_get_split_tables(void);
 

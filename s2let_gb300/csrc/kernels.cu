@@ -1074,13 +1074,19 @@ int get_split_tables() { return g_split_tables.load(); }
 void set_df_max_maps(int maps) { g_df_max_maps.store(maps); }
 int get_df_max_maps() { return g_df_max_maps.load(); }
 
+namespace {
+// batches that try the tensor-core contractions first: every one in FP64 mode,
+// those past df_max_maps in split-precision mode
+bool on_tensor_cores(int nb) { return t_precision == 0 || nb > df_max_maps(); }
+}  // namespace
+
 void contract_l2t(const L2T &p, cudaStream_t st) {
   if (p.nb <= 0 || p.mhi < p.mlo) return;
   if (p.tb->rc) {
     contract_l2t_rc(p, st);
     return;
   }
-  if (t_precision == 1 && p.nb > df_max_maps() && contract_l2t_mixed(&p, 1, st)) return;
+  if (on_tensor_cores(p.nb) && contract_l2t_mixed(&p, 1, st)) return;
   ContractArgs a{};
   a.table = p.use_q ? p.tb->Q : p.tb->D;
   if (t_precision == 1) a.table_df = df_table(*p.tb, p.use_q, st);
@@ -1117,7 +1123,7 @@ void contract_t2l(const T2L &p, cudaStream_t st) {
     contract_t2l_rc(p, st);
     return;
   }
-  if (t_precision == 1 && p.nb > df_max_maps() && contract_t2l_mixed(&p, 1, st)) return;
+  if (on_tensor_cores(p.nb) && contract_t2l_mixed(&p, 1, st)) return;
   ContractArgs a{};
   a.table = p.use_q ? p.tb->Q : p.tb->D;
   if (t_precision == 1) a.table_df = df_table(*p.tb, p.use_q, st);
@@ -1232,8 +1238,8 @@ bool df_pair_t2l(const T2L *a, cudaStream_t st) {
 
 void contract_l2t_group(const L2T *a, int n, cudaStream_t st) {
   if (n <= 0) return;
-  if (t_precision == 1 && n <= 2 && !a[0].tb->rc) {
-    if (a[0].nb > df_max_maps()) {
+  if (n <= 2 && !a[0].tb->rc) {
+    if (on_tensor_cores(a[0].nb)) {
       if (contract_l2t_mixed(a, n, st)) return;
     } else if (n == 2 && df_pair_l2t(a, st)) {
       return;
@@ -1244,8 +1250,8 @@ void contract_l2t_group(const L2T *a, int n, cudaStream_t st) {
 
 void contract_t2l_group(const T2L *a, int n, cudaStream_t st) {
   if (n <= 0) return;
-  if (t_precision == 1 && n <= 2 && !a[0].tb->rc) {
-    if (a[0].nb > df_max_maps()) {
+  if (n <= 2 && !a[0].tb->rc) {
+    if (on_tensor_cores(a[0].nb)) {
       if (contract_t2l_mixed(a, n, st)) return;
     } else if (n == 2 && df_pair_t2l(a, st)) {
       return;

@@ -1,35 +1,43 @@
-// Split-precision contraction on tcgen05 (see mixed.h for the number format).
+// Contractions on tcgen05 by digit slicing (see mixed.h for the number format).
+//
+// Two forms: 7 slices (28 digit products, the split-precision mode's forward
+// contractions) and 8 slices (36 products, FP64 results: the FP64 mode, and the
+// adjoint contractions of both modes).
 //
 // Layout in HBM
-//   Sliced table, one per (band-limit, |n|, D or Q): for each table m, for each
-//   128-row tile rt, for each 64-wide K-chunk kc, for each digit slice j, a
-//   16 KB panel [128 rows][64 bf16] in the 128-byte-swizzled K-major image that
-//   tcgen05 reads from shared memory; rows and K are zero-padded to the panel.
-//   Row exponents eA (int8) per (m, row).
-//   Sliced coefficients, per call and per problem m: for each kc one 14 KB
-//   panel [7 slices x 16 columns][64 bf16] (16 real columns = 8 complex maps),
-//   column exponents eX (int32) per (m, column).
+//   Sliced table, one per (band-limit, |n|, kind: D or Q, read along or across):
+//     for each table m, for each 128-row tile rt, for each 64-wide K-chunk kc,
+//     for each digit slice j, a 16 KB panel [128 rows][64 bf16] in the
+//     128-byte-swizzled K-major image that tcgen05 reads from shared memory;
+//     rows and K are zero-padded to the panel.  The eighth slice has an array
+//     of its own (it is the remainder of the first seven, which both forms
+//     share).  Row exponents eA (int8) per (m, row).
+//   Sliced coefficients, per call and per problem m: for each kc one panel
+//     [S slices x NC columns][64 bf16], column exponents eX (int32) per (m,
+//     column).
 //
-// Kernel k_contract_mx<NC>: persistent, one CTA per SM, 18 warps; NC real
+// Kernel k_contract_mx<NC, S>: persistent, one CTA per SM, 18 warps; NC real
 // coefficient columns (16, 32 or 64) per table pass.
 //   warp 0    producer: cp.async.bulk of panels into a ring of 16 KB table
 //             stages (10 deep; 6 at NC = 64) and a 2-deep ring of coefficient
-//             stages (7 slices x NC columns x 64 K).
+//             stages (S slices x NC columns x 64 K).
 //   warp 1    MMA issuer: per K-chunk and digit slice j, one 128 x N x 64
 //             product (tcgen05.mma of K=16, N <= 256 each) of table slice j
-//             against the first 7-j coefficient slices, written to the
-//             accumulator columns of classes j..6 (N = NC (7-j)); two TMEM
+//             against the first S-j coefficient slices, written to the
+//             accumulator columns of classes j..S-1 (N = NC (S-j)); two TMEM
 //             accumulators alternate between tiles (one at NC = 64).
 //   warps 2-17 epilogue: four warps per TMEM lane quarter, 16 columns each:
-//             tcgen05.ld of the 7 class accumulators, double-float combine,
-//             row/column exponents, sign, per-l weight, store; the
-//             accumulator is released as soon as its values are in registers.
+//             tcgen05.ld of the S class accumulators, combine (double-float
+//             for 7, integers for 8), row/column exponents, sign, per-l
+//             weight, store; the accumulator is released as soon as its values
+//             are in registers.
 // Every wait is bounded (about 2 s); on expiry the kernel raises an error flag,
 // drains its own copies and MMAs, frees TMEM and returns.
 #include <cstdint>
 #include <map>
 #include <memory>
 #include <mutex>
+#include <set>
 #include <tuple>
 #include <vector>
 
@@ -45,7 +53,8 @@ namespace s2g {
 
 namespace {
 
-constexpr int kS = 7;                  // digit slices per operand
+constexpr int kS = 7;                  // digit slices per operand (split precision)
+constexpr int kSmax = 8;               // and of the 64-bit form (FP64 results)
 constexpr int kB0 = 6;                 // bits of the first digit (later digits: 7)
 constexpr int kPK = 64;                // K per panel
 constexpr int kPM = 128;               // rows per panel
@@ -57,26 +66,24 @@ constexpr int kThreads = 64 + 32 * kEpiWarps;
 constexpr int kMinBl = 128;            // below this the FP64 kernel is used
 constexpr long long kWaitCycles = 4000000000LL;
 
-// NC real coefficient columns per CTA (16, 32 or 64): parts x maps x {re, im}.
-// NC <= 32: two TMEM accumulators alternate between tiles; NC = 64: one
-// accumulator of 448 columns, and a shallower table ring to fit shared memory.
-template <int NC>
+// NC real coefficient columns per CTA (16, 32 or 64): parts x maps x {re, im};
+// S digit slices (7, or 8 for FP64 results).  NC <= 32: two TMEM accumulators
+// alternate between tiles; NC = 64: one accumulator of 64 S columns (all of
+// TMEM at S = 8), and a shallower table ring to fit shared memory.
+template <int NC, int S>
 struct Cfg {
   static constexpr int kAST = NC == 64 ? 6 : 10;       // table pipeline depth
   static constexpr int kNBuf = NC == 64 ? 1 : 2;       // TMEM accumulators
-  static constexpr int kPanelX = kS * NC * kPK;        // elements
-  static constexpr int kAccCols = kS * NC;             // TMEM columns per accumulator
+  static constexpr int kPanelX = S * NC * kPK;         // elements
+  static constexpr int kAccCols = S * NC;              // TMEM columns per accumulator
   static constexpr int kTmemCols = NC == 16 ? 256 : 512;
   static constexpr size_t kSmemA = (size_t)kAST * kPanelA * 2;
   static constexpr size_t kSmemX = (size_t)kXST * kPanelX * 2;
   static constexpr int kNumBars = 2 * kAST + 2 * kXST + 4 + 1;
   static constexpr size_t kSmemBytes = 1024 + kSmemA + kSmemX + kNumBars * 8 + 16;
+  static_assert(kSmemBytes <= 232448, "shared memory");
+  static_assert(kNBuf * kAccCols <= kTmemCols, "TMEM");
 };
-static_assert(Cfg<64>::kSmemBytes <= 232448, "shared memory");
-static_assert(Cfg<32>::kSmemBytes <= 232448, "shared memory");
-static_assert(Cfg<64>::kNBuf * Cfg<64>::kAccCols <= Cfg<64>::kTmemCols, "TMEM");
-static_assert(Cfg<32>::kNBuf * Cfg<32>::kAccCols <= Cfg<32>::kTmemCols, "TMEM");
-static_assert(Cfg<16>::kNBuf * Cfg<16>::kAccCols <= Cfg<16>::kTmemCols, "TMEM");
 
 struct Geom {
   int l0, nl, rows, K, nkc, nrt;
@@ -144,7 +151,42 @@ __device__ __forceinline__ void split_digits(double v, int e, uint16_t *out) {
 #pragma unroll
   for (int j = 0; j < kS; ++j) out[j] = bf16_of_int(d[j]);
 }
-
+// round(v 2^(55-e)) for |v| < 2^e (subnormals included)
+__device__ __forceinline__ long long fixed55(double v, int e) {
+  const uint64_t u = bits_of(v);
+  const int E = (int)((u >> 52) & 0x7FF);
+  const long long M = (long long)((u & 0xFFFFFFFFFFFFFull) | (E ? 1ull << 52 : 0ull));
+  const int sh = (E ? E : 1) - 1075 + 55 - e;  // v 2^(55-e) = M 2^sh, sh <= 2
+  long long q;
+  if (sh >= 0)
+    q = M << sh;
+  else if (sh > -64)
+    q = (M + (1ll << (-sh - 1))) >> (-sh);
+  else
+    q = 0;
+  return (u >> 63) ? -q : q;
+}
+// The eighth digit of a table value: what the seven leave of v 2^-e, in units
+// of 2^-55 (|digit| <= 64; with it the value is represented to 2^-56).
+__device__ __forceinline__ uint16_t eighth_digit(double v, int e) {
+  return bf16_of_int((int)(fixed55(v, e) - fixed48(v, e) * 128));
+}
+// Balanced digits of q 2^-55, |q| < 2^55, as bf16 patterns in the low halves
+// of out: adding 64 in every digit position but the first makes the base-128
+// digits of the sum the balanced ones plus 64; 2^23 + digit is read off the
+// float's bits, and subtracting 2^23 + 64 leaves the digit exactly.
+__device__ __forceinline__ void split_digits_int(long long q, uint32_t *out) {
+  q += 0x0001020408102040ll;  // 64 (1 + 2^7 + ... + 2^42)
+  const uint32_t lo = (uint32_t)q & 0xFFFFFFFu, hi = (uint32_t)(q >> 28);
+  // d_0 = q >> 49 in [-64, 64]: its field holds d_0 + 128 after the offset below
+  out[0] = __float_as_uint(__fsub_rn(__uint_as_float(0x4B000000u | ((hi >> 21) + 128u & 0xFFu)), 8388736.0f)) >> 16;
+#pragma unroll
+  for (int j = 1; j < kSmax; ++j) {
+    const uint32_t w = j < 4 ? hi : lo;
+    const int sh = j < 4 ? 21 - 7 * j : 49 - 7 * j;
+    out[j] = __float_as_uint(__fsub_rn(__uint_as_float(0x4B000000u | ((w >> sh) & 127u)), 8388672.0f)) >> 16;
+  }
+}
 
 struct TableRefM {
   int mi;
@@ -167,9 +209,13 @@ __device__ __forceinline__ TableRefM table_ref_m(int tmlo, int n, int m) {
 // table slicing (plan time)
 // ---------------------------------------------------------------------------
 
+// rows l when q (t -> l) else t; tr: the source block holds the transpose
+// (row k, column row).  panels8 (nullable with panels set, or the reverse):
+// the eighth digit's panels, one per (row tile, K-chunk).
 __global__ void __launch_bounds__(128) k_slice_table(const double *__restrict__ T,
                                                      const int64_t *__restrict__ off, int bl, int nt,
-                                                     int an, int tmlo, int q, uint16_t *__restrict__ panels,
+                                                     int an, int tmlo, int q, int tr, uint16_t *__restrict__ panels,
+                                                     uint16_t *__restrict__ panels8,
                                                      const int64_t *__restrict__ pan_off,
                                                      int8_t *__restrict__ eA,
                                                      const int64_t *__restrict__ e_off) {
@@ -177,28 +223,38 @@ __global__ void __launch_bounds__(128) k_slice_table(const double *__restrict__ 
   const Geom g = geom(bl, nt, an, tmlo + mi, q != 0);
   if (rt >= g.nrt) return;
   const double *Tm = T + off[mi];
+  const int64_t rs = tr ? 1 : g.K, ks = tr ? g.rows : 1;  // strides of the row and of k
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int kpad = g.nkc * kPK;
   for (int rr = warp; rr < kPM; rr += 4) {
     const int row = rt * kPM + rr;
     const bool live = row < g.rows;
-    int mx = 0;
-    if (live)
-      for (int k = lane; k < g.K; k += 32) mx = max(mx, exp_field(Tm[(int64_t)row * g.K + k]));
+    int e;
+    if (panels) {
+      int mx = 0;
+      if (live)
+        for (int k = lane; k < g.K; k += 32) mx = max(mx, exp_field(Tm[row * rs + k * ks]));
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    int e = block_scale(mx);
-    e = e < -126 ? -126 : (e > 126 ? 126 : e);
-    if (lane == 0) eA[e_off[mi] + row] = (int8_t)e;
+      for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+      e = block_scale(mx);
+      e = e < -126 ? -126 : (e > 126 ? 126 : e);
+      if (lane == 0) eA[e_off[mi] + row] = (int8_t)e;
+    } else {
+      e = eA[e_off[mi] + row];
+    }
     for (int k = lane; k < kpad; k += 32) {
-      const double v = (live && k < g.K) ? Tm[(int64_t)row * g.K + k] : 0.0;
-      uint16_t dg[kS];
-      split_digits(v, e, dg);
+      const double v = (live && k < g.K) ? Tm[row * rs + k * ks] : 0.0;
       const int kc = k / kPK;
-      uint16_t *p = panels + pan_off[mi] + (int64_t)(rt * g.nkc + kc) * kS * kPanelA;
+      const int64_t tile = (int64_t)(rt * g.nkc + kc);
       const int idx = swz(rr, k % kPK);
+      if (panels) {
+        uint16_t dg[kS];
+        split_digits(v, e, dg);
+        uint16_t *p = panels + pan_off[mi] + tile * kS * kPanelA;
 #pragma unroll
-      for (int j = 0; j < kS; ++j) p[(int64_t)j * kPanelA + idx] = dg[j];
+        for (int j = 0; j < kS; ++j) p[(int64_t)j * kPanelA + idx] = dg[j];
+      }
+      if (panels8) panels8[pan_off[mi] / kS + tile * kPanelA + idx] = eighth_digit(v, e);
     }
   }
 }
@@ -268,15 +324,16 @@ __device__ __forceinline__ double2 weighted(const Part &P, double2 x, int l) {
 // are read once and the panels written once.
 constexpr int kMG = 4;
 constexpr int kSliceThreads = 256;
+constexpr int kNonFinite = 1 << 20;  // column exponent of a column that holds an infinity or a NaN
 // staged index of K position k: one double2 of padding per 8, so that the
 // 16-byte reads of 8 lanes at K stride 8 fall in distinct banks
 __host__ __device__ __forceinline__ int sv_idx(int k) { return k + (k >> 3); }
 
-template <int NC>
+template <int NC, int S>
 __global__ void __launch_bounds__(kSliceThreads, 3) k_slice_x(XArgs a) {
   extern __shared__ double2 sv[];  // [kMG][a.kst]
   __shared__ int gl0[kMG], gnkc[kMG], gkc0[kMG], gls[kMG], gex[kMG][2];
-  constexpr int PX = Cfg<NC>::kPanelX;
+  constexpr int PX = Cfg<NC, S>::kPanelX;
   const int cp = blockIdx.y, pm0 = blockIdx.x * kMG, c0 = 2 * cp;
   const int part = cp / a.mpp, b = a.b0 + cp % a.mpp;
   const bool live = part < a.nparts && b < a.nb;
@@ -375,12 +432,11 @@ __global__ void __launch_bounds__(kSliceThreads, 3) k_slice_x(XArgs a) {
   if (threadIdx.x < kMG) {
     const int pm = pm0 + threadIdx.x;
     // |v| < 2^e for every value of the column (e = largest unbiased exponent + 1)
-    const int er = block_scale(gex[threadIdx.x][0]), ei = block_scale(gex[threadIdx.x][1]);
-    gex[threadIdx.x][0] = er;
-    gex[threadIdx.x][1] = ei;
-    if (pm < a.nmp) {
-      a.eX[pm * NC + c0] = er;
-      a.eX[pm * NC + c0 + 1] = ei;
+    for (int ri = 0; ri < 2; ++ri) {
+      const int mx = gex[threadIdx.x][ri];
+      const int e = S == kS ? block_scale(mx) : (mx > 1 ? mx : 1) - 1022;
+      gex[threadIdx.x][ri] = e;
+      if (pm < a.nmp) a.eX[pm * NC + c0 + ri] = mx == 2047 ? kNonFinite : e;
     }
   }
   __syncthreads();
@@ -390,19 +446,23 @@ __global__ void __launch_bounds__(kSliceThreads, 3) k_slice_x(XArgs a) {
     const int kc = rest % a.nkcmax, mi = rest / a.nkcmax;
     const int pm = pm0 + mi;
     if (pm >= a.nmp || kc < gkc0[mi] || kc >= gnkc[mi]) continue;
-    uint16_t *p = a.xpan + a.xoff[pm] * (NC / 16) + (int64_t)kc * PX;
+    uint16_t *p = a.xpan + a.xoff[pm] * (NC / 16 * S) + (int64_t)kc * PX;
     const double *col = (const double *)(sv + mi * a.kst);
 #pragma unroll 1
     for (int ri = 0; ri < 2; ++ri) {  // real part (column c0), then imaginary part (c0 + 1)
-      uint32_t pk[kS][4];
+      uint32_t pk[S][4];
       if (live) {
         const int e = gex[mi][ri];
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-          uint32_t d[kS];
-          split_digits_fp32<kS>(col[2 * sv_idx(kc * kPK + h * 8 + q) + ri], e, d);  // dfconv.h
+          const double v = col[2 * sv_idx(kc * kPK + h * 8 + q) + ri];
+          uint32_t d[S];
+          if constexpr (S == kS)
+            split_digits_fp32<kS>(v, e, d);  // dfconv.h
+          else
+            split_digits_int(fixed55(v, e), d);
 #pragma unroll
-          for (int j = 0; j < kS; ++j) {
+          for (int j = 0; j < S; ++j) {
             if (q & 1)
               pk[j][q >> 1] |= d[j] << 16;
             else
@@ -411,12 +471,12 @@ __global__ void __launch_bounds__(kSliceThreads, 3) k_slice_x(XArgs a) {
         }
       } else {
 #pragma unroll
-        for (int j = 0; j < kS; ++j)
+        for (int j = 0; j < S; ++j)
 #pragma unroll
           for (int q = 0; q < 4; ++q) pk[j][q] = 0u;
       }
 #pragma unroll
-      for (int j = 0; j < kS; ++j)
+      for (int j = 0; j < S; ++j)
         *(uint4 *)(p + swz(j * NC + c0 + ri, h * 8)) = make_uint4(pk[j][0], pk[j][1], pk[j][2], pk[j][3]);
     }
   }
@@ -519,7 +579,7 @@ __device__ __forceinline__ void tc_fence_before() {
 
 struct MxArgs {
   int q;  // 0: l -> t with D, 1: t -> l with Q
-  const uint16_t *panels;
+  const uint16_t *panels, *panels8;
   const int64_t *pan_off;
   const int8_t *eA;
   const int64_t *e_off;
@@ -574,10 +634,11 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float *v) {
 #pragma unroll
   for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
 }
-// the 7 class accumulators of 8 columns into registers (waits for the loads)
+// the S class accumulators of 8 columns into registers (waits for the loads)
+template <int S>
 __device__ __forceinline__ void load_classes8(uint32_t taddr, int ncols_per_class, float (*acc)[8]) {
 #pragma unroll
-  for (int c = 0; c < kS; ++c) tmem_ld8(taddr + (uint32_t)(c * ncols_per_class), acc[c]);
+  for (int c = 0; c < S; ++c) tmem_ld8(taddr + (uint32_t)(c * ncols_per_class), acc[c]);
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 // Combine the 7 class accumulators of 8 columns for this thread's row:
@@ -609,23 +670,74 @@ __device__ __forceinline__ void combine8(float (*acc)[8], int ea, int4 e0, int4 
       hi = -hi;
       lo = -lo;
     }
-    y[col] = join_scaled(hi, lo, ea + ex_at(e0, e1, col) - 2 * kB0);
+    const int ex = ex_at(e0, e1, col);
+    y[col] = ex == kNonFinite ? double_of(0x7FF8000000000000ull) : join_scaled(hi, lo, ea + ex - 2 * kB0);
+  }
+}
+// The same for 8 slices and FP64 results: the class sums are integers; classes
+// 0-3 and 4-7 go to two 64-bit words of 43 and 46 bits, their 71-bit sum is
+// normalised and rounded once, in integer arithmetic (an FP64 conversion and
+// sum would take three FP64 instructions per value, more than the tile's MMAs).
+__device__ __forceinline__ double join71(long long hi, long long lo, int k) {  // (hi 2^28 + lo) 2^k
+  hi += lo >> 28;
+  uint32_t l = (uint32_t)lo & 0xFFFFFFFu;
+  const unsigned long long s = (unsigned long long)hi & (1ull << 63);
+  if (s) {  // magnitude of hi 2^28 + l
+    hi = -hi - (l != 0);
+    l = (0u - l) & 0xFFFFFFFu;
+  }
+  unsigned long long a = (unsigned long long)hi;
+  int n, top;  // a normalised by n, exponent of its leading bit
+  if (a >> 28) {
+    n = __clzll((long long)a);
+    top = 63 - n + 28;
+    a = (a << n) | (n >= 28 ? (unsigned long long)l << (n - 28) : (unsigned long long)(l >> (28 - n)));
+  } else {
+    a = (a << 28) | l;
+    if (a == 0) return 0.0;
+    n = __clzll((long long)a);
+    top = 63 - n;
+    a <<= n;
+  }
+  const int E = 1023 + top + k;
+  if (E <= 0 || E >= 2046) {
+    const double d = ldexp((double)(a >> 11), top + k - 52);
+    return s ? -d : d;
+  }
+  return double_of(s | ((((unsigned long long)(E - 1)) << 52) + (a >> 11) + ((a >> 10) & 1)));
+}
+__device__ __forceinline__ void combine8_int(float (*acc)[8], int ea, int4 e0, int4 e1, double sign, double *y) {
+#pragma unroll
+  for (int col = 0; col < 8; ++col) {
+    long long hi = 0, lo = 0;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      hi += (long long)__float2int_rn(acc[c][col]) << (7 * (3 - c));
+      lo += (long long)__float2int_rn(acc[c + 4][col]) << (7 * (3 - c));
+    }
+    if (sign < 0.0) {
+      hi = -hi;
+      lo = -lo;
+    }
+    const int ex = ex_at(e0, e1, col);
+    y[col] = ex == kNonFinite ? double_of(0x7FF8000000000000ull) : join71(hi, lo, ea + ex - 2 * kB0 - 49);
   }
 }
 
-template <int NC>
+template <int NC, int S>
 __global__ void __launch_bounds__(kThreads, 1) k_contract_mx(MxArgs a) {
-  constexpr int PX = Cfg<NC>::kPanelX;
-  constexpr int ACC = Cfg<NC>::kAccCols;
-  constexpr int TMC = Cfg<NC>::kTmemCols;
-  constexpr int kAST = Cfg<NC>::kAST;
-  constexpr int NBUF = Cfg<NC>::kNBuf;
-  constexpr int kNumBars = Cfg<NC>::kNumBars;
+  using C = Cfg<NC, S>;
+  constexpr int PX = C::kPanelX;
+  constexpr int ACC = C::kAccCols;
+  constexpr int TMC = C::kTmemCols;
+  constexpr int kAST = C::kAST;
+  constexpr int NBUF = C::kNBuf;
+  constexpr int kNumBars = C::kNumBars;
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint16_t *sA = (uint16_t *)smem;
-  uint16_t *sX = (uint16_t *)(smem + Cfg<NC>::kSmemA);
-  uint64_t *bars = (uint64_t *)(smem + Cfg<NC>::kSmemA + Cfg<NC>::kSmemX);
+  uint16_t *sX = (uint16_t *)(smem + C::kSmemA);
+  uint64_t *bars = (uint64_t *)(smem + C::kSmemA + C::kSmemX);
   uint64_t *fullA = bars, *emptyA = bars + kAST, *fullX = bars + 2 * kAST, *emptyX = bars + 2 * kAST + kXST;
   uint64_t *tfull = bars + 2 * kAST + 2 * kXST, *tempty = tfull + 2, *mma_done = tfull + 4;
   volatile int *abort_flag = (volatile int *)(bars + kNumBars);
@@ -670,18 +782,20 @@ __global__ void __launch_bounds__(kThreads, 1) k_contract_mx(MxArgs a) {
     for (int t = blockIdx.x; ok && t < a.ntiles * a.ngroups; t += gridDim.x) {
       const TileInfo ti = tile_info(a, t);
       const uint16_t *pan = a.panels + a.pan_off[ti.mi] + (int64_t)ti.rt * ti.nkc * kS * kPanelA;
-      const uint16_t *xp = a.xpan + ti.g * a.xg + a.xoff[ti.pm] * (NC / 16);
+      const uint16_t *pan8 = S == kSmax ? a.panels8 + a.pan_off[ti.mi] / kS + (int64_t)ti.rt * ti.nkc * kPanelA : nullptr;
+      const uint16_t *xp = a.xpan + ti.g * a.xg + a.xoff[ti.pm] * (NC / 16 * S);
       for (int kc = ti.kc0; ok && kc < ti.nkc; ++kc) {
         const int xs = issuedX % kXST;
         if (!(ok = bar_wait(&emptyX[xs], ((issuedX / kXST) & 1) ^ 1, abort_flag, a.err))) break;
         bar_expect_tx(&fullX[xs], PX * 2);
         bulk_g2s(sX + (size_t)xs * PX, xp + (int64_t)kc * PX, PX * 2, &fullX[xs]);
         ++issuedX;
-        for (int j = 0; j < kS; ++j) {
+        for (int j = 0; j < S; ++j) {
           const int as = issuedA % kAST;
           if (!(ok = bar_wait(&emptyA[as], ((issuedA / kAST) & 1) ^ 1, abort_flag, a.err))) break;
           bar_expect_tx(&fullA[as], kPanelA * 2);
-          bulk_g2s(sA + (size_t)as * kPanelA, pan + ((int64_t)kc * kS + j) * kPanelA, kPanelA * 2, &fullA[as]);
+          const uint16_t *src = j < kS ? pan + ((int64_t)kc * kS + j) * kPanelA : pan8 + (int64_t)kc * kPanelA;
+          bulk_g2s(sA + (size_t)as * kPanelA, src, kPanelA * 2, &fullA[as]);
           ++issuedA;
         }
       }
@@ -705,13 +819,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_contract_mx(MxArgs a) {
         if (!(ok = bar_wait(&fullX[xs], (cx / kXST) & 1, abort_flag, a.err))) break;
         tc_fence_after();
         const uint64_t bdesc = sw128_desc(sX + (size_t)xs * PX);
-        for (int j = 0; j < kS; ++j) {
+        for (int j = 0; j < S; ++j) {
           const int as = ca % kAST;
           if (!(ok = bar_wait(&fullA[as], (ca / kAST) & 1, abort_flag, a.err))) break;
           tc_fence_after();
           const uint64_t adesc = sw128_desc(sA + (size_t)as * kPanelA);
-          // B rows [0, NC (7 - j)) -> accumulator columns NC j + row, in MMAs of N <= 256
-          const int ntot = NC * (kS - j);
+          // B rows [0, NC (S - j)) -> accumulator columns NC j + row, in MMAs of N <= 256
+          const int ntot = NC * (S - j);
           for (int off = 0; off < ntot; off += 256) {
             const int n = ntot - off < 256 ? ntot - off : 256;
             const uint32_t idesc = idesc_bf16(kPM, n);
@@ -781,13 +895,16 @@ __global__ void __launch_bounds__(kThreads, 1) k_contract_mx(MxArgs a) {
         const int c0 = pi * 16 + hh * 8;  // first column of this half
         double y[8];
         if (live) {
-          float acc[kS][8];
-          load_classes8(taddr + (uint32_t)c0, NC, acc);
+          float acc[S][8];
+          load_classes8<S>(taddr + (uint32_t)c0, NC, acc);
           if (hh == 1) {  // every column of this warp is in registers: hand the accumulator back
             tc_fence_before();
             bar_arrive(&tempty[ab]);
           }
-          combine8(acc, ea, hh ? ex4[2] : ex4[0], hh ? ex4[3] : ex4[1], ti.sign, y);
+          if constexpr (S == kS)
+            combine8(acc, ea, hh ? ex4[2] : ex4[0], hh ? ex4[3] : ex4[1], ti.sign, y);
+          else
+            combine8_int(acc, ea, hh ? ex4[2] : ex4[0], hh ? ex4[3] : ex4[1], ti.sign, y);
         } else {
 #pragma unroll
           for (int col = 0; col < 8; ++col) y[col] = 0.0;
@@ -846,18 +963,39 @@ struct TileList {
   int64_t work_entries = 0;  // table entries streamed per launch (all tiles)
 };
 
+// Which table a contraction reads, and how: rows of the panels are t (l -> t)
+// or l (t -> l), from D[t][l] or Q[l][t]; two of the four read it transposed.
+enum TableKind { TK_L2T_D = 0, TK_T2L_Q = 1, TK_L2T_Q = 2, TK_T2L_D = 3 };
+bool kind_rows_l(int kind) { return kind == TK_T2L_Q || kind == TK_T2L_D; }
+bool kind_of_q(int kind) { return kind == TK_T2L_Q || kind == TK_L2T_Q; }
+bool kind_transposed(int kind) { return kind == TK_L2T_Q || kind == TK_T2L_D; }
+
 struct SlicedTable {
   int bl = 0, nt = 0, an = 0, mlo = 0, nm = 0;
-  bool q = false;
-  uint16_t *panels = nullptr;
+  bool q = false;    // rows l
+  uint16_t *panels = nullptr;   // 7 digit slices
+  uint16_t *panels8 = nullptr;  // the eighth, built when an FP64 contraction first needs it
   int8_t *eA = nullptr;
   int64_t *d_pan_off = nullptr, *d_e_off = nullptr;
   size_t bytes = 0;
   std::map<std::tuple<int, int, int, int>, TileList> lists;  // (n, mlo, mhi, lmin)
+  void release() {
+    cudaFree(panels);
+    cudaFree(panels8);
+    cudaFree(eA);
+    cudaFree(d_pan_off);
+    cudaFree(d_e_off);
+    for (auto &l : lists) {
+      cudaFree(l.second.d_tiles);
+      cudaFree(l.second.d_xoff);
+    }
+  }
 };
 
 std::mutex g_mx_mu;
-std::map<std::tuple<int, int, int, int>, std::unique_ptr<SlicedTable>> g_sliced;  // (bl, an, ss, q)
+using TableKey = std::tuple<int, int, int, int>;  // (bl, an, ss, kind)
+std::map<TableKey, std::unique_ptr<SlicedTable>> g_sliced;
+std::set<TableKey> g_refused;  // optional tables that did not fit when first wanted
 size_t g_mx_bytes = 0;
 int *g_err = nullptr;
 
@@ -869,17 +1007,25 @@ T *dev_alloc(size_t n, size_t *acc) {
   return (T *)p;
 }
 
-SlicedTable &sliced(const WignerTable &tb, bool q, cudaStream_t st) {
-  auto key = std::make_tuple(tb.bl, tb.an, tb.ss, q ? 1 : 0);
+bool capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  S2G_CUDA(cudaStreamIsCapturing(st, &cap));
+  return cap != cudaStreamCaptureStatusNone;
+}
+
+// Panels of one table and kind (caller holds g_mx_mu).  The split-precision
+// forward contractions cannot do without theirs; the others (with the eighth
+// digit) are optional: the FP64 and double-float kernels take over (nullptr)
+// when table copies are switched off (s2let_gpu_set_split_tables), when less
+// than a third of the device memory would stay free, or when a stream capture
+// meets a table that no earlier call has built.  A refusal stands until the
+// plans are released, so that a program's route does not change under it.
+SlicedTable *sliced(const WignerTable &tb, int kind, bool eighth, cudaStream_t st) {
+  const TableKey key = std::make_tuple(tb.bl, tb.an, tb.ss, kind);
   auto it = g_sliced.find(key);
-  if (it != g_sliced.end()) return *it->second;
-  auto s = std::make_unique<SlicedTable>();
-  s->bl = tb.bl;
-  s->nt = tb.nt;
-  s->an = tb.an;
-  s->mlo = tb.mlo;
-  s->nm = tb.nm;
-  s->q = q;
+  if (it != g_sliced.end() && (!eighth || it->second->panels8)) return it->second.get();
+  if (eighth && (!get_split_tables() || g_refused.count(key) || capturing(st))) return nullptr;
+  const bool fresh = it == g_sliced.end(), q = kind_rows_l(kind);
   std::vector<int64_t> po(tb.nm), eo(tb.nm);
   int64_t ptot = 0, etot = 0;
   for (int mi = 0; mi < tb.nm; ++mi) {
@@ -889,30 +1035,67 @@ SlicedTable &sliced(const WignerTable &tb, bool q, cudaStream_t st) {
     ptot += (int64_t)g.nrt * g.nkc * kS * kPanelA;
     etot += (int64_t)g.nrt * kPM;
   }
+  if (eighth) {
+    const size_t need = sizeof(uint16_t) * (size_t)(ptot / kS) * (fresh ? kSmax : 1);
+    size_t fr = 0, tot = 0;
+    S2G_CUDA(cudaMemGetInfo(&fr, &tot));
+    if (fr < need + tot / 3) {
+      g_refused.insert(key);
+      return nullptr;
+    }
+  }
+  std::unique_ptr<SlicedTable> made;
+  SlicedTable *s = fresh ? nullptr : it->second.get();
   size_t by = 0;
-  s->panels = dev_alloc<uint16_t>((size_t)ptot, &by);
-  s->eA = dev_alloc<int8_t>((size_t)etot, &by);
-  s->d_pan_off = dev_alloc<int64_t>(tb.nm, &by);
-  s->d_e_off = dev_alloc<int64_t>(tb.nm, &by);
-  S2G_CUDA(cudaMemcpyAsync(s->d_pan_off, po.data(), sizeof(int64_t) * tb.nm, cudaMemcpyHostToDevice, st));
-  S2G_CUDA(cudaMemcpyAsync(s->d_e_off, eo.data(), sizeof(int64_t) * tb.nm, cudaMemcpyHostToDevice, st));
-  int nrt_max = (std::max(tb.bl, tb.nt) + kPM - 1) / kPM;
-  dim3 grid(tb.nm, nrt_max);
-  k_slice_table<<<grid, 128, 0, st>>>(q ? tb.Q : tb.D, tb.d_off, tb.bl, tb.nt, tb.an, tb.mlo, q ? 1 : 0,
-                                      s->panels, s->d_pan_off, s->eA, s->d_e_off);
-  S2G_LAUNCHED();
-  S2G_CUDA(cudaStreamSynchronize(st));
-  s->bytes = by;
+  if (fresh) {
+    made = std::make_unique<SlicedTable>();
+    s = made.get();
+    s->bl = tb.bl;
+    s->nt = tb.nt;
+    s->an = tb.an;
+    s->mlo = tb.mlo;
+    s->nm = tb.nm;
+    s->q = q;
+  }
+  uint16_t *p8 = nullptr;
+  try {
+    if (fresh) {
+      s->panels = dev_alloc<uint16_t>((size_t)ptot, &by);
+      s->eA = dev_alloc<int8_t>((size_t)etot, &by);
+      s->d_pan_off = dev_alloc<int64_t>(tb.nm, &by);
+      s->d_e_off = dev_alloc<int64_t>(tb.nm, &by);
+      S2G_CUDA(cudaMemcpyAsync(s->d_pan_off, po.data(), sizeof(int64_t) * tb.nm, cudaMemcpyHostToDevice, st));
+      S2G_CUDA(cudaMemcpyAsync(s->d_e_off, eo.data(), sizeof(int64_t) * tb.nm, cudaMemcpyHostToDevice, st));
+    }
+    if (eighth) p8 = dev_alloc<uint16_t>((size_t)(ptot / kS), &by);
+    const dim3 grid(tb.nm, (std::max(tb.bl, tb.nt) + kPM - 1) / kPM);
+    k_slice_table<<<grid, 128, 0, st>>>(kind_of_q(kind) ? tb.Q : tb.D, tb.d_off, tb.bl, tb.nt, tb.an, tb.mlo,
+                                        q ? 1 : 0, kind_transposed(kind) ? 1 : 0, fresh ? s->panels : nullptr, p8,
+                                        s->d_pan_off, s->eA, s->d_e_off);
+    S2G_LAUNCHED();
+    S2G_CUDA(cudaStreamSynchronize(st));
+  } catch (const Error &e) {
+    if (fresh) s->release();
+    cudaFree(p8);
+    if (!eighth || e.code != ERR_NOMEM) throw;
+    cudaGetLastError();
+    g_refused.insert(key);
+    return nullptr;
+  }
+  if (p8) s->panels8 = p8;
+  s->bytes += by;
   g_mx_bytes += by;
-  SlicedTable &ref = *s;
-  g_sliced.emplace(key, std::move(s));
-  return ref;
+  if (fresh) g_sliced.emplace(key, std::move(made));
+  return s;
 }
 
-const TileList &tile_list(SlicedTable &s, int n, int mlo, int mhi, int lmin, cudaStream_t st) {
+// tiles of one problem (caller holds g_mx_mu); nullptr when a stream capture
+// meets an optional one (see sliced)
+const TileList *tile_list(SlicedTable &s, int n, int mlo, int mhi, int lmin, bool optional, cudaStream_t st) {
   auto key = std::make_tuple(n, mlo, mhi, lmin);
   auto it = s.lists.find(key);
-  if (it != s.lists.end()) return it->second;
+  if (it != s.lists.end()) return &it->second;
+  if (optional && capturing(st)) return nullptr;
   TileList L;
   std::vector<int2> tiles;
   std::vector<int64_t> xoff(mhi - mlo + 1);
@@ -920,7 +1103,7 @@ const TileList &tile_list(SlicedTable &s, int n, int mlo, int mhi, int lmin, cud
   for (int m = mlo; m <= mhi; ++m) {
     const Geom g = geom(s.bl, s.nt, s.an, m, s.q);
     xoff[m - mlo] = xe;
-    xe += (int64_t)g.nkc * Cfg<16>::kPanelX;
+    xe += (int64_t)g.nkc * 16 * kPK;  // per digit slice and 16 columns
     if (g.nl <= 0) continue;
     const int lst = g.l0 > lmin ? g.l0 : lmin;
     int rt0 = 0, kc0 = 0;
@@ -947,7 +1130,7 @@ const TileList &tile_list(SlicedTable &s, int n, int mlo, int mhi, int lmin, cud
   S2G_CUDA(cudaStreamSynchronize(st));
   g_mx_bytes += by;
   s.bytes += by;
-  return s.lists.emplace(key, L).first->second;
+  return &s.lists.emplace(key, L).first->second;
 }
 
 int num_sms() {
@@ -969,7 +1152,8 @@ int *error_flag() {
 }
 
 struct Problem {
-  bool q;
+  int kind;     // TableKind
+  bool eighth;  // 8 digit slices
   const WignerTable *tb;
   int n, mlo, mhi;
   int nparts;
@@ -977,35 +1161,40 @@ struct Problem {
   int nb;
 };
 
-template <int NC>
-void run_mixed(const Problem &p, cudaStream_t st, int gpl_max) {
+// a problem's table panels and tiles
+struct Prepared {
+  SlicedTable *s = nullptr;
+  const TileList *L = nullptr;
+  int *err = nullptr;
+  int lmin = 0;
+};
+
+// False (nothing launched) when an optional problem's coefficient panels do
+// not fit in device memory.
+template <int NC, int S>
+bool run_mixed(const Problem &p, const Prepared &pr, cudaStream_t st, int gpl_max) {
+  using C = Cfg<NC, S>;
   static const bool attr = [] {  // once per instantiation (thread-safe static initialisation)
-    S2G_CUDA(cudaFuncSetAttribute(k_contract_mx<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)Cfg<NC>::kSmemBytes));
+    S2G_CUDA(cudaFuncSetAttribute(k_contract_mx<NC, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)C::kSmemBytes));
     return true;
   }();
   (void)attr;
-  int lmin = p.part[0].lmin;
-  for (int i = 1; i < p.nparts; ++i) lmin = std::min(lmin, p.part[i].lmin);
-  SlicedTable *s;
-  const TileList *L;
-  int *err;
-  {
-    std::lock_guard<std::mutex> lk(g_mx_mu);
-    s = &sliced(*p.tb, p.q, st);
-    L = &tile_list(*s, p.n, p.mlo, p.mhi, lmin, st);
-    err = error_flag();
-  }
+  const bool q = kind_rows_l(p.kind);
+  const SlicedTable *s = pr.s;
+  const TileList *L = pr.L;
+  int *err = pr.err;
+  const int lmin = pr.lmin;
   const int nmp = p.mhi - p.mlo + 1;
   const int mpp = NC / (2 * p.nparts);  // maps per part per launch
   int nkcmax = 0;
-  for (int pm = 0; pm < nmp; ++pm) nkcmax = std::max(nkcmax, geom(p.tb->bl, p.tb->nt, p.tb->an, p.mlo + pm, p.q).nkc);
+  for (int pm = 0; pm < nmp; ++pm) nkcmax = std::max(nkcmax, geom(p.tb->bl, p.tb->nt, p.tb->an, p.mlo + pm, q).nkc);
   const size_t slice_smem = sizeof(double2) * kMG * (size_t)sv_idx(nkcmax * kPK);
   constexpr int kSliceSmemMax = 232448 - 1024;  // the opt-in maximum less the static arrays
   S2G_REQUIRE(slice_smem <= (size_t)kSliceSmemMax, ERR_INVALID,
               "coefficient slicing: K too large for shared-memory staging");
   static const bool attr_x = [] {
-    S2G_CUDA(cudaFuncSetAttribute(k_slice_x<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSliceSmemMax));
+    S2G_CUDA(cudaFuncSetAttribute(k_slice_x<NC, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSliceSmemMax));
     return true;
   }();
   (void)attr_x;
@@ -1013,13 +1202,18 @@ void run_mixed(const Problem &p, cudaStream_t st, int gpl_max) {
   // map groups run up to gpl_max at a time in one launch (their tiles
   // interleaved, the table read once from HBM and again from L2)
   const int gpl = ngroups < gpl_max ? ngroups : gpl_max;
-  // coefficient panels: the tile list's offsets count 16-column panels; an
-  // NC-column panel is NC/16 times larger, so offsets scale by NC/16
-  const int64_t x_elems = L->x_elems * (NC / 16);
+  // coefficient panels: the tile list's offsets count one slice of 16 columns
+  const int64_t x_elems = L->x_elems * (NC / 16 * S);
   uint16_t *xpan = nullptr;
   int *eX = nullptr;
   const int64_t *xoff = L->d_xoff;
-  S2G_CUDA(cudaMallocAsync((void **)&xpan, sizeof(uint16_t) * (size_t)(x_elems ? x_elems * gpl : 1), st));
+  const cudaError_t got =
+      cudaMallocAsync((void **)&xpan, sizeof(uint16_t) * (size_t)(x_elems ? x_elems * gpl : 1), st);
+  if (got == cudaErrorMemoryAllocation && p.eighth) {
+    cudaGetLastError();
+    return false;
+  }
+  S2G_CUDA(got);
   S2G_CUDA(cudaMallocAsync((void **)&eX, sizeof(int) * (size_t)nmp * NC * gpl, st));
   const double entries = (double)L->work_entries;
   for (int g0 = 0; g0 < ngroups; g0 += gpl) {
@@ -1031,11 +1225,11 @@ void run_mixed(const Problem &p, cudaStream_t st, int gpl_max) {
       double xby = 0;
       if (timing_enabled()) {
         fl += 4.0 * entries * nbg * p.nparts;
-        by += entries * 2.0 * kS + (double)x_elems * 2.0 + 16.0 * nbg * p.nparts * (double)p.tb->nt * nmp;
-        xby = (double)x_elems * 2.0 * (1.0 + 8.0 / (2.0 * kS));  // panels written + FP64 values read
+        by += entries * 2.0 * S + (double)x_elems * 2.0 + 16.0 * nbg * p.nparts * (double)p.tb->nt * nmp;
+        xby = (double)x_elems * 2.0 * (1.0 + 8.0 / (2.0 * S));  // panels written + FP64 values read
       }
       XArgs xa{};
-      xa.q = p.q ? 1 : 0;
+      xa.q = q ? 1 : 0;
       xa.bl = p.tb->bl;
       xa.nt = p.tb->nt;
       xa.an = p.tb->an;
@@ -1053,14 +1247,15 @@ void run_mixed(const Problem &p, cudaStream_t st, int gpl_max) {
       xa.nkcmax = nkcmax;
       xa.kst = sv_idx(nkcmax * kPK);
       KTimer kx(KC_SLICE, st, 0.0, xby);
-      k_slice_x<NC><<<dim3((nmp + kMG - 1) / kMG, NC / 2), kSliceThreads, slice_smem, st>>>(xa);
+      k_slice_x<NC, S><<<dim3((nmp + kMG - 1) / kMG, NC / 2), kSliceThreads, slice_smem, st>>>(xa);
       S2G_LAUNCHED();
     }
     if (L->ntiles == 0) continue;
     KTimer kt(KC_MIXED, st, fl, by);
     MxArgs ma{};
-    ma.q = p.q ? 1 : 0;
+    ma.q = q ? 1 : 0;
     ma.panels = s->panels;
+    ma.panels8 = s->panels8;
     ma.pan_off = s->d_pan_off;
     ma.eA = s->eA;
     ma.e_off = s->d_e_off;
@@ -1087,11 +1282,12 @@ void run_mixed(const Problem &p, cudaStream_t st, int gpl_max) {
     ma.err = err;
     const int nwork = L->ntiles * ng;
     const int grid = nwork < num_sms() ? nwork : num_sms();
-    k_contract_mx<NC><<<grid, kThreads, Cfg<NC>::kSmemBytes, st>>>(ma);
+    k_contract_mx<NC, S><<<grid, kThreads, C::kSmemBytes, st>>>(ma);
     S2G_LAUNCHED();
   }
   cudaFreeAsync(xpan, st);
   cudaFreeAsync(eX, st);
+  return true;
 }
 
 // Columns per table pass (2 (re, im) x maps x parts) and map groups per launch.
@@ -1099,7 +1295,8 @@ void run_mixed(const Problem &p, cudaStream_t st, int gpl_max) {
 // (larger batches loop over map groups), 4 groups per launch.  With tuning
 // on, the candidates below are timed per (band-limit bucket, column bucket,
 // direction) and the fastest kept.
-void run_problem(const Problem &p, cudaStream_t st) {
+template <int S>
+bool run_shapes(const Problem &p, const Prepared &pr, cudaStream_t st) {
   struct Shape {
     int nc, gpl;
   };
@@ -1109,16 +1306,28 @@ void run_problem(const Problem &p, cudaStream_t st) {
   // a candidate narrower than one part's two columns cannot hold a map
   const int first = 2 * p.nparts > 16 ? (2 * p.nparts > 32 ? 4 : 2) : 0;
   const auto run = [&](const Shape &sh) {
-    if (sh.nc == 16)
-      run_mixed<16>(p, st, sh.gpl);
-    else if (sh.nc == 32)
-      run_mixed<32>(p, st, sh.gpl);
-    else
-      run_mixed<64>(p, st, sh.gpl);
+    if (sh.nc == 16) return run_mixed<16, S>(p, pr, st, sh.gpl);
+    if (sh.nc == 32) return run_mixed<32, S>(p, pr, st, sh.gpl);
+    return run_mixed<64, S>(p, pr, st, sh.gpl);
   };
-  const int c = tuned(TF_MIXED, tune_bucket(p.tb->bl), tune_bucket(cols), p.q ? 1 : 0, 7 - first, def - first, st,
-                      [&](int i) { run(kCand[first + i]); });
-  run(kCand[first + c]);
+  const int c = tuned(TF_MIXED, tune_bucket(p.tb->bl), tune_bucket(cols), p.kind + (S == kSmax ? 4 : 0), 7 - first,
+                      def - first, st, [&](int i) { run(kCand[first + i]); });
+  return run(kCand[first + c]);
+}
+
+// false when the problem's optional table panels are not to be had
+bool run_problem(const Problem &p, cudaStream_t st) {
+  Prepared pr;
+  pr.lmin = p.part[0].lmin;
+  for (int i = 1; i < p.nparts; ++i) pr.lmin = std::min(pr.lmin, p.part[i].lmin);
+  {
+    std::lock_guard<std::mutex> lk(g_mx_mu);
+    pr.s = sliced(*p.tb, p.kind, p.eighth, st);
+    if (pr.s) pr.L = tile_list(*pr.s, p.n, p.mlo, p.mhi, pr.lmin, p.eighth, st);
+    if (!pr.L) return false;
+    pr.err = error_flag();
+  }
+  return p.eighth ? run_shapes<kSmax>(p, pr, st) : run_shapes<kS>(p, pr, st);
 }
 
 Part part_of(const L2T &a) {
@@ -1161,31 +1370,29 @@ bool same_problem(const A &x, const A &y) {
 
 }  // namespace
 
-bool contract_l2t_mixed(const L2T *a, int nparts, cudaStream_t st) {
-  if (nparts < 1 || nparts > kMaxParts) return false;
-  if (a[0].use_q || a[0].tb->bl < kMinBl || a[0].nb <= 0 || a[0].mhi < a[0].mlo) return false;
-  for (int i = 1; i < nparts; ++i)
-    if (!same_problem(a[0], a[i])) return false;
-  Problem p{};
-  p.q = false;
-  p.tb = a[0].tb;
-  p.n = a[0].n;
-  p.mlo = a[0].mlo;
-  p.mhi = a[0].mhi;
-  p.nb = a[0].nb;
-  p.nparts = nparts;
-  for (int i = 0; i < nparts; ++i) p.part[i] = part_of(a[i]);
-  run_problem(p, st);
-  return true;
-}
+namespace {
+// The split-precision mode's forward contractions take 7 slices; the FP64 mode
+// and the adjoints of both modes 8.  Eight slices hold every value to 2^-56 of
+// its row's (column's) power of two; the dropped products (i + j = 8) and the
+// representation errors add about 2^-56 per term, summed exactly: classes 0-2
+// are exact up to reduction ranges of 1365 (longer ones stay on the FP64
+// kernels), the rounding of the others is below 2^-45-21 of the result.  An FP64
+// sum rounds each partial sum to 2^-53 of it.  Measured against a 64-bit
+// reference, errors equal the FP64 kernels' to 1 % at L = 128 to 1024 (7.6e-13 /
+// 7.5e-13 of f_wav at L = 1024), and px2wav + wav2px of 2 maps at L = 1024, N = 4
+// contracts in 15.8 ms against 64.9 on the FP64 pipe.
+constexpr int kMaxK8 = 1365;
 
-bool contract_t2l_mixed(const T2L *a, int nparts, cudaStream_t st) {
+template <class A>
+bool contract_mixed(const A *a, int nparts, int kind, cudaStream_t st) {
   if (nparts < 1 || nparts > kMaxParts) return false;
-  if (!a[0].use_q || a[0].tb->bl < kMinBl || a[0].nb <= 0 || a[0].mhi < a[0].mlo) return false;
+  if (a[0].tb->bl < kMinBl || a[0].nb <= 0 || a[0].mhi < a[0].mlo) return false;
   for (int i = 1; i < nparts; ++i)
     if (!same_problem(a[0], a[i])) return false;
   Problem p{};
-  p.q = true;
+  p.kind = kind;
+  p.eighth = t_precision == 0 || kind_transposed(kind);
+  if (p.eighth && std::max(a[0].tb->bl, a[0].tb->nt) > kMaxK8) return false;
   p.tb = a[0].tb;
   p.n = a[0].n;
   p.mlo = a[0].mlo;
@@ -1193,24 +1400,22 @@ bool contract_t2l_mixed(const T2L *a, int nparts, cudaStream_t st) {
   p.nb = a[0].nb;
   p.nparts = nparts;
   for (int i = 0; i < nparts; ++i) p.part[i] = part_of(a[i]);
-  run_problem(p, st);
-  return true;
+  return run_problem(p, st);
+}
+}  // namespace
+
+bool contract_l2t_mixed(const L2T *a, int nparts, cudaStream_t st) {
+  return contract_mixed(a, nparts, a[0].use_q ? TK_L2T_Q : TK_L2T_D, st);
+}
+bool contract_t2l_mixed(const T2L *a, int nparts, cudaStream_t st) {
+  return contract_mixed(a, nparts, a[0].use_q ? TK_T2L_Q : TK_T2L_D, st);
 }
 
 void release_sliced_tables() {
   std::lock_guard<std::mutex> lk(g_mx_mu);
-  for (auto &kv : g_sliced) {
-    SlicedTable &s = *kv.second;
-    cudaFree(s.panels);
-    cudaFree(s.eA);
-    cudaFree(s.d_pan_off);
-    cudaFree(s.d_e_off);
-    for (auto &l : s.lists) {
-      cudaFree(l.second.d_tiles);
-      cudaFree(l.second.d_xoff);
-    }
-  }
+  for (auto &kv : g_sliced) kv.second->release();
   g_sliced.clear();
+  g_refused.clear();
   g_mx_bytes = 0;
 }
 

@@ -1,14 +1,17 @@
-// Split-precision Legendre/Wigner contraction on the tcgen05 tensor cores.
+// Legendre/Wigner contractions on the tcgen05 tensor cores by digit slicing.
 //
 // Every FP64 operand row (a table row, a coefficient column) is written as
-// 2^e * sum_{i<7} d_i 2^{-6-7i} with integer digits |d_i| <= 64 held exactly in
-// bf16.  The 28 digit products with i + j <= 6 are accumulated in FP32 by
-// tcgen05.mma; a class c = i + j sums at most c + 1 products of magnitude
-// <= 2^12 over K <= 1024 terms, so classes 0..2 are exact integers and the
-// rounding of the others sits below 2^-45 of the result.  The epilogue
-// combines the classes in FP64.  Truncation error: about 2^-41 of
-// max|row| * max|column| per term (measured 2.5e-12 normwise on adversarial
-// synthetic rows; the FP64 oracle tolerance of the path is 1e-10).
+// 2^e * sum_{i<S} d_i 2^{-6-7i} with integer digits |d_i| <= 64 held exactly in
+// bf16.  The digit products with i + j < S (28 for S = 7, 36 for S = 8) are
+// accumulated in FP32 by tcgen05.mma; a class c = i + j sums at most c + 1
+// products of magnitude <= 2^12 over K <= 1024 terms, so classes 0..2 are exact
+// integers and the rounding of the others sits below 2^-45 of the result.
+// S = 7 (split precision): the epilogue combines the classes in double-float;
+// truncation error about 2^-41 of max|row| * max|column| per term (measured
+// 2.5e-12 normwise on adversarial synthetic rows; the oracle tolerance of the
+// path is 1e-10).  S = 8 (FP64 mode, adjoints): combined in integers and rounded
+// once, 2^-56 of max|row| * max|column| per term, no more than the rounding of
+// an FP64 sum.  A column that holds an infinity or a NaN gives NaN.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -18,8 +21,9 @@
 namespace s2g {
 
 // True when the contraction ran on the tensor cores; false when the problem is
-// outside the split-precision kernel's domain (small band-limit, adjoint table
-// orientation) and the caller must run the FP64 kernel.
+// outside the kernel's domain (small band-limit, a reduction too long for FP64
+// results, no room for the optional table panels) and the caller must run the
+// FP64 or double-float kernel.
 // nparts (1 or 2) problems that differ only in their coefficients, weights,
 // lmin and outputs (scales sharing one band-limit and n) share one pass over
 // the table.
