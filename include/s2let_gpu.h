@@ -415,7 +415,7 @@ const char *s2let_gpu_last_error_string(void);
 
 /* Arithmetic used by subsequent calls of this thread.
  *   0 = FP64 (default): FP64 inputs, outputs and rounding error throughout.
- *       On stored Wigner tables from band-limit 128 the contractions run on
+ *       On stored Wigner tables from band-limit 64 the contractions run on
  *       the tensor cores in eight bf16 digit slices (55-bit operands, products
  *       summed exactly but for terms below 2^-56 of the operands' scales), as
  *       long as a third of the device memory stays free beside the sliced
@@ -424,8 +424,9 @@ const char *s2let_gpu_last_error_string(void);
  *   1 = split precision (within 1e-10 of the FP64 path): on stored Wigner
  *       tables the Legendre/Wigner contraction of batches of two maps or
  *       more runs on the tensor cores (seven bf16 digit slices; eight for the
- *       adjoints); one-map calls (s2let_gpu_set_df_max_maps) and band-limits
- *       below 128 contract in double-float arithmetic on the FP32 pipe;
+ *       adjoints and band-limits 64 to 127); one-map calls
+ *       (s2let_gpu_set_df_max_maps) and smaller band-limits contract in
+ *       double-float arithmetic on the FP32 pipe;
  *       recomputed tables regenerate and contract in double-float; ring and
  *       gamma DFTs as in the FP64 mode. */
 int s2let_gpu_set_precision(int mode);

@@ -63,7 +63,12 @@ constexpr int kMaxParts = 2;           // scales sharing one table pass
 constexpr int kXST = 2;                // coefficient pipeline depth
 constexpr int kEpiWarps = 16;          // four warps per TMEM lane quarter, one 16-column chunk each
 constexpr int kThreads = 64 + 32 * kEpiWarps;
-constexpr int kMinBl = 128;            // below this the FP64 kernel is used
+constexpr int kMinBl = 128;            // 7 slices from this band-limit
+// 8 slices from this band-limit, whatever the batch (so that a map's result does
+// not depend on its batch).  Per contraction at bl = 64, FP64 kernel against
+// slicing + contraction: 1 map 16 / 26 us, 8 complex maps 50 / 28, 32 maps 77 /
+// 38; at bl = 32 8 maps 28 / 29, 32 maps 37 / 30.
+constexpr int kMinBl8 = 64;
 constexpr long long kWaitCycles = 4000000000LL;
 
 // NC real coefficient columns per CTA (16, 32 or 64): parts x maps x {re, im};
@@ -1371,7 +1376,8 @@ bool same_problem(const A &x, const A &y) {
 }  // namespace
 
 namespace {
-// The split-precision mode's forward contractions take 7 slices; the FP64 mode
+// The split-precision mode's forward contractions take 7 slices (8 below
+// band-limit 128, where double-float would be the alternative); the FP64 mode
 // and the adjoints of both modes 8.  Eight slices hold every value to 2^-56 of
 // its row's (column's) power of two; the dropped products (i + j = 8) and the
 // representation errors add about 2^-56 per term, summed exactly: classes 0-2
@@ -1386,12 +1392,12 @@ constexpr int kMaxK8 = 1365;
 template <class A>
 bool contract_mixed(const A *a, int nparts, int kind, cudaStream_t st) {
   if (nparts < 1 || nparts > kMaxParts) return false;
-  if (a[0].tb->bl < kMinBl || a[0].nb <= 0 || a[0].mhi < a[0].mlo) return false;
+  if (a[0].tb->bl < kMinBl8 || a[0].nb <= 0 || a[0].mhi < a[0].mlo) return false;
   for (int i = 1; i < nparts; ++i)
     if (!same_problem(a[0], a[i])) return false;
   Problem p{};
   p.kind = kind;
-  p.eighth = t_precision == 0 || kind_transposed(kind);
+  p.eighth = t_precision == 0 || kind_transposed(kind) || a[0].tb->bl < kMinBl;
   if (p.eighth && std::max(a[0].tb->bl, a[0].tb->nt) > kMaxK8) return false;
   p.tb = a[0].tb;
   p.n = a[0].n;

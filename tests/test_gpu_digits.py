@@ -15,8 +15,8 @@ from conftest import rel_err
 from s2let_gb300.capi import make_parameters
 
 TOL = 1e-12
-# L, N, spin, real, sampling: L = 128 (+-1: one row tile and K-chunk edge), 192, 193 (K = 3 x 64 and past it), 257
-CASES = [(128, 3, 0, True, 0), (129, 2, 1, False, 0), (128, 2, 0, True, 1), (192, 1, 0, False, 0),
+# L, N, spin, real, sampling: L = 64 (the smallest), 128 (+-1: one row tile and K-chunk edge), 192, 193 (K = 3 x 64 and past it), 257
+CASES = [(64, 3, 0, True, 0), (65, 2, 1, False, 1), (100, 4, 0, True, 0), (128, 3, 0, True, 0), (129, 2, 1, False, 0), (128, 2, 0, True, 1), (192, 1, 0, False, 0),
          (193, 4, 0, True, 0), (160, 3, 2, False, 1), (257, 2, 0, True, 0)]
 
 
