@@ -7,30 +7,43 @@
 // Layout in HBM
 //   Sliced table, one per (band-limit, |n|, kind: D or Q, read along or across):
 //     for each table m, for each 128-row tile rt, for each 64-wide K-chunk kc,
-//     for each digit slice j, a 16 KB panel [128 rows][64 bf16] in the
-//     128-byte-swizzled K-major image that tcgen05 reads from shared memory;
-//     rows and K are zero-padded to the panel.  The eighth slice has an array
-//     of its own (it is the remainder of the first seven, which both forms
-//     share).  Row exponents eA (int8) per (m, row).
+//     for each digit slice j, an 8 KB block [4 K groups][128 rows][16 bytes] of
+//     digits + 64; rows and K are zero-padded to the block.  One byte per digit:
+//     7 or 8 bytes per table entry, half of what bf16 panels take, so that the
+//     table stream (the bound of small batches) and the L2-to-SM traffic (of
+//     large ones) halve.  The eighth slice has an array of its own (it is the
+//     remainder of the first seven, which both forms share).  Row exponents eA
+//     (int8) per (m, row).
 //   Sliced coefficients, per call and per problem m: for each kc one panel
 //     [S slices x NC columns][64 bf16], column exponents eX (int32) per (m,
 //     column).
 //
-// Kernel k_contract_mx<NC, S>: persistent, one CTA per SM, 18 warps; NC real
+// Kernel k_contract_mx<NC, S>: persistent, one CTA per SM; NC real
 // coefficient columns (16, 32 or 64) per table pass.
-//   warp 0    producer: cp.async.bulk of panels into a ring of 16 KB table
-//             stages (10 deep; 6 at NC = 64) and a 2-deep ring of coefficient
-//             stages (S slices x NC columns x 64 K).
+//   warp 0    producer: cp.async.bulk of digit blocks into a ring of 8 KB stages
+//             and of coefficient panels into a 2-deep ring (S slices x NC
+//             columns x 64 K).
+//   converter warps (5; 2 at NC = 64): digit block -> 16 KB panel [128 rows][64
+//             bf16] in the 128-byte-swizzled K-major image that tcgen05 reads,
+//             in a ring of 16 KB stages: a byte permute puts digit + 64 under the
+//             exponent of 128 (bf16 has 8 significant bits), one packed
+//             subtraction of 192 leaves the digit, 2 instructions per 2 digits.
 //   warp 1    MMA issuer: per K-chunk and digit slice j, one 128 x N x 64
 //             product (tcgen05.mma of K=16, N <= 256 each) of table slice j
 //             against the first S-j coefficient slices, written to the
 //             accumulator columns of classes j..S-1 (N = NC (S-j)); two TMEM
 //             accumulators alternate between tiles (one at NC = 64).
-//   warps 2-17 epilogue: four warps per TMEM lane quarter, 16 columns each:
+//   epilogue warps (NC / 4): one per TMEM lane quarter and 16 columns:
 //             tcgen05.ld of the S class accumulators, combine (double-float
 //             for 7, integers for 8), row/column exponents, sign, per-l
 //             weight, store; the accumulator is released as soon as its values
 //             are in registers.
+// Measured (2 maps at L = 1024, N = 4, FP64, 16 columns): 13.0 ms against 15.8 with
+// bf16 panels in HBM; 32 maps, split precision, 64 columns: 32.2 against 33.5.
+// With a quarter of the MMAs the 16-column launches take 24 % less, without the
+// conversion's stores 10 %, without the combination 4 %: no single unit paces
+// them (DRAM 38 % busy, tensor pipe 17 %); what is left is the latency of 32
+// MMAs of N <= 128 per K-chunk behind one another.
 // Every wait is bounded (about 2 s); on expiry the kernel raises an error flag,
 // drains its own copies and MMAs, frees TMEM and returns.
 #include <cstdint>
@@ -58,11 +71,9 @@ constexpr int kSmax = 8;               // and of the 64-bit form (FP64 results)
 constexpr int kB0 = 6;                 // bits of the first digit (later digits: 7)
 constexpr int kPK = 64;                // K per panel
 constexpr int kPM = 128;               // rows per panel
-constexpr int kPanelA = kPM * kPK;     // 8192 elements, 16 KB
+constexpr int kPanelA = kPM * kPK;     // digits of a block, elements of a panel
+constexpr int kGrpK = 16;              // consecutive K of one row in a digit block
 constexpr int kMaxParts = 2;           // scales sharing one table pass
-constexpr int kXST = 2;                // coefficient pipeline depth
-constexpr int kEpiWarps = 16;          // four warps per TMEM lane quarter, one 16-column chunk each
-constexpr int kThreads = 64 + 32 * kEpiWarps;
 constexpr int kMinBl = 128;            // 7 slices from this band-limit
 // 8 slices from this band-limit, whatever the batch (so that a map's result does
 // not depend on its batch).  Per contraction at bl = 64, FP64 kernel against
@@ -74,19 +85,34 @@ constexpr long long kWaitCycles = 4000000000LL;
 // NC real coefficient columns per CTA (16, 32 or 64): parts x maps x {re, im};
 // S digit slices (7, or 8 for FP64 results).  NC <= 32: two TMEM accumulators
 // alternate between tiles; NC = 64: one accumulator of 64 S columns (all of
-// TMEM at S = 8), and a shallower table ring to fit shared memory.
+// TMEM at S = 8).  The table rings take what the coefficient stages leave of
+// shared memory; the digit blocks in flight (48 KB and more) cover the latency
+// at an SM's share of the HBM bandwidth (28 KB).
 template <int NC, int S>
 struct Cfg {
-  static constexpr int kAST = NC == 64 ? 6 : 10;       // table pipeline depth
-  static constexpr int kNBuf = NC == 64 ? 1 : 2;       // TMEM accumulators
-  static constexpr int kPanelX = S * NC * kPK;         // elements
-  static constexpr int kAccCols = S * NC;              // TMEM columns per accumulator
+  static constexpr int kXST = NC == 16 ? 3 : 2;                                    // coefficient ring
+  static constexpr int kAST = NC == 64 ? 3 : 5;                                    // panel ring
+  static constexpr int kRST = NC == 64 ? (S == 8 ? 6 : 8) : (NC == 32 ? 10 : 12);  // digit-block ring
+  static constexpr int kNBuf = NC == 64 ? 1 : 2;                                   // TMEM accumulators
+  static constexpr int kConvWarps = NC == 64 ? 2 : 5;  // 2: 640 threads, so that 96 registers hold the epilogue
+  static constexpr int kEpiWarps = NC / 4;  // one per TMEM lane quarter and 16-column chunk
+  static constexpr int kThreads = 32 * (2 + kConvWarps + kEpiWarps);
+  static constexpr int kPanelX = S * NC * kPK;  // elements
+  static constexpr int kAccCols = S * NC;       // TMEM columns per accumulator
   static constexpr int kTmemCols = NC == 16 ? 256 : 512;
   static constexpr size_t kSmemA = (size_t)kAST * kPanelA * 2;
+  static constexpr size_t kSmemR = (size_t)kRST * kPanelA;
   static constexpr size_t kSmemX = (size_t)kXST * kPanelX * 2;
-  static constexpr int kNumBars = 2 * kAST + 2 * kXST + 4 + 1;
-  static constexpr size_t kSmemBytes = 1024 + kSmemA + kSmemX + kNumBars * 8 + 16;
+  static constexpr int kNumBars = 2 * kAST + 2 * kRST + 2 * kXST + 4 + 1;
+  static constexpr size_t kSmemBytes = 1024 + kSmemA + kSmemX + kSmemR + kNumBars * 8 + 16;
   static_assert(kSmemBytes <= 232448, "shared memory");
+  // The converter warps take blocks out of order, and a parity wait tells only
+  // neighbouring phases of a stage apart.  A warp waits for block c after its
+  // block c - kConvWarps, whose panel stage was free, so the MMAs (in order) had
+  // consumed every block up to c - kConvWarps - kAST: the panel stage of c is at
+  // most one phase behind if kConvWarps <= kAST, and the digit block before c in
+  // its stage (c - kRST) has been loaded if kConvWarps + kAST <= kRST.
+  static_assert(kConvWarps <= kAST && kConvWarps + kAST <= kRST, "ring depths");
   static_assert(kNBuf * kAccCols <= kTmemCols, "TMEM");
 };
 
@@ -128,10 +154,6 @@ __device__ __forceinline__ void int_digits(long long q, int *d) {
   }
   d[0] = (int)q;
 }
-__device__ __forceinline__ uint16_t bf16_of_int(int d) {
-  // |d| <= 64: exact in bf16 (top half of the fp32 pattern)
-  return (uint16_t)(__float_as_uint((float)d) >> 16);
-}
 // round(v 2^(48-e)) for |v| < 2^e, from the significand bits (no FP64 work)
 __device__ __forceinline__ long long fixed48(double v, int e) {
   const uint64_t u = bits_of(v);
@@ -149,13 +171,6 @@ __device__ __forceinline__ long long fixed48(double v, int e) {
   return (u >> 63) ? -q : q;
 }
 
-// digits of v 2^-e as bf16 bit patterns
-__device__ __forceinline__ void split_digits(double v, int e, uint16_t *out) {
-  int d[kS];
-  int_digits(fixed48(v, e), d);
-#pragma unroll
-  for (int j = 0; j < kS; ++j) out[j] = bf16_of_int(d[j]);
-}
 // round(v 2^(55-e)) for |v| < 2^e (subnormals included)
 __device__ __forceinline__ long long fixed55(double v, int e) {
   const uint64_t u = bits_of(v);
@@ -173,9 +188,7 @@ __device__ __forceinline__ long long fixed55(double v, int e) {
 }
 // The eighth digit of a table value: what the seven leave of v 2^-e, in units
 // of 2^-55 (|digit| <= 64; with it the value is represented to 2^-56).
-__device__ __forceinline__ uint16_t eighth_digit(double v, int e) {
-  return bf16_of_int((int)(fixed55(v, e) - fixed48(v, e) * 128));
-}
+__device__ __forceinline__ int eighth_digit(double v, int e) { return (int)(fixed55(v, e) - fixed48(v, e) * 128); }
 // Balanced digits of q 2^-55, |q| < 2^55, as bf16 patterns in the low halves
 // of out: adding 64 in every digit position but the first makes the base-128
 // digits of the sum the balanced ones plus 64; 2^23 + digit is read off the
@@ -216,11 +229,11 @@ __device__ __forceinline__ TableRefM table_ref_m(int tmlo, int n, int m) {
 
 // rows l when q (t -> l) else t; tr: the source block holds the transpose
 // (row k, column row).  panels8 (nullable with panels set, or the reverse):
-// the eighth digit's panels, one per (row tile, K-chunk).
+// the eighth digit's blocks, one per (row tile, K-chunk).
 __global__ void __launch_bounds__(128) k_slice_table(const double *__restrict__ T,
                                                      const int64_t *__restrict__ off, int bl, int nt,
-                                                     int an, int tmlo, int q, int tr, uint16_t *__restrict__ panels,
-                                                     uint16_t *__restrict__ panels8,
+                                                     int an, int tmlo, int q, int tr, uint8_t *__restrict__ panels,
+                                                     uint8_t *__restrict__ panels8,
                                                      const int64_t *__restrict__ pan_off,
                                                      int8_t *__restrict__ eA,
                                                      const int64_t *__restrict__ e_off) {
@@ -251,15 +264,15 @@ __global__ void __launch_bounds__(128) k_slice_table(const double *__restrict__ 
       const double v = (live && k < g.K) ? Tm[row * rs + k * ks] : 0.0;
       const int kc = k / kPK;
       const int64_t tile = (int64_t)(rt * g.nkc + kc);
-      const int idx = swz(rr, k % kPK);
+      const int idx = (k % kPK / kGrpK * kPM + rr) * kGrpK + k % kGrpK;
       if (panels) {
-        uint16_t dg[kS];
-        split_digits(v, e, dg);
-        uint16_t *p = panels + pan_off[mi] + tile * kS * kPanelA;
+        int dg[kS];
+        int_digits(fixed48(v, e), dg);
+        uint8_t *p = panels + pan_off[mi] + tile * kS * kPanelA;
 #pragma unroll
-        for (int j = 0; j < kS; ++j) p[(int64_t)j * kPanelA + idx] = dg[j];
+        for (int j = 0; j < kS; ++j) p[(int64_t)j * kPanelA + idx] = (uint8_t)(dg[j] + 64);
       }
-      if (panels8) panels8[pan_off[mi] / kS + tile * kPanelA + idx] = eighth_digit(v, e);
+      if (panels8) panels8[pan_off[mi] / kS + tile * kPanelA + idx] = (uint8_t)(eighth_digit(v, e) + 64);
     }
   }
 }
@@ -526,7 +539,7 @@ __device__ __noinline__ bool bar_wait_timed(uint64_t *b, uint32_t parity) {
 }
 // Bounded wait; false when the CTA is aborting or the wait expired (then it
 // raises the CTA abort flag and the global error flag).
-__device__ __noinline__ bool bar_wait(uint64_t *b, uint32_t parity, volatile int *abort_flag, int *err) {
+__device__ __noinline__ bool bar_wait_slow(uint64_t *b, uint32_t parity, volatile int *abort_flag, int *err) {
   const long long t0 = clock64();
   for (uint32_t it = 0;; ++it) {
     if (bar_try(b, parity)) return true;
@@ -539,6 +552,9 @@ __device__ __noinline__ bool bar_wait(uint64_t *b, uint32_t parity, volatile int
       }
     }
   }
+}
+__device__ __forceinline__ bool bar_wait(uint64_t *b, uint32_t parity, volatile int *abort_flag, int *err) {
+  return bar_try(b, parity) || bar_wait_slow(b, parity, abort_flag, err);
 }
 __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
@@ -582,9 +598,22 @@ __device__ __forceinline__ void tc_fence_before() {
 // the contraction
 // ---------------------------------------------------------------------------
 
+// 8 digits (bytes d + 64 of two words) as bf16: 0x4300 | x is 128 + x for x <
+// 128 and 256 for x = 128, all exact, so subtracting 192 leaves d.
+__device__ __forceinline__ uint32_t digits2_bf16(uint32_t w, uint32_t sel) {
+  const uint32_t v = __byte_perm(w, 0x43434343u, sel);
+  uint32_t r;
+  asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(v), "r"(0x43404340u));
+  return r;
+}
+__device__ __forceinline__ uint4 digits_bf16(uint32_t lo, uint32_t hi) {
+  return make_uint4(digits2_bf16(lo, 0x4140), digits2_bf16(lo, 0x4342), digits2_bf16(hi, 0x4140),
+                    digits2_bf16(hi, 0x4342));
+}
+
 struct MxArgs {
   int q;  // 0: l -> t with D, 1: t -> l with Q
-  const uint16_t *panels, *panels8;
+  const uint8_t *panels, *panels8;
   const int64_t *pan_off;
   const int8_t *eA;
   const int64_t *e_off;
@@ -612,10 +641,13 @@ struct TileInfo {
   int g;  // map group
   double sign;
 };
-__device__ __forceinline__ TileInfo tile_info(const MxArgs &a, int v) {
+// tile entry of work item v (read one item ahead of its use)
+__device__ __forceinline__ int2 tile_of(const MxArgs &a, int v) {
+  return v < a.ntiles * a.ngroups ? a.tiles[v / a.ngroups] : make_int2(0, 0);
+}
+__device__ __forceinline__ TileInfo tile_info(const MxArgs &a, int v, int2 tl) {
   TileInfo ti;
   ti.g = v % a.ngroups;
-  const int2 tl = a.tiles[v / a.ngroups];
   ti.pm = tl.x;
   ti.rt = tl.y;
   ti.m = a.mlo + ti.pm;
@@ -730,24 +762,26 @@ __device__ __forceinline__ void combine8_int(float (*acc)[8], int ea, int4 e0, i
 }
 
 template <int NC, int S>
-__global__ void __launch_bounds__(kThreads, 1) k_contract_mx(MxArgs a) {
+__global__ void __launch_bounds__(Cfg<NC, S>::kThreads, 1) k_contract_mx(MxArgs a) {
   using C = Cfg<NC, S>;
   constexpr int PX = C::kPanelX;
   constexpr int ACC = C::kAccCols;
   constexpr int TMC = C::kTmemCols;
-  constexpr int kAST = C::kAST;
+  constexpr int kAST = C::kAST, kRST = C::kRST, kXST = C::kXST;
   constexpr int NBUF = C::kNBuf;
+  constexpr int kEpi0 = 2 + C::kConvWarps;  // first epilogue warp
   constexpr int kNumBars = C::kNumBars;
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint16_t *sA = (uint16_t *)smem;
   uint16_t *sX = (uint16_t *)(smem + C::kSmemA);
-  uint64_t *bars = (uint64_t *)(smem + C::kSmemA + C::kSmemX);
-  uint64_t *fullA = bars, *emptyA = bars + kAST, *fullX = bars + 2 * kAST, *emptyX = bars + 2 * kAST + kXST;
-  uint64_t *tfull = bars + 2 * kAST + 2 * kXST, *tempty = tfull + 2, *mma_done = tfull + 4;
+  uint8_t *sR = smem + C::kSmemA + C::kSmemX;
+  uint64_t *bars = (uint64_t *)(smem + C::kSmemA + C::kSmemX + C::kSmemR);
+  uint64_t *fullA = bars, *emptyA = fullA + kAST, *fullR = emptyA + kAST, *emptyR = fullR + kRST;
+  uint64_t *fullX = emptyR + kRST, *emptyX = fullX + kXST;
+  uint64_t *tfull = emptyX + kXST, *tempty = tfull + 2, *mma_done = tfull + 4;
   volatile int *abort_flag = (volatile int *)(bars + kNumBars);
   uint32_t *tmem_slot = (uint32_t *)(bars + kNumBars) + 1;
-  int *cons = (int *)(bars + kNumBars) + 2;  // [2]: table / coefficient stages consumed
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
@@ -755,17 +789,20 @@ __global__ void __launch_bounds__(kThreads, 1) k_contract_mx(MxArgs a) {
       bar_init(&fullA[i], 1);
       bar_init(&emptyA[i], 1);
     }
+    for (int i = 0; i < kRST; ++i) {
+      bar_init(&fullR[i], 1);
+      bar_init(&emptyR[i], 1);
+    }
     for (int i = 0; i < kXST; ++i) {
       bar_init(&fullX[i], 1);
       bar_init(&emptyX[i], 1);
     }
     for (int i = 0; i < 2; ++i) {
       bar_init(&tfull[i], 1);
-      bar_init(&tempty[i], 32 * kEpiWarps);
+      bar_init(&tempty[i], 32 * C::kEpiWarps);
     }
     bar_init(mma_done, 1);
     *abort_flag = 0;
-    cons[0] = cons[1] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -780,14 +817,16 @@ __global__ void __launch_bounds__(kThreads, 1) k_contract_mx(MxArgs a) {
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
-  int issuedA = 0, issuedX = 0;
+  int issuedR = 0, issuedX = 0;
   if (warp == 0 && lane == 0) {
     // ---------------- producer ----------------
     bool ok = true;
+    int2 next = tile_of(a, blockIdx.x);
     for (int t = blockIdx.x; ok && t < a.ntiles * a.ngroups; t += gridDim.x) {
-      const TileInfo ti = tile_info(a, t);
-      const uint16_t *pan = a.panels + a.pan_off[ti.mi] + (int64_t)ti.rt * ti.nkc * kS * kPanelA;
-      const uint16_t *pan8 = S == kSmax ? a.panels8 + a.pan_off[ti.mi] / kS + (int64_t)ti.rt * ti.nkc * kPanelA : nullptr;
+      const TileInfo ti = tile_info(a, t, next);
+      next = tile_of(a, t + gridDim.x);
+      const uint8_t *pan = a.panels + a.pan_off[ti.mi] + (int64_t)ti.rt * ti.nkc * kS * kPanelA;
+      const uint8_t *pan8 = S == kSmax ? a.panels8 + a.pan_off[ti.mi] / kS + (int64_t)ti.rt * ti.nkc * kPanelA : nullptr;
       const uint16_t *xp = a.xpan + ti.g * a.xg + a.xoff[ti.pm] * (NC / 16 * S);
       for (int kc = ti.kc0; ok && kc < ti.nkc; ++kc) {
         const int xs = issuedX % kXST;
@@ -796,12 +835,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_contract_mx(MxArgs a) {
         bulk_g2s(sX + (size_t)xs * PX, xp + (int64_t)kc * PX, PX * 2, &fullX[xs]);
         ++issuedX;
         for (int j = 0; j < S; ++j) {
-          const int as = issuedA % kAST;
-          if (!(ok = bar_wait(&emptyA[as], ((issuedA / kAST) & 1) ^ 1, abort_flag, a.err))) break;
-          bar_expect_tx(&fullA[as], kPanelA * 2);
-          const uint16_t *src = j < kS ? pan + ((int64_t)kc * kS + j) * kPanelA : pan8 + (int64_t)kc * kPanelA;
-          bulk_g2s(sA + (size_t)as * kPanelA, src, kPanelA * 2, &fullA[as]);
-          ++issuedA;
+          const int rs = issuedR % kRST;
+          if (!(ok = bar_wait(&emptyR[rs], ((issuedR / kRST) & 1) ^ 1, abort_flag, a.err))) break;
+          bar_expect_tx(&fullR[rs], kPanelA);
+          const uint8_t *src = j < kS ? pan + ((int64_t)kc * kS + j) * kPanelA : pan8 + (int64_t)kc * kPanelA;
+          bulk_g2s(sR + (size_t)rs * kPanelA, src, kPanelA, &fullR[rs]);
+          ++issuedR;
         }
       }
     }
@@ -809,8 +848,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_contract_mx(MxArgs a) {
     // ---------------- MMA issuer ----------------
     int ca = 0, cx = 0, ti_n = 0;
     bool ok = true, any = false;
+    int2 next = tile_of(a, blockIdx.x);
     for (int t = blockIdx.x; ok && t < a.ntiles * a.ngroups; t += gridDim.x, ++ti_n) {
-      const TileInfo ti = tile_info(a, t);
+      const TileInfo ti = tile_info(a, t, next);
+      next = tile_of(a, t + gridDim.x);
       const int ab = ti_n % NBUF;
       if (!(ok = bar_wait(&tempty[ab], ((ti_n / NBUF) & 1) ^ 1, abort_flag, a.err))) break;
       tc_fence_after();
@@ -854,31 +895,75 @@ __global__ void __launch_bounds__(kThreads, 1) k_contract_mx(MxArgs a) {
       if (!ok) break;
       mma_commit(&tfull[ab]);
     }
-    cons[0] = ca;
-    cons[1] = cx;
     if (any) {  // every MMA of this thread has completed before TMEM is released
       mma_commit(mma_done);
       if (!bar_wait_timed(mma_done, 0)) atomicExch(a.err, 2);
     }
-  } else if (warp >= 2) {
+  } else if (warp >= 2 && warp < kEpi0) {
+    // ---------------- converters ----------------
+    // every warp takes whole blocks, warp w the w-th, (w + kConvWarps)-th, ...:
+    // the waits, the proxy fence and the arrivals (several hundred cycles a
+    // block) of the warps overlap.  Lane -> rows lane + 32 i, all 4 K groups.
+    const int w = warp - 2;
+    int done = 0;  // blocks of earlier tiles
+    bool ok = true;
+    int2 next = tile_of(a, blockIdx.x);
+    for (int t = blockIdx.x; ok && t < a.ntiles * a.ngroups; t += gridDim.x) {
+      const TileInfo ti = tile_info(a, t, next);
+      next = tile_of(a, t + gridDim.x);
+      const int n = (ti.nkc - ti.kc0) * S;
+      for (int c = done + (w - done % C::kConvWarps + C::kConvWarps) % C::kConvWarps; c < done + n;
+           c += C::kConvWarps) {
+        const int rs = c % kRST, as = c % kAST;
+        ok = bar_wait(&fullR[rs], (c / kRST) & 1, abort_flag, a.err) &&
+             bar_wait(&emptyA[as], ((c / kAST) & 1) ^ 1, abort_flag, a.err);
+        if (!__all_sync(0xffffffffu, ok)) {
+          ok = false;
+          break;
+        }
+        const uint4 *src = (const uint4 *)(sR + (size_t)rs * kPanelA) + lane;
+        uint16_t *dst = sA + (size_t)as * kPanelA;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          uint4 d[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) d[i] = src[q * kPM + 32 * i];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            *(uint4 *)(dst + swz(lane + 32 * i, q * kGrpK)) = digits_bf16(d[i].x, d[i].y);
+            *(uint4 *)(dst + swz(lane + 32 * i, q * kGrpK + 8)) = digits_bf16(d[i].z, d[i].w);
+          }
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // visible to the MMAs' reads
+        __syncwarp();
+        if (lane == 0) {
+          bar_arrive(&fullA[as]);
+          bar_arrive(&emptyR[rs]);
+        }
+      }
+      done += n;
+    }
+  } else if (warp >= kEpi0) {
     // ---------------- epilogue ----------------
     // warp -> TMEM lane quarter (warp mod 4, the quarter it may address) and one
     // 16-column chunk pi, read as two 8-column halves; the accumulator is
     // handed back right after the second half is in registers, before it is
     // combined and stored, so that the next tile's MMAs wait as little as possible
     const int quarter = warp & 3;
-    const int pi = (warp - 2) / 4;
+    const int pi = (warp - kEpi0) / 4;
     const int rr = quarter * 32 + lane;
     int ti_n = 0;
+    int2 next = tile_of(a, blockIdx.x);
     for (int t = blockIdx.x; t < a.ntiles * a.ngroups; t += gridDim.x, ++ti_n) {
-      const TileInfo ti = tile_info(a, t);
+      const TileInfo ti = tile_info(a, t, next);
+      next = tile_of(a, t + gridDim.x);
       const int ab = ti_n % NBUF;
       const bool live = ti.kc0 < ti.nkc;
       // the row and column exponents do not depend on the accumulator: read
       // them before waiting, so that their latency is not spent holding TMEM
       int ea = 0;
       int4 ex4[4];
-      if (pi < NC / 16 && live) {
+      if (live) {
         ea = (int)a.eA[a.e_off[ti.mi] + ti.rt * kPM + rr];
         const int4 *ep = (const int4 *)(a.eX + ti.g * a.eXg + ti.pm * NC + pi * 16);
 #pragma unroll
@@ -887,10 +972,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_contract_mx(MxArgs a) {
       // warp-uniform outcome: tcgen05.ld below is .sync.aligned
       if (!__all_sync(0xffffffffu, bar_wait(&tfull[ab], (ti_n / NBUF) & 1, abort_flag, a.err))) break;
       tc_fence_after();
-      if (pi >= NC / 16 || !live) {  // no columns here, or nothing accumulated: release at once
+      if (!live) {  // nothing accumulated: release at once
         tc_fence_before();
         bar_arrive(&tempty[ab]);
-        if (pi >= NC / 16) continue;
       }
       const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(ab * ACC);
       const int t_row = ti.rt * kPM + rr;
@@ -938,14 +1022,15 @@ __global__ void __launch_bounds__(kThreads, 1) k_contract_mx(MxArgs a) {
     }
   }
 
-  // producer: on abort, wait (bounded) for its own copies still in flight
+  // producer: on abort, wait (bounded) for its own copies still in flight: the
+  // last one of every stage
   __syncthreads();
   if (warp == 0 && lane == 0 && *abort_flag) {
     const long long t0 = clock64();
-    for (int i = cons[0]; i < issuedA; ++i)
-      while (!bar_try(&fullA[i % kAST], (i / kAST) & 1) && clock64() - t0 < kWaitCycles) {
+    for (int i = max(0, issuedR - kRST); i < issuedR; ++i)
+      while (!bar_try(&fullR[i % kRST], (i / kRST) & 1) && clock64() - t0 < kWaitCycles) {
       }
-    for (int i = cons[1]; i < issuedX; ++i)
+    for (int i = max(0, issuedX - kXST); i < issuedX; ++i)
       while (!bar_try(&fullX[i % kXST], (i / kXST) & 1) && clock64() - t0 < kWaitCycles) {
       }
   }
@@ -978,8 +1063,8 @@ bool kind_transposed(int kind) { return kind == TK_L2T_Q || kind == TK_T2L_D; }
 struct SlicedTable {
   int bl = 0, nt = 0, an = 0, mlo = 0, nm = 0;
   bool q = false;    // rows l
-  uint16_t *panels = nullptr;   // 7 digit slices
-  uint16_t *panels8 = nullptr;  // the eighth, built when an FP64 contraction first needs it
+  uint8_t *panels = nullptr;   // 7 digit slices
+  uint8_t *panels8 = nullptr;  // the eighth, built when an FP64 contraction first needs it
   int8_t *eA = nullptr;
   int64_t *d_pan_off = nullptr, *d_e_off = nullptr;
   size_t bytes = 0;
@@ -1041,7 +1126,7 @@ SlicedTable *sliced(const WignerTable &tb, int kind, bool eighth, cudaStream_t s
     etot += (int64_t)g.nrt * kPM;
   }
   if (eighth) {
-    const size_t need = sizeof(uint16_t) * (size_t)(ptot / kS) * (fresh ? kSmax : 1);
+    const size_t need = (size_t)(ptot / kS) * (fresh ? kSmax : 1);
     size_t fr = 0, tot = 0;
     S2G_CUDA(cudaMemGetInfo(&fr, &tot));
     if (fr < need + tot / 3) {
@@ -1062,17 +1147,17 @@ SlicedTable *sliced(const WignerTable &tb, int kind, bool eighth, cudaStream_t s
     s->nm = tb.nm;
     s->q = q;
   }
-  uint16_t *p8 = nullptr;
+  uint8_t *p8 = nullptr;
   try {
     if (fresh) {
-      s->panels = dev_alloc<uint16_t>((size_t)ptot, &by);
+      s->panels = dev_alloc<uint8_t>((size_t)ptot, &by);
       s->eA = dev_alloc<int8_t>((size_t)etot, &by);
       s->d_pan_off = dev_alloc<int64_t>(tb.nm, &by);
       s->d_e_off = dev_alloc<int64_t>(tb.nm, &by);
       S2G_CUDA(cudaMemcpyAsync(s->d_pan_off, po.data(), sizeof(int64_t) * tb.nm, cudaMemcpyHostToDevice, st));
       S2G_CUDA(cudaMemcpyAsync(s->d_e_off, eo.data(), sizeof(int64_t) * tb.nm, cudaMemcpyHostToDevice, st));
     }
-    if (eighth) p8 = dev_alloc<uint16_t>((size_t)(ptot / kS), &by);
+    if (eighth) p8 = dev_alloc<uint8_t>((size_t)(ptot / kS), &by);
     const dim3 grid(tb.nm, (std::max(tb.bl, tb.nt) + kPM - 1) / kPM);
     k_slice_table<<<grid, 128, 0, st>>>(kind_of_q(kind) ? tb.Q : tb.D, tb.d_off, tb.bl, tb.nt, tb.an, tb.mlo,
                                         q ? 1 : 0, kind_transposed(kind) ? 1 : 0, fresh ? s->panels : nullptr, p8,
@@ -1230,7 +1315,7 @@ bool run_mixed(const Problem &p, const Prepared &pr, cudaStream_t st, int gpl_ma
       double xby = 0;
       if (timing_enabled()) {
         fl += 4.0 * entries * nbg * p.nparts;
-        by += entries * 2.0 * S + (double)x_elems * 2.0 + 16.0 * nbg * p.nparts * (double)p.tb->nt * nmp;
+        by += entries * S + (double)x_elems * 2.0 + 16.0 * nbg * p.nparts * (double)p.tb->nt * nmp;
         xby = (double)x_elems * 2.0 * (1.0 + 8.0 / (2.0 * S));  // panels written + FP64 values read
       }
       XArgs xa{};
@@ -1287,7 +1372,7 @@ bool run_mixed(const Problem &p, const Prepared &pr, cudaStream_t st, int gpl_ma
     ma.err = err;
     const int nwork = L->ntiles * ng;
     const int grid = nwork < num_sms() ? nwork : num_sms();
-    k_contract_mx<NC, S><<<grid, kThreads, C::kSmemBytes, st>>>(ma);
+    k_contract_mx<NC, S><<<grid, C::kThreads, C::kSmemBytes, st>>>(ma);
     S2G_LAUNCHED();
   }
   cudaFreeAsync(xpan, st);
