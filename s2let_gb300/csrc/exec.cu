@@ -358,6 +358,23 @@ struct Sht {
 };
 Sht sht_of(const WavPlan &P) { return Sht{P.L, P.s, P.ss, P.real, P.d_w + P.w_cl, P.rc(P.L)}; }
 
+// ring DFTs between nb maps (rings contiguous in each, maps stride apart) and
+// their contiguous spectra of width sw from m = mlo
+RingJob ring_job(const void *in, void *out, int K, int64_t mstride, int nt, int sw, int mlo, int nb, int bl) {
+  RingJob j;
+  j.in = in;
+  j.out = out;
+  j.ring_stride = K;
+  j.map_stride = mstride;
+  j.rpm = nt;
+  j.spec_stride = sw;
+  j.sw = sw;
+  j.mlo = mlo;
+  j.nrings = nb * nt;
+  j.bl = bl;
+  return j;
+}
+
 // flm (nb x L^2, zero outside the computed range) <- forward transform of maps
 // (or the adjoint of the inverse)
 void sht_forward_once(const Sht &H, const void *f, int64_t fstride, double2 *flm, int nb, Scratch &S,
@@ -366,7 +383,7 @@ void sht_forward_once(const Sht &H, const void *f, int64_t fstride, double2 *flm
   const bool real = H.real;
   const int sw = real ? L : 2 * L - 1, mlo = real ? 0 : -(L - 1);
   double2 *spec = S.get<double2>((int64_t)nb * nt * sw);
-  ring_forward(f, K, fstride, nt, spec, sw, sw, mlo, nb * nt, L, H.ss, real, S.st);
+  ring_forward_many({ring_job(f, spec, K, fstride, nt, sw, mlo, nb, L)}, H.ss, real, S.st);
   S2G_CUDA(cudaMemsetAsync(flm, 0, sizeof(double2) * nb * L * L, S.st));
   T2L a{};
   a.tb = &wigner_table(L, std::abs(s), H.ss, H.rc);
@@ -415,7 +432,7 @@ void sht_inverse(const Sht &H, const double2 *flm, bool flm_half, void *f, int64
   a.omlo = mlo;
   a.nb = nb;
   contract_l2t(a, S.st);
-  ring_inverse(spec, sw, sw, mlo, f, K, fstride, nt, nb * nt, L, H.ss, real, S.st);
+  ring_inverse_many({ring_job(spec, f, K, fstride, nt, sw, mlo, nb, L)}, H.ss, real, S.st);
 }
 
 // Forward transform with one residual-refinement sweep (FP64 path, L above
@@ -508,32 +525,45 @@ struct WavPipe {
 };
 const double kSqrt2Pi = 2.5066282746310005024;
 
-// flm -> (f_wav, f_scal).  SPLIT_ANALYSIS: lm2wav.  SPLIT_SYNTH_ADJ: adjoint of wav2lm.
 // Ring DFTs per theta ring on the nn n-components (one complex DFT each) when
 // that is fewer than on the ng gamma slices (real slices pair up, two per
-// complex DFT); the gamma DFT then runs on pixels.
-bool rings_on_n(const WavPlan &P, const Scale &sd) {
+// complex DFT); the gamma DFT then runs on pixels.  With one slice there is no
+// gamma DFT: its ring DFTs read and write the spectra of the contraction.
+enum RingPath { RINGS_FUSED, RINGS_ON_N, RINGS_ON_SLICES, RINGS_ONE_SLICE };
+RingPath ring_path(const WavPlan &P, const Scale &sd) {
+  if (sd.ng == 1) return RINGS_ONE_SLICE;
   const double on_n = (double)sd.ns.size();
   const double on_g = P.real ? 0.5 * sd.ng : (double)sd.ng;
-  return on_n < on_g;
+  if (on_n >= on_g) return RINGS_ON_SLICES;
+  return ring_gamma_fusable((int)sd.ns.size(), sd.ng, sd.bl, P.ss) ? RINGS_FUSED : RINGS_ON_N;
 }
+// whether f_wav of the scale crosses the bus in groups of maps
+bool grouped_copies(RingPath path) { return path == RINGS_FUSED || path == RINGS_ON_N; }
 
 // Whether some scale of the plan runs its ring and gamma DFTs as separate
 // launches through a ring buffer (the fused launch keeps them on chip).
 bool needs_ring_buffer(const WavPlan &P) {
-  for (const Scale &sd : P.sc)
-    if (!rings_on_n(P, sd) || !ring_gamma_fusable((int)sd.ns.size(), sd.ng, sd.bl, P.ss)) return true;
+  for (const Scale &sd : P.sc) {
+    const RingPath path = ring_path(P, sd);
+    if (path == RINGS_ON_N || path == RINGS_ON_SLICES) return true;
+  }
   return false;
 }
 
-// Scale ranges [k0, k1) that share one table pass (consecutive scales with the
-// same band-limit and directions), smallest band-limits first, or largest
-// first when `largest_first`.
-std::vector<std::pair<size_t, size_t>> table_passes(const WavPlan &P, bool largest_first) {
+// Scales that share one table pass: as many consecutive ones with the same
+// band-limit and directions as the coefficient columns of one pass hold (64
+// real columns: 2 per map), two at least.
+int max_parts(int nb) { return std::min(kMaxParts, std::max(2, 32 / std::max(nb, 1))); }
+
+// Scale ranges [k0, k1) that share one table pass, smallest band-limits first,
+// or largest first when `largest_first`.
+std::vector<std::pair<size_t, size_t>> table_passes(const WavPlan &P, bool largest_first, int nb) {
   std::vector<std::pair<size_t, size_t>> passes;
   for (size_t k0 = 0; k0 < P.sc.size();) {
     size_t k1 = k0 + 1;
-    if (k1 < P.sc.size() && P.sc[k1].bl == P.sc[k0].bl && P.sc[k1].ns == P.sc[k0].ns) ++k1;
+    while (k1 < P.sc.size() && (int)(k1 - k0) < max_parts(nb) && P.sc[k1].bl == P.sc[k0].bl &&
+           P.sc[k1].ns == P.sc[k0].ns)
+      ++k1;
     passes.emplace_back(k0, k1);
     k0 = k1;
   }
@@ -541,12 +571,83 @@ std::vector<std::pair<size_t, size_t>> table_passes(const WavPlan &P, bool large
   return passes;
 }
 
+// The scales whose contractions are small (contract_is_small) run together:
+// one launch for the contractions of all of them, one for their ring DFTs.
+bool small_scale(const WavPlan &P, const Scale &sd, int nb) {
+  for (int n : sd.ns)
+    if (!contract_is_small(&P.table(sd.bl, std::abs(n)), nb)) return false;
+  return true;
+}
+
+// Jobs of ring DFTs collected for shared launches: those fused with the gamma
+// DFT by their directions and normalisation, the others all together.
+struct RingJobs {
+  struct Fused {
+    std::vector<int> ns;
+    int ng;
+    double c;
+    std::vector<GammaJob> jobs;
+  };
+  std::vector<RingJob> plain;
+  std::vector<Fused> fused;
+  void add(const Scale &sd, double c, const GammaJob &j) {
+    for (Fused &f : fused)
+      if (f.ns == sd.ns && f.ng == sd.ng && f.c == c) {
+        f.jobs.push_back(j);
+        return;
+      }
+    fused.push_back({sd.ns, sd.ng, c, {j}});
+  }
+  void inverse(int ss, bool real, cudaStream_t st) {
+    ring_inverse_many(plain, ss, real, st);
+    for (const Fused &f : fused) ring_inverse_gamma(f.jobs, f.ns, f.ng, real, f.c, ss, st);
+    plain.clear();
+    fused.clear();
+  }
+  void forward(int ss, bool real, cudaStream_t st) {
+    ring_forward_many(plain, ss, real, st);
+    for (const Fused &f : fused) gamma_ring_forward(f.jobs, f.ns, f.ng, real, f.c, ss, st);
+    plain.clear();
+    fused.clear();
+  }
+};
+
+// spectra and pixels of maps b0 .. b0 + nbg of one scale (G of that scale: [b][n][t][m])
+GammaJob gamma_job(const WavPlan &P, const Scale &sd, double2 *G, char *wav, size_t esz, int64_t wstride, int b0,
+                   int nbg) {
+  const int64_t W = 2 * sd.bl - 1, nt = P.nt(sd.bl), nn = (int64_t)sd.ns.size();
+  GammaJob j;
+  j.G = j.Gout = G + b0 * nn * nt * W;
+  j.gms = nn * nt * W;
+  j.gks = nt * W;
+  j.fw = wav + (size_t)sd.woff * esz + (size_t)b0 * wstride * esz;
+  j.fms = wstride;
+  j.nb = nbg;
+  j.bl = sd.bl;
+  return j;
+}
+// one slice per scale: rings against the contraction's spectra (real signals: m >= 0)
+RingJob slice_job(const WavPlan &P, const Scale &sd, double2 *G, char *wav, size_t esz, int64_t wstride, int nb,
+                  bool forward) {
+  const int W = 2 * sd.bl - 1, skip = P.real ? sd.bl - 1 : 0;
+  void *px = wav + (size_t)sd.woff * esz;
+  void *sp = G + skip;
+  RingJob j = ring_job(forward ? px : sp, forward ? sp : px, P.K(sd.bl), wstride, P.nt(sd.bl), W, 0, nb, sd.bl);
+  j.sw = W - skip;
+  j.mlo = P.real ? 0 : -(sd.bl - 1);
+  return j;
+}
+
+// flm -> (f_wav, f_scal).  SPLIT_ANALYSIS: lm2wav.  SPLIT_SYNTH_ADJ: adjoint of wav2lm.
 void wav_split(const WavPlan &P, SplitMode mode, const double2 *flm, bool flm_half, void *f_wav,
                int64_t wstride, void *f_scal, int64_t sstride, int nb, Scratch &S, WavPipe *pipe = nullptr) {
   const bool real = P.real;
   const int L = P.L;
   const size_t esz = real ? sizeof(double) : sizeof(double2);
   const bool adj = (mode == SPLIT_SYNTH_ADJ);
+  char *wav = (char *)f_wav;
+  std::vector<L2T> small;  // contractions that share launches
+  RingJobs rings;
   // scaling function: spin-0 transform at bl_scal
   {
     const int bs = P.bl_scal, Ks = P.K(bs), nts = P.nt(bs);
@@ -571,95 +672,135 @@ void wav_split(const WavPlan &P, SplitMode mode, const double2 *flm, bool flm_ha
     a.ow = sw;
     a.omlo = mlo;
     a.nb = nb;
-    contract_l2t(a, S.st);
-    ring_inverse(spec, sw, sw, mlo, f_scal, Ks, sstride, nts, nb * nts, bs, P.ss, real, S.st);
+    small.push_back(a);
+    rings.plain.push_back(ring_job(spec, f_scal, Ks, sstride, nts, sw, mlo, nb, bs));
   }
-  // G buffers [b][n][t][m] (spectral width W = 2bl-1), ring buffers [b][n or g][t][p]
-  const int64_t Wmax = 2 * P.max_bl - 1, Kmax = 2 * P.max_bl, ntmax = P.nt(P.max_bl);
-  const int64_t gsz = (int64_t)nb * P.max_nn * ntmax * Wmax;
-  double2 *Gbuf = S.get<double2>(2 * gsz);
-  // ring buffers only for the scales whose ring and gamma DFTs are separate launches
-  double2 *spec = needs_ring_buffer(P) ? S.get<double2>((int64_t)nb * std::max(P.max_ng, P.max_nn) * ntmax * Kmax)
-                                       : nullptr;
-  // with host copies the largest scales go first, so that most of f_wav can
-  // cross the bus while the smaller scales are transformed
-  const std::vector<std::pair<size_t, size_t>> passes = table_passes(P, pipe != nullptr);
-  for (const auto &pk : passes) {
-    const size_t k0 = pk.first, k1 = pk.second;
-    const int ngrp = (int)(k1 - k0);
-    const int bl = P.sc[k0].bl, W = 2 * bl - 1, nn = (int)P.sc[k0].ns.size();
-    const int nt = P.nt(bl), K = P.K(bl);
-    for (int i = 0; i < nn; ++i) {
-      L2T grp[2];
-      for (int q = 0; q < ngrp; ++q) {
-        const Scale &sd = P.sc[k0 + q];
-        const int n = sd.ns[i];
-        L2T &a = grp[q];
-        a = L2T{};
-        a.tb = &P.table(bl, std::abs(n));
-        a.n = n;
-        a.use_q = adj;
-        a.mlo = (real && n == 0) ? 0 : -(bl - 1);
-        a.mhi = bl - 1;
-        a.x = flm;
-        a.xs = (int64_t)L * L;
-        a.xL = L;
-        a.x_half = flm_half;
-        if (P.axisym) {
-          a.w = P.d_w + sd.w_axi;
-          a.wkind = P.wkind(sd.w_axi, bl);
-          a.wscale = adj ? 2.0 * kPi / K * kSqrt2Pi : 1.0 / kSqrt2Pi;
-        } else {
-          a.w = P.d_w + sd.w_split[i];
-          a.wkind = P.wkind(sd.w_split[i], bl);
-          a.wscale = adj ? 4.0 * kPi * kPi / K : 1.0;
-        }
-        a.lmin = std::max((real || P.axisym) ? 0 : std::abs(P.s), sd.lsup_split[i]);
-        a.out = Gbuf + q * gsz + (int64_t)i * nt * W;
-        a.os = (int64_t)nn * nt * W;
-        a.ow = W;
-        a.omlo = -(bl - 1);
-        a.nb = nb;
-      }
-      contract_l2t_group(grp, ngrp, S.st);
+  const auto norm = [&](const Scale &sd) { return adj && !P.axisym ? 1.0 / sd.ng : 1.0; };
+  // the contraction of direction i of a scale into G ([b][n][t][m], spectral width W = 2bl-1)
+  const auto problem = [&](const Scale &sd, int i, double2 *G) {
+    const int bl = sd.bl, W = 2 * bl - 1, n = sd.ns[i], nt = P.nt(bl), K = P.K(bl);
+    L2T a{};
+    a.tb = &P.table(bl, std::abs(n));
+    a.n = n;
+    a.use_q = adj;
+    a.mlo = (real && n == 0) ? 0 : -(bl - 1);
+    a.mhi = bl - 1;
+    a.x = flm;
+    a.xs = (int64_t)L * L;
+    a.xL = L;
+    a.x_half = flm_half;
+    if (P.axisym) {
+      a.w = P.d_w + sd.w_axi;
+      a.wkind = P.wkind(sd.w_axi, bl);
+      a.wscale = adj ? 2.0 * kPi / K * kSqrt2Pi : 1.0 / kSqrt2Pi;
+    } else {
+      a.w = P.d_w + sd.w_split[i];
+      a.wkind = P.wkind(sd.w_split[i], bl);
+      a.wscale = adj ? 4.0 * kPi * kPi / K : 1.0;
     }
-    for (int q = 0; q < ngrp; ++q) {
-      const Scale &sd = P.sc[k0 + q];
-      const int ng = sd.ng;
-      const double c = adj && !P.axisym ? 1.0 / ng : 1.0;
-      char *out = (char *)f_wav + (size_t)sd.woff * esz;
-      const double2 *Gq = Gbuf + q * gsz;
-      if (rings_on_n(P, sd)) {
-        // F_n(t, p) = sum_m G_n(t, m) e^{i m phi_p}; spec holds F[b][i][t][p].
-        // With host copies, in groups of maps, each group copied out when done.
-        const int G = pipe ? pipe->group : nb;
-        for (int b0 = 0; b0 < nb; b0 += G) {
-          const int nbg = std::min(G, nb - b0);
-          const double2 *Gb = Gq + (int64_t)b0 * nn * nt * W;
-          if (ring_gamma_fusable(nn, ng, bl, P.ss)) {  // one launch, the n-components stay on chip
-            ring_inverse_gamma(Gb, (int64_t)nn * nt * W, (int64_t)nt * W, sd.ns, ng, real, c,
-                               out + (size_t)b0 * wstride * esz, wstride, nbg, bl, P.ss, S.st);
-            if (pipe) pipe->out(S.st, f_wav, wstride, sd.woff, b0, nbg);
-            continue;
-          }
+    a.lmin = std::max((real || P.axisym) ? 0 : std::abs(P.s), sd.lsup_split[i]);
+    a.out = G + (int64_t)i * nt * W;
+    a.os = (int64_t)sd.ns.size() * nt * W;
+    a.ow = W;
+    a.omlo = -(bl - 1);
+    a.nb = nb;
+    return a;
+  };
+  double2 *spec = nullptr;  // ring buffer [b][n or g][t][p] of the separate ring and gamma launches
+  // ring and gamma DFTs of one scale, its spectra complete in G; launches shared
+  // through `rings` where the scale's path allows it
+  const auto to_pixels = [&](const Scale &sd, double2 *G, bool share) {
+    const int bl = sd.bl, W = 2 * bl - 1, nn = (int)sd.ns.size(), ng = sd.ng, nt = P.nt(bl), K = P.K(bl);
+    const double c = norm(sd);
+    char *out = wav + (size_t)sd.woff * esz;
+    const RingPath path = ring_path(P, sd);
+    const int group = pipe && !share && grouped_copies(path) ? pipe->group : nb;
+    for (int b0 = 0; b0 < nb; b0 += group) {
+      const int nbg = std::min(group, nb - b0);
+      switch (path) {
+        case RINGS_FUSED:  // one launch, the n-components stay on chip
+          rings.add(sd, c, gamma_job(P, sd, G, wav, esz, wstride, b0, nbg));
+          break;
+        case RINGS_ONE_SLICE:
+          rings.plain.push_back(slice_job(P, sd, G, wav, esz, wstride, nb, false));
+          break;
+        case RINGS_ON_N: {
+          // F_n(t, p) = sum_m G_n(t, m) e^{i m phi_p}; spec holds F[b][i][t][p]
           double2 *sb = spec + (int64_t)b0 * nn * nt * K;
+          std::vector<RingJob> jobs;
           for (int i = 0; i < nn; ++i) {
             const bool herm = real && sd.ns[i] == 0;  // real signal, n = 0: only m >= 0 computed
-            ring_inverse_c(Gb + (int64_t)i * nt * W + (herm ? bl - 1 : 0), W, (int64_t)nn * nt * W, nt,
-                           herm ? bl : W, herm ? 0 : -(bl - 1), herm, sb + (int64_t)i * nt * K, K,
-                           (int64_t)nn * nt * K, nt, nbg * nt, bl, P.ss, S.st);
+            RingJob j = ring_job(G + ((int64_t)b0 * nn + i) * nt * W + (herm ? bl - 1 : 0), sb + (int64_t)i * nt * K,
+                                 K, (int64_t)nn * nt * K, nt, W, herm ? 0 : -(bl - 1), nbg, bl);
+            j.spec_map_stride = (int64_t)nn * nt * W;
+            j.spec_rpm = nt;
+            j.sw = herm ? bl : W;
+            j.herm = herm;
+            jobs.push_back(j);
           }
-          gamma_px_synthesis(sb, out + (size_t)b0 * wstride * esz, wstride, sd.d_ns, nn, ng, bl, P.ss, nbg, real,
-                             c, S.st);
-          if (pipe) pipe->out(S.st, f_wav, wstride, sd.woff, b0, nbg);
+          ring_inverse_many(jobs, P.ss, false, S.st);
+          gamma_px_synthesis(sb, out + (size_t)b0 * wstride * esz, wstride, sd.d_ns, nn, ng, bl, P.ss, nbg, real, c,
+                             S.st);
+          break;
         }
-      } else {
-        const int sw = real ? bl : W, mlo = real ? 0 : -(bl - 1);
-        gamma_synthesis(Gq, spec, sd.d_ns, nn, ng, bl, P.ss, nb, real, c, S.st);
-        ring_inverse(spec, sw, sw, mlo, out, K, wstride, ng * nt, nb * ng * nt, bl, P.ss, real, S.st);
-        if (pipe) pipe->out(S.st, f_wav, wstride, sd.woff, 0, nb);
+        case RINGS_ON_SLICES: {
+          const int sw = real ? bl : W, mlo = real ? 0 : -(bl - 1);
+          gamma_synthesis(G, spec, sd.d_ns, nn, ng, bl, P.ss, nb, real, c, S.st);
+          RingJob j = ring_job(spec, out, K, wstride, ng * nt, sw, mlo, nb, bl);
+          ring_inverse_many({j}, P.ss, real, S.st);
+          break;
+        }
+      }
+      if (!share) {
+        rings.inverse(P.ss, real, S.st);
+        if (pipe) pipe->out(S.st, f_wav, wstride, sd.woff, b0, nbg);
       }
     }
+  };
+  const int64_t Kmax = 2 * P.max_bl, ntmax = P.nt(P.max_bl);
+  if (needs_ring_buffer(P)) spec = S.get<double2>((int64_t)nb * std::max(P.max_ng, P.max_nn) * ntmax * Kmax);
+  const auto gsize = [&](const Scale &sd) { return (int64_t)nb * (int64_t)sd.ns.size() * P.nt(sd.bl) * (2 * sd.bl - 1); };
+  const auto run_small = [&] {
+    std::vector<std::pair<const Scale *, double2 *>> sc;
+    for (const Scale &sd : P.sc)
+      if (small_scale(P, sd, nb)) {
+        double2 *G = S.get<double2>(gsize(sd));
+        for (size_t i = 0; i < sd.ns.size(); ++i) small.push_back(problem(sd, (int)i, G));
+        sc.emplace_back(&sd, G);
+      }
+    contract_l2t_many(small, S.st);
+    for (const auto &x : sc) to_pixels(*x.first, x.second, true);
+    rings.inverse(P.ss, real, S.st);
+    if (pipe)
+      for (const auto &x : sc) pipe->out(S.st, f_wav, wstride, x.first->woff, 0, nb);
+  };
+  // with host copies the largest scales go first, so that most of f_wav can
+  // cross the bus while the smaller scales are transformed
+  if (!pipe) run_small();
+  const auto passes = table_passes(P, pipe != nullptr, nb);
+  int64_t gtot = 0;  // spectra of one pass, reused by the next
+  for (const auto &pk : passes)
+    if (!small_scale(P, P.sc[pk.first], nb))
+      gtot = std::max(gtot, (int64_t)(pk.second - pk.first) * gsize(P.sc[pk.first]));
+  double2 *Gbuf = gtot ? S.get<double2>(gtot) : nullptr;
+  std::vector<RingJob> scal_ring;
+  if (pipe) scal_ring.swap(rings.plain);  // the scaling function goes with the small scales
+  for (const auto &pk : passes) {
+    const Scale &s0 = P.sc[pk.first];
+    if (small_scale(P, s0, nb)) continue;
+    const int ngrp = (int)(pk.second - pk.first);
+    const int64_t gsz = gsize(s0);
+    for (size_t i = 0; i < s0.ns.size(); ++i) {
+      L2T grp[kMaxParts];
+      for (int q = 0; q < ngrp; ++q) grp[q] = problem(P.sc[pk.first + q], (int)i, Gbuf + q * gsz);
+      contract_l2t_group(grp, ngrp, S.st);
+    }
+    for (int q = 0; q < ngrp; ++q) to_pixels(P.sc[pk.first + q], Gbuf + q * gsz, !pipe);
+    if (!pipe) rings.inverse(P.ss, real, S.st);
+  }
+  if (pipe) {
+    rings.plain.swap(scal_ring);
+    run_small();
   }
 }
 
@@ -672,13 +813,16 @@ void wav_merge(const WavPlan &P, MergeMode mode, const void *f_wav, int64_t wstr
   const int L = P.L;
   const size_t esz = real ? sizeof(double) : sizeof(double2);
   const bool adj = (mode == MERGE_ANALYSIS_ADJ);
+  char *wav = (char *)const_cast<void *>(f_wav);
   double2 *z = S.get<double2>((int64_t)nb * std::max<int64_t>(1, P.z_per_map));
   const int bs = P.bl_scal, Ks = P.K(bs), nts = P.nt(bs);
   double2 *zs = S.get<double2>((int64_t)nb * bs * bs);
+  std::vector<T2L> small;  // contractions that share launches
+  RingJobs rings;
   {
     const int sw = real ? bs : 2 * bs - 1, mlo = real ? 0 : -(bs - 1);
     double2 *spec = S.get<double2>((int64_t)nb * nts * sw);
-    ring_forward(f_scal, Ks, sstride, nts, spec, sw, sw, mlo, nb * nts, bs, P.ss, real, S.st);
+    rings.plain.push_back(ring_job(f_scal, spec, Ks, sstride, nts, sw, mlo, nb, bs));
     if (P.scal_lmin > 0) S2G_CUDA(cudaMemsetAsync(zs, 0, sizeof(double2) * nb * bs * bs, S.st));
     T2L a{};
     a.tb = &P.table(bs, 0);
@@ -697,88 +841,126 @@ void wav_merge(const WavPlan &P, MergeMode mode, const void *f_wav, int64_t wstr
     a.y = zs;
     a.ys = (int64_t)bs * bs;
     a.nb = nb;
-    contract_t2l(a, S.st);
+    small.push_back(a);
   }
-  const int64_t Wmax = 2 * P.max_bl - 1, Kmax = 2 * P.max_bl, ntmax = P.nt(P.max_bl);
-  const int64_t gsz = (int64_t)nb * P.max_nn * ntmax * Wmax;
-  double2 *Gbuf = S.get<double2>(2 * gsz);
-  double2 *spec = needs_ring_buffer(P) ? S.get<double2>((int64_t)nb * std::max(P.max_ng, P.max_nn) * ntmax * Kmax)
-                                       : nullptr;
-  // with host copies the largest scales go first (their pieces are queued
-  // first, see merge_order), so that their ring DFTs run while the rest of
-  // f_wav is still crossing the bus
-  const std::vector<std::pair<size_t, size_t>> passes = table_passes(P, pipe != nullptr);
-  for (const auto &pk : passes) {
-    const size_t k0 = pk.first, k1 = pk.second;
-    const int ngrp = (int)(k1 - k0);
-    const int bl = P.sc[k0].bl, W = 2 * bl - 1, nn = (int)P.sc[k0].ns.size();
-    const int nt = P.nt(bl), K = P.K(bl);
-    const int sw = real ? bl : W, mlo = real ? 0 : -(bl - 1);
-    for (int q = 0; q < ngrp; ++q) {
-      const Scale &sd = P.sc[k0 + q];
-      const int ng = sd.ng;
-      const double c = (adj || P.axisym) ? 1.0 : 1.0 / ng;
-      const char *in = (const char *)f_wav + (size_t)sd.woff * esz;
-      double2 *Gq = Gbuf + q * gsz;
-      if (rings_on_n(P, sd)) {
-        // F_n(t, p) = c sum_g e^{-i n gamma_g} f_g(t, p), then one DFT per (n, t).
-        // With host copies, in groups of maps, each after its copy has landed.
-        const int G = pipe ? pipe->group : nb;
-        for (int b0 = 0; b0 < nb; b0 += G) {
-          const int nbg = std::min(G, nb - b0);
-          if (pipe) pipe->wait(S.st, sd.woff, b0);
-          if (ring_gamma_fusable(nn, ng, bl, P.ss)) {  // one launch, the n-components stay on chip
-            gamma_ring_forward(in + (size_t)b0 * wstride * esz, wstride, sd.ns, ng, real, c,
-                               Gq + (int64_t)b0 * nn * nt * W, (int64_t)nn * nt * W, (int64_t)nt * W, nbg, bl, P.ss,
-                               S.st);
-            continue;
-          }
+  const auto norm = [&](const Scale &sd) { return (adj || P.axisym) ? 1.0 : 1.0 / sd.ng; };
+  const auto problem = [&](const Scale &sd, int i, const double2 *G) {
+    const int bl = sd.bl, W = 2 * bl - 1, n = sd.ns[i], nt = P.nt(bl), K = P.K(bl);
+    T2L a{};
+    a.tb = &P.table(bl, std::abs(n));
+    a.n = n;
+    a.use_q = !adj;
+    a.mlo = (real && n == 0) ? 0 : -(bl - 1);
+    a.mhi = bl - 1;
+    a.in = G + (int64_t)i * nt * W;
+    a.is = (int64_t)sd.ns.size() * nt * W;
+    a.iw = W;
+    a.imlo = -(bl - 1);
+    if (P.axisym) {
+      a.w = P.d_w + sd.w_axi;
+      a.wkind = P.wkind(sd.w_axi, bl);
+      a.wscale = adj ? 1.0 / kSqrt2Pi : 2.0 * kPi / K * kSqrt2Pi;
+      a.lmin = sd.lsup_merge[i];
+    } else {
+      a.w = nullptr;
+      a.wscale = adj ? 1.0 : 4.0 * kPi * kPi / K;
+      a.lmin = std::max(real ? 0 : std::abs(P.s), sd.lsup_merge[i]);
+    }
+    a.y = z + sd.z_off[i];
+    a.ys = P.z_per_map;
+    a.nb = nb;
+    return a;
+  };
+  double2 *spec = nullptr;  // ring buffer of the separate ring and gamma launches
+  // ring and gamma DFTs of one scale into G, the launches shared through `rings`
+  // where the scale's path allows it
+  const auto to_spectra = [&](const Scale &sd, double2 *G, bool share) {
+    const int bl = sd.bl, W = 2 * bl - 1, nn = (int)sd.ns.size(), ng = sd.ng, nt = P.nt(bl), K = P.K(bl);
+    const double c = norm(sd);
+    const char *in = wav + (size_t)sd.woff * esz;
+    const RingPath path = ring_path(P, sd);
+    const int group = pipe && grouped_copies(path) ? pipe->group : nb;
+    if (share && pipe)
+      for (int b0 = 0; b0 < nb; b0 += group) pipe->wait(S.st, sd.woff, b0);
+    const int step = share ? nb : group;
+    for (int b0 = 0; b0 < nb; b0 += step) {
+      const int nbg = std::min(step, nb - b0);
+      // with host copies, in groups of maps, each after its copy has landed
+      if (pipe && !share) pipe->wait(S.st, sd.woff, b0);
+      switch (path) {
+        case RINGS_FUSED:  // one launch, the n-components stay on chip
+          rings.add(sd, c, gamma_job(P, sd, G, wav, esz, wstride, b0, nbg));
+          break;
+        case RINGS_ONE_SLICE:
+          rings.plain.push_back(slice_job(P, sd, G, wav, esz, wstride, nb, true));
+          break;
+        case RINGS_ON_N: {
+          // F_n(t, p) = c sum_g e^{-i n gamma_g} f_g(t, p), then one DFT per (n, t)
           double2 *sb = spec + (int64_t)b0 * nn * nt * K;
           gamma_px_analysis(in + (size_t)b0 * wstride * esz, wstride, sb, sd.d_ns, nn, ng, bl, P.ss, nbg, real, c,
                             S.st);
-          for (int i = 0; i < nn; ++i)
-            ring_forward_c(sb + (int64_t)i * nt * K, K, (int64_t)nn * nt * K, nt,
-                           Gq + (int64_t)b0 * nn * nt * W + (int64_t)i * nt * W, W, (int64_t)nn * nt * W, nt, W,
-                           -(bl - 1), nbg * nt, bl, P.ss, S.st);
+          std::vector<RingJob> jobs;
+          for (int i = 0; i < nn; ++i) {
+            RingJob j = ring_job(sb + (int64_t)i * nt * K, G + ((int64_t)b0 * nn + i) * nt * W, K,
+                                 (int64_t)nn * nt * K, nt, W, -(bl - 1), nbg, bl);
+            j.spec_map_stride = (int64_t)nn * nt * W;
+            j.spec_rpm = nt;
+            jobs.push_back(j);
+          }
+          ring_forward_many(jobs, P.ss, false, S.st);
+          break;
         }
-      } else {
-        if (pipe) pipe->wait(S.st, sd.woff, 0);
-        ring_forward(in, K, wstride, ng * nt, spec, sw, sw, mlo, nb * ng * nt, bl, P.ss, real, S.st);
-        gamma_analysis(spec, Gq, sd.d_ns, nn, ng, bl, P.ss, nb, real, c, S.st);
+        case RINGS_ON_SLICES: {
+          const int sw = real ? bl : W, mlo = real ? 0 : -(bl - 1);
+          ring_forward_many({ring_job(in, spec, K, wstride, ng * nt, sw, mlo, nb, bl)}, P.ss, real, S.st);
+          gamma_analysis(spec, G, sd.d_ns, nn, ng, bl, P.ss, nb, real, c, S.st);
+          break;
+        }
       }
+      if (!share) rings.forward(P.ss, real, S.st);
     }
-    for (int i = 0; i < nn; ++i) {
-      T2L grp[2];
-      for (int q = 0; q < ngrp; ++q) {
-        const Scale &sd = P.sc[k0 + q];
-        const int n = sd.ns[i];
-        T2L &a = grp[q];
-        a = T2L{};
-        a.tb = &P.table(bl, std::abs(n));
-        a.n = n;
-        a.use_q = !adj;
-        a.mlo = (real && n == 0) ? 0 : -(bl - 1);
-        a.mhi = bl - 1;
-        a.in = Gbuf + q * gsz + (int64_t)i * nt * W;
-        a.is = (int64_t)nn * nt * W;
-        a.iw = W;
-        a.imlo = -(bl - 1);
-        if (P.axisym) {
-          a.w = P.d_w + sd.w_axi;
-          a.wkind = P.wkind(sd.w_axi, bl);
-          a.wscale = adj ? 1.0 / kSqrt2Pi : 2.0 * kPi / K * kSqrt2Pi;
-          a.lmin = sd.lsup_merge[i];
-        } else {
-          a.w = nullptr;
-          a.wscale = adj ? 1.0 : 4.0 * kPi * kPi / K;
-          a.lmin = std::max(real ? 0 : std::abs(P.s), sd.lsup_merge[i]);
-        }
-        a.y = z + sd.z_off[i];
-        a.ys = P.z_per_map;
-        a.nb = nb;
+  };
+  const int64_t Kmax = 2 * P.max_bl, ntmax = P.nt(P.max_bl);
+  if (needs_ring_buffer(P)) spec = S.get<double2>((int64_t)nb * std::max(P.max_ng, P.max_nn) * ntmax * Kmax);
+  const auto gsize = [&](const Scale &sd) { return (int64_t)nb * (int64_t)sd.ns.size() * P.nt(sd.bl) * (2 * sd.bl - 1); };
+  const auto run_small = [&] {
+    for (const Scale &sd : P.sc)
+      if (small_scale(P, sd, nb)) {
+        double2 *G = S.get<double2>(gsize(sd));
+        to_spectra(sd, G, true);
+        for (size_t i = 0; i < sd.ns.size(); ++i) small.push_back(problem(sd, (int)i, G));
       }
+    rings.forward(P.ss, real, S.st);
+    contract_t2l_many(small, S.st);
+  };
+  // with host copies the largest scales go first (their pieces are queued
+  // first), so that their ring DFTs run while the rest of f_wav is still
+  // crossing the bus
+  if (!pipe) run_small();
+  const auto passes = table_passes(P, pipe != nullptr, nb);
+  int64_t gtot = 0;  // spectra of one pass, reused by the next
+  for (const auto &pk : passes)
+    if (!small_scale(P, P.sc[pk.first], nb))
+      gtot = std::max(gtot, (int64_t)(pk.second - pk.first) * gsize(P.sc[pk.first]));
+  double2 *Gbuf = gtot ? S.get<double2>(gtot) : nullptr;
+  std::vector<RingJob> scal_ring;
+  if (pipe) scal_ring.swap(rings.plain);  // the scaling function goes with the small scales
+  for (const auto &pk : passes) {
+    const Scale &s0 = P.sc[pk.first];
+    if (small_scale(P, s0, nb)) continue;
+    const int ngrp = (int)(pk.second - pk.first);
+    const int64_t gsz = gsize(s0);
+    for (int q = 0; q < ngrp; ++q) to_spectra(P.sc[pk.first + q], Gbuf + q * gsz, !pipe);
+    if (!pipe) rings.forward(P.ss, real, S.st);
+    for (size_t i = 0; i < s0.ns.size(); ++i) {
+      T2L grp[kMaxParts];
+      for (int q = 0; q < ngrp; ++q) grp[q] = problem(P.sc[pk.first + q], (int)i, Gbuf + q * gsz);
       contract_t2l_group(grp, ngrp, S.st);
     }
+  }
+  if (pipe) {
+    rings.plain.swap(scal_ring);
+    run_small();
   }
   merge_lmn(flm, L, (int64_t)L * L, z, P.z_per_map, P.d_pairs, P.npairs, P.d_w, zs, (int64_t)bs * bs, bs,
             real, accumulate, nb, S.st);
@@ -1365,10 +1547,10 @@ int host_batch(const char *fn, s2g::Op op, const s2let_parameters_t *p, bool rea
         copy_async(hs + (size_t)c0 * ns * esz, 0, ds, 0, (size_t)n * ns * esz, 1, cudaMemcpyDeviceToHost, st);
       } else {
         copy_async(ds, 0, hs + (size_t)c0 * ns * esz, 0, (size_t)n * ns * esz, 1, cudaMemcpyHostToDevice, st);
-        for (const auto &pk : table_passes(P, true))  // in the order the synthesis reads them
+        for (const auto &pk : table_passes(P, true, n))  // in the order the synthesis reads them
           for (size_t k = pk.first; k < pk.second; ++k) {
             const Scale &sd = P.sc[k];
-            if (rings_on_n(P, sd)) {
+            if (grouped_copies(ring_path(P, sd))) {
               for (int b0 = 0; b0 < n; b0 += pipe.group) pipe.in(dw, nw, sd.woff, b0, std::min(pipe.group, n - b0));
             } else {
               pipe.in(dw, nw, sd.woff, 0, n);

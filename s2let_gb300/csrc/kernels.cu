@@ -12,6 +12,7 @@
 #include <map>
 #include <mutex>
 #include <type_traits>
+#include <vector>
 
 #include "autotune.h"
 #include "common.h"
@@ -98,6 +99,21 @@ struct ContractArgs {
   int lmin2;
 };
 
+// Problems of one launch: blockIdx.x runs over the m of all of them, problem q
+// has first[q] .. first[q + 1].  The contractions of the small band-limits (a
+// few microseconds each, and a launch each before) go in one.
+constexpr int kMaxBatch = 16;
+struct ContractBatch {
+  int n;
+  int first[kMaxBatch + 1];
+  ContractArgs a[kMaxBatch];
+};
+__device__ __forceinline__ int problem_of(const ContractBatch &g) {
+  int q = 0;
+  while (q + 1 < g.n && (int)blockIdx.x >= g.first[q + 1]) ++q;
+  return q;
+}
+
 __device__ __forceinline__ double2 weight_at(const ContractArgs &a, int l) {
   double2 w = a.w ? a.w[l] : make_double2(1.0, 0.0);
   if (a.wconj) w.y = -w.y;
@@ -107,10 +123,12 @@ __device__ __forceinline__ double2 weight_at(const ContractArgs &a, int l) {
 // MODE 0: l->t with D (A[t][l] = D[t][l-l0])     MODE 1: l->t with Q^T (A[t][l] = Q[l-l0][t])
 // MODE 2: t->l with Q (A[l][t] = Q[l-l0][t])     MODE 3: t->l with D^T (A[l][t] = D[t][l-l0])
 template <int MODE, int NBT>
-__global__ void __launch_bounds__(CT_M) k_contract(ContractArgs a) {
+__global__ void __launch_bounds__(CT_M) k_contract(const __grid_constant__ ContractBatch g) {
   __shared__ double sA[CT_M][CT_K + 1];
   __shared__ double2 sX[CT_K][NBT];
-  const int m = a.mlo + blockIdx.x;
+  const int prob = problem_of(g);
+  const ContractArgs &a = g.a[prob];
+  const int m = a.mlo + (int)blockIdx.x - g.first[prob];
   const int am = m < 0 ? -m : m;
   const int l0 = am > a.an ? am : a.an;
   const int bl = a.bl;
@@ -331,10 +349,12 @@ constexpr int DFC_R = 8;    // rows per lane (MODE 0, 2; half that from 4 maps p
 constexpr int DFC_LPR = 8;  // lanes per row (MODE 0, 2)
 
 template <int MODE, int NBT, class E>
-__global__ void __launch_bounds__(CT_M) k_contract_df(ContractArgs a) {
+__global__ void __launch_bounds__(CT_M) k_contract_df(const __grid_constant__ ContractBatch gb) {
   extern __shared__ float4 sx[];  // [k - kbeg][b]
   __shared__ int sxm[NBT];
-  const int m = a.mlo + blockIdx.x;
+  const int prob = problem_of(gb);
+  const ContractArgs &a = gb.a[prob];
+  const int m = a.mlo + (int)blockIdx.x - gb.first[prob];
   const int am = m < 0 ? -m : m;
   const int l0 = am > a.an ? am : a.an;
   const int bl = a.bl;
@@ -543,21 +563,22 @@ void contract_work(const ContractArgs &a, int nm, double *flops, double *bytes, 
 constexpr size_t kDfcSmemMax = 200 * 1024;
 
 template <int MODE, int NBT, class E>
-void launch_contract_df_e(dim3 grid, size_t smem, const ContractArgs &a, cudaStream_t st) {
+void launch_contract_df_e(dim3 grid, size_t smem, const ContractBatch &g, cudaStream_t st) {
   static bool attr = [] {
     S2G_CUDA(cudaFuncSetAttribute(k_contract_df<MODE, NBT, E>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)kDfcSmemMax));
     return true;
   }();
   (void)attr;
-  k_contract_df<MODE, NBT, E><<<grid, CT_M, smem, st>>>(a);
+  k_contract_df<MODE, NBT, E><<<grid, CT_M, smem, st>>>(g);
 }
+// every problem of the batch reads the same form of table
 template <int MODE, int NBT>
-void launch_contract_df(dim3 grid, size_t smem, const ContractArgs &a, cudaStream_t st) {
-  if (a.table_df)
-    launch_contract_df_e<MODE, NBT, float2>(grid, smem, a, st);
+void launch_contract_df(dim3 grid, size_t smem, const ContractBatch &g, cudaStream_t st) {
+  if (g.a[0].table_df)
+    launch_contract_df_e<MODE, NBT, float2>(grid, smem, g, st);
   else
-    launch_contract_df_e<MODE, NBT, double>(grid, smem, a, st);
+    launch_contract_df_e<MODE, NBT, double>(grid, smem, g, st);
 }
 
 // Double-float copies of stored Wigner tables for the double-float
@@ -601,47 +622,69 @@ const float2 *df_table(const WignerTable &tb, bool q, cudaStream_t st) {
   return p;
 }
 
+ContractBatch batch_of(const ContractArgs &a, int nm) {
+  ContractBatch g;
+  g.n = 1;
+  g.first[0] = 0;
+  g.first[1] = nm;
+  g.a[0] = a;
+  return g;
+}
+
+// rows: the most output rows of any problem of the batch
 template <int MODE>
-void launch_contract_nbt(const ContractArgs &a, int nm, int rows, int nbt, cudaStream_t st) {
-  dim3 grid(nm, ceil_div(rows, CT_M), ceil_div(a.nb, nbt));
+void launch_contract_nbt(const ContractBatch &g, int rows, int nbt, cudaStream_t st) {
+  const int nb = g.a[0].nb;
+  dim3 grid(g.first[g.n], ceil_div(rows, CT_M), ceil_div(nb, nbt));
   if (t_precision == 1) {  // split precision: the double-float kernel
     // shared memory: the split coefficient columns over the reduction range
-    const int kmax = a.bl > a.nt ? a.bl : a.nt;
+    int kmax = 0;
+    for (int q = 0; q < g.n; ++q) kmax = std::max(kmax, std::max(g.a[q].bl, g.a[q].nt));
     while (nbt > 1 && (size_t)kmax * nbt * sizeof(float4) > kDfcSmemMax) nbt /= 2;
     S2G_REQUIRE((size_t)kmax * sizeof(float4) <= kDfcSmemMax, ERR_UNSUPPORTED,
                 "reduction range too long for the double-float contraction");
-    grid.z = ceil_div(a.nb, nbt);
+    grid.z = ceil_div(nb, nbt);
     const size_t smem = (size_t)kmax * nbt * sizeof(float4);
     switch (nbt) {
-      case 8: launch_contract_df<MODE, 8>(grid, smem, a, st); break;
-      case 4: launch_contract_df<MODE, 4>(grid, smem, a, st); break;
-      case 2: launch_contract_df<MODE, 2>(grid, smem, a, st); break;
-      default: launch_contract_df<MODE, 1>(grid, smem, a, st); break;
+      case 8: launch_contract_df<MODE, 8>(grid, smem, g, st); break;
+      case 4: launch_contract_df<MODE, 4>(grid, smem, g, st); break;
+      case 2: launch_contract_df<MODE, 2>(grid, smem, g, st); break;
+      default: launch_contract_df<MODE, 1>(grid, smem, g, st); break;
     }
     S2G_LAUNCHED();
     return;
   }
   switch (nbt) {
-  case 8: k_contract<MODE, 8><<<grid, CT_M, 0, st>>>(a); break;
-  case 4: k_contract<MODE, 4><<<grid, CT_M, 0, st>>>(a); break;
-  case 2: k_contract<MODE, 2><<<grid, CT_M, 0, st>>>(a); break;
-  default: k_contract<MODE, 1><<<grid, CT_M, 0, st>>>(a); break;
+  case 8: k_contract<MODE, 8><<<grid, CT_M, 0, st>>>(g); break;
+  case 4: k_contract<MODE, 4><<<grid, CT_M, 0, st>>>(g); break;
+  case 2: k_contract<MODE, 2><<<grid, CT_M, 0, st>>>(g); break;
+  default: k_contract<MODE, 1><<<grid, CT_M, 0, st>>>(g); break;
   }
   S2G_LAUNCHED();
 }
 
 // maps per CTA: the largest power of two up to 8 that the batch fills, or the
-// autotuned choice among those (per mode, band-limit bucket and batch bucket)
+// autotuned choice among those (per mode, bucket of the largest band-limit and
+// batch bucket)
 template <int MODE>
-void launch_contract(const ContractArgs &a, int nm, int rows, cudaStream_t st) {
+void launch_contract(const ContractBatch &g, int rows, cudaStream_t st) {
   static const int kCand[4] = {1, 2, 4, 8};
-  const int ncand = a.nb >= 8 ? 4 : (a.nb >= 4 ? 3 : (a.nb >= 2 ? 2 : 1));
-  const int c = tuned(TF_CONTRACT, MODE + 4 * t_precision, tune_bucket(a.bl), tune_bucket(a.nb), ncand, ncand - 1,
-                      st, [&](int i) { launch_contract_nbt<MODE>(a, nm, rows, kCand[i], st); });
+  const int nb = g.a[0].nb;
+  const int ncand = nb >= 8 ? 4 : (nb >= 4 ? 3 : (nb >= 2 ? 2 : 1));
+  int bl = 0;
+  for (int q = 0; q < g.n; ++q) bl = std::max(bl, g.a[q].bl);
+  const int c = tuned(TF_CONTRACT, MODE + 4 * t_precision, tune_bucket(bl), tune_bucket(nb), ncand, ncand - 1, st,
+                      [&](int i) { launch_contract_nbt<MODE>(g, rows, kCand[i], st); });
   double fl = 0, by = 0;
-  if (timing_enabled()) contract_work(a, nm, &fl, &by);
+  if (timing_enabled())
+    for (int q = 0; q < g.n; ++q) {
+      double f1 = 0, b1 = 0;
+      contract_work(g.a[q], g.first[q + 1] - g.first[q], &f1, &b1);
+      fl += f1;
+      by += b1;
+    }
   KTimer kt(KC_CONTRACT, st, fl, by);
-  launch_contract_nbt<MODE>(a, nm, rows, kCand[c], st);
+  launch_contract_nbt<MODE>(g, rows, kCand[c], st);
 }
 
 // two parts on one table (double-float kernel, split precision): columns =
@@ -665,10 +708,11 @@ void launch_contract_df_pair(const ContractArgs &a, int nm, int rows, cudaStream
   }
   KTimer kt(KC_CONTRACT, st, fl, by);
   const dim3 grid(nm, ceil_div(rows, CT_M), 1);
+  const ContractBatch g = batch_of(a, nm);
   switch (nbt) {
-    case 8: launch_contract_df<MODE, 8>(grid, smem, a, st); break;
-    case 4: launch_contract_df<MODE, 4>(grid, smem, a, st); break;
-    default: launch_contract_df<MODE, 2>(grid, smem, a, st); break;
+    case 8: launch_contract_df<MODE, 8>(grid, smem, g, st); break;
+    case 4: launch_contract_df<MODE, 4>(grid, smem, g, st); break;
+    default: launch_contract_df<MODE, 2>(grid, smem, g, st); break;
   }
   S2G_LAUNCHED();
 }
@@ -1080,13 +1124,8 @@ namespace {
 bool on_tensor_cores(int nb) { return t_precision == 0 || nb > df_max_maps(); }
 }  // namespace
 
-void contract_l2t(const L2T &p, cudaStream_t st) {
-  if (p.nb <= 0 || p.mhi < p.mlo) return;
-  if (p.tb->rc) {
-    contract_l2t_rc(p, st);
-    return;
-  }
-  if (on_tensor_cores(p.nb) && contract_l2t_mixed(&p, 1, st)) return;
+namespace {
+ContractArgs args_of(const L2T &p, cudaStream_t st) {
   ContractArgs a{};
   a.table = p.use_q ? p.tb->Q : p.tb->D;
   if (t_precision == 1) a.table_df = df_table(*p.tb, p.use_q, st);
@@ -1110,20 +1149,9 @@ void contract_l2t(const L2T &p, cudaStream_t st) {
   a.dw = p.ow;
   a.d_mlo = p.omlo;
   a.nb = p.nb;
-  const int nm = p.mhi - p.mlo + 1;
-  if (p.use_q)
-    launch_contract<1>(a, nm, a.nt, st);
-  else
-    launch_contract<0>(a, nm, a.nt, st);
+  return a;
 }
-
-void contract_t2l(const T2L &p, cudaStream_t st) {
-  if (p.nb <= 0 || p.mhi < p.mlo) return;
-  if (p.tb->rc) {
-    contract_t2l_rc(p, st);
-    return;
-  }
-  if (on_tensor_cores(p.nb) && contract_t2l_mixed(&p, 1, st)) return;
+ContractArgs args_of(const T2L &p, cudaStream_t st) {
   ContractArgs a{};
   a.table = p.use_q ? p.tb->Q : p.tb->D;
   if (t_precision == 1) a.table_df = df_table(*p.tb, p.use_q, st);
@@ -1145,120 +1173,132 @@ void contract_t2l(const T2L &p, cudaStream_t st) {
   a.dst = p.y;
   a.ds = p.ys;
   a.nb = p.nb;
-  const int nm = p.mhi - p.mlo + 1;
-  if (p.use_q)
-    launch_contract<2>(a, nm, a.bl, st);
-  else
-    launch_contract<3>(a, nm, a.bl, st);
+  return a;
 }
-
+int rows_of(const L2T &p) { return p.tb->nt; }
+int rows_of(const T2L &p) { return p.tb->bl; }
+void launch_batch(const L2T &p, const ContractBatch &g, int rows, cudaStream_t st) {
+  if (p.use_q)
+    launch_contract<1>(g, rows, st);
+  else
+    launch_contract<0>(g, rows, st);
+}
+void launch_batch(const T2L &p, const ContractBatch &g, int rows, cudaStream_t st) {
+  if (p.use_q)
+    launch_contract<2>(g, rows, st);
+  else
+    launch_contract<3>(g, rows, st);
+}
 // split precision, two scales of one band-limit and n on a stored table, a
 // batch the double-float kernel takes: both parts in one pass over the table
-bool df_pair_l2t(const L2T *a, cudaStream_t st) {
-  const L2T &p = a[0], &q = a[1];
-  if (p.tb != q.tb || p.tb->rc || p.use_q != q.use_q || p.n != q.n || p.mlo != q.mlo || p.mhi != q.mhi ||
-      p.xs != q.xs || p.xL != q.xL || p.x_half != q.x_half || p.wscale != q.wscale || p.wconj != q.wconj ||
-      p.os != q.os || p.ow != q.ow || p.omlo != q.omlo || p.nb != q.nb || p.nb > 4 || p.nb < 1 || p.mhi < p.mlo)
-    return false;
-  ContractArgs c{};
-  c.table = p.use_q ? p.tb->Q : p.tb->D;
-  c.table_df = df_table(*p.tb, p.use_q, st);
-  c.off = p.tb->d_off;
-  c.bl = p.tb->bl;
-  c.nt = p.tb->nt;
-  c.an = p.tb->an;
-  c.tmlo = p.tb->mlo;
-  c.n = p.n;
-  c.mlo = p.mlo;
-  c.lmin = p.lmin;
-  c.w = p.w;
-  c.wscale = p.wscale;
-  c.wconj = p.wconj;
-  c.src = p.x;
-  c.ss = p.xs;
-  c.sw_or_xL = p.xL;
-  c.x_half = p.x_half;
-  c.dst = p.out;
-  c.ds = p.os;
-  c.dw = p.ow;
-  c.d_mlo = p.omlo;
-  c.nb = p.nb;
+bool same_pair(const L2T &p, const L2T &q) {
+  return p.tb == q.tb && !p.tb->rc && p.use_q == q.use_q && p.n == q.n && p.mlo == q.mlo && p.mhi == q.mhi &&
+         p.xs == q.xs && p.xL == q.xL && p.x_half == q.x_half && p.wscale == q.wscale && p.wconj == q.wconj &&
+         p.os == q.os && p.ow == q.ow && p.omlo == q.omlo && p.nb == q.nb && p.nb <= 4 && p.nb >= 1 &&
+         p.mhi >= p.mlo;
+}
+bool same_pair(const T2L &p, const T2L &q) {
+  return p.tb == q.tb && !p.tb->rc && p.use_q == q.use_q && p.n == q.n && p.mlo == q.mlo && p.mhi == q.mhi &&
+         p.is == q.is && p.iw == q.iw && p.imlo == q.imlo && p.wscale == q.wscale && p.wconj == q.wconj &&
+         p.ys == q.ys && p.nb == q.nb && p.nb <= 4 && p.nb >= 1 && p.mhi >= p.mlo;
+}
+const double2 *source_of(const L2T &p) { return p.x; }
+const double2 *source_of(const T2L &p) { return p.in; }
+double2 *dest_of(const L2T &p) { return p.out; }
+double2 *dest_of(const T2L &p) { return p.y; }
+template <class A>
+bool df_pair(const A &p, const A &q, cudaStream_t st) {
+  if (!same_pair(p, q)) return false;
+  ContractArgs c = args_of(p, st);
   c.nparts = 2;
-  c.src2 = q.x;
-  c.dst2 = q.out;
+  c.src2 = source_of(q);
+  c.dst2 = dest_of(q);
   c.w2 = q.w;
   c.lmin2 = q.lmin;
   const int nm = p.mhi - p.mlo + 1;
-  if (p.use_q)
-    launch_contract_df_pair<1>(c, nm, c.nt, st);
-  else
-    launch_contract_df_pair<0>(c, nm, c.nt, st);
+  if constexpr (std::is_same<A, L2T>::value) {
+    if (p.use_q)
+      launch_contract_df_pair<1>(c, nm, c.nt, st);
+    else
+      launch_contract_df_pair<0>(c, nm, c.nt, st);
+  } else {
+    if (p.use_q)
+      launch_contract_df_pair<2>(c, nm, c.bl, st);
+    else
+      launch_contract_df_pair<3>(c, nm, c.bl, st);
+  }
   return true;
 }
+void contract_rc(const L2T &p, cudaStream_t st) { contract_l2t_rc(p, st); }
+void contract_rc(const T2L &p, cudaStream_t st) { contract_t2l_rc(p, st); }
+bool contract_tensor(const L2T *p, int n, cudaStream_t st) { return contract_l2t_mixed(p, n, st); }
+bool contract_tensor(const T2L *p, int n, cudaStream_t st) { return contract_t2l_mixed(p, n, st); }
 
-bool df_pair_t2l(const T2L *a, cudaStream_t st) {
-  const T2L &p = a[0], &q = a[1];
-  if (p.tb != q.tb || p.tb->rc || p.use_q != q.use_q || p.n != q.n || p.mlo != q.mlo || p.mhi != q.mhi ||
-      p.is != q.is || p.iw != q.iw || p.imlo != q.imlo || p.wscale != q.wscale || p.wconj != q.wconj ||
-      p.ys != q.ys || p.nb != q.nb || p.nb > 4 || p.nb < 1 || p.mhi < p.mlo)
-    return false;
-  ContractArgs c{};
-  c.table = p.use_q ? p.tb->Q : p.tb->D;
-  c.table_df = df_table(*p.tb, p.use_q, st);
-  c.off = p.tb->d_off;
-  c.bl = p.tb->bl;
-  c.nt = p.tb->nt;
-  c.an = p.tb->an;
-  c.tmlo = p.tb->mlo;
-  c.n = p.n;
-  c.mlo = p.mlo;
-  c.lmin = p.lmin;
-  c.w = p.w;
-  c.wscale = p.wscale;
-  c.wconj = p.wconj;
-  c.src = p.in;
-  c.ss = p.is;
-  c.sw_or_xL = p.iw;
-  c.s_mlo = p.imlo;
-  c.dst = p.y;
-  c.ds = p.ys;
-  c.nb = p.nb;
-  c.nparts = 2;
-  c.src2 = q.in;
-  c.dst2 = q.y;
-  c.w2 = q.w;
-  c.lmin2 = q.lmin;
-  const int nm = p.mhi - p.mlo + 1;
-  if (p.use_q)
-    launch_contract_df_pair<2>(c, nm, c.bl, st);
-  else
-    launch_contract_df_pair<3>(c, nm, c.bl, st);
-  return true;
-}
-
-void contract_l2t_group(const L2T *a, int n, cudaStream_t st) {
-  if (n <= 0) return;
-  if (n <= 2 && !a[0].tb->rc) {
-    if (on_tensor_cores(a[0].nb)) {
-      if (contract_l2t_mixed(a, n, st)) return;
-    } else if (n == 2 && df_pair_l2t(a, st)) {
-      return;
-    }
+template <class A>
+void contract_one(const A &p, cudaStream_t st) {
+  if (p.nb <= 0 || p.mhi < p.mlo) return;
+  if (p.tb->rc) {
+    contract_rc(p, st);
+    return;
   }
-  for (int i = 0; i < n; ++i) contract_l2t(a[i], st);
+  if (on_tensor_cores(p.nb) && contract_tensor(&p, 1, st)) return;
+  launch_batch(p, batch_of(args_of(p, st), p.mhi - p.mlo + 1), rows_of(p), st);
 }
-
-void contract_t2l_group(const T2L *a, int n, cudaStream_t st) {
+template <class A>
+void contract_group(const A *a, int n, cudaStream_t st) {
   if (n <= 0) return;
-  if (n <= 2 && !a[0].tb->rc) {
-    if (on_tensor_cores(a[0].nb)) {
-      if (contract_t2l_mixed(a, n, st)) return;
-    } else if (n == 2 && df_pair_t2l(a, st)) {
-      return;
-    }
+  if (!a[0].tb->rc && on_tensor_cores(a[0].nb) && contract_tensor(a, n, st)) return;
+  const bool pairs = t_precision == 1 && !a[0].tb->rc && !on_tensor_cores(a[0].nb);
+  for (int i = 0; i < n; ++i) {
+    if (pairs && i + 1 < n && df_pair(a[i], a[i + 1], st))
+      ++i;
+    else
+      contract_one(a[i], st);
   }
-  for (int i = 0; i < n; ++i) contract_t2l(a[i], st);
 }
+template <class A>
+void contract_many(const std::vector<A> &v, cudaStream_t st) {
+  ContractBatch g;
+  const A *p0 = nullptr;
+  int rows = 0;
+  g.n = 0;
+  g.first[0] = 0;
+  const auto flush = [&] {
+    if (g.n) launch_batch(*p0, g, rows, st);
+    g.n = rows = 0;
+  };
+  for (const A &p : v) {
+    if (p.nb <= 0 || p.mhi < p.mlo) continue;
+    if (!contract_is_small(p.tb, p.nb)) {
+      contract_one(p, st);
+      continue;
+    }
+    const ContractArgs a = args_of(p, st);
+    if (g.n && (g.n == kMaxBatch || p.use_q != p0->use_q || p.nb != p0->nb ||
+                (a.table_df == nullptr) != (g.a[0].table_df == nullptr)))
+      flush();
+    p0 = g.n ? p0 : &p;
+    g.a[g.n] = a;
+    g.first[g.n + 1] = g.first[g.n] + p.mhi - p.mlo + 1;
+    rows = std::max(rows, rows_of(p));
+    ++g.n;
+  }
+  flush();
+}
+}  // namespace
+
+// Tables whose contractions run in the FP64 or double-float kernel with a small
+// CTA count: below the tensor cores' band-limit, and for the double-float one-map
+// calls up to 128 (255 CTAs of one row block; larger ones fill the GPU alone).
+bool contract_is_small(const WignerTable *tb, int nb) {
+  return !tb->rc && tb->bl <= (on_tensor_cores(nb) ? kTensorMinBl - 1 : 128);
+}
+void contract_l2t(const L2T &p, cudaStream_t st) { contract_one(p, st); }
+void contract_t2l(const T2L &p, cudaStream_t st) { contract_one(p, st); }
+void contract_l2t_group(const L2T *a, int n, cudaStream_t st) { contract_group(a, n, st); }
+void contract_t2l_group(const T2L *a, int n, cudaStream_t st) { contract_group(a, n, st); }
+void contract_l2t_many(const std::vector<L2T> &v, cudaStream_t st) { contract_many(v, st); }
+void contract_t2l_many(const std::vector<T2L> &v, cudaStream_t st) { contract_many(v, st); }
 
 void gamma_synthesis(const double2 *G, double2 *spec, const int *ns, int nn, int ng, int bl, int ss, int nb,
                      bool real, double c, cudaStream_t st) {

@@ -18,11 +18,23 @@ namespace s2g {
 // real != 0: rings are real; spectra hold m >= 0 only (mlo = 0) and are
 // Hermitian-completed on the inverse.  Spectrum rows have width `sw`.
 // Ring r lives at (r / rpm) * map_stride + (r % rpm) * ring_stride elements.
-void ring_forward(const void *rings, int64_t ring_stride, int64_t map_stride, int rpm, double2 *spec,
-                  int64_t spec_stride, int sw, int mlo, int nrings, int bl, int ss, bool real, cudaStream_t st);
-void ring_inverse(const double2 *spec, int64_t spec_stride, int sw, int mlo, void *rings,
-                  int64_t ring_stride, int64_t map_stride, int rpm, int nrings, int bl, int ss, bool real,
-                  cudaStream_t st);
+// Spectrum of ring r: (r / spec_rpm) * spec_map_stride + (r % spec_rpm) * spec_stride.
+// herm (complex inverse): columns m < 0 are conj of m > 0 (a real-valued ring held
+// as complex).  Several independent DFTs (of any band-limits, all real or all
+// complex) share a launch.
+struct RingJob {
+  const void *in = nullptr;  // forward: rings; inverse: spectra
+  void *out = nullptr;
+  int64_t ring_stride = 0, map_stride = 0;
+  int rpm = 1;
+  int64_t spec_stride = 0, spec_map_stride = 0;
+  int spec_rpm = 1 << 30;
+  int sw = 0, mlo = 0;
+  bool herm = false;
+  int nrings = 0, bl = 0;
+};
+void ring_forward_many(const std::vector<RingJob> &jobs, int ss, bool real, cudaStream_t st);
+void ring_inverse_many(const std::vector<RingJob> &jobs, int ss, bool real, cudaStream_t st);
 
 // Contraction over l producing ring spectra ("l -> t", t < tb->nt):
 //   out[b][t][m - omlo] = sum_l A_m[t][l] x_b(l, m) w(l)
@@ -31,16 +43,6 @@ void ring_inverse(const double2 *spec, int64_t spec_stride, int sw, int mlo, voi
 // (band-limit xL >= bl); when x_half, x holds m >= 0 only and
 // x(l,-m) = (-1)^m conj(x(l,m)).  w(l) = wre/wim arrays (nullable => 1) times
 // wscale, conjugated when wconj.  Rows l < lmin contribute nothing.
-// Complex rings with two-level spectrum addressing: spectrum of ring r at
-// spec + (r / spec_rpm) * spec_map_stride + (r % spec_rpm) * spec_stride.
-// herm (inverse): columns m < 0 are conj of m > 0 (a real-valued ring held as complex).
-void ring_forward_c(const double2 *rings, int64_t ring_stride, int64_t map_stride, int rpm, double2 *spec,
-                    int64_t spec_stride, int64_t spec_map_stride, int spec_rpm, int sw, int mlo, int nrings, int bl,
-                    int ss, cudaStream_t st);
-void ring_inverse_c(const double2 *spec, int64_t spec_stride, int64_t spec_map_stride, int spec_rpm, int sw,
-                    int mlo, bool herm, double2 *rings, int64_t ring_stride, int64_t map_stride, int rpm, int nrings,
-                    int bl, int ss, cudaStream_t st);
-
 // Kind of a per-l weight array: every entry real, every entry imaginary, or
 // general complex.  The directional weights are a real profile times 1 or i
 // (odd or even N), the axisymmetric and scaling weights are real.
@@ -78,8 +80,10 @@ void set_df_max_maps(int maps);
 int get_df_max_maps();
 
 void contract_l2t(const L2T &a, cudaStream_t st);
-// n problems on the same table (same band-limit, n, m range and batch): one
-// table pass on the split-precision path when n <= 2, else one call each.
+// n <= kMaxParts problems on the same table (same band-limit, n, m range and
+// batch): one table pass on the tensor cores, or in double-float two at a time,
+// else one call each.
+constexpr int kMaxParts = 8;
 void contract_l2t_group(const L2T *a, int n, cudaStream_t st);
 
 // Contraction over t producing harmonic coefficients ("t -> l"):
@@ -106,6 +110,12 @@ struct T2L {
 };
 void contract_t2l(const T2L &a, cudaStream_t st);
 void contract_t2l_group(const T2L *a, int n, cudaStream_t st);
+// Independent problems (any tables, one direction, one batch size): those on
+// small tables (contract_is_small) share launches, the others run one by one.
+bool contract_is_small(const WignerTable *tb, int nb);
+constexpr int kTensorMinBl = 64;  // smallest band-limit on the tensor cores
+void contract_l2t_many(const std::vector<L2T> &v, cudaStream_t st);
+void contract_t2l_many(const std::vector<T2L> &v, cudaStream_t st);
 
 // gamma synthesis: spec[b][g][t][m - (real?0:-(bl-1))] from coefficients
 // G[b][k][t][m + bl - 1] of directions ns[k], t < grid_rings(bl, ss); real:
@@ -138,10 +148,19 @@ void gamma_px_analysis(const void *in, int64_t in_ms, double2 *F, const int *ns,
 //   gamma_ring_forward:  F_k = c sum_g e^{-i n_k gamma_g} f_g, then the
 //                        forward ring DFT of every F_k to G (all m)
 bool ring_gamma_fusable(int nn, int ng, int bl, int ss);
-void ring_inverse_gamma(const double2 *G, int64_t gms, int64_t gks, const std::vector<int> &ns, int ng, bool real,
-                        double c, void *fw, int64_t fms, int nb, int bl, int ss, cudaStream_t st);
-void gamma_ring_forward(const void *fw, int64_t fms, const std::vector<int> &ns, int ng, bool real, double c,
-                        double2 *Gout, int64_t gms, int64_t gks, int nb, int bl, int ss, cudaStream_t st);
+// Each job is one scale's rings; all jobs of a call have the same directions.
+struct GammaJob {
+  const double2 *G = nullptr;  // synthesis: spectra in
+  double2 *Gout = nullptr;     // analysis: spectra out
+  int64_t gms = 0, gks = 0;
+  void *fw = nullptr;  // the gamma slices (analysis: read)
+  int64_t fms = 0;
+  int nb = 0, bl = 0;
+};
+void ring_inverse_gamma(const std::vector<GammaJob> &jobs, const std::vector<int> &ns, int ng, bool real, double c,
+                        int ss, cudaStream_t st);
+void gamma_ring_forward(const std::vector<GammaJob> &jobs, const std::vector<int> &ns, int ng, bool real, double c,
+                        int ss, cudaStream_t st);
 
 // FP32 storage conversions: `rows` rows of n values, row r at src + r ss and
 // dst + r ds (elements; complex values as interleaved pairs).  Widening is

@@ -73,13 +73,12 @@ constexpr int kPK = 64;                // K per panel
 constexpr int kPM = 128;               // rows per panel
 constexpr int kPanelA = kPM * kPK;     // digits of a block, elements of a panel
 constexpr int kGrpK = 16;              // consecutive K of one row in a digit block
-constexpr int kMaxParts = 2;           // scales sharing one table pass
 constexpr int kMinBl = 128;            // 7 slices from this band-limit
 // 8 slices from this band-limit, whatever the batch (so that a map's result does
 // not depend on its batch).  Per contraction at bl = 64, FP64 kernel against
 // slicing + contraction: 1 map 16 / 26 us, 8 complex maps 50 / 28, 32 maps 77 /
 // 38; at bl = 32 8 maps 28 / 29, 32 maps 37 / 30.
-constexpr int kMinBl8 = 64;
+constexpr int kMinBl8 = kTensorMinBl;
 constexpr long long kWaitCycles = 4000000000LL;
 
 // NC real coefficient columns per CTA (16, 32 or 64): parts x maps x {re, im};

@@ -70,22 +70,43 @@ struct RingArgs {
   const int4 *chirp, *bhat, *tw;
 };
 
+// Jobs of one launch: blocks (fused: clusters) first[q] .. first[q + 1] belong to
+// job q.  The scales of small band-limits, a few microseconds each, share launches.
+constexpr int kMaxJobs = 16;
+struct RingGroup {
+  int n;
+  int first[kMaxJobs + 1];
+  RingArgs a[kMaxJobs];
+};
+
 // One launch of ring DFTs fused with the gamma DFT (k_ring_inverse_gamma,
 // k_gamma_ring_forward): NN <= kFuseMaxNN n-components per ring.
 constexpr int kFuseMaxNN = 8;
 constexpr int kFuseMaxTw = 128;
-struct GammaFuse {
+struct GammaItem {
+  RingArgs a;
   const double2 *G;  // synthesis input: spectrum of component k of ring (b, t) at G + b gms + k gks + t W
   double2 *Gout;     // analysis output, the same addressing (all m from -(bl-1))
   int64_t gms, gks;
   int W, nt;
-  int herm_k;  // real signals: the component with n = 0 (m >= 0 stored, at offset bl-1), else -1
-  void *fw;    // gamma slice g of ring (b, t) at fw + b fms + g npx + t K (double, or double2 unless real)
+  void *fw;  // gamma slice g of ring (b, t) at fw + b fms + g npx + t K (double, or double2 unless real)
   int64_t fms, npx;
-  int ng, real;
-  int et;                // the twiddles below are over 2^et
+};
+struct GammaFuse {
+  int n;
+  int first[kMaxJobs + 1];
+  GammaItem it[kMaxJobs];
+  int herm_k;  // real signals: the component with n = 0 (m >= 0 stored, at offset bl-1), else -1
+  int ng;
+  int et;               // the twiddles below are over 2^et
   int4 tw[kFuseMaxTw];  // [g NN + k] twiddles with their normalisation
 };
+template <class G>
+__device__ __forceinline__ int job_of(const G &g, int block) {
+  int q = 0;
+  while (q + 1 < g.n && block >= g.first[q + 1]) ++q;
+  return q;
+}
 
 // element offset of ring r (rings of a map are ring_stride apart, maps map_stride)
 __device__ __forceinline__ int64_t ring_base(const RingArgs &a, int r) {
@@ -310,11 +331,13 @@ __device__ __forceinline__ double2 nan2() {
 constexpr int kRingThreads = 256;
 
 template <bool REAL>
-__global__ void __launch_bounds__(kRingThreads, 3) k_ring_forward(RingArgs a) {
+__global__ void __launch_bounds__(kRingThreads, 3) k_ring_forward(const __grid_constant__ RingGroup grp) {
   extern __shared__ longlong2 buf[];
   __shared__ int s_mx;
+  const int job = job_of(grp, blockIdx.x), blk = blockIdx.x - grp.first[job];
+  const RingArgs &a = grp.a[job];
   const int K = a.K, P = a.P, logP = a.logP;
-  const int r0 = REAL ? 2 * blockIdx.x : blockIdx.x;
+  const int r0 = REAL ? 2 * blk : blk;
   const bool has1 = REAL && (r0 + 1 < a.nrings);
   int em = 0;
   for (int j = threadIdx.x; j < K; j += blockDim.x) {
@@ -368,12 +391,14 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_ring_forward(RingArgs a) {
 }
 
 template <bool REAL>
-__global__ void __launch_bounds__(kRingThreads, 3) k_ring_inverse(RingArgs a) {
+__global__ void __launch_bounds__(kRingThreads, 3) k_ring_inverse(const __grid_constant__ RingGroup grp) {
   extern __shared__ longlong2 buf[];
   __shared__ int s_mx;
+  const int job = job_of(grp, blockIdx.x), blk = blockIdx.x - grp.first[job];
+  const RingArgs &a = grp.a[job];
   constexpr int BITS = REAL ? 60 : 61;  // A + i B of two rings
   const int K = a.K, P = a.P, logP = a.logP, bl = a.bl;
-  const int r0 = REAL ? 2 * blockIdx.x : blockIdx.x;
+  const int r0 = REAL ? 2 * blk : blk;
   const bool has1 = REAL && (r0 + 1 < a.nrings);
   const double2 *s0 = a.spec_in + spec_base(a, r0);
   int em = 0;
@@ -458,15 +483,17 @@ __device__ __forceinline__ int cluster_max_int(cg::cluster_group &cl, int *slot,
 }
 
 template <int NN, bool REAL>
-__global__ void __launch_bounds__(kRingThreads, 3) k_ring_inverse_gamma(RingArgs a, const __grid_constant__ GammaFuse gf) {
+__global__ void __launch_bounds__(kRingThreads, 3) k_ring_inverse_gamma(const __grid_constant__ GammaFuse grp) {
   extern __shared__ longlong2 buf[];
   __shared__ int s_mx, s_em, s_k;
   cg::cluster_group cl = cg::this_cluster();
   const int k = (int)cl.block_rank();
-  const int r = blockIdx.x / NN;
+  const int job = job_of(grp, blockIdx.x / NN), r = blockIdx.x / NN - grp.first[job];
+  const GammaItem &gf = grp.it[job];
+  const RingArgs &a = gf.a;
   const int b = r / gf.nt, t = r - b * gf.nt;
   const int K = a.K, P = a.P, logP = a.logP, bl = a.bl;
-  const bool herm = (k == gf.herm_k);
+  const bool herm = (k == grp.herm_k);
   const int sw = herm ? bl : gf.W, mlo = herm ? 0 : -(bl - 1);
   const double2 *s0 = gf.G + (int64_t)b * gf.gms + (int64_t)k * gf.gks + (int64_t)t * gf.W + (herm ? bl - 1 : 0);
   int em = 0;
@@ -501,7 +528,7 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_ring_inverse_gamma(RingArgs
     kj[j] = *cl.map_shared_rank(&s_k, j);
     km = max(km, kj[j]);
   }
-  const int ko = km + 2 + gf.et;
+  const int ko = km + 2 + grp.et;
   const bool bad = em == kExpNonFinite;
   const int chunk = (K + NN - 1) / NN;
   const int p1 = min(K, (k + 1) * chunk);
@@ -514,15 +541,15 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_ring_inverse_gamma(RingArgs
     longlong2 z[NN];
 #pragma unroll
     for (int j = 0; j < NN; ++j) z[j] = fx_sar(*cl.map_shared_rank(buf + i, j), min(63, km - kj[j]));
-    for (int g = 0; 2 * g <= gf.ng; ++g) {
-      const int g2 = gf.ng - g;  // the conjugate partner (g = 0 and g2 == g have none)
+    for (int g = 0; 2 * g <= grp.ng; ++g) {
+      const int g2 = grp.ng - g;  // the conjugate partner (g = 0 and g2 == g have none)
       const int64_t o = obase + (int64_t)g * gf.npx + p, o2 = obase + (int64_t)g2 * gf.npx + p;
       const bool pair = g > 0 && g2 != g;
       if (REAL) {
         long long A = 0, B = 0;
 #pragma unroll
         for (int j = 0; j < NN; ++j) {
-          const int4 w = gf.tw[g * NN + j];
+          const int4 w = grp.tw[g * NN + j];
           A = fx_mac4(A, z[j].x, w.x, w.y);
           B = fx_mac4(B, z[j].y, w.z, w.w);
         }
@@ -532,7 +559,7 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_ring_inverse_gamma(RingArgs
         longlong2 U = make_longlong2(0, 0), V = make_longlong2(0, 0);
 #pragma unroll
         for (int j = 0; j < NN; ++j) {
-          const int4 w = gf.tw[g * NN + j];
+          const int4 w = grp.tw[g * NN + j];
           U = make_longlong2(fx_mac4(U.x, z[j].x, w.x, w.y), fx_mac4(U.y, z[j].y, w.x, w.y));
           V = make_longlong2(fx_mac4(V.x, z[j].x, w.z, w.w), fx_mac4(V.y, z[j].y, w.z, w.w));
         }
@@ -546,12 +573,14 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_ring_inverse_gamma(RingArgs
 }
 
 template <int NN, bool REAL>
-__global__ void __launch_bounds__(kRingThreads, 3) k_gamma_ring_forward(RingArgs a, const __grid_constant__ GammaFuse gf) {
+__global__ void __launch_bounds__(kRingThreads, 3) k_gamma_ring_forward(const __grid_constant__ GammaFuse grp) {
   extern __shared__ longlong2 buf[];
   __shared__ int s_mx, s_em;
   cg::cluster_group cl = cg::this_cluster();
   const int k = (int)cl.block_rank();
-  const int r = blockIdx.x / NN;
+  const int job = job_of(grp, blockIdx.x / NN), r = blockIdx.x / NN - grp.first[job];
+  const GammaItem &gf = grp.it[job];
+  const RingArgs &a = gf.a;
   const int b = r / gf.nt, t = r - b * gf.nt;
   const int K = a.K, P = a.P, logP = a.logP;
   const int chunk = (K + NN - 1) / NN;
@@ -559,7 +588,7 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_gamma_ring_forward(RingArgs
   const int64_t ibase = (int64_t)b * gf.fms + (int64_t)t * K;
   int em = 0;
   for (int p = p0 + threadIdx.x; p < p1; p += blockDim.x)
-    for (int g = 0; g < gf.ng; ++g) {
+    for (int g = 0; g < grp.ng; ++g) {
       const int64_t o = ibase + (int64_t)g * gf.npx + p;
       if (REAL)
         em = max(em, exp_field(((const double *)gf.fw)[o]));
@@ -578,8 +607,8 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_gamma_ring_forward(RingArgs
     longlong2 acc[NN];
 #pragma unroll
     for (int j = 0; j < NN; ++j) acc[j] = make_longlong2(0, 0);
-    for (int g = 0; 2 * g <= gf.ng; ++g) {
-      const int g2 = gf.ng - g;
+    for (int g = 0; 2 * g <= grp.ng; ++g) {
+      const int g2 = grp.ng - g;
       const bool pair = g > 0 && g2 != g;
       const int64_t o = ibase + (int64_t)g * gf.npx + p, o2 = ibase + (int64_t)g2 * gf.npx + p;
       if (REAL) {
@@ -588,7 +617,7 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_gamma_ring_forward(RingArgs
         const long long Pp = fa + fb, Q = fa - fb;
 #pragma unroll
         for (int j = 0; j < NN; ++j) {
-          const int4 w = gf.tw[g * NN + j];
+          const int4 w = grp.tw[g * NN + j];
           acc[j] = make_longlong2(fx_mac4(acc[j].x, Pp, w.x, w.y), fx_mac4(acc[j].y, Q, w.z, w.w));
         }
       } else {
@@ -597,7 +626,7 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_gamma_ring_forward(RingArgs
         const longlong2 Pp = fx_add(fa, fb), Q = fx_sub(fa, fb);
 #pragma unroll
         for (int j = 0; j < NN; ++j) {
-          const int4 w = gf.tw[g * NN + j];
+          const int4 w = grp.tw[g * NN + j];
           // C P + i S Q
           acc[j] = make_longlong2(fx_mac4(fx_mac4(acc[j].x, Pp.x, w.x, w.y), -Q.y, w.z, w.w),
                                   fx_mac4(fx_mac4(acc[j].y, Pp.y, w.x, w.y), Q.x, w.z, w.w));
@@ -612,7 +641,7 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_gamma_ring_forward(RingArgs
   cl.sync();  // every component's buffer is complete
   const int sh = bluestein(buf, a, &s_mx);
   // split to 61 bits, over 4 in the gamma sums as after a scaled chirp, times 2^et
-  const int k0 = core_exponent(a, e, 61, sh) + gf.et;
+  const int k0 = core_exponent(a, e, 61, sh) + grp.et;
   double2 *out = gf.Gout + (int64_t)b * gf.gms + (int64_t)k * gf.gks + (int64_t)t * gf.W;
   for (int c = threadIdx.x; c < gf.W; c += blockDim.x) {
     const int m = c - (a.bl - 1);
@@ -647,18 +676,32 @@ size_t ring_smem(int P) { return sizeof(longlong2) * (size_t)P; }
 
 // Shared memory of the ring kernels: one P-point buffer of 16-byte values,
 // with a carveout just large enough for the resident buffers (three at P =
-// 4096), so that the rest of the SM's L1 keeps the twiddle table (48 KB there).
+// 4096), so that the rest of the SM's L1 keeps the twiddles.  Set when a
+// kernel's buffer size changes.
 void ring_smem_attrs(const void *kernel, size_t smem) {
+  static std::mutex mu;
+  static std::map<const void *, size_t> set;
+  std::lock_guard<std::mutex> lk(mu);
+  size_t &cur = set[kernel];
+  if (cur == smem) return;
   if (smem > 48 * 1024) S2G_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   constexpr double kMaxSmemPerSm = 228.0 * 1024.0;
   const int pct = std::min(100, (int)std::ceil(100.0 * 3.0 * (double)(smem + 2048) / kMaxSmemPerSm) + 1);
   S2G_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, pct));
+  cur = smem;
+}
+
+int largest_P(const RingGroup &g) {
+  int P = 0;
+  for (int q = 0; q < g.n; ++q) P = std::max(P, g.a[q].P);
+  return P;
 }
 
 template <class KF>
-void launch_ring(KF kernel, const RingArgs &a, int nblk, cudaStream_t st) {
-  ring_smem_attrs((const void *)kernel, ring_smem(a.P));
-  kernel<<<nblk, ring_threads(a.P), ring_smem(a.P), st>>>(a);
+void launch_ring(KF kernel, const RingGroup &g, cudaStream_t st) {
+  const int P = largest_P(g);
+  ring_smem_attrs((const void *)kernel, ring_smem(P));
+  kernel<<<g.first[g.n], ring_threads(P), ring_smem(P), st>>>(g);
   S2G_LAUNCHED();
 }
 
@@ -671,24 +714,47 @@ double ring_work(const RingArgs &a, int nblk) {
   return (double)nblk * 12.0 * (2.0 * passes * 0.75 * P + P + 2.0 * a.K);
 }
 
-void run_ring_forward(const RingArgs &a, int nrings, bool real, cudaStream_t st) {
-  const int nblk = real ? (nrings + 1) / 2 : nrings;
-  KTimer kt(KC_RING, st, timing_enabled() ? ring_work(a, nblk) : 0.0,
-            (double)nrings * a.K * (real ? 8.0 : 16.0) + (double)nrings * a.sw * 16.0);
-  if (real)
-    launch_ring(k_ring_forward<true>, a, nblk, st);
-  else
-    launch_ring(k_ring_forward<false>, a, nblk, st);
-}
-
-void run_ring_inverse(const RingArgs &a, int nrings, bool real, cudaStream_t st) {
-  const int nblk = real ? (nrings + 1) / 2 : nrings;
-  KTimer kt(KC_RING, st, timing_enabled() ? ring_work(a, nblk) : 0.0,
-            (double)nrings * a.K * (real ? 8.0 : 16.0) + (double)nrings * a.sw * 16.0);
-  if (real)
-    launch_ring(k_ring_inverse<true>, a, nblk, st);
-  else
-    launch_ring(k_ring_inverse<false>, a, nblk, st);
+// launches of up to kMaxJobs jobs
+template <class LAUNCH>
+void run_rings(const std::vector<RingJob> &jobs, int ss, bool real, bool forward, LAUNCH &&launch, cudaStream_t st) {
+  RingGroup g;
+  double fl = 0, by = 0;
+  g.n = 0;
+  g.first[0] = 0;
+  const auto flush = [&] {
+    if (!g.n) return;
+    KTimer kt(KC_RING, st, fl, by);
+    launch(g);
+    g.n = 0;
+    fl = by = 0;
+  };
+  for (const RingJob &j : jobs) {
+    if (j.nrings <= 0) continue;
+    RingArgs a = ring_args(ring_fft(grid_ring_len(j.bl, ss)), j.bl, j.nrings);
+    a.ring_stride = j.ring_stride;
+    a.map_stride = j.map_stride;
+    a.rpm = j.rpm;
+    a.spec_stride = j.spec_stride;
+    a.spec_map_stride = j.spec_map_stride;
+    a.spec_rpm = j.spec_rpm;
+    a.herm = j.herm ? 1 : 0;
+    a.sw = j.sw;
+    a.mlo = j.mlo;
+    if (forward) {
+      a.rings = j.in;
+      a.spec_out = (double2 *)j.out;
+    } else {
+      a.spec_in = (const double2 *)j.in;
+      a.rings_out = (double2 *)j.out;
+    }
+    const int nblk = real ? (j.nrings + 1) / 2 : j.nrings;
+    if (timing_enabled()) fl += ring_work(a, nblk);
+    by += (double)j.nrings * a.K * (real ? 8.0 : 16.0) + (double)j.nrings * a.sw * 16.0;
+    g.a[g.n] = a;
+    g.first[g.n + 1] = g.first[g.n] + nblk;
+    if (++g.n == kMaxJobs) flush();
+  }
+  flush();
 }
 
 // Twiddles of the fused gamma DFT: synthesis c e^{i n_k gamma_g} (x2 for
@@ -726,11 +792,13 @@ cudaLaunchConfig_t fused_config(int nctas, int nn, int P, cudaLaunchAttribute *a
 }
 
 template <class KF>
-void launch_fused(KF kernel, const RingArgs &a, const GammaFuse &gf, int nrings, int nn, cudaStream_t st) {
-  ring_smem_attrs((const void *)kernel, ring_smem(a.P));
+void launch_fused(KF kernel, const GammaFuse &gf, int nn, cudaStream_t st) {
+  int P = 0;
+  for (int q = 0; q < gf.n; ++q) P = std::max(P, gf.it[q].a.P);
+  ring_smem_attrs((const void *)kernel, ring_smem(P));
   cudaLaunchAttribute at[1];
-  const cudaLaunchConfig_t cfg = fused_config(nrings * nn, nn, a.P, at, st);
-  S2G_CUDA(cudaLaunchKernelEx(&cfg, kernel, a, gf));
+  const cudaLaunchConfig_t cfg = fused_config(gf.first[gf.n] * nn, nn, P, at, st);
+  S2G_CUDA(cudaLaunchKernelEx(&cfg, kernel, gf));
   S2G_LAUNCHED();
 }
 
@@ -775,151 +843,108 @@ bool ring_gamma_fusable(int nn, int ng, int bl, int ss) {
 }
 
 namespace {
-// the parts of a fused launch that both directions share
-GammaFuse gamma_fuse(const RingArgs &a, int64_t gms, int64_t gks, const std::vector<int> &ns, int ng, bool real,
-                     double c, void *fw, int64_t fms, int nt, bool synth) {
-  GammaFuse gf{};
-  gf.gms = gms;
-  gf.gks = gks;
-  gf.W = 2 * a.bl - 1;
-  gf.nt = nt;
-  gf.herm_k = -1;
-  gf.fw = fw;
-  gf.fms = fms;
-  gf.npx = (int64_t)nt * a.K;
-  gf.ng = ng;
-  gf.real = real ? 1 : 0;
-  fuse_twiddles(gf, ns, ng, real, c, synth);
-  return gf;
-}
 // multiply-adds of the gamma products: 3 per real product, (ng + 1)/2 slice pairs
 double gamma_work(double px, int ng, int nn, bool real) { return px * ((ng + 1) / 2) * nn * (real ? 6.0 : 12.0); }
+
+// launches of up to kMaxJobs jobs of one direction
+template <class LAUNCH>
+void run_fused(const std::vector<GammaJob> &jobs, const std::vector<int> &ns, int ng, bool real, double c, int ss,
+               bool synth, LAUNCH &&launch, cudaStream_t st) {
+  const int nn = (int)ns.size();
+  GammaFuse g;
+  double fl = 0, by = 0;
+  g.n = 0;
+  g.first[0] = 0;
+  g.ng = ng;
+  g.herm_k = -1;
+  for (int k = 0; k < nn; ++k)
+    if (synth && real && ns[k] == 0) g.herm_k = k;
+  const auto flush = [&] {
+    if (!g.n) return;
+    KTimer kt(KC_RING, st, fl, by);
+    launch(g);
+    g.n = 0;
+    fl = by = 0;
+  };
+  bool tw = false;
+  for (const GammaJob &j : jobs) {
+    S2G_REQUIRE(ring_gamma_fusable(nn, ng, j.bl, ss), ERR_UNSUPPORTED, "fused ring/gamma DFT: unsupported shape");
+    const int nt = grid_rings(j.bl, ss), nrings = j.nb * nt;
+    if (nrings <= 0) continue;
+    if (!tw) fuse_twiddles(g, ns, ng, real, c, synth);
+    tw = true;
+    GammaItem &it = g.it[g.n];
+    it.a = ring_args(ring_fft(grid_ring_len(j.bl, ss)), j.bl, nrings);
+    it.G = j.G;
+    it.Gout = j.Gout;
+    it.gms = j.gms;
+    it.gks = j.gks;
+    it.W = 2 * j.bl - 1;
+    it.nt = nt;
+    it.fw = j.fw;
+    it.fms = j.fms;
+    it.npx = (int64_t)nt * it.a.K;
+    const double px = (double)nrings * it.a.K;
+    if (timing_enabled()) fl += ring_work(it.a, nrings * nn) + gamma_work(px, ng, nn, real);
+    by += (double)nrings * nn * it.W * 16.0 + px * ng * (real ? 8.0 : 16.0);
+    g.first[g.n + 1] = g.first[g.n] + nrings;
+    if (++g.n == kMaxJobs) flush();
+  }
+  flush();
+}
 }  // namespace
 
-void ring_inverse_gamma(const double2 *G, int64_t gms, int64_t gks, const std::vector<int> &ns, int ng, bool real,
-                        double c, void *fw, int64_t fms, int nb, int bl, int ss, cudaStream_t st) {
-  const int nn = (int)ns.size();
-  S2G_REQUIRE(ring_gamma_fusable(nn, ng, bl, ss), ERR_UNSUPPORTED, "fused ring/gamma DFT: unsupported shape");
-  const int nt = grid_rings(bl, ss), nrings = nb * nt;
-  if (nrings <= 0) return;
-  const RingArgs a = ring_args(ring_fft(grid_ring_len(bl, ss)), bl, nrings);
-  GammaFuse gf = gamma_fuse(a, gms, gks, ns, ng, real, c, fw, fms, nt, true);
-  gf.G = G;
-  for (int k = 0; k < nn; ++k)
-    if (real && ns[k] == 0) gf.herm_k = k;
-  const double px = (double)nrings * a.K;
-  KTimer kt(KC_RING, st, timing_enabled() ? ring_work(a, nrings * nn) + gamma_work(px, ng, nn, real) : 0.0,
-            (double)nrings * nn * gf.W * 16.0 + px * ng * (real ? 8.0 : 16.0));
-  switch (nn) {
-#define S2G_FUSE(N)                                                          \
-  case N:                                                                    \
-    if (real)                                                                \
-      launch_fused(k_ring_inverse_gamma<N, true>, a, gf, nrings, N, st);    \
-    else                                                                     \
-      launch_fused(k_ring_inverse_gamma<N, false>, a, gf, nrings, N, st);   \
+void ring_inverse_gamma(const std::vector<GammaJob> &jobs, const std::vector<int> &ns, int ng, bool real, double c,
+                        int ss, cudaStream_t st) {
+  run_fused(jobs, ns, ng, real, c, ss, true, [&](const GammaFuse &gf) {
+    switch ((int)ns.size()) {
+#define S2G_FUSE(N)                                               \
+  case N:                                                         \
+    if (real)                                                     \
+      launch_fused(k_ring_inverse_gamma<N, true>, gf, N, st);    \
+    else                                                          \
+      launch_fused(k_ring_inverse_gamma<N, false>, gf, N, st);   \
     break;
-    S2G_FUSE(2) S2G_FUSE(3) S2G_FUSE(4) S2G_FUSE(5) S2G_FUSE(6) S2G_FUSE(7) S2G_FUSE(8)
+      S2G_FUSE(2) S2G_FUSE(3) S2G_FUSE(4) S2G_FUSE(5) S2G_FUSE(6) S2G_FUSE(7) S2G_FUSE(8)
 #undef S2G_FUSE
-    default: break;
-  }
+      default: break;
+    }
+  }, st);
 }
 
-void gamma_ring_forward(const void *fw, int64_t fms, const std::vector<int> &ns, int ng, bool real, double c,
-                        double2 *Gout, int64_t gms, int64_t gks, int nb, int bl, int ss, cudaStream_t st) {
-  const int nn = (int)ns.size();
-  S2G_REQUIRE(ring_gamma_fusable(nn, ng, bl, ss), ERR_UNSUPPORTED, "fused ring/gamma DFT: unsupported shape");
-  const int nt = grid_rings(bl, ss), nrings = nb * nt;
-  if (nrings <= 0) return;
-  const RingArgs a = ring_args(ring_fft(grid_ring_len(bl, ss)), bl, nrings);
-  GammaFuse gf = gamma_fuse(a, gms, gks, ns, ng, real, c, const_cast<void *>(fw), fms, nt, false);
-  gf.Gout = Gout;
-  const double px = (double)nrings * a.K;
-  KTimer kt(KC_RING, st, timing_enabled() ? ring_work(a, nrings * nn) + gamma_work(px, ng, nn, real) : 0.0,
-            (double)nrings * nn * gf.W * 16.0 + px * ng * (real ? 8.0 : 16.0));
-  switch (nn) {
-#define S2G_FUSE(N)                                                          \
-  case N:                                                                    \
-    if (real)                                                                \
-      launch_fused(k_gamma_ring_forward<N, true>, a, gf, nrings, N, st);    \
-    else                                                                     \
-      launch_fused(k_gamma_ring_forward<N, false>, a, gf, nrings, N, st);   \
+void gamma_ring_forward(const std::vector<GammaJob> &jobs, const std::vector<int> &ns, int ng, bool real, double c,
+                        int ss, cudaStream_t st) {
+  run_fused(jobs, ns, ng, real, c, ss, false, [&](const GammaFuse &gf) {
+    switch ((int)ns.size()) {
+#define S2G_FUSE(N)                                               \
+  case N:                                                         \
+    if (real)                                                     \
+      launch_fused(k_gamma_ring_forward<N, true>, gf, N, st);    \
+    else                                                          \
+      launch_fused(k_gamma_ring_forward<N, false>, gf, N, st);   \
     break;
-    S2G_FUSE(2) S2G_FUSE(3) S2G_FUSE(4) S2G_FUSE(5) S2G_FUSE(6) S2G_FUSE(7) S2G_FUSE(8)
+      S2G_FUSE(2) S2G_FUSE(3) S2G_FUSE(4) S2G_FUSE(5) S2G_FUSE(6) S2G_FUSE(7) S2G_FUSE(8)
 #undef S2G_FUSE
-    default: break;
-  }
+      default: break;
+    }
+  }, st);
 }
 
-void ring_forward(const void *rings, int64_t ring_stride, int64_t map_stride, int rpm, double2 *spec,
-                  int64_t spec_stride, int sw, int mlo, int nrings, int bl, int ss, bool real, cudaStream_t st) {
-  if (nrings <= 0) return;
-  const RingFFT &rf = ring_fft(grid_ring_len(bl, ss));
-  RingArgs a = ring_args(rf, bl, nrings);
-  a.rings = rings;
-  a.ring_stride = ring_stride;
-  a.map_stride = map_stride;
-  a.rpm = rpm;
-  a.spec_out = spec;
-  a.spec_stride = spec_stride;
-  a.sw = sw;
-  a.mlo = mlo;
-  run_ring_forward(a, nrings, real, st);
+void ring_forward_many(const std::vector<RingJob> &jobs, int ss, bool real, cudaStream_t st) {
+  run_rings(jobs, ss, real, true, [&](const RingGroup &g) {
+    if (real)
+      launch_ring(k_ring_forward<true>, g, st);
+    else
+      launch_ring(k_ring_forward<false>, g, st);
+  }, st);
 }
-
-void ring_inverse(const double2 *spec, int64_t spec_stride, int sw, int mlo, void *rings,
-                  int64_t ring_stride, int64_t map_stride, int rpm, int nrings, int bl, int ss, bool real,
-                  cudaStream_t st) {
-  if (nrings <= 0) return;
-  const RingFFT &rf = ring_fft(grid_ring_len(bl, ss));
-  RingArgs a = ring_args(rf, bl, nrings);
-  a.spec_in = spec;
-  a.spec_stride = spec_stride;
-  a.sw = sw;
-  a.mlo = mlo;
-  a.rings_out = (double2 *)rings;
-  a.ring_stride = ring_stride;
-  a.map_stride = map_stride;
-  a.rpm = rpm;
-  run_ring_inverse(a, nrings, real, st);
-}
-
-void ring_forward_c(const double2 *rings, int64_t ring_stride, int64_t map_stride, int rpm, double2 *spec,
-                    int64_t spec_stride, int64_t spec_map_stride, int spec_rpm, int sw, int mlo, int nrings, int bl,
-                    int ss, cudaStream_t st) {
-  if (nrings <= 0) return;
-  const RingFFT &rf = ring_fft(grid_ring_len(bl, ss));
-  RingArgs a = ring_args(rf, bl, nrings);
-  a.rings = rings;
-  a.ring_stride = ring_stride;
-  a.map_stride = map_stride;
-  a.rpm = rpm;
-  a.spec_out = spec;
-  a.spec_stride = spec_stride;
-  a.spec_map_stride = spec_map_stride;
-  a.spec_rpm = spec_rpm;
-  a.sw = sw;
-  a.mlo = mlo;
-  run_ring_forward(a, nrings, false, st);
-}
-
-void ring_inverse_c(const double2 *spec, int64_t spec_stride, int64_t spec_map_stride, int spec_rpm, int sw,
-                    int mlo, bool herm, double2 *rings, int64_t ring_stride, int64_t map_stride, int rpm, int nrings,
-                    int bl, int ss, cudaStream_t st) {
-  if (nrings <= 0) return;
-  const RingFFT &rf = ring_fft(grid_ring_len(bl, ss));
-  RingArgs a = ring_args(rf, bl, nrings);
-  a.spec_in = spec;
-  a.spec_stride = spec_stride;
-  a.spec_map_stride = spec_map_stride;
-  a.spec_rpm = spec_rpm;
-  a.herm = herm ? 1 : 0;
-  a.sw = sw;
-  a.mlo = mlo;
-  a.rings_out = rings;
-  a.ring_stride = ring_stride;
-  a.map_stride = map_stride;
-  a.rpm = rpm;
-  run_ring_inverse(a, nrings, false, st);
+void ring_inverse_many(const std::vector<RingJob> &jobs, int ss, bool real, cudaStream_t st) {
+  run_rings(jobs, ss, real, false, [&](const RingGroup &g) {
+    if (real)
+      launch_ring(k_ring_inverse<true>, g, st);
+    else
+      launch_ring(k_ring_inverse<false>, g, st);
+  }, st);
 }
 
 }  // namespace s2g
