@@ -457,10 +457,12 @@ int s2let_gpu_get_df_max_maps(void);
  *       the free device memory (S2LET_GPU_TABLE_BUDGET_GB overrides), else the
  *       largest band-limits recomputed;
  *   1 = stored tables always;
- *   2 = recomputed always: the kernels regenerate the Wigner d values from
- *       double-double checkpoints every 64 degrees (≈ 1/50 of the memory) and
- *       apply the forward quadrature as a separate operator (FP64, or
- *       double-float at split precision).
+ *   2 = recomputed at L and at every scale from band-limit 64 (smaller scales'
+ *       tables take a few MB and are shared by all plans): the kernels
+ *       regenerate the Wigner d values from double-double checkpoints every 64
+ *       degrees (≈ 1/50 of the memory) and apply the forward quadrature as a
+ *       separate operator (on the tensor cores in eight digit slices, or in
+ *       double-float at split precision up to band-limit 512).
  * Returns the status. */
 int s2let_gpu_set_table_mode(int mode);
 int s2let_gpu_get_table_mode(void);

@@ -27,13 +27,6 @@ __device__ __forceinline__ float2 df_add(float2 a, float2 b) {
   return s;
 }
 __device__ __forceinline__ float2 df_neg(float2 a) { return make_float2(-a.x, -a.y); }
-// a + b renormalised (fast two-sum of the result: |lo| <= ulp(hi) / 2), for
-// accumulators summing many terms, where the unnormalised lo would grow
-__device__ __forceinline__ float2 df_add_norm(float2 a, float2 b) {
-  const float2 s = df_add(a, b);
-  const float h = __fadd_rn(s.x, s.y);
-  return make_float2(h, __fsub_rn(s.y, __fsub_rn(h, s.x)));
-}
 // a*b + c*d (double-float in, double-float out)
 __device__ __forceinline__ float2 df_dot2(float2 a, float2 b, float2 c, float2 d) {
   const float p1 = __fmul_rn(a.x, b.x);
@@ -85,10 +78,25 @@ __device__ __forceinline__ float2 df_mul(float2 a, float2 b) {
   return make_float2(p, e);
 }
 
-// s += v x (double-float real times complex), the accumulator renormalised
-// after each add (for sums of many terms)
-__device__ __forceinline__ void df_mac(float4 &s, float2 v, float4 x) {
-  s = dmk(df_add_norm(dre(s), df_mul(v, dre(x))), df_add_norm(dim_(s), df_mul(v, dim_(x))));
+// Dot2 step (Ogita, Rump and Oishi, SIAM J. Sci. Comput. 26, 2005): (s, c) += a x,
+// a and x double-float reals, s carried by TwoSum, its rounding errors and the
+// products' low parts gathered in c; s + c is the sum as if computed in twice the
+// working precision
+__device__ __forceinline__ void dot2_mac(float &s, float &c, float2 av, float xh, float xl) {
+  const float p = __fmul_rn(av.x, xh);
+  const float q = __fmaf_rn(av.x, xh, -p);
+  const float t = __fadd_rn(s, p);
+  const float v = __fsub_rn(t, s);
+  const float r = __fadd_rn(__fsub_rn(s, __fsub_rn(t, v)), __fsub_rn(p, v));
+  s = t;
+  c = __fadd_rn(c, __fadd_rn(q, r));
+  c = __fmaf_rn(av.x, xl, c);
+  c = __fmaf_rn(av.y, xh, c);
+}
+// complex sums (re.s, re.c, im.s, im.c) += v x
+__device__ __forceinline__ void dot2_cmac(float4 &s, float2 v, float4 x) {
+  dot2_mac(s.x, s.y, v, x.x, x.y);
+  dot2_mac(s.z, s.w, v, x.z, x.w);
 }
 
 }  // namespace

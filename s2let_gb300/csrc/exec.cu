@@ -119,6 +119,11 @@ struct PlanSpec {
   bool merge_conj = false;        // merge multiplies by conj(psi) (else psi)
 };
 
+// Scales up to this band-limit keep stored tables beside a recomputed larger one
+// (4 MB per direction at 63, shared by every parameter set, against 2 to 100 us of
+// recomputation a scale): their contractions then share launches.
+constexpr int kStoredMaxBl = 63;
+
 std::unique_ptr<WavPlan> build_plan(const PlanSpec &ps) {
   auto P = std::make_unique<WavPlan>();
   P->L = ps.L;
@@ -231,7 +236,8 @@ std::unique_ptr<WavPlan> build_plan(const PlanSpec &ps) {
         total += b;
       }
     if (t_table_mode == 2) {
-      for (auto &kv : need) P->rc_bl.push_back(kv.first);
+      for (auto &kv : need)
+        if (kv.first > kStoredMaxBl || kv.first == L) P->rc_bl.push_back(kv.first);
     } else if (t_table_mode == 0) {
       const int64_t budget = table_budget_bytes();
       for (auto it = need.rbegin(); it != need.rend() && total > budget; ++it) {
@@ -571,6 +577,23 @@ std::vector<std::pair<size_t, size_t>> table_passes(const WavPlan &P, bool large
   return passes;
 }
 
+// Directions (indices into ns) whose contractions go together: each by itself on
+// a stored table, n and -n on a recomputed one (they share its rows).
+std::vector<std::vector<int>> table_directions(const WavPlan &P, const Scale &sd) {
+  std::vector<std::vector<int>> out;
+  for (int i = 0; i < (int)sd.ns.size(); ++i) {
+    std::vector<int> *with = nullptr;
+    if (P.rc(sd.bl))
+      for (auto &d : out)
+        if (std::abs(sd.ns[d[0]]) == std::abs(sd.ns[i])) with = &d;
+    if (with)
+      with->push_back(i);
+    else
+      out.push_back({i});
+  }
+  return out;
+}
+
 // The scales whose contractions are small (contract_is_small) run together:
 // one launch for the contractions of all of them, one for their ring DFTs.
 bool small_scale(const WavPlan &P, const Scale &sd, int nb) {
@@ -790,10 +813,11 @@ void wav_split(const WavPlan &P, SplitMode mode, const double2 *flm, bool flm_ha
     if (small_scale(P, s0, nb)) continue;
     const int ngrp = (int)(pk.second - pk.first);
     const int64_t gsz = gsize(s0);
-    for (size_t i = 0; i < s0.ns.size(); ++i) {
-      L2T grp[kMaxParts];
-      for (int q = 0; q < ngrp; ++q) grp[q] = problem(P.sc[pk.first + q], (int)i, Gbuf + q * gsz);
-      contract_l2t_group(grp, ngrp, S.st);
+    for (const auto &dirs : table_directions(P, s0)) {
+      std::vector<L2T> grp;
+      for (int i : dirs)
+        for (int q = 0; q < ngrp; ++q) grp.push_back(problem(P.sc[pk.first + q], i, Gbuf + q * gsz));
+      contract_l2t_group(grp.data(), (int)grp.size(), S.st);
     }
     for (int q = 0; q < ngrp; ++q) to_pixels(P.sc[pk.first + q], Gbuf + q * gsz, !pipe);
     if (!pipe) rings.inverse(P.ss, real, S.st);
@@ -952,10 +976,11 @@ void wav_merge(const WavPlan &P, MergeMode mode, const void *f_wav, int64_t wstr
     const int64_t gsz = gsize(s0);
     for (int q = 0; q < ngrp; ++q) to_spectra(P.sc[pk.first + q], Gbuf + q * gsz, !pipe);
     if (!pipe) rings.forward(P.ss, real, S.st);
-    for (size_t i = 0; i < s0.ns.size(); ++i) {
-      T2L grp[kMaxParts];
-      for (int q = 0; q < ngrp; ++q) grp[q] = problem(P.sc[pk.first + q], (int)i, Gbuf + q * gsz);
-      contract_t2l_group(grp, ngrp, S.st);
+    for (const auto &dirs : table_directions(P, s0)) {
+      std::vector<T2L> grp;
+      for (int i : dirs)
+        for (int q = 0; q < ngrp; ++q) grp.push_back(problem(P.sc[pk.first + q], i, Gbuf + q * gsz));
+      contract_t2l_group(grp.data(), (int)grp.size(), S.st);
     }
   }
   if (pipe) {

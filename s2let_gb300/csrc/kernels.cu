@@ -275,18 +275,6 @@ __device__ __forceinline__ float2 df_split_unit(double v) {
 __device__ __forceinline__ float2 unit_df(double v) { return df_split_unit(v); }
 __device__ __forceinline__ float2 unit_df(float2 v) { return v; }
 
-// Dot2 step: (s, c) += a * x, a and x double-float reals
-__device__ __forceinline__ void dot2_mac(float &s, float &c, float2 av, float xh, float xl) {
-  const float p = __fmul_rn(av.x, xh);
-  const float q = __fmaf_rn(av.x, xh, -p);
-  const float t = __fadd_rn(s, p);
-  const float v = __fsub_rn(t, s);
-  const float r = __fadd_rn(__fsub_rn(s, __fsub_rn(t, v)), __fsub_rn(p, v));
-  s = t;
-  c = __fadd_rn(c, __fadd_rn(q, r));
-  c = __fmaf_rn(av.x, xl, c);
-  c = __fmaf_rn(av.y, xh, c);
-}
 // (s, c) += (s2, c2), symmetric in its two operands: TwoSum's error r is
 // exact and c + c2 commutes, so both lanes of a butterfly step get the same
 // bits (the lane that stores a sum then does not matter)
@@ -1229,8 +1217,8 @@ bool df_pair(const A &p, const A &q, cudaStream_t st) {
   }
   return true;
 }
-void contract_rc(const L2T &p, cudaStream_t st) { contract_l2t_rc(p, st); }
-void contract_rc(const T2L &p, cudaStream_t st) { contract_t2l_rc(p, st); }
+void contract_rc(const L2T *p, int n, cudaStream_t st) { contract_l2t_rc(p, n, st); }
+void contract_rc(const T2L *p, int n, cudaStream_t st) { contract_t2l_rc(p, n, st); }
 bool contract_tensor(const L2T *p, int n, cudaStream_t st) { return contract_l2t_mixed(p, n, st); }
 bool contract_tensor(const T2L *p, int n, cudaStream_t st) { return contract_t2l_mixed(p, n, st); }
 
@@ -1238,7 +1226,7 @@ template <class A>
 void contract_one(const A &p, cudaStream_t st) {
   if (p.nb <= 0 || p.mhi < p.mlo) return;
   if (p.tb->rc) {
-    contract_rc(p, st);
+    contract_rc(&p, 1, st);
     return;
   }
   if (on_tensor_cores(p.nb) && contract_tensor(&p, 1, st)) return;
@@ -1247,8 +1235,12 @@ void contract_one(const A &p, cudaStream_t st) {
 template <class A>
 void contract_group(const A *a, int n, cudaStream_t st) {
   if (n <= 0) return;
-  if (!a[0].tb->rc && on_tensor_cores(a[0].nb) && contract_tensor(a, n, st)) return;
-  const bool pairs = t_precision == 1 && !a[0].tb->rc && !on_tensor_cores(a[0].nb);
+  if (a[0].tb->rc) {
+    contract_rc(a, n, st);
+    return;
+  }
+  if (on_tensor_cores(a[0].nb) && contract_tensor(a, n, st)) return;
+  const bool pairs = t_precision == 1 && !on_tensor_cores(a[0].nb);
   for (int i = 0; i < n; ++i) {
     if (pairs && i + 1 < n && df_pair(a[i], a[i + 1], st))
       ++i;
@@ -1267,8 +1259,12 @@ void contract_many(const std::vector<A> &v, cudaStream_t st) {
     if (g.n) launch_batch(*p0, g, rows, st);
     g.n = rows = 0;
   };
+  std::vector<A> rc;
+  for (const A &p : v)
+    if (p.tb->rc) rc.push_back(p);
+  contract_rc(rc.data(), (int)rc.size(), st);
   for (const A &p : v) {
-    if (p.nb <= 0 || p.mhi < p.mlo) continue;
+    if (p.nb <= 0 || p.mhi < p.mlo || p.tb->rc) continue;
     if (!contract_is_small(p.tb, p.nb)) {
       contract_one(p, st);
       continue;

@@ -80,9 +80,10 @@ void set_df_max_maps(int maps);
 int get_df_max_maps();
 
 void contract_l2t(const L2T &a, cudaStream_t st);
-// n <= kMaxParts problems on the same table (same band-limit, n, m range and
-// batch): one table pass on the tensor cores, or in double-float two at a time,
-// else one call each.
+// n problems on the same table, n <= kMaxParts of one direction (same band-limit,
+// n, m range and batch) on a stored table: one table pass on the tensor cores, or
+// in double-float two at a time, else one call each; any directions n and -n on a
+// recomputed one.
 constexpr int kMaxParts = 8;
 void contract_l2t_group(const L2T *a, int n, cudaStream_t st);
 

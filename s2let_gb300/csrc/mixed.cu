@@ -115,18 +115,25 @@ struct Cfg {
   static_assert(kNBuf * kAccCols <= kTmemCols, "TMEM");
 };
 
+// What a launch computes.
+enum MxMode {
+  MX_L2T = 0,   // sums over l: rows t, K = l
+  MX_T2L = 1,   // sums over theta: rows l, K = t
+  MX_QUAD = 2,  // the quadrature operator on ring spectra: rows t, K = t', one block per parity of m + n
+};
+
 struct Geom {
   int l0, nl, rows, K, nkc, nrt;
 };
 // Tile geometry of one m block of a table with nt theta samples: l -> t has
 // rows t < nt and reduction K = l - l0; t -> l has rows l - l0 and K = t.
-__host__ __device__ inline Geom geom(int bl, int nt, int an, int m, bool q) {
+__host__ __device__ inline Geom geom(int bl, int nt, int an, int m, int mode) {
   Geom g;
   const int am = m < 0 ? -m : m;
-  g.l0 = am > an ? am : an;
+  g.l0 = mode == MX_QUAD ? 0 : (am > an ? am : an);
   g.nl = bl - g.l0 > 0 ? bl - g.l0 : 0;
-  g.rows = q ? g.nl : nt;
-  g.K = q ? nt : g.nl;
+  g.rows = mode == MX_T2L ? g.nl : nt;
+  g.K = mode == MX_L2T ? g.nl : nt;
   g.nkc = g.nl > 0 ? (g.K + kPK - 1) / kPK : 0;
   g.nrt = (g.rows + kPM - 1) / kPM;  // l -> t keeps its rows (written as zeros) when nl = 0
   return g;
@@ -226,18 +233,17 @@ __device__ __forceinline__ TableRefM table_ref_m(int tmlo, int n, int m) {
 // table slicing (plan time)
 // ---------------------------------------------------------------------------
 
-// rows l when q (t -> l) else t; tr: the source block holds the transpose
-// (row k, column row).  panels8 (nullable with panels set, or the reverse):
+// mode: MxMode; tr: the source block holds the transpose (row k, column row).  panels8 (nullable with panels set, or the reverse):
 // the eighth digit's blocks, one per (row tile, K-chunk).
 __global__ void __launch_bounds__(128) k_slice_table(const double *__restrict__ T,
                                                      const int64_t *__restrict__ off, int bl, int nt,
-                                                     int an, int tmlo, int q, int tr, uint8_t *__restrict__ panels,
+                                                     int an, int tmlo, int mode, int tr, uint8_t *__restrict__ panels,
                                                      uint8_t *__restrict__ panels8,
                                                      const int64_t *__restrict__ pan_off,
                                                      int8_t *__restrict__ eA,
                                                      const int64_t *__restrict__ e_off) {
   const int mi = blockIdx.x, rt = blockIdx.y;
-  const Geom g = geom(bl, nt, an, tmlo + mi, q != 0);
+  const Geom g = geom(bl, nt, an, tmlo + mi, mode);
   if (rt >= g.nrt) return;
   const double *Tm = T + off[mi];
   const int64_t rs = tr ? 1 : g.K, ks = tr ? g.rows : 1;  // strides of the row and of k
@@ -296,7 +302,7 @@ struct Part {
 };
 
 struct XArgs {
-  int q;  // 0: l -> t (K = l - l0), 1: t -> l (K = t)
+  int mode;  // MxMode
   int bl, nt, an, mlo, lmin;  // lmin: smallest lmin over the parts
   int nparts;
   Part part[kMaxParts];
@@ -358,10 +364,10 @@ __global__ void __launch_bounds__(kSliceThreads, 3) k_slice_x(XArgs a) {
     const int pm = pm0 + threadIdx.x;
     int l0 = 0, nkc = 0, kc0 = 0, ls = 0;
     if (pm < a.nmp) {
-      const Geom g = geom(a.bl, a.nt, a.an, a.mlo + pm, a.q != 0);
+      const Geom g = geom(a.bl, a.nt, a.an, a.mlo + pm, a.mode);
       l0 = g.l0;
       nkc = g.nkc;
-      if (!a.q) {
+      if (a.mode == MX_L2T) {
         const int lst = g.l0 > a.lmin ? g.l0 : a.lmin;
         kc0 = lst >= a.bl ? g.nkc : (lst - g.l0) / kPK;
         // first degree with a value: below its part's lmin the column is zero
@@ -384,7 +390,7 @@ __global__ void __launch_bounds__(kSliceThreads, 3) k_slice_x(XArgs a) {
     double2 *col = sv + mi * a.kst;
     int er = 0, ei = 0;
     constexpr int kStep = kSliceThreads / kMG, kU = 4;  // kU loads in flight per thread
-    if (!a.q) {
+    if (a.mode == MX_L2T) {
       // every lane walks the same degrees, so the kMG m of one degree are adjacent
       int lb = a.bl;
       for (int i = 0; i < kMG; ++i)
@@ -611,7 +617,7 @@ __device__ __forceinline__ uint4 digits_bf16(uint32_t lo, uint32_t hi) {
 }
 
 struct MxArgs {
-  int q;  // 0: l -> t with D, 1: t -> l with Q
+  int mode;  // MxMode
   const uint8_t *panels, *panels8;
   const int64_t *pan_off;
   const int8_t *eA;
@@ -650,15 +656,20 @@ __device__ __forceinline__ TileInfo tile_info(const MxArgs &a, int v, int2 tl) {
   ti.pm = tl.x;
   ti.rt = tl.y;
   ti.m = a.mlo + ti.pm;
-  const TableRefM r = table_ref_m(a.tmlo, a.n, ti.m);
-  ti.mi = r.mi;
-  ti.sign = r.sign;
-  const Geom g = geom(a.bl, a.nt, a.an, ti.m, a.q != 0);
+  if (a.mode == MX_QUAD) {
+    ti.mi = (ti.m + a.an) & 1;
+    ti.sign = 1.0;
+  } else {
+    const TableRefM r = table_ref_m(a.tmlo, a.n, ti.m);
+    ti.mi = r.mi;
+    ti.sign = r.sign;
+  }
+  const Geom g = geom(a.bl, a.nt, a.an, ti.m, a.mode);
   ti.l0 = g.l0;
   ti.nkc = g.nkc;
   const int lst = g.l0 > a.lmin ? g.l0 : a.lmin;
   ti.kc0 = 0;
-  if (!a.q) ti.kc0 = lst >= a.bl ? g.nkc : (lst - g.l0) / kPK;
+  if (a.mode == MX_L2T) ti.kc0 = lst >= a.bl ? g.nkc : (lst - g.l0) / kPK;
   return ti;
 }
 
@@ -1005,7 +1016,7 @@ __global__ void __launch_bounds__(Cfg<NC, S>::kThreads, 1) k_contract_mx(MxArgs 
           const int b = a.b0 + ti.g * a.mpp + cp % a.mpp;
           if (part >= a.nparts || b >= a.nb) continue;
           const Part &P = a.part[part];
-          if (!a.q) {
+          if (a.mode != MX_T2L) {
             if (t_row < a.nt)
               P.dst[(int64_t)b * P.ds + (int64_t)t_row * P.dw + (ti.m - P.d_mlo)] =
                   make_double2(y[2 * bb], y[2 * bb + 1]);
@@ -1054,14 +1065,19 @@ struct TileList {
 
 // Which table a contraction reads, and how: rows of the panels are t (l -> t)
 // or l (t -> l), from D[t][l] or Q[l][t]; two of the four read it transposed.
-enum TableKind { TK_L2T_D = 0, TK_T2L_Q = 1, TK_L2T_Q = 2, TK_T2L_D = 3 };
-bool kind_rows_l(int kind) { return kind == TK_T2L_Q || kind == TK_T2L_D; }
+// TK_W and TK_WT: the quadrature operators W_+ and W_- of a recomputed table's
+// grid, and their transposes.
+enum TableKind { TK_L2T_D = 0, TK_T2L_Q = 1, TK_L2T_Q = 2, TK_T2L_D = 3, TK_W = 4, TK_WT = 5 };
+MxMode kind_mode(int kind) {
+  if (kind >= TK_W) return MX_QUAD;
+  return kind == TK_T2L_Q || kind == TK_T2L_D ? MX_T2L : MX_L2T;
+}
 bool kind_of_q(int kind) { return kind == TK_T2L_Q || kind == TK_L2T_Q; }
-bool kind_transposed(int kind) { return kind == TK_L2T_Q || kind == TK_T2L_D; }
+bool kind_transposed(int kind) { return kind == TK_L2T_Q || kind == TK_T2L_D || kind == TK_WT; }
 
 struct SlicedTable {
   int bl = 0, nt = 0, an = 0, mlo = 0, nm = 0;
-  bool q = false;    // rows l
+  int mode = MX_L2T;
   uint8_t *panels = nullptr;   // 7 digit slices
   uint8_t *panels8 = nullptr;  // the eighth, built when an FP64 contraction first needs it
   int8_t *eA = nullptr;
@@ -1110,15 +1126,19 @@ bool capturing(cudaStream_t st) {
 // meets a table that no earlier call has built.  A refusal stands until the
 // plans are released, so that a program's route does not change under it.
 SlicedTable *sliced(const WignerTable &tb, int kind, bool eighth, cudaStream_t st) {
-  const TableKey key = std::make_tuple(tb.bl, tb.an, tb.ss, kind);
+  const int mode = kind_mode(kind);
+  // the quadrature operators belong to the grid: one block per parity
+  const bool quad = mode == MX_QUAD;
+  const int nm = quad ? 2 : tb.nm, tmlo = quad ? 0 : tb.mlo;
+  const TableKey key = std::make_tuple(tb.bl, quad ? -1 : tb.an, tb.ss, kind);
   auto it = g_sliced.find(key);
   if (it != g_sliced.end() && (!eighth || it->second->panels8)) return it->second.get();
   if (eighth && (!get_split_tables() || g_refused.count(key) || capturing(st))) return nullptr;
-  const bool fresh = it == g_sliced.end(), q = kind_rows_l(kind);
-  std::vector<int64_t> po(tb.nm), eo(tb.nm);
+  const bool fresh = it == g_sliced.end();
+  std::vector<int64_t> po(nm), eo(nm);
   int64_t ptot = 0, etot = 0;
-  for (int mi = 0; mi < tb.nm; ++mi) {
-    const Geom g = geom(tb.bl, tb.nt, tb.an, tb.mlo + mi, q);
+  for (int mi = 0; mi < nm; ++mi) {
+    const Geom g = geom(tb.bl, tb.nt, tb.an, tmlo + mi, mode);
     po[mi] = ptot;
     eo[mi] = etot;
     ptot += (int64_t)g.nrt * g.nkc * kS * kPanelA;
@@ -1142,26 +1162,33 @@ SlicedTable *sliced(const WignerTable &tb, int kind, bool eighth, cudaStream_t s
     s->bl = tb.bl;
     s->nt = tb.nt;
     s->an = tb.an;
-    s->mlo = tb.mlo;
-    s->nm = tb.nm;
-    s->q = q;
+    s->mlo = tmlo;
+    s->nm = nm;
+    s->mode = mode;
   }
   uint8_t *p8 = nullptr;
   try {
     if (fresh) {
       s->panels = dev_alloc<uint8_t>((size_t)ptot, &by);
       s->eA = dev_alloc<int8_t>((size_t)etot, &by);
-      s->d_pan_off = dev_alloc<int64_t>(tb.nm, &by);
-      s->d_e_off = dev_alloc<int64_t>(tb.nm, &by);
-      S2G_CUDA(cudaMemcpyAsync(s->d_pan_off, po.data(), sizeof(int64_t) * tb.nm, cudaMemcpyHostToDevice, st));
-      S2G_CUDA(cudaMemcpyAsync(s->d_e_off, eo.data(), sizeof(int64_t) * tb.nm, cudaMemcpyHostToDevice, st));
+      s->d_pan_off = dev_alloc<int64_t>(nm, &by);
+      s->d_e_off = dev_alloc<int64_t>(nm, &by);
+      S2G_CUDA(cudaMemcpyAsync(s->d_pan_off, po.data(), sizeof(int64_t) * nm, cudaMemcpyHostToDevice, st));
+      S2G_CUDA(cudaMemcpyAsync(s->d_e_off, eo.data(), sizeof(int64_t) * nm, cudaMemcpyHostToDevice, st));
     }
     if (eighth) p8 = dev_alloc<uint8_t>((size_t)(ptot / kS), &by);
-    const dim3 grid(tb.nm, (std::max(tb.bl, tb.nt) + kPM - 1) / kPM);
-    k_slice_table<<<grid, 128, 0, st>>>(kind_of_q(kind) ? tb.Q : tb.D, tb.d_off, tb.bl, tb.nt, tb.an, tb.mlo,
-                                        q ? 1 : 0, kind_transposed(kind) ? 1 : 0, fresh ? s->panels : nullptr, p8,
-                                        s->d_pan_off, s->eA, s->d_e_off);
+    const dim3 grid(nm, (std::max(tb.bl, tb.nt) + kPM - 1) / kPM);
+    int64_t *d_woff = nullptr;  // the operators' blocks from W_+
+    if (quad) {
+      const int64_t woff[2] = {0, (int64_t)(((intptr_t)tb.W[1] - (intptr_t)tb.W[0]) / (intptr_t)sizeof(double))};
+      S2G_CUDA(cudaMallocAsync((void **)&d_woff, sizeof woff, st));
+      S2G_CUDA(cudaMemcpyAsync(d_woff, woff, sizeof woff, cudaMemcpyHostToDevice, st));
+    }
+    k_slice_table<<<grid, 128, 0, st>>>(quad ? tb.W[0] : (kind_of_q(kind) ? tb.Q : tb.D), quad ? d_woff : tb.d_off,
+                                        tb.bl, tb.nt, tb.an, tmlo, mode, kind_transposed(kind) ? 1 : 0,
+                                        fresh ? s->panels : nullptr, p8, s->d_pan_off, s->eA, s->d_e_off);
     S2G_LAUNCHED();
+    if (d_woff) cudaFreeAsync(d_woff, st);
     S2G_CUDA(cudaStreamSynchronize(st));
   } catch (const Error &e) {
     if (fresh) s->release();
@@ -1190,16 +1217,16 @@ const TileList *tile_list(SlicedTable &s, int n, int mlo, int mhi, int lmin, boo
   std::vector<int64_t> xoff(mhi - mlo + 1);
   int64_t xe = 0, work = 0;
   for (int m = mlo; m <= mhi; ++m) {
-    const Geom g = geom(s.bl, s.nt, s.an, m, s.q);
+    const Geom g = geom(s.bl, s.nt, s.an, m, s.mode);
     xoff[m - mlo] = xe;
     xe += (int64_t)g.nkc * 16 * kPK;  // per digit slice and 16 columns
     if (g.nl <= 0) continue;
     const int lst = g.l0 > lmin ? g.l0 : lmin;
     int rt0 = 0, kc0 = 0;
-    if (s.q) {
+    if (s.mode == MX_T2L) {
       if (lst >= s.bl) continue;
       rt0 = (lst - g.l0) / kPM;
-    } else {
+    } else if (s.mode == MX_L2T) {
       kc0 = lst >= s.bl ? g.nkc : (lst - g.l0) / kPK;
     }
     for (int rt = rt0; rt < g.nrt; ++rt) {
@@ -1269,7 +1296,7 @@ bool run_mixed(const Problem &p, const Prepared &pr, cudaStream_t st, int gpl_ma
     return true;
   }();
   (void)attr;
-  const bool q = kind_rows_l(p.kind);
+  const int mode = kind_mode(p.kind);
   const SlicedTable *s = pr.s;
   const TileList *L = pr.L;
   int *err = pr.err;
@@ -1277,7 +1304,7 @@ bool run_mixed(const Problem &p, const Prepared &pr, cudaStream_t st, int gpl_ma
   const int nmp = p.mhi - p.mlo + 1;
   const int mpp = NC / (2 * p.nparts);  // maps per part per launch
   int nkcmax = 0;
-  for (int pm = 0; pm < nmp; ++pm) nkcmax = std::max(nkcmax, geom(p.tb->bl, p.tb->nt, p.tb->an, p.mlo + pm, q).nkc);
+  for (int pm = 0; pm < nmp; ++pm) nkcmax = std::max(nkcmax, geom(p.tb->bl, p.tb->nt, p.tb->an, p.mlo + pm, mode).nkc);
   const size_t slice_smem = sizeof(double2) * kMG * (size_t)sv_idx(nkcmax * kPK);
   constexpr int kSliceSmemMax = 232448 - 1024;  // the opt-in maximum less the static arrays
   S2G_REQUIRE(slice_smem <= (size_t)kSliceSmemMax, ERR_INVALID,
@@ -1318,7 +1345,7 @@ bool run_mixed(const Problem &p, const Prepared &pr, cudaStream_t st, int gpl_ma
         xby = (double)x_elems * 2.0 * (1.0 + 8.0 / (2.0 * S));  // panels written + FP64 values read
       }
       XArgs xa{};
-      xa.q = q ? 1 : 0;
+      xa.mode = mode;
       xa.bl = p.tb->bl;
       xa.nt = p.tb->nt;
       xa.an = p.tb->an;
@@ -1335,14 +1362,14 @@ bool run_mixed(const Problem &p, const Prepared &pr, cudaStream_t st, int gpl_ma
       xa.nmp = nmp;
       xa.nkcmax = nkcmax;
       xa.kst = sv_idx(nkcmax * kPK);
-      KTimer kx(KC_SLICE, st, 0.0, xby);
+      KTimer kx(mode == MX_QUAD ? KC_QUAD : KC_SLICE, st, 0.0, xby);
       k_slice_x<NC, S><<<dim3((nmp + kMG - 1) / kMG, NC / 2), kSliceThreads, slice_smem, st>>>(xa);
       S2G_LAUNCHED();
     }
     if (L->ntiles == 0) continue;
-    KTimer kt(KC_MIXED, st, fl, by);
+    KTimer kt(mode == MX_QUAD ? KC_QUAD : KC_MIXED, st, fl, by);
     MxArgs ma{};
-    ma.q = q ? 1 : 0;
+    ma.mode = mode;
     ma.panels = s->panels;
     ma.panels8 = s->panels8;
     ma.pan_off = s->d_pan_off;
@@ -1499,6 +1526,34 @@ bool contract_l2t_mixed(const L2T *a, int nparts, cudaStream_t st) {
 }
 bool contract_t2l_mixed(const T2L *a, int nparts, cudaStream_t st) {
   return contract_mixed(a, nparts, a[0].use_q ? TK_T2L_Q : TK_T2L_D, st);
+}
+
+bool quadrature_mixed(const WignerTable &tb, bool trans, const QuadIO *io, int n, int mlo, int mhi, int64_t is, int iw,
+                      int i_mlo, int64_t os, int ow, int o_mlo, int nb, cudaStream_t st) {
+  if (n < 1 || n > kMaxParts || nb <= 0 || mhi < mlo) return false;
+  if (tb.bl < kMinBl8 || std::max(tb.bl, tb.nt) > kMaxK8) return false;
+  Problem p{};
+  p.kind = trans ? TK_WT : TK_W;
+  p.eighth = true;
+  p.tb = &tb;
+  p.n = tb.an & 1;
+  p.mlo = mlo;
+  p.mhi = mhi;
+  p.nb = nb;
+  p.nparts = n;
+  for (int i = 0; i < n; ++i) {
+    Part &P = p.part[i];
+    P.src = io[i].in;
+    P.ss = is;
+    P.sw = iw;
+    P.s_mlo = i_mlo;
+    P.wscale = 1.0;
+    P.dst = io[i].out;
+    P.ds = os;
+    P.dw = ow;
+    P.d_mlo = o_mlo;
+  }
+  return run_problem(p, st);
 }
 
 void release_sliced_tables() {

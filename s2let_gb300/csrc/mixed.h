@@ -30,6 +30,16 @@ namespace s2g {
 bool contract_l2t_mixed(const L2T *a, int nparts, cudaStream_t st);
 bool contract_t2l_mixed(const T2L *a, int nparts, cudaStream_t st);
 
+// The quadrature operator W_eps(m) (trans: its transpose) of a recomputed table's
+// grid on the ring spectra of n <= kMaxParts problems, m in [mlo, mhi]: in eight
+// digit slices, with FP64 rounding error in both modes; false as above.
+struct QuadIO {
+  const double2 *in;
+  double2 *out;
+};
+bool quadrature_mixed(const WignerTable &tb, bool trans, const QuadIO *io, int n, int mlo, int mhi, int64_t is, int iw,
+                      int i_mlo, int64_t os, int ow, int o_mlo, int nb, cudaStream_t st);
+
 void release_sliced_tables();
 size_t sliced_table_bytes();
 // Reads and clears the device flag raised by a split-precision launch whose

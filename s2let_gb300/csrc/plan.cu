@@ -10,6 +10,7 @@
 
 #include "common.h"
 #include "plan.h"
+#include "recompute.h"
 
 namespace s2g {
 
@@ -545,6 +546,12 @@ std::unique_ptr<WignerTable> build_table(int bl, int an, int ss, bool rc) {
     for (int t = 0; t < nt; ++t) uq[t] = make_double2(ang[t].u_hi, ang[t].north ? 1.0 : 0.0);
     tb->uq = dev_alloc<double2>(nt);
     S2G_CUDA(cudaMemcpy(tb->uq, uq.data(), sizeof(double2) * nt, cudaMemcpyHostToDevice));
+    std::vector<int64_t> roff(tb->nm + 1, 0);
+    for (int mi = 0; mi < tb->nm; ++mi) roff[mi + 1] = roff[mi] + std::max(0, bl - tb->l0(tb->mlo + mi));
+    tb->d_roff = dev_alloc<int64_t>(tb->nm + 1);
+    S2G_CUDA(cudaMemcpy(tb->d_roff, roff.data(), sizeof(int64_t) * (tb->nm + 1), cudaMemcpyHostToDevice));
+    tb->rec = build_rec(bl, an, tb->mlo, tb->nm, tb->d_roff, roff.back());
+    g_bytes += sizeof(RcRec) * (size_t)roff.back();
     k_wigner_ckpt<<<ceil_div(nthr, 128), 128>>>(tb->ck, tb->ck_e, tb->d_coff, bl, nt, an, tb->mlo, tb->nm, d_hi,
                                                 d_lo, d_ex, d_ang);
     S2G_LAUNCHED();
@@ -656,6 +663,8 @@ void release_plans() {
     cudaFree(kv.second->ck_e);
     cudaFree(kv.second->d_coff);
     cudaFree(kv.second->uq);
+    cudaFree(kv.second->rec);
+    cudaFree(kv.second->d_roff);
   }
   for (auto &kv : g_wmat) {
     cudaFree(kv.second.first);

@@ -35,6 +35,12 @@ namespace s2g {
 constexpr int kSeg = 64;
 constexpr int kCkZeroExp = -100000;  // exponent of an all-zero checkpoint
 
+// The rescaled recursion of a recomputed table at one (m, l) (recompute.cu):
+// p' north of the equator (-p' south), q' north and south, lam
+struct alignas(16) RcRec {
+  double p, qn, qs, lam;
+};
+
 struct WignerTable {
   int bl = 0, an = 0, ss = 0, nt = 0, mlo = 0, nm = 0;
   bool rc = false;
@@ -48,6 +54,8 @@ struct WignerTable {
   double2 *ck = nullptr;
   int *ck_e = nullptr;
   double2 *uq = nullptr;
+  RcRec *rec = nullptr;  // degree l at [roff[mi] + l - l0], 32 B per (m, l)
+  int64_t *d_roff = nullptr;
   const double *W[2] = {nullptr, nullptr};
   int64_t elems() const { return off.empty() ? 0 : off.back(); }
   int l0(int m) const { return (m < 0 ? -m : m) > an ? (m < 0 ? -m : m) : an; }

@@ -8,9 +8,19 @@
 //   d^{l+1} = (q_l + p_l u) d^l - c2_l d^{l-1}
 //   north: p_l = -r l(l+1), q_l = r (l(l+1) - m n);  south: p_l = r l(l+1), q_l = -r (l(l+1) + m n)
 //   r = (2l+1) / (l S_{l+1}),  c2_l = (l+1) S_l / (l S_{l+1}),  S_l = sqrt((l^2-m^2)(l^2-n^2))
-// Three FP64 instructions per value; restarting every kSeg degrees from the
-// double-double checkpoints keeps the recursion's rounding growth to a few
-// ulps (a plain FP64 run over l < 2048 drifts by ~3e-12 near the poles).
+// rescaled within a segment: with d^l = lam_l w_l, lam_{lc} = lam_{lc+1} = 1 and
+// lam_{l+1} = c2_l lam_{l-1}, it is w_{l+1} = (p' u + q') w_l - w_{l-1} with (p', q') =
+// (p, q) lam_l / (c2_l lam_{l-1}): two FP64 instructions per value.  lam depends on
+// (l, m) only and is folded into the coefficients (l -> t) or the output weight (t
+// -> l).  p', q' and lam are part of the table (WignerTable::rec): computing them
+// per launch and ring tile (two square roots and two divisions per degree, and a
+// serial product over the segment) cost a third of the FP64 work.  Restarting
+// every kSeg degrees from the double-double checkpoints keeps the recursion's
+// rounding growth to a few ulps (a plain FP64 run over l < 2048 drifts by ~3e-12
+// near the poles).
+// One regenerated row serves every problem on its table at once (parts): the
+// scales of one band-limit, and directions n and -n (d_{m,-n} = (-1)^{m+n}
+// d_{-m,n}), up to 4 parts per launch.
 // Values are carried scaled by 2^-E, one scale per ring and segment, applied
 // once per segment: to the partial sums (l -> t) or to the inputs (t -> l).
 //
@@ -19,6 +29,7 @@
 //   k_apply_w  the forward quadrature W_eps(m) (or its transpose) on ring spectra: the
 //              stored path's Q = D^T W becomes D^T applied after W (FP64 tiled GEMM)
 #include <algorithm>
+#include <vector>
 
 #include "autotune.h"
 #include "common.h"
@@ -35,61 +46,99 @@ namespace {
 constexpr int kRcT = 128;  // threads per CTA: rings per tile
 static_assert(kRcT == 2 * kSeg, "t -> l maps two threads per degree of a segment");
 
+constexpr int kRcParts = 4;
+// One problem on the table: row mt of the table is its m = mt, or -mt (neg).
+struct RcPart {
+  int mlo, mhi, lmin;
+  int neg;
+  const double2 *w;
+  const double2 *src;  // l -> t: x (l^2 + l + m);  t -> l: spectra [t][m - s_mlo]
+  double2 *dst;        // l -> t: spectra [t][m - d_mlo];  t -> l: y (l^2 + l + m)
+};
 struct RcArgs {
-  int bl, nt, an, tmlo, n;
+  int bl, nt, an, tmlo;
   const int64_t *coff;
   const double2 *ck;
   const int *ck_e;
   const double2 *uq;
-  int mlo, lmin;
-  const double2 *w;
+  const RcRec *rec;
+  const int64_t *roff;
+  int np, lmin;  // parts, smallest lmin
+  RcPart part[kRcParts];
   double wscale;
   int wconj;
-  const double2 *src;  // l -> t: x (l^2 + l + m);  t -> l: spectra [t][m - s_mlo]
   int64_t ss;
   int sw, s_mlo, x_half;
-  double2 *dst;  // l -> t: spectra [t][m - d_mlo];  t -> l: y (l^2 + l + m)
   int64_t ds;
   int dw, d_mlo;
-  int nb;
+  int nb, mpc;  // maps, maps per CTA: column c = part c / mpc, map b0 + c % mpc
 };
 
+// explicit roundings: every instantiation (columns per CTA) gives the same bits
 __device__ __forceinline__ double2 cmul_(double2 a, double2 b) {
-  return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+  return make_double2(__fma_rn(a.x, b.x, __dmul_rn(-a.y, b.y)), __fma_rn(a.x, b.y, __dmul_rn(a.y, b.x)));
 }
-__device__ __forceinline__ double2 weight_of(const RcArgs &a, int l) {
-  double2 w = a.w ? a.w[l] : make_double2(1.0, 0.0);
+__device__ __forceinline__ double2 weight_of(const RcArgs &a, const RcPart &P, int l) {
+  double2 w = P.w ? P.w[l] : make_double2(1.0, 0.0);
   if (a.wconj) w.y = -w.y;
   return make_double2(w.x * a.wscale, w.y * a.wscale);
 }
-
-// table row (mirror for n < 0, or n = 0 and m < 0 on a table holding m >= 0)
-struct RcRef {
-  int mi, mt;
+// m of a part at table row mt, whether the part has it, and its sign
+struct RcM {
+  int m;
+  bool on;
   double sign;
 };
-__device__ __forceinline__ RcRef rc_ref(const RcArgs &a, int m) {
-  RcRef r;
-  if (a.n > 0 || (a.n == 0 && m >= 0)) {
-    r.mi = m - a.tmlo;
-    r.sign = 1.0;
-  } else {
-    r.mi = -m - a.tmlo;
-    r.sign = ((m + a.an) & 1) ? -1.0 : 1.0;
-  }
-  r.mt = a.tmlo + r.mi;
+__device__ __forceinline__ RcM rc_m(const RcArgs &a, const RcPart &P, int mt) {
+  RcM r;
+  r.m = P.neg ? -mt : mt;
+  r.on = r.m >= P.mlo && r.m <= P.mhi;
+  r.sign = P.neg && ((r.m + a.an) & 1) ? -1.0 : 1.0;
   return r;
 }
+// l -> t coefficient of a column: x(l, m) w(l) f
+__device__ __forceinline__ double2 rc_coef(const RcArgs &a, const RcPart &P, int m, int b, int l, double f) {
+  const int64_t base = (int64_t)b * a.ss + (int64_t)l * l + l;
+  double2 v;
+  if (a.x_half && m < 0) {
+    v = P.src[base - m];
+    v.y = -v.y;
+    if (m & 1) v = make_double2(-v.x, -v.y);
+  } else {
+    v = P.src[base + m];
+  }
+  const double2 w = weight_of(a, P, l);
+  return cmul_(v, make_double2(w.x * f, w.y * f));
+}
 
-// recursion coefficients of degree l for (m, an): cn = (p, q) north, cs = (p, q) south
-__device__ __forceinline__ void rec_coef(int l, int m, int an, double2 &cn, double2 &cs, double &c2) {
-  const double dl = l, ll1 = dl * (dl + 1.0), mn = (double)m * an, m2 = (double)m * m, n2 = (double)an * an;
-  const double s1 = sqrt(((dl + 1.0) * (dl + 1.0) - m2) * ((dl + 1.0) * (dl + 1.0) - n2));
-  const double s0 = sqrt((dl * dl - m2) * (dl * dl - n2));
-  const double r = (2.0 * dl + 1.0) / (dl * s1);
-  cn = make_double2(-r * ll1, r * (ll1 - mn));
-  cs = make_double2(r * ll1, -r * (ll1 + mn));
-  c2 = (dl + 1.0) * s0 / (dl * s1);
+// The rescaled recursion of every (m, segment): rec[roff[mi] + l - l0] = (p', q'
+// north, q' south, lam) of degree l (p', q' unused at a segment's first degree).
+__global__ void k_rc_rec(RcRec *__restrict__ rec, const int64_t *__restrict__ roff, int bl, int an, int mlo,
+                         int nm, int maxseg) {
+  const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (gid >= (int64_t)nm * maxseg) return;
+  const int mi = (int)(gid / maxseg), c = (int)(gid % maxseg);
+  const int m = mlo + mi, am = m < 0 ? -m : m, l0 = am > an ? am : an;
+  const int lc = l0 + c * kSeg, n = min(kSeg, bl - lc);
+  if (n <= 0) return;
+  RcRec *out = rec + roff[mi] + c * kSeg;
+  out[0] = RcRec{0.0, 0.0, 0.0, 1.0};
+  double lam0 = 1.0, lam1 = 1.0;  // lam of degrees lc + i - 1 and lc + i
+  for (int i = 1; i < n; ++i) {
+    const double dl = lc + i, ll1 = dl * (dl + 1.0), mn = (double)m * an, m2 = (double)m * m, n2 = (double)an * an;
+    const double s1 = sqrt(((dl + 1.0) * (dl + 1.0) - m2) * ((dl + 1.0) * (dl + 1.0) - n2));
+    const double s0 = sqrt((dl * dl - m2) * (dl * dl - n2));
+    const double r = (2.0 * dl + 1.0) / (dl * s1), c2 = (dl + 1.0) * s0 / (dl * s1);
+    const double f = lam1 / (c2 * lam0);
+    out[i] = RcRec{-r * ll1 * f, r * (ll1 - mn) * f, -r * (ll1 + mn) * f, lam1};
+    const double lam2 = c2 * lam0;
+    lam0 = lam1;
+    lam1 = lam2;
+  }
+}
+// p' (negated south of the equator), q' of one degree
+__device__ __forceinline__ double2 rec_pq(const RcRec &r, bool north) {
+  return north ? make_double2(r.p, r.qn) : make_double2(-r.p, r.qs);
 }
 
 __device__ __forceinline__ int exp_bits(double v) { return (int)((__double_as_longlong(v) >> 52) & 0x7FF); }
@@ -103,19 +152,16 @@ __device__ __forceinline__ double pow2(int E) { return E < -1074 ? 0.0 : ldexp(1
 // ---------------------------------------------------------------------------
 
 template <int NBT>
-__global__ void __launch_bounds__(kRcT) k_rc_l2t(RcArgs a) {
-  __shared__ double2 scn[kSeg], scs[kSeg];
-  __shared__ double sc2[kSeg];
+__global__ void __launch_bounds__(kRcT) k_rc_l2t(const __grid_constant__ RcArgs a) {
+  __shared__ RcRec srec[kSeg];
   __shared__ double2 sx[kSeg][NBT];
-  const int m = a.mlo + blockIdx.x;
-  const int am = m < 0 ? -m : m;
-  const RcRef r = rc_ref(a, m);
-  const int amt = r.mt < 0 ? -r.mt : r.mt;
+  const int mt = a.tmlo + blockIdx.x;
+  const int amt = mt < 0 ? -mt : mt;
   const int l0 = amt > a.an ? amt : a.an, bl = a.bl, nl = bl - l0;
   const int lst = l0 > a.lmin ? l0 : a.lmin;
   const int t = blockIdx.y * kRcT + threadIdx.x;
   const bool live = t < a.nt;
-  const int b0 = blockIdx.z * NBT;
+  const int b0 = blockIdx.z * a.mpc;
   double2 acc[NBT];
 #pragma unroll
   for (int b = 0; b < NBT; ++b) acc[b] = make_double2(0.0, 0.0);
@@ -128,29 +174,23 @@ __global__ void __launch_bounds__(kRcT) k_rc_l2t(RcArgs a) {
   }
   if (nl > 0 && lst < bl) {
     const int nseg = (nl + kSeg - 1) / kSeg, c0 = (lst - l0) / kSeg;
-    const double2 *ck = a.ck + a.coff[r.mi];
-    const int *cke = a.ck_e + a.coff[r.mi];
-    const double2 *cc = north ? scn : scs;
+    const double2 *ck = a.ck + a.coff[blockIdx.x];
+    const int *cke = a.ck_e + a.coff[blockIdx.x];
+    const RcRec *rec = a.rec + a.roff[blockIdx.x];
     for (int c = c0; c < nseg; ++c) {
       const int lc = l0 + c * kSeg, n = min(kSeg, bl - lc);
       __syncthreads();
-      for (int i = threadIdx.x; i < n; i += kRcT)
-        if (i >= 1) rec_coef(lc + i, r.mt, a.an, scn[i], scs[i], sc2[i]);
+      for (int i = threadIdx.x; i < n; i += kRcT) srec[i] = rec[c * kSeg + i];
+      __syncthreads();
       for (int i = threadIdx.x; i < kSeg * NBT; i += kRcT) {
-        const int kk = i / NBT, b = i % NBT, l = lc + kk;
+        const int kk = i / NBT, col = i % NBT, l = lc + kk, p = col / a.mpc, b = b0 + col % a.mpc;
         double2 v = make_double2(0.0, 0.0);
-        if (kk < n && l >= lst && b0 + b < a.nb) {
-          const int64_t base = (int64_t)(b0 + b) * a.ss + (int64_t)l * l + l;
-          if (a.x_half && m < 0) {
-            v = a.src[base - m];
-            v.y = -v.y;
-            if (am & 1) v = make_double2(-v.x, -v.y);
-          } else {
-            v = a.src[base + m];
-          }
-          v = cmul_(v, weight_of(a, l));
+        if (kk < n && p < a.np && b < a.nb) {
+          const RcPart &P = a.part[p];
+          const RcM rm = rc_m(a, P, mt);
+          if (rm.on && l >= P.lmin) v = rc_coef(a, P, rm.m, b, l, srec[kk].lam);
         }
-        sx[kk][b] = v;
+        sx[kk][col] = v;
       }
       __syncthreads();
       if (!live) continue;
@@ -169,9 +209,9 @@ __global__ void __launch_bounds__(kRcT) k_rc_l2t(RcArgs a) {
         }
       }
       for (int i = 1; i + 1 < n; ++i) {
-        const double2 k = cc[i];
+        const double2 k = rec_pq(srec[i], north);
         const double xt = fma(k.x, u, k.y);
-        const double vn = fma(xt, v, -sc2[i] * vp);
+        const double vn = fma(xt, v, -vp);
         vp = v;
         v = vn;
         if (exp_bits(v) > 1023 + kRenorm) {  // flush at the old scale, continue at the new one
@@ -202,10 +242,13 @@ __global__ void __launch_bounds__(kRcT) k_rc_l2t(RcArgs a) {
   }
   if (!live) return;
 #pragma unroll
-  for (int b = 0; b < NBT; ++b) {
-    if (b0 + b >= a.nb) break;
-    a.dst[(int64_t)(b0 + b) * a.ds + (int64_t)t * a.dw + (m - a.d_mlo)] =
-        make_double2(acc[b].x * r.sign, acc[b].y * r.sign);
+  for (int col = 0; col < NBT; ++col) {
+    const int p = col / a.mpc, b = b0 + col % a.mpc;
+    if (p >= a.np || b >= a.nb) continue;
+    const RcM rm = rc_m(a, a.part[p], mt);
+    if (!rm.on) continue;
+    a.part[p].dst[(int64_t)b * a.ds + (int64_t)t * a.dw + (rm.m - a.d_mlo)] =
+        make_double2(acc[col].x * rm.sign, acc[col].y * rm.sign);
   }
 }
 
@@ -220,35 +263,34 @@ size_t rc_t2l_smem() {
   return sizeof(double) * kRcT * kTileLd + sizeof(double2) * kRcT * NBT;
 }
 
-// grid: x = m, y = segment, z = batch chunk.  Threads generate one ring's row of
-// the tile each, then contract as (degree li = tid % kSeg, half bh = tid / kSeg):
-// with NBT >= 2 each half takes half of the maps over all rings of the tile;
-// with NBT = 1 each half takes half of the rings, and the halves add up at the end.
+// grid: x = table row, y = segment, z = batch chunk.  Threads generate one ring's
+// row of the tile each, then contract as (degree li = tid % kSeg, half bh = tid /
+// kSeg): with NBT >= 2 each half takes half of the columns over all rings of the
+// tile; with NBT = 1 each half takes half of the rings, and the halves add up at
+// the end.
 template <int NBT>
-__global__ void __launch_bounds__(kRcT) k_rc_t2l(RcArgs a) {
-  static_assert(NBT == 1 || NBT % 2 == 0, "one map, or two map halves");
+__global__ void __launch_bounds__(kRcT) k_rc_t2l(const __grid_constant__ RcArgs a) {
+  static_assert(NBT == 1 || NBT % 2 == 0, "one column, or two column halves");
   constexpr int NH = NBT == 1 ? 1 : NBT / 2;
   constexpr bool SPLIT_T = NBT == 1;
   extern __shared__ double smem_rc[];
   double *tile = smem_rc;                                   // [kRcT][kTileLd]
   double2 *sg = (double2 *)(smem_rc + kRcT * kTileLd);      // [kRcT][NBT]
-  __shared__ double2 scn[kSeg], scs[kSeg];
-  __shared__ double sc2[kSeg];
-  const int m = a.mlo + blockIdx.x, c = blockIdx.y;
-  const RcRef r = rc_ref(a, m);
-  const int amt = r.mt < 0 ? -r.mt : r.mt;
+  __shared__ RcRec srec[kSeg];
+  const int mt = a.tmlo + blockIdx.x, c = blockIdx.y;
+  const int amt = mt < 0 ? -mt : mt;
   const int l0 = amt > a.an ? amt : a.an, bl = a.bl, nl = bl - l0;
   const int lst = l0 > a.lmin ? l0 : a.lmin;
   const int nseg = nl > 0 ? (nl + kSeg - 1) / kSeg : 0;
   if (c >= nseg) return;
   const int lc = l0 + c * kSeg, n = min(kSeg, bl - lc);
   if (lc + n <= lst) return;  // every degree of the segment is below lmin: no output
-  const int b0 = blockIdx.z * NBT;
+  const int b0 = blockIdx.z * a.mpc;
   const int tid = threadIdx.x;
-  for (int i = tid; i < n; i += kRcT)
-    if (i >= 1) rec_coef(lc + i, r.mt, a.an, scn[i], scs[i], sc2[i]);
-  const double2 *ck = a.ck + a.coff[r.mi] + (int64_t)c * a.nt;
-  const int *cke = a.ck_e + a.coff[r.mi] + (int64_t)c * a.nt;
+  const RcRec *rec = a.rec + a.roff[blockIdx.x] + c * kSeg;
+  for (int i = tid; i < n; i += kRcT) srec[i] = rec[i];
+  const double2 *ck = a.ck + a.coff[blockIdx.x] + (int64_t)c * a.nt;
+  const int *cke = a.ck_e + a.coff[blockIdx.x] + (int64_t)c * a.nt;
   const int li = tid % kSeg, bh = tid / kSeg;
   double2 acc[NH];
 #pragma unroll
@@ -263,15 +305,15 @@ __global__ void __launch_bounds__(kRcT) k_rc_t2l(RcArgs a) {
     if (E >= -1074 - 2 * kRenorm) {
       const double2 q = a.uq[t];
       const double u = q.x;
-      const double2 *cc = q.y != 0.0 ? scn : scs;
+      const bool north = q.y != 0.0;
       const double2 ab = ck[t];
       double vp = ab.x, v = ab.y;
       row[0] = vp;
       if (n > 1) row[1] = v;
       for (int i = 1; i + 1 < n; ++i) {
-        const double2 k = cc[i];
+        const double2 k = rec_pq(srec[i], north);
         const double xt = fma(k.x, u, k.y);
-        const double vn = fma(xt, v, -sc2[i] * vp);
+        const double vn = fma(xt, v, -vp);
         vp = v;
         v = vn;
         if (exp_bits(v) > 1023 + kRenorm) {  // keep one scale per row: rescale what is written
@@ -288,13 +330,15 @@ __global__ void __launch_bounds__(kRcT) k_rc_t2l(RcArgs a) {
       for (int i = 0; i < kSeg; ++i) row[i] = 0.0;
     }
 #pragma unroll
-    for (int b = 0; b < NBT; ++b) {
+    for (int col = 0; col < NBT; ++col) {
+      const int p = col / a.mpc, b = b0 + col % a.mpc;
       double2 g = make_double2(0.0, 0.0);
-      if (t < a.nt && b0 + b < a.nb && scale != 0.0) {
-        g = a.src[(int64_t)(b0 + b) * a.ss + (int64_t)t * a.sw + (m - a.s_mlo)];
+      if (t < a.nt && p < a.np && b < a.nb && scale != 0.0) {
+        const RcM rm = rc_m(a, a.part[p], mt);
+        if (rm.on) g = a.part[p].src[(int64_t)b * a.ss + (int64_t)t * a.sw + (rm.m - a.s_mlo)];
         g = make_double2(g.x * scale, g.y * scale);
       }
-      sg[tid * NBT + b] = g;
+      sg[tid * NBT + col] = g;
     }
     __syncthreads();
     const int tl_end = min(kRcT, a.nt - t0);
@@ -321,14 +365,18 @@ __global__ void __launch_bounds__(kRcT) k_rc_t2l(RcArgs a) {
     acc[0].y += red[li].y;
   }
   const int l = lc + li;
-  if (li >= n || l < lst) return;
-  const double2 wt = weight_of(a, l);
+  if (li >= n) return;
+  const double lam = srec[li].lam;  // the rescaled recursion's lam_l
 #pragma unroll
   for (int j = 0; j < NH; ++j) {
-    const int b = b0 + (SPLIT_T ? 0 : bh * NH) + j;
-    if (b >= a.nb) break;
-    const double2 v = make_double2(acc[j].x * r.sign, acc[j].y * r.sign);
-    a.dst[(int64_t)b * a.ds + (int64_t)l * l + l + m] = cmul_(v, wt);
+    const int col = (SPLIT_T ? 0 : bh * NH) + j, p = col / a.mpc, b = b0 + col % a.mpc;
+    if (p >= a.np || b >= a.nb) continue;
+    const RcPart &P = a.part[p];
+    const RcM rm = rc_m(a, P, mt);
+    if (!rm.on || l < P.lmin) continue;
+    const double sl = rm.sign * lam;
+    P.dst[(int64_t)b * a.ds + (int64_t)l * l + l + rm.m] =
+        cmul_(make_double2(acc[j].x * sl, acc[j].y * sl), weight_of(a, P, l));
   }
 }
 
@@ -348,7 +396,7 @@ __global__ void __launch_bounds__(kRcT) k_rc_t2l(RcArgs a) {
 // lower rescaling threshold (2^kRenormDf) so that they stay in the float
 // range.  Coefficients (l -> t) and spectra (t -> l) enter as double-float
 // scaled by the largest power of two of their block (segment or tile, per
-// map).  Accumulators are renormalised after each add.
+// map).  The sums are Dot2 sums (dfarith.h).
 // ---------------------------------------------------------------------------
 
 constexpr int kRenormDf = 60;
@@ -359,50 +407,19 @@ __device__ __forceinline__ float2 df_of(double v) {  // |v| within the float ran
   return make_float2(h, l);
 }
 __device__ __forceinline__ float2 df_scale(float2 a, int k) { return make_float2(scale_pow2(a.x, k), scale_pow2(a.y, k)); }
-// Rescaled recursion of one segment (double-float kernels): with v_l =
-// lam_l w_l, lam_{lc} = lam_{lc+1} = 1 and lam_{l+1} = c2_l lam_{l-1}, the
-// three-term step v_{l+1} = (p u + q) v_l - c2_l v_{l-1} becomes
-// w_{l+1} = (p' u + q') w_l - w_{l-1} with (p', q') = (p, q) lam_l / (c2_l
-// lam_{l-1}): two FP64 instructions per value instead of three.  lam depends
-// on (l, m) only, so it is folded into the coefficients (l -> t) or the output
-// weight (t -> l).  On entry cn / cs / c2 hold the coefficients of degrees
-// lc + i, i in [1, n); on exit cn / cs the rescaled pairs and lam[i], i < n.
-// Called by all threads of the block (contains barriers).
-__device__ void rescale_segment(double2 *cn, double2 *cs, const double *c2, double *lam, int n) {
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    lam[0] = 1.0;
-    if (n > 1) lam[1] = 1.0;
-    for (int i = 1; i + 1 < n; ++i) lam[i + 1] = c2[i] * lam[i - 1];
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < n; i += blockDim.x)
-    if (i >= 1) {
-      const double f = lam[i] / (c2[i] * lam[i - 1]);
-      cn[i] = make_double2(cn[i].x * f, cn[i].y * f);
-      cs[i] = make_double2(cs[i].x * f, cs[i].y * f);
-    }
-  __syncthreads();
-}
-
-
-
 template <int NBT>
-__global__ void __launch_bounds__(kRcT) k_rc_l2t_df(RcArgs a) {
-  __shared__ double2 scn[kSeg], scs[kSeg];
-  __shared__ double sc2[kSeg], slam[kSeg];
+__global__ void __launch_bounds__(kRcT) k_rc_l2t_df(const __grid_constant__ RcArgs a) {
+  __shared__ RcRec srec[kSeg];
   __shared__ double2 sxd[kSeg][NBT];  // weighted coefficients of the segment
   __shared__ float4 sx[kSeg][NBT];    // the same as double-float, scaled by 2^-sxs[b]
   __shared__ int sxm[NBT], sxs[NBT];
-  const int m = a.mlo + blockIdx.x;
-  const int am = m < 0 ? -m : m;
-  const RcRef r = rc_ref(a, m);
-  const int amt = r.mt < 0 ? -r.mt : r.mt;
+  const int mt = a.tmlo + blockIdx.x;
+  const int amt = mt < 0 ? -mt : mt;
   const int l0 = amt > a.an ? amt : a.an, bl = a.bl, nl = bl - l0;
   const int lst = l0 > a.lmin ? l0 : a.lmin;
   const int t = blockIdx.y * kRcT + threadIdx.x;
   const bool live = t < a.nt;
-  const int b0 = blockIdx.z * NBT;
+  const int b0 = blockIdx.z * a.mpc;
   double2 acc[NBT];
 #pragma unroll
   for (int b = 0; b < NBT; ++b) acc[b] = make_double2(0.0, 0.0);
@@ -415,30 +432,22 @@ __global__ void __launch_bounds__(kRcT) k_rc_l2t_df(RcArgs a) {
   }
   if (nl > 0 && lst < bl) {
     const int nseg = (nl + kSeg - 1) / kSeg, c0 = (lst - l0) / kSeg;
-    const double2 *ck = a.ck + a.coff[r.mi];
-    const int *cke = a.ck_e + a.coff[r.mi];
-    const double2 *cc = north ? scn : scs;
+    const double2 *ck = a.ck + a.coff[blockIdx.x];
+    const int *cke = a.ck_e + a.coff[blockIdx.x];
+    const RcRec *rec = a.rec + a.roff[blockIdx.x];
     for (int c = c0; c < nseg; ++c) {
       const int lc = l0 + c * kSeg, n = min(kSeg, bl - lc);
       __syncthreads();
-      for (int i = threadIdx.x; i < n; i += kRcT)
-        if (i >= 1) rec_coef(lc + i, r.mt, a.an, scn[i], scs[i], sc2[i]);
+      for (int i = threadIdx.x; i < n; i += kRcT) srec[i] = rec[c * kSeg + i];
       if (threadIdx.x < NBT) sxm[threadIdx.x] = 0;
-      rescale_segment(scn, scs, sc2, slam, n);
+      __syncthreads();
       for (int i = threadIdx.x; i < kSeg * NBT; i += kRcT) {
-        const int kk = i / NBT, b = i % NBT, l = lc + kk;
+        const int kk = i / NBT, b = i % NBT, l = lc + kk, p = b / a.mpc, bm = b0 + b % a.mpc;
         double2 v = make_double2(0.0, 0.0);
-        if (kk < n && l >= lst && b0 + b < a.nb) {
-          const int64_t base = (int64_t)(b0 + b) * a.ss + (int64_t)l * l + l;
-          if (a.x_half && m < 0) {
-            v = a.src[base - m];
-            v.y = -v.y;
-            if (am & 1) v = make_double2(-v.x, -v.y);
-          } else {
-            v = a.src[base + m];
-          }
-          const double2 wl = weight_of(a, l);
-          v = cmul_(v, make_double2(wl.x * slam[kk], wl.y * slam[kk]));
+        if (kk < n && p < a.np && bm < a.nb) {
+          const RcPart &P = a.part[p];
+          const RcM rm = rc_m(a, P, mt);
+          if (rm.on && l >= P.lmin) v = rc_coef(a, P, rm.m, bm, l, srec[kk].lam);
         }
         sxd[kk][b] = v;
         atomicMax(&sxm[b], max(exp_bits(v.x), exp_bits(v.y)));
@@ -462,12 +471,12 @@ __global__ void __launch_bounds__(kRcT) k_rc_l2t_df(RcArgs a) {
 #pragma unroll
         for (int b = 0; b < NBT; ++b) {
           sum[b] = make_float4(0.f, 0.f, 0.f, 0.f);
-          df_mac(sum[b], dvp, sx[0][b]);
-          if (n > 1) df_mac(sum[b], dv, sx[1][b]);
+          dot2_cmac(sum[b], dvp, sx[0][b]);
+          if (n > 1) dot2_cmac(sum[b], dv, sx[1][b]);
         }
       }
       for (int i = 1; i + 1 < n; ++i) {
-        const double2 k = cc[i];
+        const double2 k = rec_pq(srec[i], north);
         const double xt = fma(k.x, u, k.y);
         const double vn = fma(xt, v, -vp);  // rescaled recursion
         vp = v;
@@ -486,7 +495,7 @@ __global__ void __launch_bounds__(kRcT) k_rc_l2t_df(RcArgs a) {
         }
         const float2 dv = df_of(v);
 #pragma unroll
-        for (int b = 0; b < NBT; ++b) df_mac(sum[b], dv, sx[i + 1][b]);
+        for (int b = 0; b < NBT; ++b) dot2_cmac(sum[b], dv, sx[i + 1][b]);
       }
 #pragma unroll
       for (int b = 0; b < NBT; ++b) {
@@ -498,10 +507,13 @@ __global__ void __launch_bounds__(kRcT) k_rc_l2t_df(RcArgs a) {
   }
   if (!live) return;
 #pragma unroll
-  for (int b = 0; b < NBT; ++b) {
-    if (b0 + b >= a.nb) break;
-    a.dst[(int64_t)(b0 + b) * a.ds + (int64_t)t * a.dw + (m - a.d_mlo)] =
-        make_double2(acc[b].x * r.sign, acc[b].y * r.sign);
+  for (int col = 0; col < NBT; ++col) {
+    const int p = col / a.mpc, b = b0 + col % a.mpc;
+    if (p >= a.np || b >= a.nb) continue;
+    const RcM rm = rc_m(a, a.part[p], mt);
+    if (!rm.on) continue;
+    a.part[p].dst[(int64_t)b * a.ds + (int64_t)t * a.dw + (rm.m - a.d_mlo)] =
+        make_double2(acc[col].x * rm.sign, acc[col].y * rm.sign);
   }
 }
 
@@ -516,32 +528,30 @@ size_t rc_t2l_df_smem() {
 // sums over the tile's rings share one power of two and are flushed to FP64
 // once per tile.
 template <int NBT>
-__global__ void __launch_bounds__(kRcT) k_rc_t2l_df(RcArgs a) {
-  static_assert(NBT == 1 || NBT % 2 == 0, "one map, or two map halves");
+__global__ void __launch_bounds__(kRcT) k_rc_t2l_df(const __grid_constant__ RcArgs a) {
+  static_assert(NBT == 1 || NBT % 2 == 0, "one column, or two column halves");
   constexpr int NH = NBT == 1 ? 1 : NBT / 2;
   constexpr bool SPLIT_T = NBT == 1;
   extern __shared__ float2 smem_df[];
   float2 *tile = smem_df;                                  // [kRcT][kTileLd]
   float4 *sg = (float4 *)(smem_df + kRcT * kTileLd);       // [kRcT][NBT]
-  __shared__ double2 scn[kSeg], scs[kSeg];
-  __shared__ double sc2[kSeg], slam[kSeg];
+  __shared__ RcRec srec[kSeg];
   __shared__ int sgm[NBT];
-  const int m = a.mlo + blockIdx.x, c = blockIdx.y;
-  const RcRef r = rc_ref(a, m);
-  const int amt = r.mt < 0 ? -r.mt : r.mt;
+  const int mt = a.tmlo + blockIdx.x, c = blockIdx.y;
+  const int amt = mt < 0 ? -mt : mt;
   const int l0 = amt > a.an ? amt : a.an, bl = a.bl, nl = bl - l0;
   const int lst = l0 > a.lmin ? l0 : a.lmin;
   const int nseg = nl > 0 ? (nl + kSeg - 1) / kSeg : 0;
   if (c >= nseg) return;
   const int lc = l0 + c * kSeg, n = min(kSeg, bl - lc);
   if (lc + n <= lst) return;  // every degree of the segment is below lmin: no output
-  const int b0 = blockIdx.z * NBT;
+  const int b0 = blockIdx.z * a.mpc;
   const int tid = threadIdx.x;
-  for (int i = tid; i < n; i += kRcT)
-    if (i >= 1) rec_coef(lc + i, r.mt, a.an, scn[i], scs[i], sc2[i]);
-  rescale_segment(scn, scs, sc2, slam, n);
-  const double2 *ck = a.ck + a.coff[r.mi] + (int64_t)c * a.nt;
-  const int *cke = a.ck_e + a.coff[r.mi] + (int64_t)c * a.nt;
+  const RcRec *rec = a.rec + a.roff[blockIdx.x] + c * kSeg;
+  for (int i = tid; i < n; i += kRcT) srec[i] = rec[i];
+  __syncthreads();
+  const double2 *ck = a.ck + a.coff[blockIdx.x] + (int64_t)c * a.nt;
+  const int *cke = a.ck_e + a.coff[blockIdx.x] + (int64_t)c * a.nt;
   const int li = tid % kSeg, bh = tid / kSeg;
   double2 acc[NH];
 #pragma unroll
@@ -555,13 +565,13 @@ __global__ void __launch_bounds__(kRcT) k_rc_t2l_df(RcArgs a) {
     if (on) {
       const double2 q = a.uq[t];
       const double u = q.x;
-      const double2 *cc = q.y != 0.0 ? scn : scs;
+      const bool north = q.y != 0.0;
       const double2 ab = ck[t];
       double vp = ab.x, v = ab.y;
       row[0] = df_of(vp);
       if (n > 1) row[1] = df_of(v);
       for (int i = 1; i + 1 < n; ++i) {
-        const double2 k = cc[i];
+        const double2 k = rec_pq(srec[i], north);
         const double xt = fma(k.x, u, k.y);
         const double vn = fma(xt, v, -vp);  // rescaled recursion
         vp = v;
@@ -585,8 +595,10 @@ __global__ void __launch_bounds__(kRcT) k_rc_t2l_df(RcArgs a) {
 #pragma unroll
     for (int b = 0; b < NBT; ++b) {
       g[b] = make_double2(0.0, 0.0);
-      if (on && b0 + b < a.nb) {
-        g[b] = a.src[(int64_t)(b0 + b) * a.ss + (int64_t)t * a.sw + (m - a.s_mlo)];
+      const int p = b / a.mpc, bm = b0 + b % a.mpc;
+      if (on && p < a.np && bm < a.nb) {
+        const RcM rm = rc_m(a, a.part[p], mt);
+        if (rm.on) g[b] = a.part[p].src[(int64_t)bm * a.ss + (int64_t)t * a.sw + (rm.m - a.s_mlo)];
         const int ex = max(exp_bits(g[b].x), exp_bits(g[b].y));
         if (ex > 0) atomicMax(&sgm[b], ex + E);
       }
@@ -608,7 +620,7 @@ __global__ void __launch_bounds__(kRcT) k_rc_t2l_df(RcArgs a) {
     for (int tl = tl_lo; tl < tl_hi; ++tl) {
       const float2 d = tile[tl * kTileLd + li];
 #pragma unroll
-      for (int j = 0; j < NH; ++j) df_mac(sum[j], d, sg[tl * NBT + (SPLIT_T ? 0 : bh * NH) + j]);
+      for (int j = 0; j < NH; ++j) dot2_cmac(sum[j], d, sg[tl * NBT + (SPLIT_T ? 0 : bh * NH) + j]);
     }
 #pragma unroll
     for (int j = 0; j < NH; ++j) {
@@ -629,15 +641,18 @@ __global__ void __launch_bounds__(kRcT) k_rc_t2l_df(RcArgs a) {
     acc[0].y += red[li].y;
   }
   const int l = lc + li;
-  if (li >= n || l < lst) return;
-  const double2 wt = weight_of(a, l);
-  const double sl = r.sign * slam[li];  // the rescaled recursion's lam_l
+  if (li >= n) return;
+  const double lam = srec[li].lam;  // the rescaled recursion's lam_l
 #pragma unroll
   for (int j = 0; j < NH; ++j) {
-    const int b = b0 + (SPLIT_T ? 0 : bh * NH) + j;
-    if (b >= a.nb) break;
-    const double2 v = make_double2(acc[j].x * sl, acc[j].y * sl);
-    a.dst[(int64_t)b * a.ds + (int64_t)l * l + l + m] = cmul_(v, wt);
+    const int col = (SPLIT_T ? 0 : bh * NH) + j, p = col / a.mpc, b = b0 + col % a.mpc;
+    if (p >= a.np || b >= a.nb) continue;
+    const RcPart &P = a.part[p];
+    const RcM rm = rc_m(a, P, mt);
+    if (!rm.on || l < P.lmin) continue;
+    const double sl = rm.sign * lam;
+    P.dst[(int64_t)b * a.ds + (int64_t)l * l + l + rm.m] =
+        cmul_(make_double2(acc[j].x * sl, acc[j].y * sl), weight_of(a, P, l));
   }
 }
 
@@ -650,11 +665,21 @@ __global__ void __launch_bounds__(kRcT) k_rc_t2l_df(RcArgs a) {
 // A = W (trans = 0) or W^T (trans = 1).  Columns are the (map, m) pairs of the
 // parity, each complex column two real ones.  64 x 64 output tile per CTA.
 constexpr int AW_T = 64, AW_K = 16;
-__global__ void __launch_bounds__(256) k_apply_w(const double *__restrict__ Wp, const double *__restrict__ Wm,
-                                                 int trans, int nt, int an, int mlo, int mhi,
-                                                 const double2 *__restrict__ in, int64_t is, int iw, int i_mlo,
-                                                 double2 *__restrict__ out, int64_t os, int ow, int o_mlo, int nb) {
-  const int par = blockIdx.z;
+// problems of one launch (blockIdx.z = parity + 2 problem), strides in common
+constexpr int kWItems = kMaxParts;
+struct WItems {
+  int n;
+  const double2 *in[kWItems];
+  double2 *out[kWItems];
+  int mlo[kWItems], mhi[kWItems];
+};
+__global__ void __launch_bounds__(256) k_apply_w(const double *__restrict__ Wp, const double *__restrict__ Wm, int trans,
+                                          int nt, int an, const __grid_constant__ WItems items, int64_t is, int iw,
+                                          int i_mlo, int64_t os, int ow, int o_mlo, int nb) {
+  const int par = blockIdx.z & 1, item = blockIdx.z >> 1;
+  const int mlo = items.mlo[item], mhi = items.mhi[item];
+  const double2 *__restrict__ in = items.in[item];
+  double2 *__restrict__ out = items.out[item];
   const int m_first = ((mlo + an) & 1) == par ? mlo : mlo + 1;
   if (m_first > mhi) return;
   const int nmp = (mhi - m_first) / 2 + 1;  // m's of this parity
@@ -722,17 +747,17 @@ __global__ void __launch_bounds__(256) k_apply_w(const double *__restrict__ Wp, 
 // The same operator in double-float (split-precision path).  Per K-slab of
 // AWD_K: W values as double-float pairs (unscaled: the operator's entries sit
 // well inside the float range), each real column's slab as double-float
-// scaled by its largest power of two; the slab's partial sums (renormalised
-// double-float) are flushed into FP64 accumulators with that power of two.
-// About 15 FP32 instructions per multiply-add against one FP64 instruction at
-// 1/64 of the rate.
+// scaled by its largest power of two; the slab's partial sums (Dot2) are flushed
+// into FP64 accumulators with that power of two.  12 FP32 instructions per
+// multiply-add against one FP64 instruction at 1/64 of the rate.
 constexpr int AWD_K = 32;
-__global__ void __launch_bounds__(256) k_apply_w_df(const double *__restrict__ Wp, const double *__restrict__ Wm,
-                                                    int trans, int nt, int an, int mlo, int mhi,
-                                                    const double2 *__restrict__ in, int64_t is, int iw, int i_mlo,
-                                                    double2 *__restrict__ out, int64_t os, int ow, int o_mlo,
-                                                    int nb) {
-  const int par = blockIdx.z;
+__global__ void __launch_bounds__(256) k_apply_w_df(const double *__restrict__ Wp, const double *__restrict__ Wm, int trans,
+                                          int nt, int an, const __grid_constant__ WItems items, int64_t is, int iw,
+                                          int i_mlo, int64_t os, int ow, int o_mlo, int nb) {
+  const int par = blockIdx.z & 1, item = blockIdx.z >> 1;
+  const int mlo = items.mlo[item], mhi = items.mhi[item];
+  const double2 *__restrict__ in = items.in[item];
+  double2 *__restrict__ out = items.out[item];
   const int m_first = ((mlo + an) & 1) == par ? mlo : mlo + 1;
   if (m_first > mhi) return;
   const int nmp = (mhi - m_first) / 2 + 1;  // m's of this parity
@@ -779,7 +804,7 @@ __global__ void __launch_bounds__(256) k_apply_w_df(const double *__restrict__ W
       sB[kk][cc] = df_split(*reinterpret_cast<const double *>(&sB[kk][cc]), sBe[cc]);
     }
     __syncthreads();
-    float2 sum[4][4];
+    float2 sum[4][4];  // Dot2 sums (s, c)
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -794,7 +819,7 @@ __global__ void __launch_bounds__(256) k_apply_w_df(const double *__restrict__ W
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) sum[i][j] = df_add_norm(sum[i][j], df_mul(x[i], y[j]));
+        for (int j = 0; j < 4; ++j) dot2_mac(sum[i][j].x, sum[i][j].y, x[i], y[j].x, y[j].y);
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -819,25 +844,42 @@ __global__ void __launch_bounds__(256) k_apply_w_df(const double *__restrict__ W
   }
 }
 
-RcArgs rc_args(const WignerTable &tb, int n, int mlo, int lmin, const double2 *w, double wscale, bool wconj,
-               int nb) {
+RcArgs rc_args(const WignerTable &tb, double wscale, bool wconj, int nb) {
   RcArgs a{};
   a.bl = tb.bl;
   a.nt = tb.nt;
   a.an = tb.an;
   a.tmlo = tb.mlo;
-  a.n = n;
   a.coff = tb.d_coff;
   a.ck = tb.ck;
   a.ck_e = tb.ck_e;
   a.uq = tb.uq;
-  a.mlo = mlo;
-  a.lmin = lmin;
-  a.w = w;
+  a.rec = tb.rec;
+  a.roff = tb.d_roff;
   a.wscale = wscale;
   a.wconj = wconj ? 1 : 0;
   a.nb = nb;
+  a.lmin = tb.bl;
   return a;
+}
+
+// The parts of one problem: n > 0 reads table row m, n < 0 row -m, n = 0 both.
+template <class A>
+std::vector<RcPart> parts_of(const A &p, const double2 *src, double2 *dst) {
+  RcPart P{};
+  P.mlo = p.mlo;
+  P.mhi = p.mhi;
+  P.lmin = p.lmin;
+  P.w = p.w;
+  P.src = src;
+  P.dst = dst;
+  P.neg = p.n < 0 ? 1 : 0;
+  if (p.n != 0 || p.mlo >= 0) return {P};
+  RcPart N = P;
+  P.mlo = 0;
+  N.mhi = std::min(p.mhi, -1);
+  N.neg = 1;
+  return {P, N};
 }
 
 // algorithmic work of one launch, as the stored path counts it (one complex x
@@ -852,24 +894,28 @@ void rc_work(const WignerTable &tb, int mlo, int mhi, int lmin, int nb, double *
   *bytes = 16.0 * nb * (double)(mhi - mlo + 1) * (tb.nt + tb.bl);
 }
 
-void apply_w(const WignerTable &tb, bool trans, int mlo, int mhi, const double2 *in, int64_t is, int iw, int i_mlo,
-             double2 *out, int64_t os, int ow, int o_mlo, int nb, cudaStream_t st) {
-  const int nm = mhi - mlo + 1;
+void apply_w(const WignerTable &tb, bool trans, const WItems &items, int64_t is, int iw, int i_mlo, int64_t os, int ow,
+             int o_mlo, int nb, cudaStream_t st) {
+  int nm = 0, nmtot = 0;
+  for (int i = 0; i < items.n; ++i) {
+    nm = std::max(nm, items.mhi[i] - items.mlo[i] + 1);
+    nmtot += items.mhi[i] - items.mlo[i] + 1;
+  }
   const int ncols = 2 * ((nm + 1) / 2) * nb;
-  KTimer kt(KC_QUAD, st, 2.0 * tb.nt * (double)tb.nt * nm * nb * 2.0, 16.0 * nb * (double)nm * tb.nt * 2.0);
-  dim3 grid(ceil_div(ncols, AW_T), ceil_div(tb.nt, AW_T), 2);
+  KTimer kt(KC_QUAD, st, 2.0 * tb.nt * (double)tb.nt * nmtot * nb * 2.0, 16.0 * nb * (double)nmtot * tb.nt * 2.0);
+  dim3 grid(ceil_div(ncols, AW_T), ceil_div(tb.nt, AW_T), 2 * items.n);
   if (t_precision == 1)  // split precision: double-float multiply-adds
-    k_apply_w_df<<<grid, 256, 0, st>>>(tb.W[0], tb.W[1], trans ? 1 : 0, tb.nt, tb.an, mlo, mhi, in, is, iw, i_mlo,
-                                       out, os, ow, o_mlo, nb);
+    k_apply_w_df<<<grid, 256, 0, st>>>(tb.W[0], tb.W[1], trans ? 1 : 0, tb.nt, tb.an, items, is, iw, i_mlo, os, ow,
+                                       o_mlo, nb);
   else
-    k_apply_w<<<grid, 256, 0, st>>>(tb.W[0], tb.W[1], trans ? 1 : 0, tb.nt, tb.an, mlo, mhi, in, is, iw, i_mlo,
-                                    out, os, ow, o_mlo, nb);
+    k_apply_w<<<grid, 256, 0, st>>>(tb.W[0], tb.W[1], trans ? 1 : 0, tb.nt, tb.an, items, is, iw, i_mlo, os, ow,
+                                    o_mlo, nb);
   S2G_LAUNCHED();
 }
 
 template <int NBT>
 void launch_l2t(const RcArgs &a, int nm, cudaStream_t st) {
-  dim3 grid(nm, ceil_div(a.nt, kRcT), ceil_div(a.nb, NBT));
+  dim3 grid(nm, ceil_div(a.nt, kRcT), ceil_div(a.nb, a.mpc));
   k_rc_l2t<NBT><<<grid, kRcT, 0, st>>>(a);
   S2G_LAUNCHED();
 }
@@ -882,14 +928,14 @@ void launch_t2l(const RcArgs &a, int nm, int maxseg, cudaStream_t st) {
     return true;
   }();
   (void)attr;
-  dim3 grid(nm, maxseg, ceil_div(a.nb, NBT));
+  dim3 grid(nm, maxseg, ceil_div(a.nb, a.mpc));
   k_rc_t2l<NBT><<<grid, kRcT, smem, st>>>(a);
   S2G_LAUNCHED();
 }
 
 template <int NBT>
 void launch_l2t_df(const RcArgs &a, int nm, cudaStream_t st) {
-  dim3 grid(nm, ceil_div(a.nt, kRcT), ceil_div(a.nb, NBT));
+  dim3 grid(nm, ceil_div(a.nt, kRcT), ceil_div(a.nb, a.mpc));
   k_rc_l2t_df<NBT><<<grid, kRcT, 0, st>>>(a);
   S2G_LAUNCHED();
 }
@@ -902,121 +948,195 @@ void launch_t2l_df(const RcArgs &a, int nm, int maxseg, cudaStream_t st) {
     return true;
   }();
   (void)attr;
-  dim3 grid(nm, maxseg, ceil_div(a.nb, NBT));
+  dim3 grid(nm, maxseg, ceil_div(a.nb, a.mpc));
   k_rc_t2l_df<NBT><<<grid, kRcT, smem, st>>>(a);
   S2G_LAUNCHED();
 }
 
 }  // namespace
 
-void contract_l2t_rc(const L2T &p, cudaStream_t st) {
+namespace {
+void run_l2t(const RcArgs &a, int nm, int nbt, cudaStream_t st) {
+  const bool df = t_precision == 1;  // split precision: the double-float kernels (same results to about 1e-13)
+  switch (nbt) {
+    case 8: df ? launch_l2t_df<8>(a, nm, st) : launch_l2t<8>(a, nm, st); break;
+    case 4: df ? launch_l2t_df<4>(a, nm, st) : launch_l2t<4>(a, nm, st); break;
+    case 2: df ? launch_l2t_df<2>(a, nm, st) : launch_l2t<2>(a, nm, st); break;
+    default: df ? launch_l2t_df<1>(a, nm, st) : launch_l2t<1>(a, nm, st); break;
+  }
+}
+void run_t2l(const RcArgs &a, int nm, int maxseg, int nbt, cudaStream_t st) {
+  const bool df = t_precision == 1;
+  switch (nbt) {
+    case 16: df ? launch_t2l_df<16>(a, nm, maxseg, st) : launch_t2l<16>(a, nm, maxseg, st); break;
+    case 8: df ? launch_t2l_df<8>(a, nm, maxseg, st) : launch_t2l<8>(a, nm, maxseg, st); break;
+    case 4: df ? launch_t2l_df<4>(a, nm, maxseg, st) : launch_t2l<4>(a, nm, maxseg, st); break;
+    case 2: df ? launch_t2l_df<2>(a, nm, maxseg, st) : launch_t2l<2>(a, nm, maxseg, st); break;
+    default: df ? launch_t2l_df<1>(a, nm, maxseg, st) : launch_t2l<1>(a, nm, maxseg, st); break;
+  }
+}
+
+// Launches over up to kRcParts parts each.  Columns per CTA (parts x maps): the
+// largest power of two up to maxcols that parts and batch fill, or the autotuned
+// choice of maps per CTA.
+// mincols: a batch takes at least so many (the t -> l kernel sums one column in
+// another order than several).
+template <class RUN>
+void launch_parts(RcArgs a, const std::vector<RcPart> &parts, const WignerTable &tb, int family, int mincols,
+                  int maxcols, cudaStream_t st, RUN &&run) {
+  for (size_t i = 0; i < parts.size(); i += kRcParts) {
+    a.np = (int)std::min<size_t>(kRcParts, parts.size() - i);
+    a.lmin = tb.bl;
+    double fl = 0, by = 0;
+    for (int p = 0; p < a.np; ++p) {
+      a.part[p] = parts[i + p];
+      a.lmin = std::min(a.lmin, a.part[p].lmin);
+      if (timing_enabled()) {
+        double f1 = 0, b1 = 0;
+        rc_work(tb, a.part[p].mlo, a.part[p].mhi, a.part[p].lmin, a.nb, &f1, &b1);
+        fl += f1;
+        by += b1;
+      }
+    }
+    const int np2 = a.np > 2 ? 4 : a.np;
+    const int c0 = a.nb > 1 && np2 < mincols ? 1 : 0;  // log2 of the fewest maps per CTA
+    int ncand = 1;
+    while ((2 << (c0 + ncand - 1)) <= a.nb && np2 << (c0 + ncand) <= maxcols) ++ncand;
+    const auto go = [&](int c) {
+      a.mpc = 1 << (c0 + c);
+      run(a, np2 << (c0 + c));
+    };
+    const int c = tuned(family, tune_bucket(tb.bl), tune_bucket(a.nb), (t_precision == 1 ? 1 : 0) + 2 * (np2 / 2),
+                        ncand, ncand - 1, st, go);
+    KTimer kt(KC_RECOMPUTE, st, fl, by);
+    go(c);
+  }
+}
+
+bool same_form(const L2T &p, const L2T &q) {
+  return p.tb == q.tb && p.use_q == q.use_q && p.xs == q.xs && p.x_half == q.x_half && p.wscale == q.wscale &&
+         p.wconj == q.wconj && p.os == q.os && p.ow == q.ow && p.omlo == q.omlo && p.nb == q.nb;
+}
+bool same_form(const T2L &p, const T2L &q) {
+  return p.tb == q.tb && p.use_q == q.use_q && p.is == q.is && p.iw == q.iw && p.imlo == q.imlo &&
+         p.wscale == q.wscale && p.wconj == q.wconj && p.ys == q.ys && p.nb == q.nb;
+}
+
+// Quadrature of n problems, as many of one m range as a pass takes.  FP64 mode: on
+// the tensor cores (the FP64 kernel competes with the recursion for the FP64 pipe).
+// Split precision: there from band-limit 513; up to 512 by the double-float kernel.
+// That one takes twice the time alone (32 maps of 64 <= L <= 320, one by one: 15.7
+// against 8.3 ms), but it shares the GPU with the other maps of a multi-map call,
+// which the tensor-core kernel's shared memory does not (20.9 against 21.8 ms).
+constexpr int kQuadDfMaxBl = 512;
+template <class A, class F>
+void quadrature(const A *p, int n, bool trans, F &&io, int64_t is, int iw, int i_mlo, int64_t os, int ow, int o_mlo,
+                cudaStream_t st) {
+  const WignerTable &tb = *p[0].tb;
+  for (int i0 = 0; i0 < n;) {
+    QuadIO q[kMaxParts];
+    int k = 0;
+    for (; k < kMaxParts && i0 + k < n && p[i0 + k].mlo == p[i0].mlo && p[i0 + k].mhi == p[i0].mhi; ++k)
+      io(i0 + k, &q[k].in, &q[k].out);
+    const bool tensor = t_precision == 0 || tb.bl > kQuadDfMaxBl;
+    if (!tensor || !quadrature_mixed(tb, trans, q, k, p[i0].mlo, p[i0].mhi, is, iw, i_mlo, os, ow, o_mlo, p[0].nb, st)) {
+      WItems w{};
+      w.n = k;
+      for (int i = 0; i < k; ++i) {
+        w.in[i] = q[i].in;
+        w.out[i] = q[i].out;
+        w.mlo[i] = p[i0].mlo;
+        w.mhi[i] = p[i0].mhi;
+      }
+      apply_w(tb, trans, w, is, iw, i_mlo, os, ow, o_mlo, p[0].nb, st);
+    }
+    i0 += k;
+  }
+}
+
+void l2t_rc(const L2T *v, int n, cudaStream_t st) {
+  const L2T &p = v[0];
   const WignerTable &tb = *p.tb;
-  const int nm = p.mhi - p.mlo + 1;
-  RcArgs a = rc_args(tb, p.n, p.mlo, p.lmin, p.w, p.wscale, p.wconj, p.nb);
-  a.src = p.x;
+  RcArgs a = rc_args(tb, p.wscale, p.wconj, p.nb);
   a.ss = p.xs;
   a.x_half = p.x_half ? 1 : 0;
-  // Q^T x = W^T (D x): D x into a scratch of the output's layout, then W^T
-  double2 *tmp = nullptr;
-  if (p.use_q) {
-    S2G_CUDA(cudaMallocAsync((void **)&tmp, sizeof(double2) * (size_t)p.nb * tb.nt * p.ow, st));
-    a.dst = tmp;
-    a.ds = (int64_t)tb.nt * p.ow;
-  } else {
-    a.dst = p.out;
-    a.ds = p.os;
-  }
   a.dw = p.ow;
   a.d_mlo = p.omlo;
-  {
-    double fl = 0, by = 0;
-    if (timing_enabled()) rc_work(tb, p.mlo, p.mhi, p.lmin, p.nb, &fl, &by);
-    // maps per CTA: the largest of 1/2/4/8 the batch fills, or the autotuned choice
-    // split precision: the double-float kernels (same results to about 1e-13)
-    const bool df = t_precision == 1;
-    const auto run = [&](int nbc) {
-      if (df) {
-        switch (nbc) {
-          case 8: launch_l2t_df<8>(a, nm, st); break;
-          case 4: launch_l2t_df<4>(a, nm, st); break;
-          case 2: launch_l2t_df<2>(a, nm, st); break;
-          default: launch_l2t_df<1>(a, nm, st); break;
-        }
-        return;
-      }
-      switch (nbc) {
-        case 8: launch_l2t<8>(a, nm, st); break;
-        case 4: launch_l2t<4>(a, nm, st); break;
-        case 2: launch_l2t<2>(a, nm, st); break;
-        default: launch_l2t<1>(a, nm, st); break;
-      }
-    };
-    static const int kCand[4] = {1, 2, 4, 8};
-    const int ncand = p.nb >= 8 ? 4 : (p.nb >= 4 ? 3 : (p.nb >= 2 ? 2 : 1));
-    const int c = tuned(TF_RC_L2T, tune_bucket(tb.bl), tune_bucket(p.nb), df ? 1 : 0, ncand, ncand - 1, st,
-                        [&](int i) { run(kCand[i]); });
-    KTimer kt(KC_RECOMPUTE, st, fl, by);
-    run(kCand[c]);
-  }
+  // Q^T x = W^T (D x): D x into scratch of the output's layout, then W^T
+  double2 *tmp = nullptr;
+  const int64_t one = (int64_t)p.nb * tb.nt * p.ow;
+  if (p.use_q) S2G_CUDA(cudaMallocAsync((void **)&tmp, sizeof(double2) * (size_t)(one * n), st));
+  a.ds = p.use_q ? (int64_t)tb.nt * p.ow : p.os;
+  std::vector<RcPart> parts;
+  for (int i = 0; i < n; ++i)
+    for (const RcPart &q : parts_of(v[i], v[i].x, p.use_q ? tmp + i * one : v[i].out)) parts.push_back(q);
+  launch_parts(a, parts, tb, TF_RC_L2T, 1, 8, st, [&](const RcArgs &x, int nbt) { run_l2t(x, tb.nm, nbt, st); });
   if (p.use_q) {
-    apply_w(tb, true, p.mlo, p.mhi, tmp, (int64_t)tb.nt * p.ow, p.ow, p.omlo, p.out, p.os, p.ow, p.omlo, p.nb, st);
+    quadrature(v, n, true, [&](int i, const double2 **in, double2 **out) {
+      *in = tmp + i * one;
+      *out = v[i].out;
+    }, a.ds, p.ow, p.omlo, p.os, p.ow, p.omlo, st);
     cudaFreeAsync(tmp, st);
   }
 }
 
-void contract_t2l_rc(const T2L &p, cudaStream_t st) {
+void t2l_rc(const T2L *v, int n, cudaStream_t st) {
+  const T2L &p = v[0];
   const WignerTable &tb = *p.tb;
-  const int nm = p.mhi - p.mlo + 1;
-  RcArgs a = rc_args(tb, p.n, p.mlo, p.lmin, p.w, p.wscale, p.wconj, p.nb);
+  RcArgs a = rc_args(tb, p.wscale, p.wconj, p.nb);
   // Q in = D^T (W in): the quadrature on the spectra first
   double2 *tmp = nullptr;
+  const int64_t one = (int64_t)p.nb * tb.nt * p.iw;
+  a.ss = p.use_q ? (int64_t)tb.nt * p.iw : p.is;
   if (p.use_q) {
-    S2G_CUDA(cudaMallocAsync((void **)&tmp, sizeof(double2) * (size_t)p.nb * tb.nt * p.iw, st));
-    apply_w(tb, false, p.mlo, p.mhi, p.in, p.is, p.iw, p.imlo, tmp, (int64_t)tb.nt * p.iw, p.iw, p.imlo, p.nb, st);
-    a.src = tmp;
-    a.ss = (int64_t)tb.nt * p.iw;
-  } else {
-    a.src = p.in;
-    a.ss = p.is;
+    S2G_CUDA(cudaMallocAsync((void **)&tmp, sizeof(double2) * (size_t)(one * n), st));
+    quadrature(v, n, false, [&](int i, const double2 **in, double2 **out) {
+      *in = v[i].in;
+      *out = tmp + i * one;
+    }, p.is, p.iw, p.imlo, a.ss, p.iw, p.imlo, st);
   }
   a.sw = p.iw;
   a.s_mlo = p.imlo;
-  a.dst = p.y;
   a.ds = p.ys;
   int maxseg = 1;
-  for (int m = p.mlo; m <= p.mhi; ++m) maxseg = std::max(maxseg, tb.nseg(m < 0 ? -m : m));
-  {
-    double fl = 0, by = 0;
-    if (timing_enabled()) rc_work(tb, p.mlo, p.mhi, p.lmin, p.nb, &fl, &by);
-    // maps per CTA: the largest of 1/2/4/8/16 the batch fills, or the autotuned choice
-    const bool df = t_precision == 1;  // split precision: the double-float kernels
-    const auto run = [&](int nbc) {
-      if (df) {
-        switch (nbc) {
-          case 16: launch_t2l_df<16>(a, nm, maxseg, st); break;
-          case 8: launch_t2l_df<8>(a, nm, maxseg, st); break;
-          case 4: launch_t2l_df<4>(a, nm, maxseg, st); break;
-          case 2: launch_t2l_df<2>(a, nm, maxseg, st); break;
-          default: launch_t2l_df<1>(a, nm, maxseg, st); break;
-        }
-        return;
-      }
-      switch (nbc) {
-        case 16: launch_t2l<16>(a, nm, maxseg, st); break;
-        case 8: launch_t2l<8>(a, nm, maxseg, st); break;
-        case 4: launch_t2l<4>(a, nm, maxseg, st); break;
-        case 2: launch_t2l<2>(a, nm, maxseg, st); break;
-        default: launch_t2l<1>(a, nm, maxseg, st); break;
-      }
-    };
-    static const int kCand[5] = {1, 2, 4, 8, 16};
-    const int ncand = p.nb >= 16 ? 5 : (p.nb >= 8 ? 4 : (p.nb >= 4 ? 3 : (p.nb >= 2 ? 2 : 1)));
-    const int c = tuned(TF_RC_T2L, tune_bucket(tb.bl), tune_bucket(p.nb), df ? 1 : 0, ncand, ncand - 1, st,
-                        [&](int i) { run(kCand[i]); });
-    KTimer kt(KC_RECOMPUTE, st, fl, by);
-    run(kCand[c]);
-  }
+  for (int m = 0; m < tb.bl; ++m) maxseg = std::max(maxseg, tb.nseg(m));
+  std::vector<RcPart> parts;
+  for (int i = 0; i < n; ++i)
+    for (const RcPart &q : parts_of(v[i], p.use_q ? tmp + i * one : v[i].in, v[i].y)) parts.push_back(q);
+  launch_parts(a, parts, tb, TF_RC_T2L, 2, 16, st,
+               [&](const RcArgs &x, int nbt) { run_t2l(x, tb.nm, maxseg, nbt, st); });
   if (tmp) cudaFreeAsync(tmp, st);
+}
+
+// problems of one form in shared launches, in order
+template <class A, class F>
+void by_form(const A *p, int n, F &&f) {
+  std::vector<A> same;
+  for (int i = 0; i < n; ++i) {
+    if (!same.empty() && !same_form(same[0], p[i])) {
+      f(same.data(), (int)same.size());
+      same.clear();
+    }
+    if (p[i].nb > 0 && p[i].mhi >= p[i].mlo) same.push_back(p[i]);
+  }
+  if (!same.empty()) f(same.data(), (int)same.size());
+}
+}  // namespace
+
+RcRec *build_rec(int bl, int an, int mlo, int nm, const int64_t *d_roff, int64_t n) {
+  RcRec *rec = nullptr;
+  S2G_CUDA(cudaMalloc(&rec, sizeof(RcRec) * (size_t)(n > 0 ? n : 1)));
+  const int maxseg = ceil_div(bl, kSeg);
+  k_rc_rec<<<ceil_div((int64_t)nm * maxseg, 128), 128>>>(rec, d_roff, bl, an, mlo, nm, maxseg);
+  S2G_LAUNCHED();
+  return rec;
+}
+
+void contract_l2t_rc(const L2T *p, int n, cudaStream_t st) {
+  by_form(p, n, [&](const L2T *v, int k) { l2t_rc(v, k, st); });
+}
+void contract_t2l_rc(const T2L *p, int n, cudaStream_t st) {
+  by_form(p, n, [&](const T2L *v, int k) { t2l_rc(v, k, st); });
 }
 
 }  // namespace s2g
