@@ -335,7 +335,7 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_ring_forward(const __grid_c
   extern __shared__ longlong2 buf[];
   __shared__ int s_mx;
   const int job = job_of(grp, blockIdx.x), blk = blockIdx.x - grp.first[job];
-  const RingArgs &a = grp.a[job];
+  const RingArgs a = grp.a[job];  // by value: read once from the parameters
   const int K = a.K, P = a.P, logP = a.logP;
   const int r0 = REAL ? 2 * blk : blk;
   const bool has1 = REAL && (r0 + 1 < a.nrings);
@@ -395,7 +395,7 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_ring_inverse(const __grid_c
   extern __shared__ longlong2 buf[];
   __shared__ int s_mx;
   const int job = job_of(grp, blockIdx.x), blk = blockIdx.x - grp.first[job];
-  const RingArgs &a = grp.a[job];
+  const RingArgs a = grp.a[job];  // by value: read once from the parameters
   constexpr int BITS = REAL ? 60 : 61;  // A + i B of two rings
   const int K = a.K, P = a.P, logP = a.logP, bl = a.bl;
   const int r0 = REAL ? 2 * blk : blk;
@@ -489,7 +489,7 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_ring_inverse_gamma(const __
   cg::cluster_group cl = cg::this_cluster();
   const int k = (int)cl.block_rank();
   const int job = job_of(grp, blockIdx.x / NN), r = blockIdx.x / NN - grp.first[job];
-  const GammaItem &gf = grp.it[job];
+  const GammaItem gf = grp.it[job];  // by value: read once from the parameters
   const RingArgs &a = gf.a;
   const int b = r / gf.nt, t = r - b * gf.nt;
   const int K = a.K, P = a.P, logP = a.logP, bl = a.bl;
@@ -579,7 +579,7 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_gamma_ring_forward(const __
   cg::cluster_group cl = cg::this_cluster();
   const int k = (int)cl.block_rank();
   const int job = job_of(grp, blockIdx.x / NN), r = blockIdx.x / NN - grp.first[job];
-  const GammaItem &gf = grp.it[job];
+  const GammaItem gf = grp.it[job];  // by value: read once from the parameters
   const RingArgs &a = gf.a;
   const int b = r / gf.nt, t = r - b * gf.nt;
   const int K = a.K, P = a.P, logP = a.logP;
@@ -674,20 +674,31 @@ RingArgs ring_args(const RingFFT &rf, int bl, int nrings) {
 int ring_threads(int P) { return std::min(kRingThreads, std::max(32, P / 4)); }
 size_t ring_smem(int P) { return sizeof(longlong2) * (size_t)P; }
 
-// Shared memory of the ring kernels: one P-point buffer of 16-byte values,
-// with a carveout just large enough for the resident buffers (three at P =
-// 4096), so that the rest of the SM's L1 keeps the twiddles.  Set when a
-// kernel's buffer size changes.
-void ring_smem_attrs(const void *kernel, size_t smem) {
+// Shared memory of the ring kernels: one P-point buffer of 16-byte values, and
+// the smallest carveout that holds the CTAs an SM's registers allow (3 of 256
+// threads at 80 registers; with the 1 KB the system takes per CTA and the static
+// arrays): 164 of 228 KB would not hold three at P = 4096, 196 does and leaves
+// the rest to the L1.  Room for only three CTAs whatever their size kept the
+// small rings' CTAs of 32 to 128 threads from filling the SM: 64 maps at
+// band-limit 128 took 1.19 ms in the ring kernels and take 0.80, at 48 0.34 and
+// 0.21; band-limit 1024 is unchanged.  Set when a kernel's buffer size changes.
+void ring_smem_attrs(const void *kernel, int P) {
+  const size_t smem = ring_smem(P);
+  const int ctas = std::min(32, 3 * kRingThreads / ring_threads(P));
   static std::mutex mu;
   static std::map<const void *, size_t> set;
   std::lock_guard<std::mutex> lk(mu);
   size_t &cur = set[kernel];
   if (cur == smem) return;
   if (smem > 48 * 1024) S2G_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  constexpr double kMaxSmemPerSm = 228.0 * 1024.0;
-  const int pct = std::min(100, (int)std::ceil(100.0 * 3.0 * (double)(smem + 2048) / kMaxSmemPerSm) + 1);
-  S2G_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, pct));
+  constexpr int kSizes[] = {8, 16, 32, 64, 100, 132, 164, 196, 228};  // KB of shared memory an SM can set aside
+  int kb = 228;
+  for (int k : kSizes)
+    if (ctas * (smem + 1024 + 256) <= (size_t)k * 1024) {
+      kb = k;
+      break;
+    }
+  S2G_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100 * kb / 228));
   cur = smem;
 }
 
@@ -700,7 +711,7 @@ int largest_P(const RingGroup &g) {
 template <class KF>
 void launch_ring(KF kernel, const RingGroup &g, cudaStream_t st) {
   const int P = largest_P(g);
-  ring_smem_attrs((const void *)kernel, ring_smem(P));
+  ring_smem_attrs((const void *)kernel, P);
   kernel<<<g.first[g.n], ring_threads(P), ring_smem(P), st>>>(g);
   S2G_LAUNCHED();
 }
@@ -795,7 +806,7 @@ template <class KF>
 void launch_fused(KF kernel, const GammaFuse &gf, int nn, cudaStream_t st) {
   int P = 0;
   for (int q = 0; q < gf.n; ++q) P = std::max(P, gf.it[q].a.P);
-  ring_smem_attrs((const void *)kernel, ring_smem(P));
+  ring_smem_attrs((const void *)kernel, P);
   cudaLaunchAttribute at[1];
   const cudaLaunchConfig_t cfg = fused_config(gf.first[gf.n] * nn, nn, P, at, st);
   S2G_CUDA(cudaLaunchKernelEx(&cfg, kernel, gf));
@@ -823,7 +834,7 @@ bool cluster_fits(int nn, int P) {
   }
   bool ok = ring_smem(P) <= 227 * 1024;
   if (ok) {
-    ring_smem_attrs(kern, ring_smem(P));
+    ring_smem_attrs(kern, P);
     cudaLaunchAttribute at[1];
     const cudaLaunchConfig_t cfg = fused_config(nn, nn, P, at, nullptr);
     int nclusters = 0;
