@@ -182,48 +182,86 @@ __device__ __forceinline__ void dif4(longlong2 &a0, longlong2 &a1, longlong2 &a2
   a3 = fx_mulc4(fx_sub(b2, b3), w3);
 }
 
-// Bluestein core.  On entry (barrier not yet passed) the even bit-reversed
-// positions hold a_j (slot_brev(j), j < P/2; the second half of the sequence
-// is zero and is not read); on exit, after a barrier, slot_brev(k) holds y_k 2^S
-// for k < P/2, y the convolution times P, S the sum of the scalings.  Returns
-// the shift applied between the transforms.  P >= 8.
-//   stages: even log2 P: a 4-point pass of (a0, 0, a2, 0) with unit twiddles,
-//   odd: a copy (stage 1 of (a0, 0)); then radix-4 passes; the last of them,
-//   the kernel-spectrum product and the first inverse pass work on the same
-//   four elements and stay in registers; inverse radix-4 passes; a last pass
-//   with unit twiddles, even outputs only.
-__device__ int bluestein(longlong2 *buf, const RingArgs &a, int *s_mx) {
+// First pass of the Bluestein core, fused with the producer: value(j) is the
+// premultiplied a_j for j < P/2 (the second half of the padded sequence is zero
+// and is not stored), written to the even bit-reversed positions and their
+// neighbours.  Even log2 P: stages 1 and 2 of (a0, 0, a2, 0) with unit twiddles,
+// where a0 and a2 are the elements j and j + P/4; odd: a copy (stage 1 of
+// (a0, 0)).  Returns the magnitude bits of what it wrote.  With last_pass this
+// leaves two sweeps over the buffer and two barriers of a ring to its neighbours:
+// 64 maps at band-limit 128 0.800 -> 0.773 ms in the ring kernels, 32 at 256 1.385
+// -> 1.350; 8 at 1024 5.12 -> 5.07 (analysis), 5.18 -> 5.20 (synthesis).
+template <class V>
+__device__ __forceinline__ int first_pass(longlong2 *buf, int P, int logP, V value) {
+  int mx = 0;
+  if (logP & 1) {
+    for (int j = threadIdx.x; j < P / 2; j += blockDim.x) {
+      const int b = slot_brev(j, logP);
+      const longlong2 v = value(j);
+      buf[b] = v;
+      buf[b ^ 1] = v;
+      mx |= high_bits(v);
+    }
+  } else {
+    for (int j = threadIdx.x; j < P / 4; j += blockDim.x) {
+      const int b = slot_brev(j, logP);
+      const longlong2 a0 = value(j), a2 = value(j + P / 4), ia = fx_mul_i(a2);
+      const longlong2 v0 = fx_add(a0, a2), v2 = fx_sub(a0, a2), v1 = fx_sub(a0, ia), v3 = fx_add(a0, ia);
+      buf[b] = v0;
+      buf[b ^ 1] = v1;
+      buf[b ^ 2] = v2;
+      buf[b ^ 3] = v3;
+      mx |= high_bits(v0) | high_bits(v1) | high_bits(v2) | high_bits(v3);
+    }
+  }
+  return mx;
+}
+// Last pass, fused with the consumer: y_k for k < P/2 from the buffer that
+// bluestein() leaves (unit twiddles; the other half of the outputs is not formed).
+__device__ __forceinline__ longlong2 last_pass(const longlong2 *buf, int P, int logP, int k) {
+  if (logP & 1) {
+    const int b = slot_brev(k, logP);
+    return fx_add(buf[b], buf[b ^ 1]);
+  }
+  const int b = slot_brev(k & (P / 4 - 1), logP);
+  const longlong2 a0 = buf[b], a1 = buf[b ^ 1], a2 = buf[b ^ 2], a3 = buf[b ^ 3];
+  return k < P / 4 ? fx_add(fx_add(a0, a2), fx_add(a1, a3)) : fx_add(fx_sub(a0, a2), fx_mul_i(fx_sub(a1, a3)));
+}
+// the same in place, for consumers that read other CTAs' buffers:
+// slot_brev(k) <- f(k, y_k) for k < n
+template <class F>
+__device__ __forceinline__ void last_pass_in_place(longlong2 *buf, int P, int logP, int n, F f) {
+  if (logP & 1) {
+    for (int k = threadIdx.x; k < n; k += blockDim.x) {
+      const int b = slot_brev(k, logP);
+      buf[b] = f(k, fx_add(buf[b], buf[b ^ 1]));
+    }
+  } else {
+    for (int k = threadIdx.x; k < P / 4; k += blockDim.x) {
+      const int b = slot_brev(k, logP);
+      const longlong2 a0 = buf[b], a1 = buf[b ^ 1], a2 = buf[b ^ 2], a3 = buf[b ^ 3];
+      if (k < n) buf[b] = f(k, fx_add(fx_add(a0, a2), fx_add(a1, a3)));
+      if (k + P / 4 < n) buf[b ^ 2] = f(k + P / 4, fx_add(fx_sub(a0, a2), fx_mul_i(fx_sub(a1, a3))));
+    }
+  }
+}
+
+// Bluestein core between first_pass (barrier not yet passed; mx its result) and
+// last_pass (barrier passed): the buffer then holds y_k 2^S before the last pass,
+// y the convolution times P, S the sum of the scalings.  Returns the shift
+// applied between the transforms.  P >= 8.
+//   radix-4 passes; the last of them, the kernel-spectrum product and the first
+//   inverse pass work on the same four elements and stay in registers; inverse
+//   radix-4 passes.
+__device__ int bluestein(longlong2 *buf, const RingArgs &a, int *s_mx, int mx) {
   const int P = a.P, logP = a.logP;
   const int4 *__restrict__ tw = a.tw;
   const Swz z = swz_of(logP);
   const int h0 = logP & 1 ? 2 : 4;
-  int mx = 0;
+  int s = logP & 1 ? 2 : 3;
+  if (s + 1 < logP) mx = 0;  // a radix-4 pass follows and tracks its own outputs
   if (threadIdx.x == 0) *s_mx = 0;
   __syncthreads();
-  int s;
-  if (logP & 1) {
-    for (int i = threadIdx.x; i < P / 2; i += blockDim.x) {
-      const int b = swz(2 * i, z);
-      const longlong2 v = buf[b];
-      buf[b ^ 1] = v;
-      if (logP == 3) mx |= high_bits(v);
-    }
-    s = 2;
-  } else {
-    for (int i = threadIdx.x; i < P / 4; i += blockDim.x) {
-      const int b = swz(4 * i, z);
-      const longlong2 a0 = buf[b], a2 = buf[b ^ 2];
-      const longlong2 v0 = fx_add(a0, a2), v2 = fx_sub(a0, a2);
-      const longlong2 ia = fx_mul_i(a2), v1 = fx_sub(a0, ia), v3 = fx_add(a0, ia);
-      buf[b] = v0;
-      buf[b ^ 2] = v2;
-      buf[b ^ 1] = v1;
-      buf[b ^ 3] = v3;
-      if (logP == 4) mx |= high_bits(v0) | high_bits(v1) | high_bits(v2) | high_bits(v3);
-    }
-    s = 3;
-  }
-  if (logP > 4) __syncthreads();
   for (; s + 1 < logP; s += 2) {
     const int h = 1 << (s - 1);
     const int q1 = swz(h, z), q2 = swz(2 * h, z), q3 = swz(3 * h, z);
@@ -286,20 +324,6 @@ __device__ int bluestein(longlong2 *buf, const RingArgs &a, int *s_mx) {
     }
     __syncthreads();
   }
-  if (s == 2) {  // stages 2 and 1, unit twiddles, even outputs only
-    for (int i = threadIdx.x; i < P / 4; i += blockDim.x) {
-      const int b = swz(4 * i, z);
-      const longlong2 a0 = buf[b], a1 = buf[b ^ 1], a2 = buf[b ^ 2], a3 = buf[b ^ 3];
-      buf[b] = fx_add(fx_add(a0, a2), fx_add(a1, a3));
-      buf[b ^ 2] = fx_add(fx_sub(a0, a2), fx_mul_i(fx_sub(a1, a3)));
-    }
-  } else {
-    for (int i = threadIdx.x; i < P / 2; i += blockDim.x) {
-      const int b = swz(2 * i, z);
-      buf[b] = fx_add(buf[b], buf[b ^ 1]);
-    }
-  }
-  __syncthreads();
   return sh;
 }
 // a value q in the buffer of a block with exponent e, split to `bits` bits, is
@@ -350,7 +374,7 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_ring_forward(const __grid_c
   }
   em = block_max_int(em);
   const int e = fx_exp(em);
-  for (int j = threadIdx.x; j < P / 2; j += blockDim.x) {
+  const int mx = first_pass(buf, P, logP, [&](int j) {
     longlong2 v = make_longlong2(0, 0);
     if (j < K) {
       double2 x;
@@ -362,24 +386,24 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_ring_forward(const __grid_c
       }
       v = fx_mulc4(fx_split2<61>(x, e), ld_once(&a.chirp[j]));  // x_j conj(c_j)
     }
-    buf[slot_brev(j, logP)] = v;
-  }
-  const int sh = bluestein(buf, a, &s_mx);
+    return v;
+  });
+  const int sh = bluestein(buf, a, &s_mx, mx);
   const int k0 = core_exponent(a, e, 61, sh);
   if (!REAL) {
     double2 *out = a.spec_out + spec_base(a, r0);
     for (int c = threadIdx.x; c < a.sw; c += blockDim.x) {
       const int m = a.mlo + c;
       const int k = m < 0 ? m + K : m;
-      const longlong2 y = fx_mulc(buf[slot_brev(k, logP)], ld_once(&a.chirp[k]));
+      const longlong2 y = fx_mulc(last_pass(buf, P, logP, k), ld_once(&a.chirp[k]));
       out[c] = em == kExpNonFinite ? nan2() : fx_join2(y, k0);
     }
   } else {
     double2 *out0 = a.spec_out + spec_base(a, r0);
     for (int m = threadIdx.x; m < a.sw; m += blockDim.x) {
       const int km = m ? K - m : 0;
-      const longlong2 zm = fx_mulc(buf[slot_brev(m, logP)], ld_once(&a.chirp[m]));
-      const longlong2 zc = fx_conj(fx_mulc(buf[slot_brev(km, logP)], ld_once(&a.chirp[km])));
+      const longlong2 zm = fx_mulc(last_pass(buf, P, logP, m), ld_once(&a.chirp[m]));
+      const longlong2 zc = fx_conj(fx_mulc(last_pass(buf, P, logP, km), ld_once(&a.chirp[km])));
       // A = (Z_m + conj Z_{-m})/2,  B = (Z_m - conj Z_{-m})/(2i)
       out0[m] = em == kExpNonFinite ? nan2() : fx_join2(fx_add(zm, zc), k0 - 1);
       if (has1) {
@@ -408,7 +432,7 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_ring_inverse(const __grid_c
   }
   em = block_max_int(em);
   const int e = fx_exp(em);
-  for (int j = threadIdx.x; j < P / 2; j += blockDim.x) {
+  const int mx = first_pass(buf, P, logP, [&](int j) {
     longlong2 v = make_longlong2(0, 0);
     if (j < K) {
       const int m = (j < bl) ? j : j - K;  // frequency of DFT bin j
@@ -433,13 +457,13 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_ring_inverse(const __grid_c
       // inverse DFT = conj(forward(conj z)):  a_j = conj(z_j) conj(c_j)
       v = fx_conj(fx_mul4(v, ld_once(&a.chirp[j])));
     }
-    buf[slot_brev(j, logP)] = v;
-  }
-  const int sh = bluestein(buf, a, &s_mx);
+    return v;
+  });
+  const int sh = bluestein(buf, a, &s_mx, mx);
   const int k0 = core_exponent(a, e, BITS, sh);
   for (int p = threadIdx.x; p < K; p += blockDim.x) {
     // f_p = c_p conj(y_p)
-    const longlong2 y = fx_mul(fx_conj(buf[slot_brev(p, logP)]), ld_once(&a.chirp[p]));
+    const longlong2 y = fx_mul(fx_conj(last_pass(buf, P, logP, p)), ld_once(&a.chirp[p]));
     const double2 f = em == kExpNonFinite ? nan2() : fx_join2(y, k0);
     if (REAL) {
       ((double *)a.rings_out)[ring_base(a, r0) + p] = f.x;
@@ -500,7 +524,7 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_ring_inverse_gamma(const __
   for (int c = threadIdx.x; c < sw; c += blockDim.x) em = emax2(em, s0[c]);
   em = cluster_max_int(cl, &s_em, em, NN);
   const int e = fx_exp(em);
-  for (int j = threadIdx.x; j < P / 2; j += blockDim.x) {
+  const int mx = first_pass(buf, P, logP, [&](int j) {
     longlong2 v = make_longlong2(0, 0);
     if (j < K) {
       const int m = (j < bl) ? j : j - K;
@@ -511,14 +535,11 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_ring_inverse_gamma(const __
         v = fx_conj(fx_split2<61>(s0[-m], e));
       v = fx_conj(fx_mul4(v, ld_once(&a.chirp[j])));
     }
-    buf[slot_brev(j, logP)] = v;
-  }
-  const int sh = bluestein(buf, a, &s_mx);
+    return v;
+  });
+  const int sh = bluestein(buf, a, &s_mx, mx);
   // F_k(p) = c_p conj(y_p), in place (p -> brev(p) is one-to-one); components < 2^61.5
-  for (int p = threadIdx.x; p < K; p += blockDim.x) {
-    const int i = slot_brev(p, logP);
-    buf[i] = fx_mul(fx_conj(buf[i]), ld_once(&a.chirp[p]));
-  }
+  last_pass_in_place(buf, P, logP, K, [&](int p, longlong2 y) { return fx_mul(fx_conj(y), ld_once(&a.chirp[p])); });
   if (threadIdx.x == 0) s_k = core_exponent(a, e, 61, sh);
   cl.sync();
   // gamma slices of this CTA's share of the pixels
@@ -639,14 +660,16 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_gamma_ring_forward(const __
     for (int j = 0; j < NN; ++j) *cl.map_shared_rank(buf + i, j) = fx_mulc(acc[j], ch);
   }
   cl.sync();  // every component's buffer is complete
-  const int sh = bluestein(buf, a, &s_mx);
+  // in place: a thread reads only the slots that it writes
+  const int mx = first_pass(buf, P, logP, [&](int j) { return buf[slot_brev(j, logP)]; });
+  const int sh = bluestein(buf, a, &s_mx, mx);
   // split to 61 bits, over 4 in the gamma sums as after a scaled chirp, times 2^et
   const int k0 = core_exponent(a, e, 61, sh) + grp.et;
   double2 *out = gf.Gout + (int64_t)b * gf.gms + (int64_t)k * gf.gks + (int64_t)t * gf.W;
   for (int c = threadIdx.x; c < gf.W; c += blockDim.x) {
     const int m = c - (a.bl - 1);
     const int q = m < 0 ? m + K : m;
-    const longlong2 y = fx_mulc(buf[slot_brev(q, logP)], ld_once(&a.chirp[q]));
+    const longlong2 y = fx_mulc(last_pass(buf, P, logP, q), ld_once(&a.chirp[q]));
     out[c] = em == kExpNonFinite ? nan2() : fx_join2(y, k0);
   }
 }
