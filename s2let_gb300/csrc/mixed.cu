@@ -195,21 +195,31 @@ __device__ __forceinline__ long long fixed55(double v, int e) {
 // The eighth digit of a table value: what the seven leave of v 2^-e, in units
 // of 2^-55 (|digit| <= 64; with it the value is represented to 2^-56).
 __device__ __forceinline__ int eighth_digit(double v, int e) { return (int)(fixed55(v, e) - fixed48(v, e) * 128); }
-// Balanced digits of q 2^-55, |q| < 2^55, as bf16 patterns in the low halves
-// of out: adding 64 in every digit position but the first makes the base-128
-// digits of the sum the balanced ones plus 64; 2^23 + digit is read off the
-// float's bits, and subtracting 2^23 + 64 leaves the digit exactly.
-__device__ __forceinline__ void split_digits_int(long long q, uint32_t *out) {
-  q += 0x0001020408102040ll;  // 64 (1 + 2^7 + ... + 2^42)
-  const uint32_t lo = (uint32_t)q & 0xFFFFFFFu, hi = (uint32_t)(q >> 28);
-  // d_0 = q >> 49 in [-64, 64]: its field holds d_0 + 128 after the offset below
-  out[0] = __float_as_uint(__fsub_rn(__uint_as_float(0x4B000000u | ((hi >> 21) + 128u & 0xFFu)), 8388736.0f)) >> 16;
-#pragma unroll
-  for (int j = 1; j < kSmax; ++j) {
-    const uint32_t w = j < 4 ? hi : lo;
-    const int sh = j < 4 ? 21 - 7 * j : 49 - 7 * j;
-    out[j] = __float_as_uint(__fsub_rn(__uint_as_float(0x4B000000u | ((w >> sh) & 127u)), 8388672.0f)) >> 16;
-  }
+// Balanced base-128 digits d_0 .. d_(S-1) of q, |q| <= 2^(7S-1), plus 64, one
+// per byte: digit S-1-b in byte b of lo for b < 4, digit S-5-b in byte b of hi.
+// Adding 64 in every digit position makes the balanced digits the 7-bit fields
+// of the sum (the first is 8 bits wide: d_0 + 64 may be 128); each word's
+// fields move apart by a step of 14 bits to 16 and one of 7 to 8.
+template <int S>
+__device__ __forceinline__ void digit_bytes(long long q, uint32_t &lo, uint32_t &hi) {
+  constexpr long long kBias = S == kS ? 0x0001020408102040ll : 0x0081020408102040ll;
+  const unsigned long long u = (unsigned long long)(q + kBias);
+  const auto bytes = [](uint32_t x, uint32_t sel, uint32_t mask) {
+    const uint32_t t = (x & 0x3FFFu) | ((x << 2) & ~0x3FFFu);
+    return ((t & sel) | ((t << 1) & ~sel)) & mask;
+  };
+  lo = bytes((uint32_t)u & 0xFFFFFFFu, 0x007F007Fu, 0x7F7F7F7Fu);
+  hi = S == kS ? bytes((uint32_t)(u >> 28), 0x00FF007Fu, 0x00FF7F7Fu)
+               : bytes((uint32_t)(u >> 28), 0x007F007Fu, 0xFF7F7F7Fu);
+}
+
+// Two digits (bytes d + 64 of w, chosen by sel) as bf16: 0x4300 | x is 128 + x
+// for x < 128 and 256 for x = 128, all exact, so subtracting 192 leaves d.
+__device__ __forceinline__ uint32_t digits2_bf16(uint32_t w, uint32_t sel) {
+  const uint32_t v = __byte_perm(w, 0x43434343u, sel);
+  uint32_t r;
+  asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(v), "r"(0x43404340u));
+  return r;
 }
 
 struct TableRefM {
@@ -314,10 +324,37 @@ struct XArgs {
   int *eX;
 };
 
+// v, negated when n is odd
+__device__ __forceinline__ double flip_sign(double v, int n) { return double_of(bits_of(v) ^ ((uint64_t)n << 63)); }
+// FP64 paths that are rarely taken stay out of line: inlined, they were executed
+// speculatively and kept the FP64 unit busy (k_slice_x from coefficients 189 us
+// instead of 137 at L = 512, 32 maps).
+__device__ __noinline__ double mul_fp64(double x, double y) { return __dmul_rn(x, y); }
+// x y rounded to nearest, by a 64 x 64-bit integer product (the 64 bits below the
+// kept high half only move results within 2^-11 units in the last place of a
+// rounding boundary); zeros, subnormals, infinities, NaN and results near the
+// ends of the range go to the FP64 unit.
+__device__ __forceinline__ double mul_int(double x, double y) {
+  const uint64_t ux = bits_of(x), uy = bits_of(y);
+  const int ex = (int)(ux >> 52) & 0x7FF, ey = (int)(uy >> 52) & 0x7FF, e = ex + ey - 1023;
+  if ((unsigned)(ex - 1) >= 2046u || (unsigned)(ey - 1) >= 2046u || (unsigned)(e - 1) >= 2044u) return mul_fp64(x, y);
+  // significands with the leading bit at the top: product in [2^62, 2^64)
+  uint64_t p = __umul64hi((ux << 11) | (1ull << 63), (uy << 11) | (1ull << 63));
+  const int n = p >> 63 ? 0 : 1;
+  p <<= n;
+  // the leading bit and a rounding carry run into the exponent field
+  return double_of(((ux ^ uy) & (1ull << 63)) | (((uint64_t)(e - n) << 52) + (p >> 11) + ((p >> 10) & 1)));
+}
 __device__ __forceinline__ double2 weight_of(const double2 *w, double wscale, int wconj, int l) {
   double2 v = w ? w[l] : make_double2(1.0, 0.0);
   if (wconj) v.y = -v.y;
   return make_double2(v.x * wscale, v.y * wscale);
+}
+// (out of line for the same reason)
+__device__ __noinline__ double2 weighted_complex(double2 x, double2 w, double wscale, int wconj) {
+  if (wconj) w.y = -w.y;
+  const double2 v = make_double2(w.x * wscale, w.y * wscale);
+  return make_double2(x.x * v.x - x.y * v.y, x.x * v.y + x.y * v.x);
 }
 // x times the part's weight at degree l (x times wscale without a weight).  A
 // real or imaginary weight takes three FP64 products instead of the eight of a
@@ -344,7 +381,16 @@ __device__ __forceinline__ double2 weighted(const Part &P, double2 x, int l) {
 // load covers 64-byte runs, and records the largest exponent field of each
 // real and imaginary column.  Phase 2 writes the digit panels: 8 consecutive
 // lanes build one 128-byte panel row from 8 K values each.  The FP64 values
-// are read once and the panels written once.
+// are read once and the panels written once; columns without a map are left
+// alone (with one map and one part, seven of eight column pairs).
+//
+// What bounds it: integer instructions and the latency of the two phases, at
+// 3-4 CTAs per SM, not the bytes (50 % of the DRAM rate from spectra, 20 % from
+// coefficients, whose panels stay in L2).  One launch at L = 512, 32 maps:
+// from spectra 195 -> 159 us with the digits spread in integers (digit_bytes)
+// instead of peeled off a double-float; from coefficients 191 -> 137 us with the
+// weight products in integers (mul_int) as well, as the FP64 unit they kept
+// busy is shared by the SM.  64 registers: the fourth CTA is worth 10 %.
 constexpr int kMG = 4;
 constexpr int kSliceThreads = 256;
 constexpr int kNonFinite = 1 << 20;  // column exponent of a column that holds an infinity or a NaN
@@ -353,13 +399,19 @@ constexpr int kNonFinite = 1 << 20;  // column exponent of a column that holds a
 __host__ __device__ __forceinline__ int sv_idx(int k) { return k + (k >> 3); }
 
 template <int NC, int S>
-__global__ void __launch_bounds__(kSliceThreads, 3) k_slice_x(XArgs a) {
+__global__ void __launch_bounds__(kSliceThreads, 4) k_slice_x(XArgs a) {
   extern __shared__ double2 sv[];  // [kMG][a.kst]
   __shared__ int gl0[kMG], gnkc[kMG], gkc0[kMG], gls[kMG], gex[kMG][2];
   constexpr int PX = Cfg<NC, S>::kPanelX;
   const int cp = blockIdx.y, pm0 = blockIdx.x * kMG, c0 = 2 * cp;
   const int part = cp / a.mpp, b = a.b0 + cp % a.mpp;
-  const bool live = part < a.nparts && b < a.nb;
+  if (part >= a.nparts || b >= a.nb) {
+    // no map in these columns: their panels are never written and their sums
+    // never stored; ordinary exponents keep the epilogue on its straight path
+    if (threadIdx.x < 2 * kMG && pm0 + (int)threadIdx.x / 2 < a.nmp)
+      a.eX[(pm0 + threadIdx.x / 2) * NC + c0 + threadIdx.x % 2] = 0;
+    return;
+  }
   if (threadIdx.x < kMG) {
     const int pm = pm0 + threadIdx.x;
     int l0 = 0, nkc = 0, kc0 = 0, ls = 0;
@@ -371,7 +423,7 @@ __global__ void __launch_bounds__(kSliceThreads, 3) k_slice_x(XArgs a) {
         const int lst = g.l0 > a.lmin ? g.l0 : a.lmin;
         kc0 = lst >= a.bl ? g.nkc : (lst - g.l0) / kPK;
         // first degree with a value: below its part's lmin the column is zero
-        ls = live && a.part[part].lmin > g.l0 ? a.part[part].lmin : g.l0;
+        ls = a.part[part].lmin > g.l0 ? a.part[part].lmin : g.l0;
       }
     }
     gl0[threadIdx.x] = l0;
@@ -382,7 +434,7 @@ __global__ void __launch_bounds__(kSliceThreads, 3) k_slice_x(XArgs a) {
   }
   for (int i = threadIdx.x; i < kMG * a.kst; i += kSliceThreads) ((int4 *)sv)[i] = make_int4(0, 0, 0, 0);
   __syncthreads();
-  if (live) {
+  {
     const Part &P = a.part[part];
     const int mi = threadIdx.x % kMG;  // fixed per thread: kSliceThreads is a multiple of kMG
     const int pm = pm0 + mi, m = a.mlo + pm, am = m < 0 ? -m : m;
@@ -398,7 +450,10 @@ __global__ void __launch_bounds__(kSliceThreads, 3) k_slice_x(XArgs a) {
       const int l0 = gl0[mi], ls = gls[mi];
       const bool neg = P.x_half && m < 0;
       const int mm = neg ? -m : m;
-      for (int l1 = lb + threadIdx.x / kMG; l1 < a.bl; l1 += kU * kStep) {
+      // warp-uniform bounds: the weights travel by shuffles
+      static_assert(kU == kMG, "lane mi forms the scaled weight of step u = mi");
+      for (int lw = lb + (threadIdx.x & ~31) / kMG; lw < a.bl; lw += kU * kStep) {
+        const int l1 = lw + (threadIdx.x & 31) / kMG;
         double2 v[kU];
 #pragma unroll
         for (int u = 0; u < kU; ++u) {
@@ -406,16 +461,25 @@ __global__ void __launch_bounds__(kSliceThreads, 3) k_slice_x(XArgs a) {
           v[u] = make_double2(0.0, 0.0);
           if (has && l >= ls && l < a.bl) v[u] = P.src[(int64_t)b * P.ss + (int64_t)l * l + l + mm];
         }
+        double r = P.wscale;  // lane mi: the scaled weight of degree l1 + mi kStep
+        if (P.w && P.wkind != WKIND_COMPLEX && l1 + mi * kStep < a.bl) {
+          const double2 w = P.w[l1 + mi * kStep];
+          r = mul_int(P.wkind == WKIND_REAL ? w.x : flip_sign(w.y, P.wconj), r);
+        }
 #pragma unroll
         for (int u = 0; u < kU; ++u) {
           const int l = l1 + u * kStep;
+          const double ru = __shfl_sync(0xffffffffu, r, u, kMG);
           if (!has || l < ls || l >= a.bl) continue;
           double2 x = v[u];
-          if (neg) {
-            x.y = -x.y;
-            if (am & 1) x = make_double2(-x.x, -x.y);
-          }
-          x = weighted(P, x, l);
+          // sign changes as bit flips (a negation can cost an FP64 instruction)
+          if (neg) x = make_double2(flip_sign(x.x, am), flip_sign(x.y, am + 1));
+          if (P.w && P.wkind == WKIND_COMPLEX)
+            x = weighted_complex(x, P.w[l], P.wscale, P.wconj);
+          else if (P.w && P.wkind == WKIND_IMAG)  // x (i r)
+            x = make_double2(flip_sign(mul_int(x.y, ru), 1), mul_int(x.x, ru));
+          else
+            x = make_double2(mul_int(x.x, ru), mul_int(x.y, ru));
           col[sv_idx(l - l0)] = x;
           er = max(er, exp_field(x.x));
           ei = max(ei, exp_field(x.y));
@@ -474,29 +538,23 @@ __global__ void __launch_bounds__(kSliceThreads, 3) k_slice_x(XArgs a) {
 #pragma unroll 1
     for (int ri = 0; ri < 2; ++ri) {  // real part (column c0), then imaginary part (c0 + 1)
       uint32_t pk[S][4];
-      if (live) {
-        const int e = gex[mi][ri];
+      const int e = gex[mi][ri];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const double v = col[2 * sv_idx(kc * kPK + h * 8 + q) + ri];
-          uint32_t d[S];
-          if constexpr (S == kS)
-            split_digits_fp32<kS>(v, e, d);  // dfconv.h
-          else
-            split_digits_int(fixed55(v, e), d);
+      for (int q = 0; q < 4; ++q) {  // K values 2 q and 2 q + 1
+        uint32_t lo[2], hi[2];
 #pragma unroll
-          for (int j = 0; j < S; ++j) {
-            if (q & 1)
-              pk[j][q >> 1] |= d[j] << 16;
-            else
-              pk[j][q >> 1] = d[j];
-          }
+        for (int r = 0; r < 2; ++r) {
+          const double v = col[2 * sv_idx(kc * kPK + h * 8 + 2 * q + r) + ri];
+          digit_bytes<S>(S == kS ? fixed48(v, e) : fixed55(v, e), lo[r], hi[r]);
         }
-      } else {
+        // bytes of one digit of both values side by side, two digits per word
+        const uint32_t w[4] = {__byte_perm(lo[0], lo[1], 0x5140), __byte_perm(lo[0], lo[1], 0x7362),
+                               __byte_perm(hi[0], hi[1], 0x5140), __byte_perm(hi[0], hi[1], 0x7362)};
 #pragma unroll
-        for (int j = 0; j < S; ++j)
-#pragma unroll
-          for (int q = 0; q < 4; ++q) pk[j][q] = 0u;
+        for (int j = 0; j < S; ++j) {
+          const int y = S - 1 - j;  // byte position of digit j
+          pk[j][q] = digits2_bf16(w[y >> 1], y & 1 ? 0x4342 : 0x4140);
+        }
       }
 #pragma unroll
       for (int j = 0; j < S; ++j)
@@ -603,14 +661,7 @@ __device__ __forceinline__ void tc_fence_before() {
 // the contraction
 // ---------------------------------------------------------------------------
 
-// 8 digits (bytes d + 64 of two words) as bf16: 0x4300 | x is 128 + x for x <
-// 128 and 256 for x = 128, all exact, so subtracting 192 leaves d.
-__device__ __forceinline__ uint32_t digits2_bf16(uint32_t w, uint32_t sel) {
-  const uint32_t v = __byte_perm(w, 0x43434343u, sel);
-  uint32_t r;
-  asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(v), "r"(0x43404340u));
-  return r;
-}
+// 8 digits, bytes d + 64 of two words, as bf16
 __device__ __forceinline__ uint4 digits_bf16(uint32_t lo, uint32_t hi) {
   return make_uint4(digits2_bf16(lo, 0x4140), digits2_bf16(lo, 0x4342), digits2_bf16(hi, 0x4140),
                     digits2_bf16(hi, 0x4342));
