@@ -562,12 +562,15 @@ int s2let_gpu_synthesis_adjoint_px2wav_batch(void *f_wav, void *f_scal, const vo
  * FP32 storage (configurations that keep maps and wavelet coefficients in
  * single precision).  The batched device-pointer entry points above with
  * `float` maps, f_wav and f_scal (complex signals as interleaved float
- * pairs), the same strides in elements.  Inputs are widened to FP64 on the
- * device, the transforms run as in the FP64-storage path at the precision set
- * by s2let_gpu_set_precision, and outputs are rounded to FP32 (so the results
- * are the FP64-storage results rounded, about 6e-8 relative).  Only the used
- * part of each f_wav row is read or written.  Device scratch: the FP64 copies
- * of the batch.  Asynchronous on `stream`; returns the status.  No counterpart
+ * pairs; 4-byte alignment), the same strides in elements.  Inputs are widened
+ * to FP64 as the kernels read them, the transforms run as in the FP64-storage
+ * path at the precision set by s2let_gpu_set_precision, and outputs are rounded
+ * to FP32 as they are written (so the results are the FP64-storage results
+ * rounded, about 6e-8 relative).  Only the used part of each f_wav row is read
+ * or written.  FP64 copies of the batch are made in device scratch only where
+ * more kernels than the ring DFTs touch the pixels: more directions than the
+ * fused ring and gamma DFT takes, and the refined FP64 forward transform above
+ * band-limit 1024.  Asynchronous on `stream`; returns the status.  No counterpart
  * in the reference (its transforms take double arrays only).
  */
 int s2let_gpu_analysis_px2wav_real_batch_f32(float *f_wav, float *f_scal, const float *f, int nbatch,
@@ -588,8 +591,8 @@ int s2let_gpu_analysis_adjoint_wav2px_batch_f32(void *f, const void *f_wav, cons
 int s2let_gpu_synthesis_adjoint_px2wav_batch_f32(void *f_wav, void *f_scal, const void *f, int nbatch,
                                                  const s2let_parameters_t *parameters, void *stream);
 /* s2let_gpu_px2wav_multi / s2let_gpu_wav2px_multi with FP32 storage: every
- * map's f, f_wav and f_scal are float arrays (device pointers), widened into
- * FP64 batch scratch and rounded back, inside the CUDA graph when use_graph. */
+ * map's f, f_wav and f_scal are float arrays (device pointers), read and written
+ * as by the FP32 batches above, inside the CUDA graph when use_graph. */
 int s2let_gpu_px2wav_multi_f32(void *const *f_wav, void *const *f_scal, void *const *f,
                                const s2let_parameters_t *params, const int *real, int nmaps, int use_graph,
                                void *stream);

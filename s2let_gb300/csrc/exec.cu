@@ -364,10 +364,12 @@ struct Sht {
 };
 Sht sht_of(const WavPlan &P) { return Sht{P.L, P.s, P.ss, P.real, P.d_w + P.w_cl, P.rc(P.L)}; }
 
-// ring DFTs between nb maps (rings contiguous in each, maps stride apart) and
-// their contiguous spectra of width sw from m = mlo
-RingJob ring_job(const void *in, void *out, int K, int64_t mstride, int nt, int sw, int mlo, int nb, int bl) {
+// ring DFTs between nb maps (rings contiguous in each, maps stride apart; f32: of
+// floats) and their contiguous spectra of width sw from m = mlo
+RingJob ring_job(const void *in, void *out, int K, int64_t mstride, int nt, int sw, int mlo, int nb, int bl,
+                 bool f32 = false) {
   RingJob j;
+  j.f32 = f32;
   j.in = in;
   j.out = out;
   j.ring_stride = K;
@@ -382,14 +384,14 @@ RingJob ring_job(const void *in, void *out, int K, int64_t mstride, int nt, int 
 }
 
 // flm (nb x L^2, zero outside the computed range) <- forward transform of maps
-// (or the adjoint of the inverse)
+// (or the adjoint of the inverse); f32: the maps hold floats
 void sht_forward_once(const Sht &H, const void *f, int64_t fstride, double2 *flm, int nb, Scratch &S,
-                      bool adjoint_of_inverse) {
+                      bool adjoint_of_inverse, bool f32 = false) {
   const int L = H.L, s = H.s, K = grid_ring_len(L, H.ss), nt = grid_rings(L, H.ss);
   const bool real = H.real;
   const int sw = real ? L : 2 * L - 1, mlo = real ? 0 : -(L - 1);
   double2 *spec = S.get<double2>((int64_t)nb * nt * sw);
-  ring_forward_many({ring_job(f, spec, K, fstride, nt, sw, mlo, nb, L)}, H.ss, real, S.st);
+  ring_forward_many({ring_job(f, spec, K, fstride, nt, sw, mlo, nb, L, f32)}, H.ss, real, S.st);
   S2G_CUDA(cudaMemsetAsync(flm, 0, sizeof(double2) * nb * L * L, S.st));
   T2L a{};
   a.tb = &wigner_table(L, std::abs(s), H.ss, H.rc);
@@ -413,7 +415,7 @@ void sht_forward_once(const Sht &H, const void *f, int64_t fstride, double2 *flm
 
 // maps <- inverse transform (or adjoint of the forward) of flm
 void sht_inverse(const Sht &H, const double2 *flm, bool flm_half, void *f, int64_t fstride, int nb,
-                 Scratch &S, bool adjoint_of_forward) {
+                 Scratch &S, bool adjoint_of_forward, bool f32 = false) {
   const int L = H.L, s = H.s, K = grid_ring_len(L, H.ss), nt = grid_rings(L, H.ss);
   const bool real = H.real;
   const int sw = real ? L : 2 * L - 1, mlo = real ? 0 : -(L - 1);
@@ -438,7 +440,7 @@ void sht_inverse(const Sht &H, const double2 *flm, bool flm_half, void *f, int64
   a.omlo = mlo;
   a.nb = nb;
   contract_l2t(a, S.st);
-  ring_inverse_many({ring_job(spec, f, K, fstride, nt, sw, mlo, nb, L)}, H.ss, real, S.st);
+  ring_inverse_many({ring_job(spec, f, K, fstride, nt, sw, mlo, nb, L, f32)}, H.ss, real, S.st);
 }
 
 // Forward transform with one residual-refinement sweep (FP64 path, L above
@@ -451,11 +453,13 @@ void sht_inverse(const Sht &H, const double2 *flm, bool flm_half, void *f, int64
 // accuracy; for other maps F(f - I(F f)) vanishes in exact arithmetic and the
 // sweep changes nothing beyond rounding.
 constexpr int kRefineL = 1024;
+bool refines(int L, bool adjoint_of_inverse) { return !adjoint_of_inverse && t_precision == 0 && L > kRefineL; }
 
 void sht_forward(const Sht &H, const void *f, int64_t fstride, double2 *flm, int nb, Scratch &S,
-                 bool adjoint_of_inverse) {
-  sht_forward_once(H, f, fstride, flm, nb, S, adjoint_of_inverse);
-  if (adjoint_of_inverse || t_precision != 0 || H.L <= kRefineL || nb <= 0) return;
+                 bool adjoint_of_inverse, bool f32 = false) {
+  sht_forward_once(H, f, fstride, flm, nb, S, adjoint_of_inverse, f32);
+  if (!refines(H.L, adjoint_of_inverse) || nb <= 0) return;
+  S2G_REQUIRE(!f32, ERR_UNSUPPORTED, "residual refinement of FP32 maps");
   const int64_t npx = (int64_t)grid_rings(H.L, H.ss) * grid_ring_len(H.L, H.ss);
   const int64_t dd = H.real ? 1 : 2;  // doubles per sample
   const int64_t L2 = (int64_t)H.L * H.L;
@@ -637,7 +641,7 @@ struct RingJobs {
 
 // spectra and pixels of maps b0 .. b0 + nbg of one scale (G of that scale: [b][n][t][m])
 GammaJob gamma_job(const WavPlan &P, const Scale &sd, double2 *G, char *wav, size_t esz, int64_t wstride, int b0,
-                   int nbg) {
+                   int nbg, bool f32) {
   const int64_t W = 2 * sd.bl - 1, nt = P.nt(sd.bl), nn = (int64_t)sd.ns.size();
   GammaJob j;
   j.G = j.Gout = G + b0 * nn * nt * W;
@@ -645,17 +649,18 @@ GammaJob gamma_job(const WavPlan &P, const Scale &sd, double2 *G, char *wav, siz
   j.gks = nt * W;
   j.fw = wav + (size_t)sd.woff * esz + (size_t)b0 * wstride * esz;
   j.fms = wstride;
+  j.f32 = f32;
   j.nb = nbg;
   j.bl = sd.bl;
   return j;
 }
 // one slice per scale: rings against the contraction's spectra (real signals: m >= 0)
 RingJob slice_job(const WavPlan &P, const Scale &sd, double2 *G, char *wav, size_t esz, int64_t wstride, int nb,
-                  bool forward) {
+                  bool forward, bool f32) {
   const int W = 2 * sd.bl - 1, skip = P.real ? sd.bl - 1 : 0;
   void *px = wav + (size_t)sd.woff * esz;
   void *sp = G + skip;
-  RingJob j = ring_job(forward ? px : sp, forward ? sp : px, P.K(sd.bl), wstride, P.nt(sd.bl), W, 0, nb, sd.bl);
+  RingJob j = ring_job(forward ? px : sp, forward ? sp : px, P.K(sd.bl), wstride, P.nt(sd.bl), W, 0, nb, sd.bl, f32);
   j.sw = W - skip;
   j.mlo = P.real ? 0 : -(sd.bl - 1);
   return j;
@@ -663,10 +668,11 @@ RingJob slice_job(const WavPlan &P, const Scale &sd, double2 *G, char *wav, size
 
 // flm -> (f_wav, f_scal).  SPLIT_ANALYSIS: lm2wav.  SPLIT_SYNTH_ADJ: adjoint of wav2lm.
 void wav_split(const WavPlan &P, SplitMode mode, const double2 *flm, bool flm_half, void *f_wav,
-               int64_t wstride, void *f_scal, int64_t sstride, int nb, Scratch &S, WavPipe *pipe = nullptr) {
+               int64_t wstride, void *f_scal, int64_t sstride, int nb, Scratch &S, WavPipe *pipe = nullptr,
+               bool f32 = false) {
   const bool real = P.real;
   const int L = P.L;
-  const size_t esz = real ? sizeof(double) : sizeof(double2);
+  const size_t esz = (real ? 1 : 2) * (f32 ? sizeof(float) : sizeof(double));
   const bool adj = (mode == SPLIT_SYNTH_ADJ);
   char *wav = (char *)f_wav;
   std::vector<L2T> small;  // contractions that share launches
@@ -696,7 +702,7 @@ void wav_split(const WavPlan &P, SplitMode mode, const double2 *flm, bool flm_ha
     a.omlo = mlo;
     a.nb = nb;
     small.push_back(a);
-    rings.plain.push_back(ring_job(spec, f_scal, Ks, sstride, nts, sw, mlo, nb, bs));
+    rings.plain.push_back(ring_job(spec, f_scal, Ks, sstride, nts, sw, mlo, nb, bs, f32));
   }
   const auto norm = [&](const Scale &sd) { return adj && !P.axisym ? 1.0 / sd.ng : 1.0; };
   // the contraction of direction i of a scale into G ([b][n][t][m], spectral width W = 2bl-1)
@@ -742,10 +748,10 @@ void wav_split(const WavPlan &P, SplitMode mode, const double2 *flm, bool flm_ha
       const int nbg = std::min(group, nb - b0);
       switch (path) {
         case RINGS_FUSED:  // one launch, the n-components stay on chip
-          rings.add(sd, c, gamma_job(P, sd, G, wav, esz, wstride, b0, nbg));
+          rings.add(sd, c, gamma_job(P, sd, G, wav, esz, wstride, b0, nbg, f32));
           break;
         case RINGS_ONE_SLICE:
-          rings.plain.push_back(slice_job(P, sd, G, wav, esz, wstride, nb, false));
+          rings.plain.push_back(slice_job(P, sd, G, wav, esz, wstride, nb, false, f32));
           break;
         case RINGS_ON_N: {
           // F_n(t, p) = sum_m G_n(t, m) e^{i m phi_p}; spec holds F[b][i][t][p]
@@ -769,7 +775,7 @@ void wav_split(const WavPlan &P, SplitMode mode, const double2 *flm, bool flm_ha
         case RINGS_ON_SLICES: {
           const int sw = real ? bl : W, mlo = real ? 0 : -(bl - 1);
           gamma_synthesis(G, spec, sd.d_ns, nn, ng, bl, P.ss, nb, real, c, S.st);
-          RingJob j = ring_job(spec, out, K, wstride, ng * nt, sw, mlo, nb, bl);
+          RingJob j = ring_job(spec, out, K, wstride, ng * nt, sw, mlo, nb, bl, f32);
           ring_inverse_many({j}, P.ss, real, S.st);
           break;
         }
@@ -832,10 +838,10 @@ void wav_split(const WavPlan &P, SplitMode mode, const double2 *flm, bool flm_ha
 // For real signals flm holds m >= 0 only.  accumulate: add to flm instead of overwriting.
 void wav_merge(const WavPlan &P, MergeMode mode, const void *f_wav, int64_t wstride, const void *f_scal,
                int64_t sstride, double2 *flm, int nb, Scratch &S, bool accumulate = false,
-               WavPipe *pipe = nullptr) {
+               WavPipe *pipe = nullptr, bool f32 = false) {
   const bool real = P.real;
   const int L = P.L;
-  const size_t esz = real ? sizeof(double) : sizeof(double2);
+  const size_t esz = (real ? 1 : 2) * (f32 ? sizeof(float) : sizeof(double));
   const bool adj = (mode == MERGE_ANALYSIS_ADJ);
   char *wav = (char *)const_cast<void *>(f_wav);
   double2 *z = S.get<double2>((int64_t)nb * std::max<int64_t>(1, P.z_per_map));
@@ -846,7 +852,7 @@ void wav_merge(const WavPlan &P, MergeMode mode, const void *f_wav, int64_t wstr
   {
     const int sw = real ? bs : 2 * bs - 1, mlo = real ? 0 : -(bs - 1);
     double2 *spec = S.get<double2>((int64_t)nb * nts * sw);
-    rings.plain.push_back(ring_job(f_scal, spec, Ks, sstride, nts, sw, mlo, nb, bs));
+    rings.plain.push_back(ring_job(f_scal, spec, Ks, sstride, nts, sw, mlo, nb, bs, f32));
     if (P.scal_lmin > 0) S2G_CUDA(cudaMemsetAsync(zs, 0, sizeof(double2) * nb * bs * bs, S.st));
     T2L a{};
     a.tb = &P.table(bs, 0);
@@ -913,10 +919,10 @@ void wav_merge(const WavPlan &P, MergeMode mode, const void *f_wav, int64_t wstr
       if (pipe && !share) pipe->wait(S.st, sd.woff, b0);
       switch (path) {
         case RINGS_FUSED:  // one launch, the n-components stay on chip
-          rings.add(sd, c, gamma_job(P, sd, G, wav, esz, wstride, b0, nbg));
+          rings.add(sd, c, gamma_job(P, sd, G, wav, esz, wstride, b0, nbg, f32));
           break;
         case RINGS_ONE_SLICE:
-          rings.plain.push_back(slice_job(P, sd, G, wav, esz, wstride, nb, true));
+          rings.plain.push_back(slice_job(P, sd, G, wav, esz, wstride, nb, true, f32));
           break;
         case RINGS_ON_N: {
           // F_n(t, p) = c sum_g e^{-i n gamma_g} f_g(t, p), then one DFT per (n, t)
@@ -936,7 +942,7 @@ void wav_merge(const WavPlan &P, MergeMode mode, const void *f_wav, int64_t wstr
         }
         case RINGS_ON_SLICES: {
           const int sw = real ? bl : W, mlo = real ? 0 : -(bl - 1);
-          ring_forward_many({ring_job(in, spec, K, wstride, ng * nt, sw, mlo, nb, bl)}, P.ss, real, S.st);
+          ring_forward_many({ring_job(in, spec, K, wstride, ng * nt, sw, mlo, nb, bl, f32)}, P.ss, real, S.st);
           gamma_analysis(spec, G, sd.d_ns, nn, ng, bl, P.ss, nb, real, c, S.st);
           break;
         }
@@ -1085,10 +1091,22 @@ namespace {
 enum Op { OP_PX2WAV, OP_WAV2PX, OP_ADJ_WAV2PX, OP_ADJ_PX2WAV, OP_LM2WAV, OP_WAV2LM, OP_ADJ_WAV2LM,
           OP_ADJ_LM2WAV };
 
+// Whether the ring kernels can read and write a pass's FP32 pixels and
+// coefficients themselves, that is whether no other kernel touches them: the
+// gamma DFT on pixels (more directions than the fused launch takes) and the
+// residual of the refined forward transform work on doubles.
+bool f32_in_place(Op op, const WavPlan &P) {
+  if (op == OP_PX2WAV && refines(P.L, false)) return false;
+  for (const Scale &sd : P.sc)
+    if (ring_path(P, sd) == RINGS_ON_N) return false;
+  return true;
+}
+
 // One wavelet transform of `nb` maps with plan P.  Pixel maps, wavelet and
-// scaling arrays are batched with their single-map sizes as strides.
+// scaling arrays are batched with their single-map sizes as strides; f32 (only
+// where f32_in_place): they hold floats.
 void run_plan(Op op, const WavPlan &P, void *px, void *lm, void *wav, int64_t nw, void *scal, int64_t ns,
-              int nb, cudaStream_t st, bool accumulate_lm = false, WavPipe *pipe = nullptr) {
+              int nb, cudaStream_t st, bool accumulate_lm = false, WavPipe *pipe = nullptr, bool f32 = false) {
   if (nb <= 0) return;
   Scratch S(st);
   const int L = P.L;
@@ -1098,30 +1116,30 @@ void run_plan(Op op, const WavPlan &P, void *px, void *lm, void *wav, int64_t nw
   double2 *flm = lm_api ? (double2 *)lm : S.get<double2>((int64_t)nb * L * L);
   switch (op) {
   case OP_PX2WAV:
-    sht_forward(sht_of(P), px, npx, flm, nb, S, false);
-    wav_split(P, SPLIT_ANALYSIS, flm, real, wav, nw, scal, ns, nb, S, pipe);
+    sht_forward(sht_of(P), px, npx, flm, nb, S, false, f32);
+    wav_split(P, SPLIT_ANALYSIS, flm, real, wav, nw, scal, ns, nb, S, pipe, f32);
     break;
   case OP_LM2WAV:
     wav_split(P, SPLIT_ANALYSIS, flm, false, wav, nw, scal, ns, nb, S);
     break;
   case OP_ADJ_PX2WAV:
-    sht_forward(sht_of(P), px, npx, flm, nb, S, true);
-    wav_split(P, SPLIT_SYNTH_ADJ, flm, real, wav, nw, scal, ns, nb, S, pipe);
+    sht_forward(sht_of(P), px, npx, flm, nb, S, true, f32);
+    wav_split(P, SPLIT_SYNTH_ADJ, flm, real, wav, nw, scal, ns, nb, S, pipe, f32);
     break;
   case OP_ADJ_LM2WAV:
     wav_split(P, SPLIT_SYNTH_ADJ, flm, false, wav, nw, scal, ns, nb, S);
     break;
   case OP_WAV2PX:
-    wav_merge(P, MERGE_SYNTHESIS, wav, nw, scal, ns, flm, nb, S, false, pipe);
-    sht_inverse(sht_of(P), flm, real, px, npx, nb, S, false);
+    wav_merge(P, MERGE_SYNTHESIS, wav, nw, scal, ns, flm, nb, S, false, pipe, f32);
+    sht_inverse(sht_of(P), flm, real, px, npx, nb, S, false, f32);
     break;
   case OP_WAV2LM:
     wav_merge(P, MERGE_SYNTHESIS, wav, nw, scal, ns, flm, nb, S, accumulate_lm);
     if (real) symmetrize_flm(flm, L, (int64_t)L * L, nb, st);
     break;
   case OP_ADJ_WAV2PX:
-    wav_merge(P, MERGE_ANALYSIS_ADJ, wav, nw, scal, ns, flm, nb, S, false, pipe);
-    sht_inverse(sht_of(P), flm, real, px, npx, nb, S, true);
+    wav_merge(P, MERGE_ANALYSIS_ADJ, wav, nw, scal, ns, flm, nb, S, false, pipe, f32);
+    sht_inverse(sht_of(P), flm, real, px, npx, nb, S, true, f32);
     break;
   case OP_ADJ_WAV2LM:
     wav_merge(P, MERGE_ANALYSIS_ADJ, wav, nw, scal, ns, flm, nb, S, accumulate_lm);
@@ -1131,10 +1149,10 @@ void run_plan(Op op, const WavPlan &P, void *px, void *lm, void *wav, int64_t nw
 }
 
 void run_directional(Op op, const s2let_parameters_t &p, bool real, void *px, void *lm, void *wav,
-                     void *scal, int nb, cudaStream_t st) {
+                     void *scal, int nb, cudaStream_t st, bool f32 = false) {
   validate(&p);
   const WavPlan &P = directional_plan(p, real);
-  run_plan(op, P, px, lm, wav, s2let_n_wav(&p), scal, s2let_n_scal(&p), nb, st);
+  run_plan(op, P, px, lm, wav, s2let_n_wav(&p), scal, s2let_n_scal(&p), nb, st, false, nullptr, f32);
 }
 
 // Plain spherical-harmonic transform on device buffers, MW (ss = 0) or MWSS
@@ -1200,9 +1218,10 @@ GroupStreams &group_streams() {
   return g;
 }
 
-// f32: every map's arrays hold floats (interleaved pairs when complex); they
-// are widened into FP64 batch scratch on the way in and rounded on the way out
-// (only the used part of f_wav), so every map goes through the scratch.
+// f32: every map's arrays hold floats (interleaved pairs when complex).  Where the
+// kernels cannot read and write those themselves (f32_in_place), every map goes
+// through FP64 scratch, widened on the way in and rounded on the way out.  Only
+// the used part of f_wav moves.
 void multi_pass_group(Op op, const std::vector<int> &g, const s2let_parameters_t *params, const int *real,
                       void *const *px, void *const *wav, void *const *scal, cudaStream_t st, bool f32);
 
@@ -1241,22 +1260,24 @@ void multi_pass_group(Op op, const std::vector<int> &g, const s2let_parameters_t
   {
     const s2let_parameters_t &p = params[g[0]];
     const bool re = real[g[0]] != 0;
-    if (g.size() == 1 && !f32) {
-      run_directional(op, p, re, px[g[0]], nullptr, wav[g[0]], scal[g[0]], 1, st);
+    const bool keep32 = f32 && f32_in_place(op, directional_plan(p, re));
+    if (g.size() == 1 && (!f32 || keep32)) {
+      run_directional(op, p, re, px[g[0]], nullptr, wav[g[0]], scal[g[0]], 1, st, f32);
       return;
     }
     const int nb = (int)g.size();
-    const size_t esz = re ? sizeof(double) : sizeof(double2);
+    const size_t rsz = keep32 ? sizeof(float) : sizeof(double);  // per real in the batch
+    const size_t esz = (re ? 1 : 2) * rsz;
     const size_t bpx = esz * s2let_n_px(&p), bw = esz * s2let_n_wav(&p), bs = esz * s2let_n_scal(&p);
-    const int64_t rpx = (int64_t)(bpx / sizeof(double)), rw = (int64_t)(bw / sizeof(double)),
-                  rs = (int64_t)(bs / sizeof(double)), rwu = f32 ? used_wav_reals(p, re) : rw;
+    const int64_t rpx = (int64_t)(bpx / rsz), rw = (int64_t)(bw / rsz), rs = (int64_t)(bs / rsz),
+                  rwu = f32 ? used_wav_reals(p, re) : rw;
     Scratch S(st);
     char *dpx = S.get<char>((int64_t)nb * bpx), *dw = S.get<char>((int64_t)nb * bw),
          *ds = S.get<char>((int64_t)nb * bs);
     const bool fwd = (op == OP_PX2WAV || op == OP_ADJ_PX2WAV);
     for (int i = 0; i < nb; ++i) {
       const int k = g[i];
-      if (f32) {
+      if (f32 && !keep32) {
         if (fwd) {
           widen_rows((const float *)px[k], 0, (double *)(dpx + i * bpx), 0, rpx, 1, st);
         } else {
@@ -1266,14 +1287,14 @@ void multi_pass_group(Op op, const std::vector<int> &g, const s2let_parameters_t
       } else if (fwd) {
         S2G_CUDA(cudaMemcpyAsync(dpx + i * bpx, px[k], bpx, cudaMemcpyDeviceToDevice, st));
       } else {
-        S2G_CUDA(cudaMemcpyAsync(dw + i * bw, wav[k], bw, cudaMemcpyDeviceToDevice, st));
+        S2G_CUDA(cudaMemcpyAsync(dw + i * bw, wav[k], rsz * rwu, cudaMemcpyDeviceToDevice, st));
         S2G_CUDA(cudaMemcpyAsync(ds + i * bs, scal[k], bs, cudaMemcpyDeviceToDevice, st));
       }
     }
-    run_directional(op, p, re, dpx, nullptr, dw, ds, nb, st);
+    run_directional(op, p, re, dpx, nullptr, dw, ds, nb, st, keep32);
     for (int i = 0; i < nb; ++i) {
       const int k = g[i];
-      if (f32) {
+      if (f32 && !keep32) {
         if (fwd) {
           narrow_rows((const double *)(dw + i * bw), 0, (float *)wav[k], 0, rwu, 1, st);
           narrow_rows((const double *)(ds + i * bs), 0, (float *)scal[k], 0, rs, 1, st);
@@ -1281,7 +1302,7 @@ void multi_pass_group(Op op, const std::vector<int> &g, const s2let_parameters_t
           narrow_rows((const double *)(dpx + i * bpx), 0, (float *)px[k], 0, rpx, 1, st);
         }
       } else if (fwd) {
-        S2G_CUDA(cudaMemcpyAsync(wav[k], dw + i * bw, bw, cudaMemcpyDeviceToDevice, st));
+        S2G_CUDA(cudaMemcpyAsync(wav[k], dw + i * bw, rsz * rwu, cudaMemcpyDeviceToDevice, st));
         S2G_CUDA(cudaMemcpyAsync(scal[k], ds + i * bs, bs, cudaMemcpyDeviceToDevice, st));
       } else {
         S2G_CUDA(cudaMemcpyAsync(px[k], dpx + i * bpx, bpx, cudaMemcpyDeviceToDevice, st));
@@ -1444,9 +1465,10 @@ int batch_directional(const char *fn, s2g::Op op, const s2let_parameters_t *p, b
   });
 }
 
-// FP32 storage: the batch widened into FP64 device scratch (only the used part
-// of each f_wav row), the FP64-storage path at the thread's precision, the
-// outputs rounded to FP32.
+// FP32 storage, at the thread's precision: the ring kernels widen what they read
+// and round what they write, or, where other kernels touch the pixels
+// (f32_in_place), the batch is widened into FP64 device scratch (only the used
+// part of each f_wav row) and the outputs are rounded from there.  Same results.
 int batch_directional_f32(const char *fn, s2g::Op op, const s2let_parameters_t *p, bool real, void *px,
                           void *wav, void *scal, int nb, void *stream) {
   return s2g::guarded(fn, [&] {
@@ -1457,6 +1479,10 @@ int batch_directional_f32(const char *fn, s2g::Op op, const s2let_parameters_t *
     if (nb == 0) return;
     S2G_REQUIRE(px && wav && scal, ERR_INVALID, "NULL buffer");
     cudaStream_t st = (cudaStream_t)stream;
+    if (f32_in_place(op, directional_plan(*p, real))) {
+      run_directional(op, *p, real, px, nullptr, wav, scal, nb, st, true);
+      return;
+    }
     const int dd = real ? 1 : 2;
     const int64_t npx = s2let_n_px(p) * dd, nw = s2let_n_wav(p) * dd, ns = s2let_n_scal(p) * dd;
     const int64_t nwu = used_wav_reals(*p, real);

@@ -31,6 +31,7 @@ struct RingJob {
   int spec_rpm = 1 << 30;
   int sw = 0, mlo = 0;
   bool herm = false;
+  bool f32 = false;  // the rings hold floats (pairs when complex)
   int nrings = 0, bl = 0;
 };
 void ring_forward_many(const std::vector<RingJob> &jobs, int ss, bool real, cudaStream_t st);
@@ -156,6 +157,7 @@ struct GammaJob {
   int64_t gms = 0, gks = 0;
   void *fw = nullptr;  // the gamma slices (analysis: read)
   int64_t fms = 0;
+  bool f32 = false;  // the gamma slices hold floats (pairs when complex)
   int nb = 0, bl = 0;
 };
 void ring_inverse_gamma(const std::vector<GammaJob> &jobs, const std::vector<int> &ns, int ng, bool real, double c,

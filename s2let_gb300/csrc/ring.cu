@@ -54,7 +54,7 @@ namespace cg = cooperative_groups;
 
 struct RingArgs {
   const void *rings;
-  double2 *rings_out;  // inverse: output rings (as double2 or double)
+  void *rings_out;  // inverse: output rings
   int64_t ring_stride;  // between rings of one map
   int64_t map_stride;   // between maps
   int rpm;              // rings per map
@@ -106,6 +106,56 @@ __device__ __forceinline__ int job_of(const G &g, int block) {
   int q = 0;
   while (q + 1 < g.n && block >= g.first[q + 1]) ++q;
   return q;
+}
+
+// Pixels in memory: doubles, or floats that are widened as they are read and
+// rounded to nearest as they are written, in integers; zeros, subnormals,
+// infinities, NaN and results outside the normal range of a float go to the
+// conversion instructions, out of line.  Complex floats are read and written as
+// two 4-byte words, so that any float pointer will do.  Widening and rounding in
+// passes of their own cost a gradient step with FP32 storage (band-limit 512, 8
+// maps) 13.08 ms instead of 12.70, and the memory of the FP64 copies.  The type
+// is a template parameter: as a run-time switch it slowed the FP64 launches by 1
+// to 8 %.
+__device__ __noinline__ double widen_any(float x) { return (double)x; }
+__device__ __noinline__ float narrow_any(double x) { return __double2float_rn(x); }
+__device__ __forceinline__ double widen(float x) {
+  const uint32_t b = __float_as_uint(x);
+  if (((b >> 23) & 0xFF) - 1u >= 254u) return widen_any(x);
+  return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7FFFFFFFu) >> 3) + (896u << 20))), (int)(b << 29));
+}
+__device__ __forceinline__ float narrow(double x) {
+  const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
+  if (((hi >> 20) & 0x7FF) - 897u >= 254u) return narrow_any(x);
+  uint32_t f = (((hi & 0x7FFFFFFFu) - (896u << 20)) << 3) | (lo >> 29);
+  const uint32_t rem = lo & 0x1FFFFFFFu;
+  f += rem > 0x10000000u || (rem == 0x10000000u && (f & 1)) ? 1u : 0u;  // the carry runs into the exponent
+  return __uint_as_float((hi & 0x80000000u) | f);
+}
+template <bool F32>
+__device__ __forceinline__ double ld_px(const void *p, int64_t i) {
+  return F32 ? widen(((const float *)p)[i]) : ((const double *)p)[i];
+}
+template <bool F32>
+__device__ __forceinline__ double2 ld_px2(const void *p, int64_t i) {
+  if (F32) return make_double2(widen(((const float *)p)[2 * i]), widen(((const float *)p)[2 * i + 1]));
+  return ((const double2 *)p)[i];
+}
+template <bool F32>
+__device__ __forceinline__ void st_px(void *p, int64_t i, double v) {
+  if (F32)
+    ((float *)p)[i] = narrow(v);
+  else
+    ((double *)p)[i] = v;
+}
+template <bool F32>
+__device__ __forceinline__ void st_px2(void *p, int64_t i, double2 v) {
+  if (F32) {
+    ((float *)p)[2 * i] = narrow(v.x);
+    ((float *)p)[2 * i + 1] = narrow(v.y);
+  } else {
+    ((double2 *)p)[i] = v;
+  }
 }
 
 // element offset of ring r (rings of a map are ring_stride apart, maps map_stride)
@@ -354,7 +404,7 @@ __device__ __forceinline__ double2 nan2() {
 
 constexpr int kRingThreads = 256;
 
-template <bool REAL>
+template <bool REAL, bool F32>
 __global__ void __launch_bounds__(kRingThreads, 3) k_ring_forward(const __grid_constant__ RingGroup grp) {
   extern __shared__ longlong2 buf[];
   __shared__ int s_mx;
@@ -366,10 +416,10 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_ring_forward(const __grid_c
   int em = 0;
   for (int j = threadIdx.x; j < K; j += blockDim.x) {
     if (REAL) {
-      em = max(em, exp_field(((const double *)a.rings)[ring_base(a, r0) + j]));
-      if (has1) em = max(em, exp_field(((const double *)a.rings)[ring_base(a, r0 + 1) + j]));
+      em = max(em, exp_field(ld_px<F32>(a.rings, ring_base(a, r0) + j)));
+      if (has1) em = max(em, exp_field(ld_px<F32>(a.rings, ring_base(a, r0 + 1) + j)));
     } else {
-      em = emax2(em, ((const double2 *)a.rings)[ring_base(a, r0) + j]);
+      em = emax2(em, ld_px2<F32>(a.rings, ring_base(a, r0) + j));
     }
   }
   em = block_max_int(em);
@@ -379,10 +429,10 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_ring_forward(const __grid_c
     if (j < K) {
       double2 x;
       if (REAL) {
-        x.x = ((const double *)a.rings)[ring_base(a, r0) + j];
-        x.y = has1 ? ((const double *)a.rings)[ring_base(a, r0 + 1) + j] : 0.0;
+        x.x = ld_px<F32>(a.rings, ring_base(a, r0) + j);
+        x.y = has1 ? ld_px<F32>(a.rings, ring_base(a, r0 + 1) + j) : 0.0;
       } else {
-        x = ((const double2 *)a.rings)[ring_base(a, r0) + j];
+        x = ld_px2<F32>(a.rings, ring_base(a, r0) + j);
       }
       v = fx_mulc4(fx_split2<61>(x, e), ld_once(&a.chirp[j]));  // x_j conj(c_j)
     }
@@ -414,7 +464,7 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_ring_forward(const __grid_c
   }
 }
 
-template <bool REAL>
+template <bool REAL, bool F32>
 __global__ void __launch_bounds__(kRingThreads, 3) k_ring_inverse(const __grid_constant__ RingGroup grp) {
   extern __shared__ longlong2 buf[];
   __shared__ int s_mx;
@@ -466,10 +516,10 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_ring_inverse(const __grid_c
     const longlong2 y = fx_mul(fx_conj(last_pass(buf, P, logP, p)), ld_once(&a.chirp[p]));
     const double2 f = em == kExpNonFinite ? nan2() : fx_join2(y, k0);
     if (REAL) {
-      ((double *)a.rings_out)[ring_base(a, r0) + p] = f.x;
-      if (has1) ((double *)a.rings_out)[ring_base(a, r0 + 1) + p] = f.y;
+      st_px<F32>(a.rings_out, ring_base(a, r0) + p, f.x);
+      if (has1) st_px<F32>(a.rings_out, ring_base(a, r0 + 1) + p, f.y);
     } else {
-      a.rings_out[ring_base(a, r0) + p] = f;
+      st_px2<F32>(a.rings_out, ring_base(a, r0) + p, f);
     }
   }
 }
@@ -506,7 +556,7 @@ __device__ __forceinline__ int cluster_max_int(cg::cluster_group &cl, int *slot,
   return r;
 }
 
-template <int NN, bool REAL>
+template <int NN, bool REAL, bool F32>
 __global__ void __launch_bounds__(kRingThreads, 3) k_ring_inverse_gamma(const __grid_constant__ GammaFuse grp) {
   extern __shared__ longlong2 buf[];
   __shared__ int s_mx, s_em, s_k;
@@ -574,8 +624,8 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_ring_inverse_gamma(const __
           A = fx_mac4(A, z[j].x, w.x, w.y);
           B = fx_mac4(B, z[j].y, w.z, w.w);
         }
-        ((double *)gf.fw)[o] = bad ? nan2().x : fx_join(A - B, ko);
-        if (pair) ((double *)gf.fw)[o2] = bad ? nan2().x : fx_join(A + B, ko);
+        st_px<F32>(gf.fw, o, bad ? nan2().x : fx_join(A - B, ko));
+        if (pair) st_px<F32>(gf.fw, o2, bad ? nan2().x : fx_join(A + B, ko));
       } else {
         longlong2 U = make_longlong2(0, 0), V = make_longlong2(0, 0);
 #pragma unroll
@@ -585,15 +635,15 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_ring_inverse_gamma(const __
           V = make_longlong2(fx_mac4(V.x, z[j].x, w.z, w.w), fx_mac4(V.y, z[j].y, w.z, w.w));
         }
         const longlong2 iV = fx_mul_i(V);
-        ((double2 *)gf.fw)[o] = bad ? nan2() : fx_join2(fx_add(U, iV), ko);
-        if (pair) ((double2 *)gf.fw)[o2] = bad ? nan2() : fx_join2(fx_sub(U, iV), ko);
+        st_px2<F32>(gf.fw, o, bad ? nan2() : fx_join2(fx_add(U, iV), ko));
+        if (pair) st_px2<F32>(gf.fw, o2, bad ? nan2() : fx_join2(fx_sub(U, iV), ko));
       }
     }
   }
   cl.sync();  // peers read this buffer until here
 }
 
-template <int NN, bool REAL>
+template <int NN, bool REAL, bool F32>
 __global__ void __launch_bounds__(kRingThreads, 3) k_gamma_ring_forward(const __grid_constant__ GammaFuse grp) {
   extern __shared__ longlong2 buf[];
   __shared__ int s_mx, s_em;
@@ -612,9 +662,9 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_gamma_ring_forward(const __
     for (int g = 0; g < grp.ng; ++g) {
       const int64_t o = ibase + (int64_t)g * gf.npx + p;
       if (REAL)
-        em = max(em, exp_field(((const double *)gf.fw)[o]));
+        em = max(em, exp_field(ld_px<F32>(gf.fw, o)));
       else
-        em = emax2(em, ((const double2 *)gf.fw)[o]);
+        em = emax2(em, ld_px2<F32>(gf.fw, o));
     }
   em = cluster_max_int(cl, &s_em, em, NN);
   const int e = fx_exp(em);
@@ -633,8 +683,8 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_gamma_ring_forward(const __
       const bool pair = g > 0 && g2 != g;
       const int64_t o = ibase + (int64_t)g * gf.npx + p, o2 = ibase + (int64_t)g2 * gf.npx + p;
       if (REAL) {
-        const long long fa = fx_split<61>(((const double *)gf.fw)[o], e);
-        const long long fb = pair ? fx_split<61>(((const double *)gf.fw)[o2], e) : 0;
+        const long long fa = fx_split<61>(ld_px<F32>(gf.fw, o), e);
+        const long long fb = pair ? fx_split<61>(ld_px<F32>(gf.fw, o2), e) : 0;
         const long long Pp = fa + fb, Q = fa - fb;
 #pragma unroll
         for (int j = 0; j < NN; ++j) {
@@ -642,8 +692,8 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_gamma_ring_forward(const __
           acc[j] = make_longlong2(fx_mac4(acc[j].x, Pp, w.x, w.y), fx_mac4(acc[j].y, Q, w.z, w.w));
         }
       } else {
-        const longlong2 fa = fx_split2<61>(((const double2 *)gf.fw)[o], e);
-        const longlong2 fb = pair ? fx_split2<61>(((const double2 *)gf.fw)[o2], e) : make_longlong2(0, 0);
+        const longlong2 fa = fx_split2<61>(ld_px2<F32>(gf.fw, o), e);
+        const longlong2 fb = pair ? fx_split2<61>(ld_px2<F32>(gf.fw, o2), e) : make_longlong2(0, 0);
         const longlong2 Pp = fx_add(fa, fb), Q = fx_sub(fa, fb);
 #pragma unroll
         for (int j = 0; j < NN; ++j) {
@@ -753,17 +803,20 @@ template <class LAUNCH>
 void run_rings(const std::vector<RingJob> &jobs, int ss, bool real, bool forward, LAUNCH &&launch, cudaStream_t st) {
   RingGroup g;
   double fl = 0, by = 0;
+  bool f32 = false;
   g.n = 0;
   g.first[0] = 0;
   const auto flush = [&] {
     if (!g.n) return;
     KTimer kt(KC_RING, st, fl, by);
-    launch(g);
+    launch(g, f32);
     g.n = 0;
     fl = by = 0;
   };
   for (const RingJob &j : jobs) {
     if (j.nrings <= 0) continue;
+    if (j.f32 != f32) flush();  // one storage type per launch
+    f32 = j.f32;
     RingArgs a = ring_args(ring_fft(grid_ring_len(j.bl, ss)), j.bl, j.nrings);
     a.ring_stride = j.ring_stride;
     a.map_stride = j.map_stride;
@@ -779,11 +832,11 @@ void run_rings(const std::vector<RingJob> &jobs, int ss, bool real, bool forward
       a.spec_out = (double2 *)j.out;
     } else {
       a.spec_in = (const double2 *)j.in;
-      a.rings_out = (double2 *)j.out;
+      a.rings_out = j.out;
     }
     const int nblk = real ? (j.nrings + 1) / 2 : j.nrings;
     if (timing_enabled()) fl += ring_work(a, nblk);
-    by += (double)j.nrings * a.K * (real ? 8.0 : 16.0) + (double)j.nrings * a.sw * 16.0;
+    by += (double)j.nrings * a.K * (real ? 8.0 : 16.0) * (j.f32 ? 0.5 : 1.0) + (double)j.nrings * a.sw * 16.0;
     g.a[g.n] = a;
     g.first[g.n + 1] = g.first[g.n] + nblk;
     if (++g.n == kMaxJobs) flush();
@@ -847,13 +900,13 @@ bool cluster_fits(int nn, int P) {
   if (it != known.end()) return it->second;
   const void *kern = nullptr;
   switch (nn) {
-    case 2: kern = (const void *)k_ring_inverse_gamma<2, false>; break;
-    case 3: kern = (const void *)k_ring_inverse_gamma<3, false>; break;
-    case 4: kern = (const void *)k_ring_inverse_gamma<4, false>; break;
-    case 5: kern = (const void *)k_ring_inverse_gamma<5, false>; break;
-    case 6: kern = (const void *)k_ring_inverse_gamma<6, false>; break;
-    case 7: kern = (const void *)k_ring_inverse_gamma<7, false>; break;
-    default: kern = (const void *)k_ring_inverse_gamma<8, false>; break;
+    case 2: kern = (const void *)k_ring_inverse_gamma<2, false, false>; break;
+    case 3: kern = (const void *)k_ring_inverse_gamma<3, false, false>; break;
+    case 4: kern = (const void *)k_ring_inverse_gamma<4, false, false>; break;
+    case 5: kern = (const void *)k_ring_inverse_gamma<5, false, false>; break;
+    case 6: kern = (const void *)k_ring_inverse_gamma<6, false, false>; break;
+    case 7: kern = (const void *)k_ring_inverse_gamma<7, false, false>; break;
+    default: kern = (const void *)k_ring_inverse_gamma<8, false, false>; break;
   }
   bool ok = ring_smem(P) <= 227 * 1024;
   if (ok) {
@@ -887,6 +940,7 @@ void run_fused(const std::vector<GammaJob> &jobs, const std::vector<int> &ns, in
   const int nn = (int)ns.size();
   GammaFuse g;
   double fl = 0, by = 0;
+  bool f32 = false;
   g.n = 0;
   g.first[0] = 0;
   g.ng = ng;
@@ -896,7 +950,7 @@ void run_fused(const std::vector<GammaJob> &jobs, const std::vector<int> &ns, in
   const auto flush = [&] {
     if (!g.n) return;
     KTimer kt(KC_RING, st, fl, by);
-    launch(g);
+    launch(g, f32);
     g.n = 0;
     fl = by = 0;
   };
@@ -905,6 +959,8 @@ void run_fused(const std::vector<GammaJob> &jobs, const std::vector<int> &ns, in
     S2G_REQUIRE(ring_gamma_fusable(nn, ng, j.bl, ss), ERR_UNSUPPORTED, "fused ring/gamma DFT: unsupported shape");
     const int nt = grid_rings(j.bl, ss), nrings = j.nb * nt;
     if (nrings <= 0) continue;
+    if (j.f32 != f32) flush();  // one storage type per launch
+    f32 = j.f32;
     if (!tw) fuse_twiddles(g, ns, ng, real, c, synth);
     tw = true;
     GammaItem &it = g.it[g.n];
@@ -920,7 +976,7 @@ void run_fused(const std::vector<GammaJob> &jobs, const std::vector<int> &ns, in
     it.npx = (int64_t)nt * it.a.K;
     const double px = (double)nrings * it.a.K;
     if (timing_enabled()) fl += ring_work(it.a, nrings * nn) + gamma_work(px, ng, nn, real);
-    by += (double)nrings * nn * it.W * 16.0 + px * ng * (real ? 8.0 : 16.0);
+    by += (double)nrings * nn * it.W * 16.0 + px * ng * (real ? 8.0 : 16.0) * (j.f32 ? 0.5 : 1.0);
     g.first[g.n + 1] = g.first[g.n] + nrings;
     if (++g.n == kMaxJobs) flush();
   }
@@ -930,14 +986,16 @@ void run_fused(const std::vector<GammaJob> &jobs, const std::vector<int> &ns, in
 
 void ring_inverse_gamma(const std::vector<GammaJob> &jobs, const std::vector<int> &ns, int ng, bool real, double c,
                         int ss, cudaStream_t st) {
-  run_fused(jobs, ns, ng, real, c, ss, true, [&](const GammaFuse &gf) {
+  run_fused(jobs, ns, ng, real, c, ss, true, [&](const GammaFuse &gf, bool f32) {
     switch ((int)ns.size()) {
 #define S2G_FUSE(N)                                               \
   case N:                                                         \
-    if (real)                                                     \
-      launch_fused(k_ring_inverse_gamma<N, true>, gf, N, st);    \
+    if (f32)                                                      \
+      real ? launch_fused(k_ring_inverse_gamma<N, true, true>, gf, N, st)           \
+           : launch_fused(k_ring_inverse_gamma<N, false, true>, gf, N, st);         \
     else                                                          \
-      launch_fused(k_ring_inverse_gamma<N, false>, gf, N, st);   \
+      real ? launch_fused(k_ring_inverse_gamma<N, true, false>, gf, N, st)          \
+           : launch_fused(k_ring_inverse_gamma<N, false, false>, gf, N, st);        \
     break;
       S2G_FUSE(2) S2G_FUSE(3) S2G_FUSE(4) S2G_FUSE(5) S2G_FUSE(6) S2G_FUSE(7) S2G_FUSE(8)
 #undef S2G_FUSE
@@ -948,14 +1006,16 @@ void ring_inverse_gamma(const std::vector<GammaJob> &jobs, const std::vector<int
 
 void gamma_ring_forward(const std::vector<GammaJob> &jobs, const std::vector<int> &ns, int ng, bool real, double c,
                         int ss, cudaStream_t st) {
-  run_fused(jobs, ns, ng, real, c, ss, false, [&](const GammaFuse &gf) {
+  run_fused(jobs, ns, ng, real, c, ss, false, [&](const GammaFuse &gf, bool f32) {
     switch ((int)ns.size()) {
 #define S2G_FUSE(N)                                               \
   case N:                                                         \
-    if (real)                                                     \
-      launch_fused(k_gamma_ring_forward<N, true>, gf, N, st);    \
+    if (f32)                                                      \
+      real ? launch_fused(k_gamma_ring_forward<N, true, true>, gf, N, st)           \
+           : launch_fused(k_gamma_ring_forward<N, false, true>, gf, N, st);         \
     else                                                          \
-      launch_fused(k_gamma_ring_forward<N, false>, gf, N, st);   \
+      real ? launch_fused(k_gamma_ring_forward<N, true, false>, gf, N, st)          \
+           : launch_fused(k_gamma_ring_forward<N, false, false>, gf, N, st);        \
     break;
       S2G_FUSE(2) S2G_FUSE(3) S2G_FUSE(4) S2G_FUSE(5) S2G_FUSE(6) S2G_FUSE(7) S2G_FUSE(8)
 #undef S2G_FUSE
@@ -965,19 +1025,19 @@ void gamma_ring_forward(const std::vector<GammaJob> &jobs, const std::vector<int
 }
 
 void ring_forward_many(const std::vector<RingJob> &jobs, int ss, bool real, cudaStream_t st) {
-  run_rings(jobs, ss, real, true, [&](const RingGroup &g) {
-    if (real)
-      launch_ring(k_ring_forward<true>, g, st);
+  run_rings(jobs, ss, real, true, [&](const RingGroup &g, bool f32) {
+    if (f32)
+      real ? launch_ring(k_ring_forward<true, true>, g, st) : launch_ring(k_ring_forward<false, true>, g, st);
     else
-      launch_ring(k_ring_forward<false>, g, st);
+      real ? launch_ring(k_ring_forward<true, false>, g, st) : launch_ring(k_ring_forward<false, false>, g, st);
   }, st);
 }
 void ring_inverse_many(const std::vector<RingJob> &jobs, int ss, bool real, cudaStream_t st) {
-  run_rings(jobs, ss, real, false, [&](const RingGroup &g) {
-    if (real)
-      launch_ring(k_ring_inverse<true>, g, st);
+  run_rings(jobs, ss, real, false, [&](const RingGroup &g, bool f32) {
+    if (f32)
+      real ? launch_ring(k_ring_inverse<true, true>, g, st) : launch_ring(k_ring_inverse<false, true>, g, st);
     else
-      launch_ring(k_ring_inverse<false>, g, st);
+      real ? launch_ring(k_ring_inverse<true, false>, g, st) : launch_ring(k_ring_inverse<false, false>, g, st);
   }, st);
 }
 
