@@ -180,10 +180,11 @@ def measured_peaks():
 # ncu capture each (DRAM bytes over the bytes the launch must move):
 # profiles/fp64_contraction_L512_N4_batch8.md (traffic grows with the table
 # size, so the ratio carries to the L=1024 launches) and
-# profiles/ring_gamma_fused_df_L1024_N4_batch8.md (the fused ring + gamma DFT
-# launches that carry most of the ring-DFT bytes: 1.437 GB of DRAM traffic for
-# 1.476 GB of spectra in and gamma slices out, per bl=1024 launch of 8 maps)
-TRAFFIC_RATIO = {"fp64_contraction": 1.126, "ring_dft": 0.974}
+# profiles/ring_gamma_fixed_point_L1024_N4_one_map.md (the fused ring + gamma DFT
+# launches that carry most of the ring-DFT bytes: 0.650 GB of DRAM traffic for
+# 0.738 GB of spectra and gamma slices, both directions of one map's two bl=1024
+# scales; the rest stays in L2)
+TRAFFIC_RATIO = {"fp64_contraction": 1.126, "ring_dft": 0.881}
 
 
 def profile_traffic(kernel, alg_bytes_per_launch):

@@ -436,7 +436,7 @@ int s2let_gpu_get_precision(void);
  * and freed by s2let_gpu_release_plans: the double-float copies of the split-
  * precision one-map contractions (the size of the FP64 tables; skipped when
  * they would leave less than 4 GiB of device memory free), and the eight-slice
- * digit panels of the FP64 mode's contractions and of the adjoints (16 bytes
+ * digit panels of the FP64 mode's contractions and of the adjoints (8 bytes
  * per table entry; skipped when less than a third of the device memory would
  * stay free).  0 = no such copies: the FP64 values are read as they are
  * (slower, no extra memory).  Process-wide.  Returns the status. */
@@ -446,8 +446,8 @@ int s2let_gpu_get_split_tables(void);
 /* Split precision on stored tables: batches of at most `maps` maps (0-4,
  * default 1, initially S2LET_GPU_DF_MAX_MAPS when set) contract in
  * double-float on the FP64 tables (8 bytes per table entry streamed, two
- * scales of one band-limit in one pass) instead of on the tensor cores (14
- * bytes per entry); 0 keeps every batch on the tensor cores.  Process-wide.
+ * scales of one band-limit in one pass) instead of on the tensor cores (7
+ * bytes per entry, expanded on chip); 0 keeps every batch on the tensor cores.  Process-wide.
  * Returns the status. */
 int s2let_gpu_set_df_max_maps(int maps);
 int s2let_gpu_get_df_max_maps(void);

@@ -26,7 +26,8 @@
 // 45 adds and shifts, against 256 FP32 instructions in double-float and 32
 // FP64 instructions at 1/64 rate.  Measured, px2wav + wav2px at L = 1024, N = 4
 // (real maps), rings and gamma DFTs: 2 maps in FP64 19.2 ms with FP64
-// butterflies, 3.8 ms so; 32 maps at split precision 60.6 ms in double-float.
+// butterflies, 3.1 ms so; 32 maps at split precision 60.6 ms in double-float,
+// 45.6 ms so.
 //
 // Table data comes as 62-bit fixed point (RingFFT, plan.h): chirp exp(i pi k^2
 // / K), the passes' twiddles level by level (the passes below the first read
@@ -113,7 +114,7 @@ __device__ __forceinline__ int job_of(const G &g, int block) {
 // infinities, NaN and results outside the normal range of a float go to the
 // conversion instructions, out of line.  Complex floats are read and written as
 // two 4-byte words, so that any float pointer will do.  Widening and rounding in
-// passes of their own cost a gradient step with FP32 storage (band-limit 512, 8
+// passes of their own cost a gradient step with FP32 storage (band-limit 256, 32
 // maps) 13.08 ms instead of 12.70, and the memory of the FP64 copies.  The type
 // is a template parameter: as a run-time switch it slowed the FP64 launches by 1
 // to 8 %.
