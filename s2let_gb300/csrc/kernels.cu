@@ -44,7 +44,7 @@ __device__ __forceinline__ double2 scl2(double2 a, double s) { return make_doubl
 constexpr int CT_M = 128;  // rows (t or l) per CTA
 constexpr int CT_K = 32;   // reduction tile
 // split precision: batches of at most this many maps contract in double-float
-// on the FP64 tables instead of streaming the tensor path's digit panels
+// instead of on the tensor cores (both sides measured at k_contract_df below)
 // (s2let_gpu_set_df_max_maps, initially S2LET_GPU_DF_MAX_MAPS or 1; 0 keeps
 // every batch on the tensor path)
 std::atomic<int> g_df_max_maps{[] {
@@ -235,9 +235,10 @@ __global__ void __launch_bounds__(CT_M) k_contract(const __grid_constant__ Contr
 
 // The same contractions in double-float on the FP32 pipe (split-precision
 // path: every contraction the tensor-core kernel does not take, and batches of
-// at most df_max_maps() maps, for which streaming the tables' 7 bf16 digit
-// panels (14 B per entry) costs more than reading 8 B per entry and
-// multiplying in double-float).
+// at most df_max_maps() maps: both read 8 B per entry, but the tensor path, in the
+// eight slices that match this accuracy, spends a 16-column tile on one map's two
+// columns.  Round trips of one map, this kernel / eight slices: band-limit 128
+// 0.22 / 0.43 ms, 256 0.64 / 0.89, 512 2.53 / 2.90, 1024 14.28 / 14.99).
 //
 // A CTA owns one m and up to 128 output rows.  It first splits its coefficient
 // columns (maps x parts; a second part is another scale on the same table)

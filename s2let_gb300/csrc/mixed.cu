@@ -39,7 +39,7 @@
 //             weight, store; the accumulator is released as soon as its values
 //             are in registers.
 // Measured (2 maps at L = 1024, N = 4, FP64, 16 columns): 13.0 ms against 15.8 with
-// bf16 panels in HBM; 32 maps, split precision, 64 columns: 32.2 against 33.5.
+// bf16 panels in HBM; 32 maps, split precision, 64 columns: 31.1 against 33.5.
 // With a quarter of the MMAs the 16-column launches take 24 % less, without the
 // conversion's stores 10 %, without the combination 4 %: no single unit paces
 // them (DRAM 38 % busy, tensor pipe 17 %); what is left is the latency of 32
