@@ -11,6 +11,7 @@
 #include "common.h"
 #include "plan.h"
 #include "recompute.h"
+#include "ringtables.h"
 
 namespace s2g {
 
@@ -375,29 +376,6 @@ __global__ void __launch_bounds__(256) k_qgemm(double *__restrict__ Q, const dou
   }
 }
 
-// host FFT (radix-2, in extended precision) for the Bluestein kernel spectrum;
-// w holds exp(-2 pi i k / n) for k < n/2
-using cxl = std::complex<long double>;
-cxl mul(cxl a, cxl b) {  // std::complex's product checks for NaN
-  return {a.real() * b.real() - a.imag() * b.imag(), a.real() * b.imag() + a.imag() * b.real()};
-}
-void host_fft(std::vector<cxl> &x, const std::vector<cxl> &w) {
-  const size_t n = x.size();
-  for (size_t i = 1, j = 0; i < n; ++i) {
-    size_t bit = n >> 1;
-    for (; j & bit; bit >>= 1) j ^= bit;
-    j ^= bit;
-    if (i < j) std::swap(x[i], x[j]);
-  }
-  for (size_t len = 2; len <= n; len <<= 1)
-    for (size_t i = 0; i < n; i += len)
-      for (size_t k = 0; k < len / 2; ++k) {
-        const cxl u = x[i + k], v = mul(x[i + k + len / 2], w[k * (n / len)]);
-        x[i + k] = u + v;
-        x[i + k + len / 2] = u - v;
-      }
-}
-
 std::mutex g_plan_mu;
 std::map<std::tuple<int, int, int, int>, std::unique_ptr<WignerTable>> g_tables;  // (bl, an, ss, rc)
 std::map<int, std::unique_ptr<RingFFT>> g_rings;
@@ -566,70 +544,23 @@ std::unique_ptr<WignerTable> build_table(int bl, int an, int ss, bool rc) {
 
 std::unique_ptr<RingFFT> build_ring(int K) {
   auto r = std::make_unique<RingFFT>();
+  const RingTables h = ring_tables(K);
   r->K = K;
-  int P = 8, logP = 3;
-  while (P < 2 * K - 1) {
-    P <<= 1;
-    ++logP;
-  }
-  r->P = P;
-  r->logP = logP;
-  const long double pi = 3.141592653589793238462643383279502884197L;
-  std::vector<cxl> chirp(K), b(P, cxl(0.0L)), tw(3 * P / 4);
-  for (long k = 0; k < K; ++k) {
-    const long double x = pi * (long double)((k * k) % (2L * K)) / (long double)K;
-    chirp[k] = {cosl(x), sinl(x)};
-  }
-  for (int k = 0; k < 3 * P / 4; ++k) {
-    if (k >= P / 4) {  // w^k = -i w^(k - P/4)
-      tw[k] = {tw[k - P / 4].imag(), -tw[k - P / 4].real()};
-    } else {
-      const long double x = 2.0L * pi * (long double)k / (long double)P;
-      tw[k] = {cosl(x), -sinl(x)};
-    }
-  }
-  b[0] = chirp[0];
-  for (int k = 1; k < K; ++k) b[k] = b[P - k] = chirp[k];
-  host_fft(b, tw);
-  long double top = 0.0L;
-  for (const cxl &v : b) top = std::max(top, std::abs(v));
-  r->eb = 0;
-  while (ldexpl(1.0L, r->eb) < top) ++r->eb;
-  const auto fixed = [](const std::vector<cxl> &v, int e) {
-    std::vector<int4> o(v.size());
-    for (size_t i = 0; i < v.size(); ++i) o[i] = fixed62(ldexpl(v[i].real(), -e), ldexpl(v[i].imag(), -e));
-    return o;
+  r->P = h.P;
+  r->logP = h.logP;
+  r->eb = h.eb;
+  const auto up = [](const std::vector<int4> &v) {
+    int4 *d = dev_alloc<int4>(v.size());
+    S2G_CUDA(cudaMemcpy(d, v.data(), sizeof(int4) * v.size(), cudaMemcpyHostToDevice));
+    return d;
   };
-  // per level h of the radix-4 passes (P/4, P/16, ...): w^j, w^2j, w^3j for j = k P / (4h), k < h
-  const int h0 = logP & 1 ? 2 : 4;
-  std::vector<cxl> levels(P - h0);
-  for (int h = h0; h <= P / 4; h *= 4)
-    for (int c = 0; c < 3; ++c)
-      for (int k = 0; k < h; ++k) levels[h - h0 + c * h + k] = tw[(c + 1) * (k * (P / (4 * h)))];
-  const auto c4 = fixed(chirp, 0), b4 = fixed(b, r->eb), t4 = fixed(levels, 0);
-  r->chirp = dev_alloc<int4>(c4.size());
-  r->bhat = dev_alloc<int4>(b4.size());
-  r->tw = dev_alloc<int4>(t4.size());
-  S2G_CUDA(cudaMemcpy(r->chirp, c4.data(), sizeof(int4) * c4.size(), cudaMemcpyHostToDevice));
-  S2G_CUDA(cudaMemcpy(r->bhat, b4.data(), sizeof(int4) * b4.size(), cudaMemcpyHostToDevice));
-  S2G_CUDA(cudaMemcpy(r->tw, t4.data(), sizeof(int4) * t4.size(), cudaMemcpyHostToDevice));
+  r->chirp = up(h.chirp);
+  r->bhat = up(h.bhat);
+  r->tw = up(h.tw);
   return r;
 }
 
 }  // namespace
-
-int4 fixed62(long double re, long double im) {
-  const auto words = [](long double v, int &h, int &l) {
-    long long q = llroundl(ldexpl(v, 62));
-    l = (int)(unsigned)(unsigned long long)q;
-    if (l == INT32_MIN) l = (int)(unsigned)(unsigned long long)++q;  // |l| < 2^31
-    h = (int)((q - l) >> 32);
-  };
-  int4 o;
-  words(re, o.x, o.y);
-  words(im, o.z, o.w);
-  return o;
-}
 
 const WignerTable &wigner_table(int bl, int an, int ss, bool rc) {
   std::lock_guard<std::mutex> lk(g_plan_mu);

@@ -69,7 +69,7 @@ inline int grid_rings(int bl, int ss) { return ss ? bl + 1 : bl; }
 inline int grid_ring_len(int bl, int ss) { return ss ? 2 * bl : 2 * bl - 1; }
 
 // Bluestein data for ring length K (odd or even), padded FFT size P = 2^logP >=
-// max(2K-1, 8), as 62-bit fixed-point constants (fxarith.h)
+// max(2K-1, 8), as 62-bit fixed-point constants (fxarith.h), on the device (ringtables.h makes them)
 struct RingFFT {
   int K = 0, P = 0, logP = 0;
   int eb = 0;             // the kernel spectrum is bhat 2^eb
@@ -80,8 +80,6 @@ struct RingFFT {
   // w^j, w^2j, w^3j (j = k P / (4h), k < h) at h - h0, + h, + 2h: P - h0 entries
   int4 *tw = nullptr;
 };
-// re + i im (magnitude at most 1) as (re.h, re.l, im.h, im.l), v = (h 2^32 + l) 2^-62, |l| < 2^31
-int4 fixed62(long double re, long double im);
 
 // rc: recomputed (checkpointed) table instead of stored D and Q
 const WignerTable &wigner_table(int bl, int an, int ss = 0, bool rc = false);

@@ -4,21 +4,9 @@
 //
 // Arithmetic.  Block fixed point on 64-bit integers (fxarith.h): each ring (or
 // pair of real rings, or ring of all n-components) is scaled by one power of
-// two from its largest exponent field, transformed in integers, and widened
-// to FP64 once per output.  Forward and inverse transform are radix-4 with a
-// factor 1/4 per stage, which keeps every magnitude bounded (|sum of four / 4|
-// <= max) without a data-dependent branch; between the two transforms the
-// block is shifted up by the headroom measured on the block itself.  A
-// rounding error of about one unit per stage against a root-mean-square
-// level that halves per stage leaves about 2^-51 of a noise-like ring's level
-// at P = 4096 (and less at smaller P) on both transforms together: the
-// accuracy of an FP64 transform of the ring, which both precision modes use.
-// Bounds (K <= P/2 samples; components, not magnitudes):
-//   after the chirp            < 2^59.5   (2^61 input / 4; |re + i im| adds half a bit)
-//   forward stages             < 2^61     (the first, unscaled stage pair doubles at most)
-//   shifted                    < 2^61     (the next two stages do not raise a magnitude)
-//   times the kernel spectrum  < 2^59.5
-//   inverse stages             < 2^61.5   (sums of four before their 1/4; last pair unscaled)
+// two from its largest exponent field, transformed in integers (ringcore.h, with
+// the bounds and the accuracy: below an FP64 transform's error), and widened to
+// FP64 once per output.  Both precision modes use it.
 // A ring that holds an infinity or a NaN comes out as NaN.
 //
 // What bounds it: the wide multiply-adds (half rate) and the integer adds of
@@ -26,8 +14,8 @@
 // 45 adds and shifts, against 256 FP32 instructions in double-float and 32
 // FP64 instructions at 1/64 rate.  Measured, px2wav + wav2px at L = 1024, N = 4
 // (real maps), rings and gamma DFTs: 2 maps in FP64 19.2 ms with FP64
-// butterflies, 3.1 ms so; 32 maps at split precision 60.6 ms in double-float,
-// 45.6 ms so.
+// butterflies, 3.2 ms so; 32 maps at split precision 60.6 ms in double-float,
+// 47 ms so.
 //
 // Table data comes as 62-bit fixed point (RingFFT, plan.h): chirp exp(i pi k^2
 // / K), the passes' twiddles level by level (the passes below the first read
@@ -43,7 +31,8 @@
 #include <vector>
 
 #include "common.h"
-#include "fxarith.h"
+#include "ringcore.h"
+#include "ringtables.h"
 #include "kernels.h"
 #include "timing.h"
 
@@ -53,7 +42,7 @@ namespace {
 
 namespace cg = cooperative_groups;
 
-struct RingArgs {
+struct RingArgs : RingCore {
   const void *rings;
   void *rings_out;  // inverse: output rings
   int64_t ring_stride;  // between rings of one map
@@ -66,9 +55,8 @@ struct RingArgs {
   int spec_rpm;             // spectra per map
   int herm;                 // complex inverse: m < 0 taken as conj of m > 0 (real-valued ring)
   int sw, mlo;
-  int nrings, bl, K, P, logP;
-  int eb;  // the kernel spectrum is bhat 2^eb
-  const int4 *chirp, *bhat, *tw;
+  int nrings, bl, K;
+  const int4 *chirp;
 };
 
 // Jobs of one launch: blocks (fused: clusters) first[q] .. first[q + 1] belong to
@@ -167,224 +155,6 @@ __device__ __forceinline__ int64_t spec_base(const RingArgs &a, int r) {
   return (int64_t)(r / a.spec_rpm) * a.spec_map_stride + (int64_t)(r % a.spec_rpm) * a.spec_stride;
 }
 
-// Shared-memory layout: element i of the P = 2^lg point buffer (16-byte
-// complex values, no padding) lives at swz(i) = i ^ X(i), where X(i) XORs bits
-// 3-4 of i into bits 1-2, bits 3-5 into bits 0-2 and bits lg-3..lg-1 into bits
-// 0-2 (the last term only for lg > 6).  X depends only on bits >= 3 and sets
-// only bits 0-2, so swz is a bijection and its own inverse, and it is linear
-// over GF(2): swz(a ^ b) = swz(a) ^ swz(b).  Every access pattern below (bit-
-// reversed scatter and gather, the radix-4 passes at every span, stride-4 and
-// linear sweeps) then touches 8 distinct 16-byte bank groups per quarter warp
-// for P >= 256 (checked by enumerating the patterns on the CPU), without the
-// 1/8 padding a skewed layout needs.
-struct Swz {
-  int top;  // lg - 3 when lg > 6, else 31 (the term vanishes for non-negative i)
-};
-__device__ __forceinline__ Swz swz_of(int logP) { return Swz{logP > 6 ? logP - 3 : 31}; }
-__device__ __forceinline__ int swz(int i, Swz z) {
-  return i ^ ((i >> 2) & 6) ^ ((i >> 3) & 7) ^ ((i >> z.top) & 7);
-}
-__device__ __forceinline__ int brev(int k, int logP) { return (int)(__brev((unsigned)k) >> (32 - logP)); }
-// buffer slot of bit-reversed position k
-__device__ __forceinline__ int slot_brev(int k, int logP) { return swz(brev(k, logP), swz_of(logP)); }
-
-// Read-only table loads with an L1 eviction priority: the twiddle table is
-// read by every pass of every ring on the SM (kept: evict_last); the chirp and
-// the chirp-kernel spectrum are read once per ring (evict_first).
-__device__ __forceinline__ int4 ld_keep(const int4 *p) {
-  int4 v;
-  asm("ld.global.nc.L1::evict_last.v4.s32 {%0, %1, %2, %3}, [%4];"
-      : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-      : "l"(p));
-  return v;
-}
-__device__ __forceinline__ int4 ld_once(const int4 *p) {
-  int4 v;
-  asm("ld.global.nc.L1::evict_first.v4.s32 {%0, %1, %2, %3}, [%4];"
-      : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-      : "l"(p));
-  return v;
-}
-
-// bits of the high word's magnitude (headroom tracking)
-__device__ __forceinline__ int high_bits(longlong2 v) {
-  const int x = (int)(v.x >> 32), y = (int)(v.y >> 32);
-  return (x ^ (x >> 31)) | (y ^ (y >> 31));
-}
-
-// forward butterfly on bit-reversed data: stages s and s + 1 with
-// w1 = w^2j (elements 1), w2 = w^j (elements 2), w3 = w^3j (elements 3), over 4
-__device__ __forceinline__ void dit4(longlong2 &a0, longlong2 &a1, longlong2 &a2, longlong2 &a3, int4 w1, int4 w2,
-                                     int4 w3) {
-  const longlong2 t0 = fx_sar(a0, 2), t1 = fx_mul4(a1, w1), t2 = fx_mul4(a2, w2), t3 = fx_mul4(a3, w3);
-  const longlong2 b0 = fx_add(t0, t1), b1 = fx_sub(t0, t1), b2 = fx_add(t2, t3), b3 = fx_mul_i(fx_sub(t2, t3));
-  a0 = fx_add(b0, b2);
-  a2 = fx_sub(b0, b2);
-  a1 = fx_sub(b1, b3);
-  a3 = fx_add(b1, b3);
-}
-// inverse butterfly, natural to bit-reversed order, over 4
-__device__ __forceinline__ void dif4(longlong2 &a0, longlong2 &a1, longlong2 &a2, longlong2 &a3, int4 w1, int4 w2,
-                                     int4 w3) {
-  const longlong2 b0 = fx_add(a0, a2), b1 = fx_add(a1, a3), b2 = fx_sub(a0, a2), b3 = fx_mul_i(fx_sub(a1, a3));
-  a0 = fx_sar(fx_add(b0, b1), 2);
-  a1 = fx_mulc4(fx_sub(b0, b1), w1);
-  a2 = fx_mulc4(fx_add(b2, b3), w2);
-  a3 = fx_mulc4(fx_sub(b2, b3), w3);
-}
-
-// First pass of the Bluestein core, fused with the producer: value(j) is the
-// premultiplied a_j for j < P/2 (the second half of the padded sequence is zero
-// and is not stored), written to the even bit-reversed positions and their
-// neighbours.  Even log2 P: stages 1 and 2 of (a0, 0, a2, 0) with unit twiddles,
-// where a0 and a2 are the elements j and j + P/4; odd: a copy (stage 1 of
-// (a0, 0)).  Returns the magnitude bits of what it wrote.  With last_pass this
-// leaves two sweeps over the buffer and two barriers of a ring to its neighbours:
-// 64 maps at band-limit 128 0.800 -> 0.773 ms in the ring kernels, 32 at 256 1.385
-// -> 1.350; 8 at 1024 5.12 -> 5.07 (analysis), 5.18 -> 5.20 (synthesis).
-template <class V>
-__device__ __forceinline__ int first_pass(longlong2 *buf, int P, int logP, V value) {
-  int mx = 0;
-  if (logP & 1) {
-    for (int j = threadIdx.x; j < P / 2; j += blockDim.x) {
-      const int b = slot_brev(j, logP);
-      const longlong2 v = value(j);
-      buf[b] = v;
-      buf[b ^ 1] = v;
-      mx |= high_bits(v);
-    }
-  } else {
-    for (int j = threadIdx.x; j < P / 4; j += blockDim.x) {
-      const int b = slot_brev(j, logP);
-      const longlong2 a0 = value(j), a2 = value(j + P / 4), ia = fx_mul_i(a2);
-      const longlong2 v0 = fx_add(a0, a2), v2 = fx_sub(a0, a2), v1 = fx_sub(a0, ia), v3 = fx_add(a0, ia);
-      buf[b] = v0;
-      buf[b ^ 1] = v1;
-      buf[b ^ 2] = v2;
-      buf[b ^ 3] = v3;
-      mx |= high_bits(v0) | high_bits(v1) | high_bits(v2) | high_bits(v3);
-    }
-  }
-  return mx;
-}
-// Last pass, fused with the consumer: y_k for k < P/2 from the buffer that
-// bluestein() leaves (unit twiddles; the other half of the outputs is not formed).
-__device__ __forceinline__ longlong2 last_pass(const longlong2 *buf, int P, int logP, int k) {
-  if (logP & 1) {
-    const int b = slot_brev(k, logP);
-    return fx_add(buf[b], buf[b ^ 1]);
-  }
-  const int b = slot_brev(k & (P / 4 - 1), logP);
-  const longlong2 a0 = buf[b], a1 = buf[b ^ 1], a2 = buf[b ^ 2], a3 = buf[b ^ 3];
-  return k < P / 4 ? fx_add(fx_add(a0, a2), fx_add(a1, a3)) : fx_add(fx_sub(a0, a2), fx_mul_i(fx_sub(a1, a3)));
-}
-// the same in place, for consumers that read other CTAs' buffers:
-// slot_brev(k) <- f(k, y_k) for k < n
-template <class F>
-__device__ __forceinline__ void last_pass_in_place(longlong2 *buf, int P, int logP, int n, F f) {
-  if (logP & 1) {
-    for (int k = threadIdx.x; k < n; k += blockDim.x) {
-      const int b = slot_brev(k, logP);
-      buf[b] = f(k, fx_add(buf[b], buf[b ^ 1]));
-    }
-  } else {
-    for (int k = threadIdx.x; k < P / 4; k += blockDim.x) {
-      const int b = slot_brev(k, logP);
-      const longlong2 a0 = buf[b], a1 = buf[b ^ 1], a2 = buf[b ^ 2], a3 = buf[b ^ 3];
-      if (k < n) buf[b] = f(k, fx_add(fx_add(a0, a2), fx_add(a1, a3)));
-      if (k + P / 4 < n) buf[b ^ 2] = f(k + P / 4, fx_add(fx_sub(a0, a2), fx_mul_i(fx_sub(a1, a3))));
-    }
-  }
-}
-
-// Bluestein core between first_pass (barrier not yet passed; mx its result) and
-// last_pass (barrier passed): the buffer then holds y_k 2^S before the last pass,
-// y the convolution times P, S the sum of the scalings.  Returns the shift
-// applied between the transforms.  P >= 8.
-//   radix-4 passes; the last of them, the kernel-spectrum product and the first
-//   inverse pass work on the same four elements and stay in registers; inverse
-//   radix-4 passes.
-__device__ int bluestein(longlong2 *buf, const RingArgs &a, int *s_mx, int mx) {
-  const int P = a.P, logP = a.logP;
-  const int4 *__restrict__ tw = a.tw;
-  const Swz z = swz_of(logP);
-  const int h0 = logP & 1 ? 2 : 4;
-  int s = logP & 1 ? 2 : 3;
-  if (s + 1 < logP) mx = 0;  // a radix-4 pass follows and tracks its own outputs
-  if (threadIdx.x == 0) *s_mx = 0;
-  __syncthreads();
-  for (; s + 1 < logP; s += 2) {
-    const int h = 1 << (s - 1);
-    const int q1 = swz(h, z), q2 = swz(2 * h, z), q3 = swz(3 * h, z);
-    const bool track = s + 3 == logP;
-    for (int i = threadIdx.x; i < P / 4; i += blockDim.x) {
-      const int jp = i & (h - 1);
-      const int b = swz(((i >> (s - 1)) << (s + 1)) + jp, z);
-      const int4 *w = tw + (h - h0) + jp;
-      const int4 w2 = ld_keep(w), w1 = ld_keep(w + h), w3 = ld_keep(w + 2 * h);
-      longlong2 a0 = buf[b], a1 = buf[b ^ q1], a2 = buf[b ^ q2], a3 = buf[b ^ q3];
-      dit4(a0, a1, a2, a3, w1, w2, w3);
-      buf[b] = a0;
-      buf[b ^ q1] = a1;
-      buf[b ^ q2] = a2;
-      buf[b ^ q3] = a3;
-      if (track) mx |= high_bits(a0) | high_bits(a1) | high_bits(a2) | high_bits(a3);
-    }
-    if (!track) __syncthreads();
-  }
-  mx = __reduce_or_sync(0xffffffffu, mx);
-  if ((threadIdx.x & 31) == 0) atomicOr(s_mx, mx);
-  __syncthreads();
-  const int sh = max(0, __clz(*s_mx) - 3);  // components < 2^61 afterwards
-  {  // last forward pass, kernel spectrum, first inverse pass
-    const int h = P / 4;
-    const int q1 = swz(h, z), q2 = swz(2 * h, z), q3 = swz(3 * h, z);
-    for (int i = threadIdx.x; i < h; i += blockDim.x) {
-      const int b = swz(i, z);
-      longlong2 a0 = fx_shl(buf[b], sh), a1 = fx_shl(buf[b ^ q1], sh), a2 = fx_shl(buf[b ^ q2], sh),
-                a3 = fx_shl(buf[b ^ q3], sh);
-      const int4 *w = tw + (h - h0) + i;
-      const int4 w2 = ld_once(w), w1 = ld_once(w + h), w3 = ld_once(w + 2 * h);
-      dit4(a0, a1, a2, a3, w1, w2, w3);
-      a0 = fx_mul4(a0, ld_once(&a.bhat[i]));
-      a1 = fx_mul4(a1, ld_once(&a.bhat[i + h]));
-      a2 = fx_mul4(a2, ld_once(&a.bhat[i + 2 * h]));
-      a3 = fx_mul4(a3, ld_once(&a.bhat[i + 3 * h]));
-      dif4(a0, a1, a2, a3, w1, w2, w3);
-      buf[b] = a0;
-      buf[b ^ q1] = a1;
-      buf[b ^ q2] = a2;
-      buf[b ^ q3] = a3;
-    }
-    __syncthreads();
-  }
-  for (s = logP - 2; s >= 3; s -= 2) {
-    const int h = 1 << (s - 2);
-    const int q1 = swz(h, z), q2 = swz(2 * h, z), q3 = swz(3 * h, z);
-    for (int i = threadIdx.x; i < P / 4; i += blockDim.x) {
-      const int jp = i & (h - 1);
-      const int b = swz(((i >> (s - 2)) << s) + jp, z);
-      const int4 *w = tw + (h - h0) + jp;
-      const int4 w2 = ld_keep(w), w1 = ld_keep(w + h), w3 = ld_keep(w + 2 * h);
-      longlong2 a0 = buf[b], a1 = buf[b ^ q1], a2 = buf[b ^ q2], a3 = buf[b ^ q3];
-      dif4(a0, a1, a2, a3, w1, w2, w3);
-      buf[b] = a0;
-      buf[b ^ q1] = a1;
-      buf[b ^ q2] = a2;
-      buf[b ^ q3] = a3;
-    }
-    __syncthreads();
-  }
-  return sh;
-}
-// a value q in the buffer of a block with exponent e, split to `bits` bits, is
-// q 2^k after the chirp (over 4) and the core: 2 per radix-4 pass and product,
-// the shift, the kernel spectrum's exponent, and the 1/P of the transforms
-__device__ __forceinline__ int core_exponent(const RingArgs &a, int e, int bits, int sh) {
-  const int passes = (a.logP - 1) >> 1;  // radix-4 passes of one direction
-  return e - bits + 2 + 4 * passes + 2 + a.eb - sh - a.logP;
-}
-
 // block-wide max of an int (blockDim.x <= 1024)
 __device__ int block_max_int(int v) {
   __shared__ int redi[32];
@@ -408,12 +178,13 @@ constexpr int kRingThreads = 256;
 template <bool REAL, bool F32>
 __global__ void __launch_bounds__(kRingThreads, 3) k_ring_forward(const __grid_constant__ RingGroup grp) {
   extern __shared__ longlong2 buf[];
-  __shared__ int s_mx;
+  __shared__ int s_mx[kRingSlots];
   const int job = job_of(grp, blockIdx.x), blk = blockIdx.x - grp.first[job];
   const RingArgs a = grp.a[job];  // by value: read once from the parameters
   const int K = a.K, P = a.P, logP = a.logP;
   const int r0 = REAL ? 2 * blk : blk;
   const bool has1 = REAL && (r0 + 1 < a.nrings);
+  if (threadIdx.x < kRingSlots) s_mx[threadIdx.x] = 0;  // before the barriers of the maximum
   int em = 0;
   for (int j = threadIdx.x; j < K; j += blockDim.x) {
     if (REAL) {
@@ -425,7 +196,7 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_ring_forward(const __grid_c
   }
   em = block_max_int(em);
   const int e = fx_exp(em);
-  const int mx = first_pass(buf, P, logP, [&](int j) {
+  first_pass(RingThreads{}, buf, P, logP, [&](int j) {
     longlong2 v = make_longlong2(0, 0);
     if (j < K) {
       double2 x;
@@ -435,12 +206,12 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_ring_forward(const __grid_c
       } else {
         x = ld_px2<F32>(a.rings, ring_base(a, r0) + j);
       }
-      v = fx_mulc4(fx_split2<61>(x, e), ld_once(&a.chirp[j]));  // x_j conj(c_j)
+      v = fx_mulc4(fx_split2<62>(x, e), ld_once(&a.chirp[j]));  // x_j conj(c_j) / 4
     }
     return v;
   });
-  const int sh = bluestein(buf, a, &s_mx, mx);
-  const int k0 = core_exponent(a, e, 61, sh);
+  const int sh = bluestein(RingThreads{}, buf, a, s_mx);
+  const int k0 = core_exponent(a, e - 60, sh);
   if (!REAL) {
     double2 *out = a.spec_out + spec_base(a, r0);
     for (int c = threadIdx.x; c < a.sw; c += blockDim.x) {
@@ -453,13 +224,13 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_ring_forward(const __grid_c
     double2 *out0 = a.spec_out + spec_base(a, r0);
     for (int m = threadIdx.x; m < a.sw; m += blockDim.x) {
       const int km = m ? K - m : 0;
-      const longlong2 zm = fx_mulc(last_pass(buf, P, logP, m), ld_once(&a.chirp[m]));
-      const longlong2 zc = fx_conj(fx_mulc(last_pass(buf, P, logP, km), ld_once(&a.chirp[km])));
+      const longlong2 zm = fx_mulc2(last_pass(buf, P, logP, m), ld_once(&a.chirp[m]));
+      const longlong2 zc = fx_conj(fx_mulc2(last_pass(buf, P, logP, km), ld_once(&a.chirp[km])));
       // A = (Z_m + conj Z_{-m})/2,  B = (Z_m - conj Z_{-m})/(2i)
-      out0[m] = em == kExpNonFinite ? nan2() : fx_join2(fx_add(zm, zc), k0 - 1);
+      out0[m] = em == kExpNonFinite ? nan2() : fx_join2(fx_add(zm, zc), k0);
       if (has1) {
         const longlong2 d = fx_sub(zm, zc);
-        out0[a.spec_stride + m] = em == kExpNonFinite ? nan2() : fx_join2(make_longlong2(d.y, -d.x), k0 - 1);
+        out0[a.spec_stride + m] = em == kExpNonFinite ? nan2() : fx_join2(make_longlong2(d.y, -d.x), k0);
       }
     }
   }
@@ -468,14 +239,15 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_ring_forward(const __grid_c
 template <bool REAL, bool F32>
 __global__ void __launch_bounds__(kRingThreads, 3) k_ring_inverse(const __grid_constant__ RingGroup grp) {
   extern __shared__ longlong2 buf[];
-  __shared__ int s_mx;
+  __shared__ int s_mx[kRingSlots];
   const int job = job_of(grp, blockIdx.x), blk = blockIdx.x - grp.first[job];
   const RingArgs a = grp.a[job];  // by value: read once from the parameters
-  constexpr int BITS = REAL ? 60 : 61;  // A + i B of two rings
+  constexpr int BITS = REAL ? 61 : 62;  // A + i B of two rings
   const int K = a.K, P = a.P, logP = a.logP, bl = a.bl;
   const int r0 = REAL ? 2 * blk : blk;
   const bool has1 = REAL && (r0 + 1 < a.nrings);
   const double2 *s0 = a.spec_in + spec_base(a, r0);
+  if (threadIdx.x < kRingSlots) s_mx[threadIdx.x] = 0;  // before the barriers of the maximum
   int em = 0;
   for (int c = threadIdx.x; c < a.sw; c += blockDim.x) {
     em = emax2(em, s0[c]);
@@ -483,7 +255,7 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_ring_inverse(const __grid_c
   }
   em = block_max_int(em);
   const int e = fx_exp(em);
-  const int mx = first_pass(buf, P, logP, [&](int j) {
+  first_pass(RingThreads{}, buf, P, logP, [&](int j) {
     longlong2 v = make_longlong2(0, 0);
     if (j < K) {
       const int m = (j < bl) ? j : j - K;  // frequency of DFT bin j
@@ -510,8 +282,8 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_ring_inverse(const __grid_c
     }
     return v;
   });
-  const int sh = bluestein(buf, a, &s_mx, mx);
-  const int k0 = core_exponent(a, e, BITS, sh);
+  const int sh = bluestein(RingThreads{}, buf, a, s_mx);
+  const int k0 = core_exponent(a, e - BITS + 2, sh);
   for (int p = threadIdx.x; p < K; p += blockDim.x) {
     // f_p = c_p conj(y_p)
     const longlong2 y = fx_mul(fx_conj(last_pass(buf, P, logP, p)), ld_once(&a.chirp[p]));
@@ -560,7 +332,7 @@ __device__ __forceinline__ int cluster_max_int(cg::cluster_group &cl, int *slot,
 template <int NN, bool REAL, bool F32>
 __global__ void __launch_bounds__(kRingThreads, 3) k_ring_inverse_gamma(const __grid_constant__ GammaFuse grp) {
   extern __shared__ longlong2 buf[];
-  __shared__ int s_mx, s_em, s_k;
+  __shared__ int s_mx[kRingSlots], s_em, s_k;
   cg::cluster_group cl = cg::this_cluster();
   const int k = (int)cl.block_rank();
   const int job = job_of(grp, blockIdx.x / NN), r = blockIdx.x / NN - grp.first[job];
@@ -571,27 +343,29 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_ring_inverse_gamma(const __
   const bool herm = (k == grp.herm_k);
   const int sw = herm ? bl : gf.W, mlo = herm ? 0 : -(bl - 1);
   const double2 *s0 = gf.G + (int64_t)b * gf.gms + (int64_t)k * gf.gks + (int64_t)t * gf.W + (herm ? bl - 1 : 0);
+  if (threadIdx.x < kRingSlots) s_mx[threadIdx.x] = 0;  // before the barriers of the maximum
   int em = 0;
   for (int c = threadIdx.x; c < sw; c += blockDim.x) em = emax2(em, s0[c]);
   em = cluster_max_int(cl, &s_em, em, NN);
   const int e = fx_exp(em);
-  const int mx = first_pass(buf, P, logP, [&](int j) {
+  first_pass(RingThreads{}, buf, P, logP, [&](int j) {
     longlong2 v = make_longlong2(0, 0);
     if (j < K) {
       const int m = (j < bl) ? j : j - K;
       const int c = m - mlo;
       if (c >= 0 && c < sw)
-        v = fx_split2<61>(s0[c], e);
+        v = fx_split2<62>(s0[c], e);
       else if (herm && m < 0 && -m < sw)
-        v = fx_conj(fx_split2<61>(s0[-m], e));
+        v = fx_conj(fx_split2<62>(s0[-m], e));
       v = fx_conj(fx_mul4(v, ld_once(&a.chirp[j])));
     }
     return v;
   });
-  const int sh = bluestein(buf, a, &s_mx, mx);
-  // F_k(p) = c_p conj(y_p), in place (p -> brev(p) is one-to-one); components < 2^61.5
-  last_pass_in_place(buf, P, logP, K, [&](int p, longlong2 y) { return fx_mul(fx_conj(y), ld_once(&a.chirp[p])); });
-  if (threadIdx.x == 0) s_k = core_exponent(a, e, 61, sh);
+  const int sh = bluestein(RingThreads{}, buf, a, s_mx);
+  // F_k(p) / 2 = c_p conj(y_p) / 2, in place (p -> brev(p) is one-to-one); components < 2^61.5
+  last_pass_in_place(RingThreads{}, buf, P, logP, K,
+                     [&](int p, longlong2 y) { return fx_mul2(fx_conj(y), ld_once(&a.chirp[p])); });
+  if (threadIdx.x == 0) s_k = core_exponent(a, e - 60, sh) + 1;
   cl.sync();
   // gamma slices of this CTA's share of the pixels
   int kj[NN], km = INT_MIN;
@@ -647,7 +421,7 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_ring_inverse_gamma(const __
 template <int NN, bool REAL, bool F32>
 __global__ void __launch_bounds__(kRingThreads, 3) k_gamma_ring_forward(const __grid_constant__ GammaFuse grp) {
   extern __shared__ longlong2 buf[];
-  __shared__ int s_mx, s_em;
+  __shared__ int s_mx[kRingSlots], s_em;
   cg::cluster_group cl = cg::this_cluster();
   const int k = (int)cl.block_rank();
   const int job = job_of(grp, blockIdx.x / NN), r = blockIdx.x / NN - grp.first[job];
@@ -658,6 +432,7 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_gamma_ring_forward(const __
   const int chunk = (K + NN - 1) / NN;
   const int p0 = k * chunk, p1 = min(K, p0 + chunk);
   const int64_t ibase = (int64_t)b * gf.fms + (int64_t)t * K;
+  if (threadIdx.x < kRingSlots) s_mx[threadIdx.x] = 0;  // before the barriers of the maximum
   int em = 0;
   for (int p = p0 + threadIdx.x; p < p1; p += blockDim.x)
     for (int g = 0; g < grp.ng; ++g) {
@@ -674,7 +449,7 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_gamma_ring_forward(const __
   // gamma_g and gamma_{ng-g} have conjugate twiddles w = C + i S and C - i S:
   // each pair contributes C (f_g + f_{ng-g}) + i S (f_g - f_{ng-g}).  The
   // twiddles' magnitudes sum to at most 1 over g (et), so F_k / 4 stays below
-  // 2^59.5 and the chirp is applied at full scale.
+  // 2^59.5 and leaves the chirp twice as large.
   for (int p = p0 + threadIdx.x; p < p1; p += blockDim.x) {
     longlong2 acc[NN];
 #pragma unroll
@@ -708,14 +483,13 @@ __global__ void __launch_bounds__(kRingThreads, 3) k_gamma_ring_forward(const __
     const int4 ch = ld_once(&a.chirp[p]);
     const int i = slot_brev(p, logP);
 #pragma unroll
-    for (int j = 0; j < NN; ++j) *cl.map_shared_rank(buf + i, j) = fx_mulc(acc[j], ch);
+    for (int j = 0; j < NN; ++j) *cl.map_shared_rank(buf + i, j) = fx_product<3, true>(acc[j], ch);
   }
   cl.sync();  // every component's buffer is complete
   // in place: a thread reads only the slots that it writes
-  const int mx = first_pass(buf, P, logP, [&](int j) { return buf[slot_brev(j, logP)]; });
-  const int sh = bluestein(buf, a, &s_mx, mx);
-  // split to 61 bits, over 4 in the gamma sums as after a scaled chirp, times 2^et
-  const int k0 = core_exponent(a, e, 61, sh) + grp.et;
+  first_pass(RingThreads{}, buf, P, logP, [&](int j) { return buf[slot_brev(j, logP)]; });
+  const int sh = bluestein(RingThreads{}, buf, a, s_mx);
+  const int k0 = core_exponent(a, e - 60 + grp.et, sh);
   double2 *out = gf.Gout + (int64_t)b * gf.gms + (int64_t)k * gf.gks + (int64_t)t * gf.W;
   for (int c = threadIdx.x; c < gf.W; c += blockDim.x) {
     const int m = c - (a.bl - 1);

@@ -1,0 +1,172 @@
+"""Host run of the ring transforms' fixed-point core (s2let_gb300/csrc/ringcore.h
+with the constants of ringtables.h): every kind of ring that loses or keeps bits
+in a scaled transform, against an extended-precision Bluestein transform, and
+beside an FP64 one.  The bound is the FP64 transform's own error of the same
+ring: fixed point must not be the less accurate of the two."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CSRC = os.path.join(HERE, "..", "s2let_gb300", "csrc")
+CUDA = next((os.path.join(d, "include") for d in (os.environ.get("CUDA_HOME", ""), "/usr/local/cuda")
+             if d and os.path.exists(os.path.join(d, "include", "cuda_runtime.h"))), None)
+
+HARNESS = r"""
+#include <cstdio>
+#include <cstdlib>
+#include <random>
+#include <string>
+#include "ringcore.h"
+#include "ringtables.h"
+using namespace s2g;
+using cd = std::complex<double>;
+template <class T> using vec = std::vector<std::complex<T>>;
+
+// forward DFT by Bluestein in precision T, its constants computed in T
+template <class T> std::complex<T> mulc_(std::complex<T> a, std::complex<T> b) {
+  return {a.real() * b.real() - a.imag() * b.imag(), a.real() * b.imag() + a.imag() * b.real()};
+}
+template <class T> void fft_(vec<T> &x, const vec<T> &w) {
+  const size_t n = x.size();
+  for (size_t i = 1, j = 0; i < n; ++i) {
+    size_t bit = n >> 1;
+    for (; j & bit; bit >>= 1) j ^= bit;
+    j ^= bit;
+    if (i < j) std::swap(x[i], x[j]);
+  }
+  for (size_t len = 2; len <= n; len <<= 1)
+    for (size_t i = 0; i < n; i += len)
+      for (size_t k = 0; k < len / 2; ++k) {
+        const auto u = x[i + k], v = mulc_(x[i + k + len / 2], w[k * (n / len)]);
+        x[i + k] = u + v;
+        x[i + k + len / 2] = u - v;
+      }
+}
+template <class T> vec<T> bluestein_ref(const vec<T> &x, int P) {
+  const int K = (int)x.size();
+  const T pi = (T)3.141592653589793238462643383279502884197L;
+  vec<T> c(K), w(P / 2), a(P), b(P);
+  for (long k = 0; k < K; ++k) {
+    const T t = pi * (T)((k * k) % (2L * K)) / (T)K;
+    c[k] = {std::cos(t), std::sin(t)};
+  }
+  for (int k = 0; k < P / 2; ++k) w[k] = {std::cos(2 * pi * (T)k / (T)P), -std::sin(2 * pi * (T)k / (T)P)};
+  for (int k = 0; k < K; ++k) {
+    a[k] = mulc_(x[k], std::conj(c[k]));
+    b[k] = c[k];
+    if (k) b[P - k] = c[k];
+  }
+  fft_(a, w);
+  fft_(b, w);
+  for (int k = 0; k < P; ++k) a[k] = std::conj(mulc_(a[k], b[k]));
+  fft_(a, w);  // conj(FFT(conj .)) is the inverse
+  vec<T> y(K);
+  for (int k = 0; k < K; ++k) y[k] = mulc_(std::conj(a[k]), std::conj(c[k])) / (T)P;
+  return y;
+}
+// as k_ring_forward<false>
+std::vector<cd> fixed_point(const std::vector<cd> &x, const RingTables &t) {
+  const int K = (int)x.size();
+  const RingCore a{t.P, t.logP, t.eb, t.bhat.data(), t.tw.data()};
+  std::vector<longlong2> buf(t.P);
+  int em = 0, slots[kRingSlots] = {};
+  for (const cd &v : x) em = std::max(em, std::max(exp_field(v.real()), exp_field(v.imag())));
+  const int e = fx_exp(em);
+  first_pass(RingThreads{}, buf.data(), t.P, t.logP, [&](int j) {
+    return j < K ? fx_mulc4(fx_split2<62>(make_double2(x[j].real(), x[j].imag()), e), t.chirp[j]) : make_longlong2(0, 0);
+  });
+  const int k0 = core_exponent(a, e - 60, bluestein(RingThreads{}, buf.data(), a, slots));
+  std::vector<cd> y(K);
+  for (int k = 0; k < K; ++k) {
+    const double2 v = fx_join2(fx_mulc(last_pass(buf.data(), t.P, t.logP, k), t.chirp[k]), k0);
+    y[k] = {v.x, v.y};
+  }
+  return y;
+}
+double err(const std::vector<cd> &y, const vec<long double> &r) {
+  long double e = 0, n = 0;
+  for (size_t k = 0; k < y.size(); ++k) {
+    e += std::norm(std::complex<long double>(y[k].real(), y[k].imag()) - r[k]);
+    n += std::norm(r[k]);
+  }
+  return (double)sqrtl(e / n);
+}
+int main(int argc, char **argv) {
+  const int K = atoi(argv[1]);
+  const RingTables t = ring_tables(K);
+  std::mt19937_64 g(K);
+  std::normal_distribution<double> nd;
+  const auto noise = [&] { return cd(nd(g), nd(g)); };
+  const auto show = [&](const std::string &name, auto f) {
+    std::vector<cd> x(K);
+    vec<long double> xl(K);
+    for (int k = 0; k < K; ++k) {
+      x[k] = f(k, std::min(k, K - k));
+      xl[k] = {x[k].real(), x[k].imag()};
+    }
+    const auto r = bluestein_ref<long double>(xl, t.P);
+    if (K < 200) {  // the reference against the plain sum
+      for (int k = 0; k < K; ++k) {
+        std::complex<long double> s = 0;
+        for (int j = 0; j < K; ++j) {
+          const long double q = 2 * 3.141592653589793238462643383279502884197L * ((long)j * k % K) / K;
+          s += xl[j] * std::complex<long double>(cosl(q), -sinl(q));
+        }
+        long double n = 0;
+        for (const auto &v : xl) n += std::norm(v);
+        if (std::abs(s - r[k]) > 1e-17L * sqrtl(n * K)) exit(2);
+      }
+    }
+    std::printf("%s %.3e %.3e\n", name.c_str(), err(fixed_point(x, t), r), err(bluestein_ref<double>(x, t.P), r));
+  };
+  const double pi = 3.14159265358979323846;
+  show("white", [&](int, int) { return noise(); });
+  show("real-pair", [&](int, int) { return cd(nd(g), 1e-3 * nd(g)); });
+  for (int p = 1; p <= 6; ++p)
+    show("steep" + std::to_string(p), [&](int, int m) { return noise() * std::pow(1.0 + m, -0.7 * p); });
+  show("smooth", [&](int, int m) { return cd(std::pow(1.0 + m, -3.0), 0); });
+  show("decay", [&](int k, int) { return cd(std::exp(-30.0 * k / K), 0); });
+  show("delta", [&](int k, int) { return cd(k == K / 3 ? 1.37 : 0.0, 0); });
+  show("delta0", [&](int k, int) { return cd(k == 0 ? 1.37 : 0.0, 0.1 * (k == 0)); });
+  show("sparse", [&](int k, int) { return k % (K / 5) == 1 ? noise() : cd(0, 0); });
+  show("constant", [&](int, int) { return cd(1, 0); });
+  show("offset", [&](int, int) { return cd(1e6 + nd(g), nd(g)); });
+  show("mode", [&](int k, int) { const double a = 2 * pi * ((long)k * (K / 5) % K) / K; return cd(cos(a), sin(a)); });
+  for (int s : {1, -1})
+    show(s > 0 ? "chirp" : "chirp-conj", [&](int k, int) {
+      const double a = s * pi * ((long)k * k % (2L * K)) / K;
+      return 0.93 * cd(cos(a), sin(a));
+    });
+  show("chirp+noise", [&](int k, int) {
+    const double a = pi * ((long)k * k % (2L * K)) / K;
+    return cd(cos(a), sin(a)) + 1e-3 * noise();
+  });
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def harness(tmp_path_factory):
+    if shutil.which("g++") is None or CUDA is None:
+        pytest.skip("needs g++ and the CUDA headers")
+    d = tmp_path_factory.mktemp("ringcore")
+    (d / "h.cpp").write_text(HARNESS)
+    subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", f"-I{CSRC}", f"-I{CUDA}", str(d / "h.cpp"), "-o",
+                    str(d / "h")], check=True)
+    return str(d / "h")
+
+
+# ring lengths: padded lengths 256 to 8192, log2 even and odd, just below a
+# power of two and just above one (odd on MW, even on MWSS sampling)
+@pytest.mark.parametrize("K", [127, 128, 200, 255, 361, 511, 723, 767, 1023, 1024, 1025, 1533, 2047, 2049, 2600, 4095])
+def test_not_less_accurate_than_fp64(harness, K):
+    out = subprocess.run([harness, str(K)], capture_output=True, text=True)
+    assert out.returncode == 0, out.returncode
+    for line in out.stdout.splitlines():
+        name, fixed, fp64 = line.split()
+        # an FP64 transform may be exact on a ring (a spike at its first sample); half a
+        # unit of the rounded outputs is always allowed
+        assert float(fixed) <= max(float(fp64), 2.0 ** -53), line
