@@ -34,6 +34,7 @@
 #include "ringcore.h"
 #include "ringtables.h"
 #include "kernels.h"
+#include "smemlimit.h"
 #include "timing.h"
 
 namespace s2g {
@@ -529,16 +530,10 @@ size_t ring_smem(int P) { return sizeof(longlong2) * (size_t)P; }
 // the rest to the L1.  Room for only three CTAs whatever their size kept the
 // small rings' CTAs of 32 to 128 threads from filling the SM: 64 maps at
 // band-limit 128 took 1.19 ms in the ring kernels and take 0.80, at 48 0.34 and
-// 0.21; band-limit 1024 is unchanged.  Set when a kernel's buffer size changes.
+// 0.21; band-limit 1024 is unchanged.
 void ring_smem_attrs(const void *kernel, int P) {
   const size_t smem = ring_smem(P);
   const int ctas = std::min(32, 3 * kRingThreads / ring_threads(P));
-  static std::mutex mu;
-  static std::map<const void *, size_t> set;
-  std::lock_guard<std::mutex> lk(mu);
-  size_t &cur = set[kernel];
-  if (cur == smem) return;
-  if (smem > 48 * 1024) S2G_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   constexpr int kSizes[] = {8, 16, 32, 64, 100, 132, 164, 196, 228};  // KB of shared memory an SM can set aside
   int kb = 228;
   for (int k : kSizes)
@@ -546,8 +541,11 @@ void ring_smem_attrs(const void *kernel, int P) {
       kb = k;
       break;
     }
-  S2G_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100 * kb / 228));
-  cur = smem;
+  static SharedMemoryLimits limits;
+  limits.prepare(
+      kernel, smem, 100 * kb / 228,
+      [&](size_t b) { S2G_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b)); },
+      [&](int c) { S2G_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, c)); });
 }
 
 int largest_P(const RingGroup &g) {
@@ -690,8 +688,11 @@ bool cluster_fits(int nn, int P) {
     const cudaLaunchConfig_t cfg = fused_config(nn, nn, P, at, nullptr);
     int nclusters = 0;
     const cudaError_t e = cudaOccupancyMaxActiveClusters(&nclusters, kern, &cfg);
-    if (e != cudaSuccess) cudaGetLastError();  // a refusal only means: not fusable here
-    ok = e == cudaSuccess && nclusters > 0;
+    if (e != cudaSuccess) {  // not fusable in this call; asked again by the next
+      cudaGetLastError();
+      return false;
+    }
+    ok = nclusters > 0;
   }
   known[key] = ok;
   return ok;
