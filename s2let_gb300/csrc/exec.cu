@@ -598,12 +598,16 @@ std::vector<std::vector<int>> table_directions(const WavPlan &P, const Scale &sd
   return out;
 }
 
-// The scales whose contractions are small (contract_is_small) run together:
+// The scales whose contractions are small (contract_small_max) run together:
 // one launch for the contractions of all of them, one for their ring DFTs.
-bool small_scale(const WavPlan &P, const Scale &sd, int nb) {
-  for (int n : sd.ns)
-    if (!contract_is_small(&P.table(sd.bl, std::abs(n)), nb)) return false;
-  return true;
+// Asked once per call: the answer depends on a switch of the process
+// (s2let_gpu_set_df_max_maps) that another thread may turn meanwhile, and the
+// spectra are allocated by it.
+std::vector<char> small_scales(const WavPlan &P, int nb) {
+  const int limit = contract_small_max(nb);
+  std::vector<char> out;
+  for (const Scale &sd : P.sc) out.push_back(!P.rc(sd.bl) && sd.bl <= limit);
+  return out;
 }
 
 // Jobs of ring DFTs collected for shared launches: those fused with the gamma
@@ -789,10 +793,12 @@ void wav_split(const WavPlan &P, SplitMode mode, const double2 *flm, bool flm_ha
   const int64_t Kmax = 2 * P.max_bl, ntmax = P.nt(P.max_bl);
   if (needs_ring_buffer(P)) spec = S.get<double2>((int64_t)nb * std::max(P.max_ng, P.max_nn) * ntmax * Kmax);
   const auto gsize = [&](const Scale &sd) { return (int64_t)nb * (int64_t)sd.ns.size() * P.nt(sd.bl) * (2 * sd.bl - 1); };
+  const std::vector<char> is_small = small_scales(P, nb);
   const auto run_small = [&] {
     std::vector<std::pair<const Scale *, double2 *>> sc;
-    for (const Scale &sd : P.sc)
-      if (small_scale(P, sd, nb)) {
+    for (size_t k = 0; k < P.sc.size(); ++k)
+      if (is_small[k]) {
+        const Scale &sd = P.sc[k];
         double2 *G = S.get<double2>(gsize(sd));
         for (size_t i = 0; i < sd.ns.size(); ++i) small.push_back(problem(sd, (int)i, G));
         sc.emplace_back(&sd, G);
@@ -809,14 +815,14 @@ void wav_split(const WavPlan &P, SplitMode mode, const double2 *flm, bool flm_ha
   const auto passes = table_passes(P, pipe != nullptr, nb);
   int64_t gtot = 0;  // spectra of one pass, reused by the next
   for (const auto &pk : passes)
-    if (!small_scale(P, P.sc[pk.first], nb))
+    if (!is_small[pk.first])
       gtot = std::max(gtot, (int64_t)(pk.second - pk.first) * gsize(P.sc[pk.first]));
   double2 *Gbuf = gtot ? S.get<double2>(gtot) : nullptr;
   std::vector<RingJob> scal_ring;
   if (pipe) scal_ring.swap(rings.plain);  // the scaling function goes with the small scales
   for (const auto &pk : passes) {
     const Scale &s0 = P.sc[pk.first];
-    if (small_scale(P, s0, nb)) continue;
+    if (is_small[pk.first]) continue;
     const int ngrp = (int)(pk.second - pk.first);
     const int64_t gsz = gsize(s0);
     for (const auto &dirs : table_directions(P, s0)) {
@@ -953,9 +959,11 @@ void wav_merge(const WavPlan &P, MergeMode mode, const void *f_wav, int64_t wstr
   const int64_t Kmax = 2 * P.max_bl, ntmax = P.nt(P.max_bl);
   if (needs_ring_buffer(P)) spec = S.get<double2>((int64_t)nb * std::max(P.max_ng, P.max_nn) * ntmax * Kmax);
   const auto gsize = [&](const Scale &sd) { return (int64_t)nb * (int64_t)sd.ns.size() * P.nt(sd.bl) * (2 * sd.bl - 1); };
+  const std::vector<char> is_small = small_scales(P, nb);
   const auto run_small = [&] {
-    for (const Scale &sd : P.sc)
-      if (small_scale(P, sd, nb)) {
+    for (size_t k = 0; k < P.sc.size(); ++k)
+      if (is_small[k]) {
+        const Scale &sd = P.sc[k];
         double2 *G = S.get<double2>(gsize(sd));
         to_spectra(sd, G, true);
         for (size_t i = 0; i < sd.ns.size(); ++i) small.push_back(problem(sd, (int)i, G));
@@ -970,14 +978,14 @@ void wav_merge(const WavPlan &P, MergeMode mode, const void *f_wav, int64_t wstr
   const auto passes = table_passes(P, pipe != nullptr, nb);
   int64_t gtot = 0;  // spectra of one pass, reused by the next
   for (const auto &pk : passes)
-    if (!small_scale(P, P.sc[pk.first], nb))
+    if (!is_small[pk.first])
       gtot = std::max(gtot, (int64_t)(pk.second - pk.first) * gsize(P.sc[pk.first]));
   double2 *Gbuf = gtot ? S.get<double2>(gtot) : nullptr;
   std::vector<RingJob> scal_ring;
   if (pipe) scal_ring.swap(rings.plain);  // the scaling function goes with the small scales
   for (const auto &pk : passes) {
     const Scale &s0 = P.sc[pk.first];
-    if (small_scale(P, s0, nb)) continue;
+    if (is_small[pk.first]) continue;
     const int ngrp = (int)(pk.second - pk.first);
     const int64_t gsz = gsize(s0);
     for (int q = 0; q < ngrp; ++q) to_spectra(P.sc[pk.first + q], Gbuf + q * gsz, !pipe);

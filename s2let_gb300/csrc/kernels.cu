@@ -1268,7 +1268,7 @@ void contract_many(const std::vector<A> &v, cudaStream_t st) {
   contract_rc(rc.data(), (int)rc.size(), st);
   for (const A &p : v) {
     if (p.nb <= 0 || p.mhi < p.mlo || p.tb->rc) continue;
-    if (!contract_is_small(p.tb, p.nb)) {
+    if (p.tb->bl > contract_small_max(p.nb)) {
       contract_one(p, st);
       continue;
     }
@@ -1289,9 +1289,7 @@ void contract_many(const std::vector<A> &v, cudaStream_t st) {
 // Tables whose contractions run in the FP64 or double-float kernel with a small
 // CTA count: below the tensor cores' band-limit, and for the double-float one-map
 // calls up to 128 (255 CTAs of one row block; larger ones fill the GPU alone).
-bool contract_is_small(const WignerTable *tb, int nb) {
-  return !tb->rc && tb->bl <= (on_tensor_cores(nb) ? kTensorMinBl - 1 : 128);
-}
+int contract_small_max(int nb) { return on_tensor_cores(nb) ? kTensorMinBl - 1 : 128; }
 void contract_l2t(const L2T &p, cudaStream_t st) { contract_one(p, st); }
 void contract_t2l(const T2L &p, cudaStream_t st) { contract_one(p, st); }
 void contract_l2t_group(const L2T *a, int n, cudaStream_t st) { contract_group(a, n, st); }

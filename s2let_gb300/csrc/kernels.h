@@ -113,8 +113,9 @@ struct T2L {
 void contract_t2l(const T2L &a, cudaStream_t st);
 void contract_t2l_group(const T2L *a, int n, cudaStream_t st);
 // Independent problems (any tables, one direction, one batch size): those on
-// small tables (contract_is_small) share launches, the others run one by one.
-bool contract_is_small(const WignerTable *tb, int nb);
+// stored tables up to band-limit contract_small_max(nb) share launches, the
+// others run one by one.
+int contract_small_max(int nb);
 constexpr int kTensorMinBl = 64;  // smallest band-limit on the tensor cores
 void contract_l2t_many(const std::vector<L2T> &v, cudaStream_t st);
 void contract_t2l_many(const std::vector<T2L> &v, cudaStream_t st);
