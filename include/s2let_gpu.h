@@ -438,10 +438,18 @@ int s2let_gpu_get_precision(void);
  * they would leave less than 4 GiB of device memory free), and the eight-slice
  * digit panels of the FP64 mode's contractions and of the adjoints (8 bytes
  * per table entry; skipped when less than a third of the device memory would
- * stay free).  0 = no such copies: the FP64 values are read as they are
- * (slower, no extra memory).  Process-wide.  Returns the status. */
+ * stay free, S2LET_GPU_PANEL_RESERVE_GB overrides the third; scratch that earlier
+ * calls left in the memory pool counts as free).  Skipped panels are asked for
+ * again half a second later.  An allocation of this library that finds no memory
+ * takes panels back, until the plans are released; those that a CUDA graph holds
+ * stay.  0 = no such copies: the FP64 values are read as they are (slower, no
+ * extra memory).  Process-wide.  Returns the status. */
 int s2let_gpu_set_split_tables(int on);
 int s2let_gpu_get_split_tables(void);
+/* Tables whose digit panels were skipped or taken back for want of memory and not
+ * built since: their contractions run on the FP64 pipe (or in double-float), several
+ * times slower.  0 = none. */
+int s2let_gpu_refused_tables(void);
 
 /* Split precision on stored tables: batches of at most `maps` maps (0-4,
  * default 1, initially S2LET_GPU_DF_MAX_MAPS when set) contract in

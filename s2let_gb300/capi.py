@@ -134,6 +134,7 @@ GPU_SIGNATURES = {
     "s2let_gpu_set_precision": (I, [I]),
     "s2let_gpu_set_split_tables": (I, [I]),
     "s2let_gpu_get_split_tables": (I, []),
+    "s2let_gpu_refused_tables": (I, []),
     "s2let_gpu_set_df_max_maps": (I, [I]),
     "s2let_gpu_get_df_max_maps": (I, []),
     "s2let_gpu_get_precision": (I, []),

@@ -54,6 +54,11 @@ extern std::atomic<uint64_t> g_launches;
       throw ::s2g::Error(::s2g::ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e_)); \
   } while (0)
 
+// cudaMalloc and cudaMallocAsync that, out of memory, give back the optional table
+// panels (mixed.cu) and try once more: a call that fits without them still does.
+cudaError_t device_malloc(void **p, size_t bytes);
+cudaError_t device_malloc_async(void **p, size_t bytes, cudaStream_t st);
+
 inline int ceil_div(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
 
 constexpr double kPi = 3.141592653589793238462643383279502884197;

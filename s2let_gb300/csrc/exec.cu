@@ -1006,13 +1006,14 @@ void wav_merge(const WavPlan &P, MergeMode mode, const void *f_wav, int64_t wstr
 }
 
 // Device bytes that stored tables of one plan may take: 60 % of the memory
-// free when the plan is built (S2LET_GPU_TABLE_BUDGET_GB overrides).
+// free when the plan is built (S2LET_GPU_TABLE_BUDGET_GB overrides), optional
+// panels of earlier plans counted as free: they make way (device_malloc).
 int64_t table_budget_bytes() {
   const char *e = getenv("S2LET_GPU_TABLE_BUDGET_GB");
   if (e && e[0]) return (int64_t)(atof(e) * 1073741824.0);
   size_t fr = 0, tot = 0;
   if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) return INT64_MAX;
-  return (int64_t)(0.6 * (double)fr);
+  return (int64_t)(0.6 * (double)(fr + optional_panel_bytes()));
 }
 
 // (-1)^s sqrt((2l+1)/4pi) on the device, cached per (L, s)
@@ -1782,6 +1783,7 @@ int s2let_gpu_set_split_tables(int on) {
   return 0;
 }
 int s2let_gpu_get_split_tables(void) { return s2g::get_split_tables(); }
+int s2let_gpu_refused_tables(void) { return s2g::refused_tables(); }
 int s2let_gpu_set_df_max_maps(int maps) {
   if (maps < 0 || maps > 4) {
     s2g::set_status(s2g::ERR_INVALID, "s2let_gpu_set_df_max_maps: 0 to 4 maps");

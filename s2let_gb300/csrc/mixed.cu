@@ -46,11 +46,12 @@
 // MMAs of N <= 128 per K-chunk behind one another.
 // Every wait is bounded (about 2 s); on expiry the kernel raises an error flag,
 // drains its own copies and MMAs, frees TMEM and returns.
+#include <chrono>
 #include <cstdint>
+#include <cstdlib>
 #include <map>
 #include <memory>
 #include <mutex>
-#include <set>
 #include <tuple>
 #include <vector>
 
@@ -60,6 +61,7 @@
 #include "kernels.h"
 #include "mixed.h"
 #include "plan.h"
+#include "runtime.h"
 #include "timing.h"
 
 namespace s2g {
@@ -1133,7 +1135,10 @@ struct SlicedTable {
   uint8_t *panels8 = nullptr;  // the eighth, built when an FP64 contraction first needs it
   int8_t *eA = nullptr;
   int64_t *d_pan_off = nullptr, *d_e_off = nullptr;
-  size_t bytes = 0;
+  size_t bytes = 0, bytes8 = 0;  // of everything; of panels8
+  int users = 0;                 // calls between looking the panels up and their last launch
+  bool forward7 = false;         // the split-precision forward contractions read panels
+  bool captured = false;         // a graph holds the panels' addresses
   std::map<std::tuple<int, int, int, int>, TileList> lists;  // (n, mlo, mhi, lmin)
   void release() {
     cudaFree(panels);
@@ -1151,16 +1156,20 @@ struct SlicedTable {
 std::mutex g_mx_mu;
 using TableKey = std::tuple<int, int, int, int>;  // (bl, an, ss, kind)
 std::map<TableKey, std::unique_ptr<SlicedTable>> g_sliced;
-std::set<TableKey> g_refused;  // optional tables that did not fit when first wanted
+// Optional panels that did not fit when last wanted: asked for again after
+// kAskAgain, or (given back by an allocation that needed the room) not before the
+// plans are released.
+struct Refusal {
+  std::chrono::steady_clock::time_point when;
+  bool given_back;
+};
+constexpr std::chrono::milliseconds kAskAgain{500};
+std::map<TableKey, Refusal> g_refused;
 size_t g_mx_bytes = 0;
 int *g_err = nullptr;
 
-template <class T>
-T *dev_alloc(size_t n, size_t *acc) {
-  void *p = nullptr;
-  S2G_CUDA(cudaMalloc(&p, sizeof(T) * (n ? n : 1)));
-  *acc += sizeof(T) * (n ? n : 1);
-  return (T *)p;
+void refuse(const TableKey &key, bool given_back) {
+  g_refused[key] = Refusal{std::chrono::steady_clock::now(), given_back};
 }
 
 bool capturing(cudaStream_t st) {
@@ -1169,13 +1178,88 @@ bool capturing(cudaStream_t st) {
   return cap != cudaStreamCaptureStatusNone;
 }
 
+// Frees the optional panels that nothing uses (caller holds g_mx_mu): the eighth
+// slices, and all slices of a table that the split-precision forward contractions do
+// not read.  Not those that a call is about to launch with or a graph holds.  False
+// when there were none.
+bool give_back_panels() {
+  std::vector<TableKey> keys;
+  for (auto &kv : g_sliced) {
+    const SlicedTable &s = *kv.second;
+    if (s.panels8 && s.users == 0 && !s.captured) keys.push_back(kv.first);
+  }
+  if (keys.empty()) return false;
+  if (cudaDeviceSynchronize() != cudaSuccess) {  // launches that still read them
+    cudaGetLastError();
+    return false;
+  }
+  for (const TableKey &key : keys) {
+    SlicedTable &s = *g_sliced[key];
+    if (s.forward7) {
+      cudaFree(s.panels8);
+      s.panels8 = nullptr;
+      s.bytes -= s.bytes8;
+      g_mx_bytes -= s.bytes8;
+      s.bytes8 = 0;
+    } else {
+      g_mx_bytes -= s.bytes;
+      s.release();
+      g_sliced.erase(key);
+    }
+    refuse(key, true);
+  }
+  return true;
+}
+
+// Caller holds g_mx_mu; optional: no room is made for it.
+template <class T>
+T *dev_alloc(size_t n, size_t *acc, bool optional = false) {
+  void *p = nullptr;
+  const size_t bytes = sizeof(T) * (n ? n : 1);
+  cudaError_t e = cudaMalloc(&p, bytes);
+  if (e == cudaErrorMemoryAllocation && !optional && give_back_panels()) {
+    cudaGetLastError();
+    e = cudaMalloc(&p, bytes);
+  }
+  S2G_CUDA(e);
+  *acc += bytes;
+  return (T *)p;
+}
+
+// Device memory that must stay free beside optional panels: a third of it, or
+// S2LET_GPU_PANEL_RESERVE_GB.
+size_t panel_reserve(size_t total) {
+  const char *e = getenv("S2LET_GPU_PANEL_RESERVE_GB");
+  return e && e[0] ? (size_t)(atof(e) * 1073741824.0) : total / 3;
+}
+// Whether `need` bytes of optional panels leave that much free.  What the
+// stream-ordered pool holds without using it (the scratch of earlier calls) counts
+// as free, and is released when it is wanted.
+bool panels_fit(size_t need) {
+  size_t fr = 0, tot = 0;
+  S2G_CUDA(cudaMemGetInfo(&fr, &tot));
+  const size_t want = need + panel_reserve(tot);
+  if (fr >= want) return true;
+  int dev = 0;
+  S2G_CUDA(cudaGetDevice(&dev));
+  cudaMemPool_t pool;
+  S2G_CUDA(cudaDeviceGetDefaultMemPool(&pool, dev));
+  uint64_t held = 0, used = 0;
+  S2G_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held));
+  S2G_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used));
+  if (fr + (size_t)(held - used) < want) return false;
+  S2G_CUDA(cudaMemPoolTrimTo(pool, 0));
+  S2G_CUDA(cudaMemGetInfo(&fr, &tot));
+  return fr >= want;
+}
+
 // Panels of one table and kind (caller holds g_mx_mu).  The split-precision
 // forward contractions cannot do without theirs; the others (with the eighth
 // digit) are optional: the FP64 and double-float kernels take over (nullptr)
-// when table copies are switched off (s2let_gpu_set_split_tables), when less
-// than a third of the device memory would stay free, or when a stream capture
-// meets a table that no earlier call has built.  A refusal stands until the
-// plans are released, so that a program's route does not change under it.
+// when table copies are switched off (s2let_gpu_set_split_tables), when a third of
+// the device memory would not stay free (panels_fit), or when a stream capture
+// meets a table that no earlier call has built.  A refusal is looked at again
+// kAskAgain later.
 SlicedTable *sliced(const WignerTable &tb, int kind, bool eighth, cudaStream_t st) {
   const int mode = kind_mode(kind);
   // the quadrature operators belong to the grid: one block per parity
@@ -1184,7 +1268,13 @@ SlicedTable *sliced(const WignerTable &tb, int kind, bool eighth, cudaStream_t s
   const TableKey key = std::make_tuple(tb.bl, quad ? -1 : tb.an, tb.ss, kind);
   auto it = g_sliced.find(key);
   if (it != g_sliced.end() && (!eighth || it->second->panels8)) return it->second.get();
-  if (eighth && (!get_split_tables() || g_refused.count(key) || capturing(st))) return nullptr;
+  if (eighth) {
+    if (!get_split_tables() || capturing(st)) return nullptr;
+    const auto no = g_refused.find(key);
+    if (no != g_refused.end() &&
+        (no->second.given_back || std::chrono::steady_clock::now() - no->second.when < kAskAgain))
+      return nullptr;
+  }
   const bool fresh = it == g_sliced.end();
   std::vector<int64_t> po(nm), eo(nm);
   int64_t ptot = 0, etot = 0;
@@ -1196,17 +1286,14 @@ SlicedTable *sliced(const WignerTable &tb, int kind, bool eighth, cudaStream_t s
     etot += (int64_t)g.nrt * kPM;
   }
   if (eighth) {
-    const size_t need = (size_t)(ptot / kS) * (fresh ? kSmax : 1);
-    size_t fr = 0, tot = 0;
-    S2G_CUDA(cudaMemGetInfo(&fr, &tot));
-    if (fr < need + tot / 3) {
-      g_refused.insert(key);
+    if (!panels_fit((size_t)(ptot / kS) * (fresh ? kSmax : 1))) {
+      refuse(key, false);
       return nullptr;
     }
   }
   std::unique_ptr<SlicedTable> made;
   SlicedTable *s = fresh ? nullptr : it->second.get();
-  size_t by = 0;
+  size_t by = 0, by8 = 0;
   if (fresh) {
     made = std::make_unique<SlicedTable>();
     s = made.get();
@@ -1220,14 +1307,14 @@ SlicedTable *sliced(const WignerTable &tb, int kind, bool eighth, cudaStream_t s
   uint8_t *p8 = nullptr;
   try {
     if (fresh) {
-      s->panels = dev_alloc<uint8_t>((size_t)ptot, &by);
-      s->eA = dev_alloc<int8_t>((size_t)etot, &by);
-      s->d_pan_off = dev_alloc<int64_t>(nm, &by);
-      s->d_e_off = dev_alloc<int64_t>(nm, &by);
+      s->panels = dev_alloc<uint8_t>((size_t)ptot, &by, eighth);
+      s->eA = dev_alloc<int8_t>((size_t)etot, &by, eighth);
+      s->d_pan_off = dev_alloc<int64_t>(nm, &by, eighth);
+      s->d_e_off = dev_alloc<int64_t>(nm, &by, eighth);
       S2G_CUDA(cudaMemcpyAsync(s->d_pan_off, po.data(), sizeof(int64_t) * nm, cudaMemcpyHostToDevice, st));
       S2G_CUDA(cudaMemcpyAsync(s->d_e_off, eo.data(), sizeof(int64_t) * nm, cudaMemcpyHostToDevice, st));
     }
-    if (eighth) p8 = dev_alloc<uint8_t>((size_t)(ptot / kS), &by);
+    if (eighth) p8 = dev_alloc<uint8_t>((size_t)(ptot / kS), &by8, true);
     const dim3 grid(nm, (std::max(tb.bl, tb.nt) + kPM - 1) / kPM);
     int64_t *d_woff = nullptr;  // the operators' blocks from W_+
     if (quad) {
@@ -1246,12 +1333,16 @@ SlicedTable *sliced(const WignerTable &tb, int kind, bool eighth, cudaStream_t s
     cudaFree(p8);
     if (!eighth || e.code != ERR_NOMEM) throw;
     cudaGetLastError();
-    g_refused.insert(key);
+    refuse(key, false);
     return nullptr;
   }
-  if (p8) s->panels8 = p8;
-  s->bytes += by;
-  g_mx_bytes += by;
+  if (p8) {
+    s->panels8 = p8;
+    s->bytes8 = by8;
+    g_refused.erase(key);
+  }
+  s->bytes += by + by8;
+  g_mx_bytes += by + by8;
   if (fresh) g_sliced.emplace(key, std::move(made));
   return s;
 }
@@ -1371,17 +1462,18 @@ bool run_mixed(const Problem &p, const Prepared &pr, cudaStream_t st, int gpl_ma
   const int gpl = ngroups < gpl_max ? ngroups : gpl_max;
   // coefficient panels: the tile list's offsets count one slice of 16 columns
   const int64_t x_elems = L->x_elems * (NC / 16 * S);
-  uint16_t *xpan = nullptr;
-  int *eX = nullptr;
   const int64_t *xoff = L->d_xoff;
-  const cudaError_t got =
-      cudaMallocAsync((void **)&xpan, sizeof(uint16_t) * (size_t)(x_elems ? x_elems * gpl : 1), st);
-  if (got == cudaErrorMemoryAllocation && p.eighth) {
-    cudaGetLastError();
-    return false;
+  Scratch scratch(st);
+  uint16_t *xpan;
+  int *eX;
+  if (p.eighth) {
+    xpan = scratch.try_get<uint16_t>(x_elems * gpl);
+    eX = xpan ? scratch.try_get<int>((int64_t)nmp * NC * gpl) : nullptr;
+    if (!eX) return false;
+  } else {
+    xpan = scratch.get<uint16_t>(x_elems * gpl);
+    eX = scratch.get<int>((int64_t)nmp * NC * gpl);
   }
-  S2G_CUDA(got);
-  S2G_CUDA(cudaMallocAsync((void **)&eX, sizeof(int) * (size_t)nmp * NC * gpl, st));
   const double entries = (double)L->work_entries;
   for (int g0 = 0; g0 < ngroups; g0 += gpl) {
     const int ng = ngroups - g0 < gpl ? ngroups - g0 : gpl;
@@ -1452,8 +1544,6 @@ bool run_mixed(const Problem &p, const Prepared &pr, cudaStream_t st, int gpl_ma
     k_contract_mx<NC, S><<<grid, C::kThreads, C::kSmemBytes, st>>>(ma);
     S2G_LAUNCHED();
   }
-  cudaFreeAsync(xpan, st);
-  cudaFreeAsync(eX, st);
   return true;
 }
 
@@ -1487,12 +1577,24 @@ bool run_problem(const Problem &p, cudaStream_t st) {
   Prepared pr;
   pr.lmin = p.part[0].lmin;
   for (int i = 1; i < p.nparts; ++i) pr.lmin = std::min(pr.lmin, p.part[i].lmin);
+  struct User {  // keeps the panels until the launches are in the stream
+    SlicedTable *s = nullptr;
+    ~User() {
+      if (!s) return;
+      std::lock_guard<std::mutex> lk(g_mx_mu);
+      --s->users;
+    }
+  } user;
   {
     std::lock_guard<std::mutex> lk(g_mx_mu);
     pr.s = sliced(*p.tb, p.kind, p.eighth, st);
     if (pr.s) pr.L = tile_list(*pr.s, p.n, p.mlo, p.mhi, pr.lmin, p.eighth, st);
     if (!pr.L) return false;
     pr.err = error_flag();
+    ++pr.s->users;
+    user.s = pr.s;
+    if (!p.eighth) pr.s->forward7 = true;
+    if (capturing(st)) pr.s->captured = true;
   }
   return p.eighth ? run_shapes<kSmax>(p, pr, st) : run_shapes<kS>(p, pr, st);
 }
@@ -1613,6 +1715,38 @@ void release_sliced_tables() {
   g_sliced.clear();
   g_refused.clear();
   g_mx_bytes = 0;
+}
+
+size_t optional_panel_bytes() {
+  std::lock_guard<std::mutex> lk(g_mx_mu);
+  size_t n = 0;
+  for (auto &kv : g_sliced) {
+    const SlicedTable &s = *kv.second;
+    if (s.panels8 && !s.captured) n += s.forward7 ? s.bytes8 : s.bytes;
+  }
+  return n;
+}
+
+int refused_tables() {
+  std::lock_guard<std::mutex> lk(g_mx_mu);
+  return (int)g_refused.size();
+}
+
+cudaError_t device_malloc(void **p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  std::lock_guard<std::mutex> lk(g_mx_mu);
+  return give_back_panels() ? cudaMalloc(p, bytes) : e;
+}
+
+cudaError_t device_malloc_async(void **p, size_t bytes, cudaStream_t st) {
+  const cudaError_t e = cudaMallocAsync(p, bytes, st);
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  if (capturing(st)) return e;
+  std::lock_guard<std::mutex> lk(g_mx_mu);
+  return give_back_panels() ? cudaMallocAsync(p, bytes, st) : e;
 }
 
 size_t sliced_table_bytes() {

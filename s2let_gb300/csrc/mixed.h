@@ -42,6 +42,10 @@ bool quadrature_mixed(const WignerTable &tb, bool trans, const QuadIO *io, int n
 
 void release_sliced_tables();
 size_t sliced_table_bytes();
+// bytes of optional panels that an allocation may take back (device_malloc)
+size_t optional_panel_bytes();
+// tables whose optional panels were last refused for want of memory
+int refused_tables();
 // Reads and clears the device flag raised by a split-precision launch whose
 // bounded wait expired (1: pipeline wait, 2: MMA drain); 0 when none did.
 int mixed_error_flag_read_and_clear();

@@ -384,7 +384,7 @@ size_t g_bytes = 0;
 template <class T>
 T *dev_alloc(size_t n) {
   T *p = nullptr;
-  S2G_CUDA(cudaMalloc(&p, sizeof(T) * (n ? n : 1)));
+  S2G_CUDA(device_malloc((void **)&p, sizeof(T) * (n ? n : 1)));
   g_bytes += sizeof(T) * (n ? n : 1);
   return p;
 }

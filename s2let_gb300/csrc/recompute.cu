@@ -37,6 +37,7 @@
 #include "kernels.h"
 #include "mixed.h"
 #include "recompute.h"
+#include "runtime.h"
 #include "timing.h"
 
 namespace s2g {
@@ -1063,9 +1064,9 @@ void l2t_rc(const L2T *v, int n, cudaStream_t st) {
   a.dw = p.ow;
   a.d_mlo = p.omlo;
   // Q^T x = W^T (D x): D x into scratch of the output's layout, then W^T
-  double2 *tmp = nullptr;
+  Scratch S(st);
   const int64_t one = (int64_t)p.nb * tb.nt * p.ow;
-  if (p.use_q) S2G_CUDA(cudaMallocAsync((void **)&tmp, sizeof(double2) * (size_t)(one * n), st));
+  double2 *tmp = p.use_q ? S.get<double2>(one * n) : nullptr;
   a.ds = p.use_q ? (int64_t)tb.nt * p.ow : p.os;
   std::vector<RcPart> parts;
   for (int i = 0; i < n; ++i)
@@ -1076,7 +1077,6 @@ void l2t_rc(const L2T *v, int n, cudaStream_t st) {
       *in = tmp + i * one;
       *out = v[i].out;
     }, a.ds, p.ow, p.omlo, p.os, p.ow, p.omlo, st);
-    cudaFreeAsync(tmp, st);
   }
 }
 
@@ -1085,11 +1085,12 @@ void t2l_rc(const T2L *v, int n, cudaStream_t st) {
   const WignerTable &tb = *p.tb;
   RcArgs a = rc_args(tb, p.wscale, p.wconj, p.nb);
   // Q in = D^T (W in): the quadrature on the spectra first
+  Scratch S(st);
   double2 *tmp = nullptr;
   const int64_t one = (int64_t)p.nb * tb.nt * p.iw;
   a.ss = p.use_q ? (int64_t)tb.nt * p.iw : p.is;
   if (p.use_q) {
-    S2G_CUDA(cudaMallocAsync((void **)&tmp, sizeof(double2) * (size_t)(one * n), st));
+    tmp = S.get<double2>(one * n);
     quadrature(v, n, false, [&](int i, const double2 **in, double2 **out) {
       *in = v[i].in;
       *out = tmp + i * one;
@@ -1105,7 +1106,6 @@ void t2l_rc(const T2L *v, int n, cudaStream_t st) {
     for (const RcPart &q : parts_of(v[i], p.use_q ? tmp + i * one : v[i].in, v[i].y)) parts.push_back(q);
   launch_parts(a, parts, tb, TF_RC_T2L, 2, 16, st,
                [&](const RcArgs &x, int nbt) { run_t2l(x, tb.nm, maxseg, nbt, st); });
-  if (tmp) cudaFreeAsync(tmp, st);
 }
 
 // problems of one form in shared launches, in order
@@ -1125,7 +1125,7 @@ void by_form(const A *p, int n, F &&f) {
 
 RcRec *build_rec(int bl, int an, int mlo, int nm, const int64_t *d_roff, int64_t n) {
   RcRec *rec = nullptr;
-  S2G_CUDA(cudaMalloc(&rec, sizeof(RcRec) * (size_t)(n > 0 ? n : 1)));
+  S2G_CUDA(device_malloc((void **)&rec, sizeof(RcRec) * (size_t)(n > 0 ? n : 1)));
   const int maxseg = ceil_div(bl, kSeg);
   k_rc_rec<<<ceil_div((int64_t)nm * maxseg, 128), 128>>>(rec, d_roff, bl, an, mlo, nm, maxseg);
   S2G_LAUNCHED();

@@ -49,7 +49,19 @@ struct Scratch {
   template <class T>
   T *get(int64_t n) {
     void *p = nullptr;
-    S2G_CUDA(cudaMallocAsync(&p, sizeof(T) * (size_t)(n > 0 ? n : 1), st));
+    S2G_CUDA(device_malloc_async(&p, sizeof(T) * (size_t)(n > 0 ? n : 1), st));
+    ptrs.push_back(p);
+    return (T *)p;
+  }
+  template <class T>
+  T *try_get(int64_t n) {  // nullptr when out of memory
+    void *p = nullptr;
+    const cudaError_t e = cudaMallocAsync(&p, sizeof(T) * (size_t)(n > 0 ? n : 1), st);
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    S2G_CUDA(e);
     ptrs.push_back(p);
     return (T *)p;
   }
