@@ -567,11 +567,11 @@ int max_parts(int nb) { return std::min(kMaxParts, std::max(2, 32 / std::max(nb,
 
 // Scale ranges [k0, k1) that share one table pass, smallest band-limits first,
 // or largest first when `largest_first`.
-std::vector<std::pair<size_t, size_t>> table_passes(const WavPlan &P, bool largest_first, int nb) {
+std::vector<std::pair<size_t, size_t>> table_passes(const WavPlan &P, bool largest_first, int parts) {
   std::vector<std::pair<size_t, size_t>> passes;
   for (size_t k0 = 0; k0 < P.sc.size();) {
     size_t k1 = k0 + 1;
-    while (k1 < P.sc.size() && (int)(k1 - k0) < max_parts(nb) && P.sc[k1].bl == P.sc[k0].bl &&
+    while (k1 < P.sc.size() && (int)(k1 - k0) < parts && P.sc[k1].bl == P.sc[k0].bl &&
            P.sc[k1].ns == P.sc[k0].ns)
       ++k1;
     passes.emplace_back(k0, k1);
@@ -608,6 +608,42 @@ std::vector<char> small_scales(const WavPlan &P, int nb) {
   std::vector<char> out;
   for (const Scale &sd : P.sc) out.push_back(!P.rc(sd.bl) && sd.bl <= limit);
   return out;
+}
+
+// Elements of the spectra [b][n][t][m] of one scale.
+int64_t spectra_size(const WavPlan &P, const Scale &sd, int nb) {
+  return (int64_t)nb * (int64_t)sd.ns.size() * P.nt(sd.bl) * (2 * sd.bl - 1);
+}
+
+// The table passes of a call and their spectra: those of one pass at a time (G,
+// reused by the next), and those of all small scales at once (small).  Where that
+// does not fit in memory, no scales are small and a pass holds two.
+struct Passes {
+  std::vector<char> is_small;
+  std::vector<std::pair<size_t, size_t>> passes;
+  double2 *small = nullptr, *G = nullptr;
+};
+Passes plan_passes(const WavPlan &P, bool largest_first, int nb, Scratch &S) {
+  Passes r;
+  r.is_small = small_scales(P, nb);
+  for (int parts : {max_parts(nb), 2}) {
+    r.passes = table_passes(P, largest_first, parts);
+    int64_t small = 0, one = 0;
+    for (const auto &pk : r.passes) {
+      int64_t n = 0;
+      for (size_t k = pk.first; k < pk.second; ++k) n += spectra_size(P, P.sc[k], nb);
+      if (r.is_small[pk.first])
+        small += n;
+      else
+        one = std::max(one, n);
+    }
+    const bool least = parts == 2 && small == 0;
+    r.small = least ? S.get<double2>(one) : S.try_get<double2>(small + one);
+    r.G = r.small + small;
+    if (r.small) break;
+    std::fill(r.is_small.begin(), r.is_small.end(), 0);
+  }
+  return r;
 }
 
 // Jobs of ring DFTs collected for shared launches: those fused with the gamma
@@ -792,16 +828,16 @@ void wav_split(const WavPlan &P, SplitMode mode, const double2 *flm, bool flm_ha
   };
   const int64_t Kmax = 2 * P.max_bl, ntmax = P.nt(P.max_bl);
   if (needs_ring_buffer(P)) spec = S.get<double2>((int64_t)nb * std::max(P.max_ng, P.max_nn) * ntmax * Kmax);
-  const auto gsize = [&](const Scale &sd) { return (int64_t)nb * (int64_t)sd.ns.size() * P.nt(sd.bl) * (2 * sd.bl - 1); };
-  const std::vector<char> is_small = small_scales(P, nb);
+  const Passes pass = plan_passes(P, pipe != nullptr, nb, S);
   const auto run_small = [&] {
     std::vector<std::pair<const Scale *, double2 *>> sc;
+    double2 *G = pass.small;
     for (size_t k = 0; k < P.sc.size(); ++k)
-      if (is_small[k]) {
+      if (pass.is_small[k]) {
         const Scale &sd = P.sc[k];
-        double2 *G = S.get<double2>(gsize(sd));
         for (size_t i = 0; i < sd.ns.size(); ++i) small.push_back(problem(sd, (int)i, G));
         sc.emplace_back(&sd, G);
+        G += spectra_size(P, sd, nb);
       }
     contract_l2t_many(small, S.st);
     for (const auto &x : sc) to_pixels(*x.first, x.second, true);
@@ -812,26 +848,20 @@ void wav_split(const WavPlan &P, SplitMode mode, const double2 *flm, bool flm_ha
   // with host copies the largest scales go first, so that most of f_wav can
   // cross the bus while the smaller scales are transformed
   if (!pipe) run_small();
-  const auto passes = table_passes(P, pipe != nullptr, nb);
-  int64_t gtot = 0;  // spectra of one pass, reused by the next
-  for (const auto &pk : passes)
-    if (!is_small[pk.first])
-      gtot = std::max(gtot, (int64_t)(pk.second - pk.first) * gsize(P.sc[pk.first]));
-  double2 *Gbuf = gtot ? S.get<double2>(gtot) : nullptr;
   std::vector<RingJob> scal_ring;
   if (pipe) scal_ring.swap(rings.plain);  // the scaling function goes with the small scales
-  for (const auto &pk : passes) {
+  for (const auto &pk : pass.passes) {
     const Scale &s0 = P.sc[pk.first];
-    if (is_small[pk.first]) continue;
+    if (pass.is_small[pk.first]) continue;
     const int ngrp = (int)(pk.second - pk.first);
-    const int64_t gsz = gsize(s0);
+    const int64_t gsz = spectra_size(P, s0, nb);
     for (const auto &dirs : table_directions(P, s0)) {
       std::vector<L2T> grp;
       for (int i : dirs)
-        for (int q = 0; q < ngrp; ++q) grp.push_back(problem(P.sc[pk.first + q], i, Gbuf + q * gsz));
+        for (int q = 0; q < ngrp; ++q) grp.push_back(problem(P.sc[pk.first + q], i, pass.G + q * gsz));
       contract_l2t_group(grp.data(), (int)grp.size(), S.st);
     }
-    for (int q = 0; q < ngrp; ++q) to_pixels(P.sc[pk.first + q], Gbuf + q * gsz, !pipe);
+    for (int q = 0; q < ngrp; ++q) to_pixels(P.sc[pk.first + q], pass.G + q * gsz, !pipe);
     if (!pipe) rings.inverse(P.ss, real, S.st);
   }
   if (pipe) {
@@ -958,15 +988,15 @@ void wav_merge(const WavPlan &P, MergeMode mode, const void *f_wav, int64_t wstr
   };
   const int64_t Kmax = 2 * P.max_bl, ntmax = P.nt(P.max_bl);
   if (needs_ring_buffer(P)) spec = S.get<double2>((int64_t)nb * std::max(P.max_ng, P.max_nn) * ntmax * Kmax);
-  const auto gsize = [&](const Scale &sd) { return (int64_t)nb * (int64_t)sd.ns.size() * P.nt(sd.bl) * (2 * sd.bl - 1); };
-  const std::vector<char> is_small = small_scales(P, nb);
+  const Passes pass = plan_passes(P, pipe != nullptr, nb, S);
   const auto run_small = [&] {
+    double2 *G = pass.small;
     for (size_t k = 0; k < P.sc.size(); ++k)
-      if (is_small[k]) {
+      if (pass.is_small[k]) {
         const Scale &sd = P.sc[k];
-        double2 *G = S.get<double2>(gsize(sd));
         to_spectra(sd, G, true);
         for (size_t i = 0; i < sd.ns.size(); ++i) small.push_back(problem(sd, (int)i, G));
+        G += spectra_size(P, sd, nb);
       }
     rings.forward(P.ss, real, S.st);
     contract_t2l_many(small, S.st);
@@ -975,25 +1005,19 @@ void wav_merge(const WavPlan &P, MergeMode mode, const void *f_wav, int64_t wstr
   // first), so that their ring DFTs run while the rest of f_wav is still
   // crossing the bus
   if (!pipe) run_small();
-  const auto passes = table_passes(P, pipe != nullptr, nb);
-  int64_t gtot = 0;  // spectra of one pass, reused by the next
-  for (const auto &pk : passes)
-    if (!is_small[pk.first])
-      gtot = std::max(gtot, (int64_t)(pk.second - pk.first) * gsize(P.sc[pk.first]));
-  double2 *Gbuf = gtot ? S.get<double2>(gtot) : nullptr;
   std::vector<RingJob> scal_ring;
   if (pipe) scal_ring.swap(rings.plain);  // the scaling function goes with the small scales
-  for (const auto &pk : passes) {
+  for (const auto &pk : pass.passes) {
     const Scale &s0 = P.sc[pk.first];
-    if (is_small[pk.first]) continue;
+    if (pass.is_small[pk.first]) continue;
     const int ngrp = (int)(pk.second - pk.first);
-    const int64_t gsz = gsize(s0);
-    for (int q = 0; q < ngrp; ++q) to_spectra(P.sc[pk.first + q], Gbuf + q * gsz, !pipe);
+    const int64_t gsz = spectra_size(P, s0, nb);
+    for (int q = 0; q < ngrp; ++q) to_spectra(P.sc[pk.first + q], pass.G + q * gsz, !pipe);
     if (!pipe) rings.forward(P.ss, real, S.st);
     for (const auto &dirs : table_directions(P, s0)) {
       std::vector<T2L> grp;
       for (int i : dirs)
-        for (int q = 0; q < ngrp; ++q) grp.push_back(problem(P.sc[pk.first + q], i, Gbuf + q * gsz));
+        for (int q = 0; q < ngrp; ++q) grp.push_back(problem(P.sc[pk.first + q], i, pass.G + q * gsz));
       contract_t2l_group(grp.data(), (int)grp.size(), S.st);
     }
   }
@@ -1607,7 +1631,7 @@ int host_batch(const char *fn, s2g::Op op, const s2let_parameters_t *p, bool rea
         copy_async(hs + (size_t)c0 * ns * esz, 0, ds, 0, (size_t)n * ns * esz, 1, cudaMemcpyDeviceToHost, st);
       } else {
         copy_async(ds, 0, hs + (size_t)c0 * ns * esz, 0, (size_t)n * ns * esz, 1, cudaMemcpyHostToDevice, st);
-        for (const auto &pk : table_passes(P, true, n))  // in the order the synthesis reads them
+        for (const auto &pk : table_passes(P, true, max_parts(n)))  // in the order the synthesis reads them
           for (size_t k = pk.first; k < pk.second; ++k) {
             const Scale &sd = P.sc[k];
             if (grouped_copies(ring_path(P, sd))) {
