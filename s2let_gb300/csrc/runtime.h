@@ -21,7 +21,9 @@ int last_status();
 void ensure_device();   // throws ERR_NO_DEVICE without a usable GPU
 cudaStream_t host_stream();  // per-thread stream of the host-pointer entry points
 
-// Runs `body`, turning exceptions into the thread's status (never exits unless asked to).
+// Runs `body`, turning exceptions into the thread's status (never exits unless asked
+// to).  The runtime's own record of a failed call (out of memory, say) is cleared: it
+// would make the thread's next launch check, here or in the caller's program, fail.
 template <class F>
 int guarded(const char *fn, F &&body) {
   try {
@@ -35,6 +37,7 @@ int guarded(const char *fn, F &&body) {
   } catch (const std::exception &e) {
     set_status(ERR_CUDA, std::string(fn) + ": " + e.what());
   }
+  cudaGetLastError();
   report_failure();
   return last_status();
 }

@@ -63,3 +63,28 @@ def test_fewer_spectra_at_once(gpu, L, nb, J_min):
     finally:
         lib.s2let_gpu_set_split_tables(1)
         lib.s2let_gpu_release_plans()
+
+
+@pytest.mark.gpu
+def test_a_call_after_one_out_of_memory(gpu):
+    """A batch whose first scratch buffer exceeds the device is refused before any
+    launch, and leaves nothing behind for the next call or the caller."""
+    torch = pytest.importorskip("torch")
+    from s2let_gb300 import torch_ops as T
+
+    lib = gpu.lib
+    p = make_parameters(48, 2.0, 2, 3, 0, 0)
+    f = torch.randn(2, gpu.sizes(p)["n_px"], dtype=torch.float64, device="cuda")
+    w0, s0 = T.px2wav(f, p)
+    st = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+    def analysis(nb, w, s):
+        return lib.s2let_gpu_analysis_px2wav_real_batch(C.c_void_p(w.data_ptr()), C.c_void_p(s.data_ptr()),
+                                                        C.c_void_p(f.data_ptr()), nb, C.byref(p), st)
+
+    w, s = torch.zeros_like(w0), torch.zeros_like(s0)
+    assert analysis(20_000_000, w, s) == 4  # 737 GB of coefficients
+    torch.cuda.synchronize()
+    assert analysis(2, w, s) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(w, w0) and torch.equal(s, s0)
