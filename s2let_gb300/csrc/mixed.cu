@@ -13,7 +13,7 @@
 //     table stream (the bound of small batches) and the L2-to-SM traffic (of
 //     large ones) halve.  The eighth slice has an array of its own (it is the
 //     remainder of the first seven, which both forms share).  Row exponents eA
-//     (int8) per (m, row).
+//     (int16) per (m, row).
 //   Sliced coefficients, per call and per problem m: for each kc one panel
 //     [S slices x NC columns][64 bf16], column exponents eX (int32) per (m,
 //     column).
@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(128) k_slice_table(const double *__restrict__ 
                                                      int an, int tmlo, int mode, int tr, uint8_t *__restrict__ panels,
                                                      uint8_t *__restrict__ panels8,
                                                      const int64_t *__restrict__ pan_off,
-                                                     int8_t *__restrict__ eA,
+                                                     int16_t *__restrict__ eA,
                                                      const int64_t *__restrict__ e_off) {
   const int mi = blockIdx.x, rt = blockIdx.y;
   const Geom g = geom(bl, nt, an, tmlo + mi, mode);
@@ -272,8 +272,7 @@ __global__ void __launch_bounds__(128) k_slice_table(const double *__restrict__ 
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
       e = block_scale(mx);
-      e = e < -126 ? -126 : (e > 126 ? 126 : e);
-      if (lane == 0) eA[e_off[mi] + row] = (int8_t)e;
+      if (lane == 0) eA[e_off[mi] + row] = (int16_t)e;
     } else {
       e = eA[e_off[mi] + row];
     }
@@ -673,7 +672,7 @@ struct MxArgs {
   int mode;  // MxMode
   const uint8_t *panels, *panels8;
   const int64_t *pan_off;
-  const int8_t *eA;
+  const int16_t *eA;
   const int64_t *e_off;
   int bl, nt, an, tmlo, n, mlo, lmin;  // lmin: smallest over the parts
   const uint16_t *xpan;
@@ -1133,7 +1132,7 @@ struct SlicedTable {
   int mode = MX_L2T;
   uint8_t *panels = nullptr;   // 7 digit slices
   uint8_t *panels8 = nullptr;  // the eighth, built when an FP64 contraction first needs it
-  int8_t *eA = nullptr;
+  int16_t *eA = nullptr;
   int64_t *d_pan_off = nullptr, *d_e_off = nullptr;
   size_t bytes = 0, bytes8 = 0;  // of everything; of panels8
   int users = 0;                 // calls between looking the panels up and their last launch
@@ -1308,7 +1307,7 @@ SlicedTable *sliced(const WignerTable &tb, int kind, bool eighth, cudaStream_t s
   try {
     if (fresh) {
       s->panels = dev_alloc<uint8_t>((size_t)ptot, &by, eighth);
-      s->eA = dev_alloc<int8_t>((size_t)etot, &by, eighth);
+      s->eA = dev_alloc<int16_t>((size_t)etot, &by, eighth);
       s->d_pan_off = dev_alloc<int64_t>(nm, &by, eighth);
       s->d_e_off = dev_alloc<int64_t>(nm, &by, eighth);
       S2G_CUDA(cudaMemcpyAsync(s->d_pan_off, po.data(), sizeof(int64_t) * nm, cudaMemcpyHostToDevice, st));
