@@ -160,5 +160,29 @@ S2G_DI double fx_join(long long q, int k) {
 }
 S2G_DI double2 fx_join2(longlong2 q, int k) { return make_double2(fx_join(q.x, k), fx_join(q.y, k)); }
 
+
+// Floats to doubles and back in integers (rounded to nearest, ties to even); zeros,
+// subnormals, infinities, NaN and results outside the normal range of a float go to
+// the conversion instructions, out of line.
+#ifdef __CUDACC__
+__device__ __noinline__ double widen_any(float x) { return (double)x; }
+__device__ __noinline__ float narrow_any(double x) { return __double2float_rn(x); }
+#else
+inline double widen_any(float x) { return (double)x; }
+inline float narrow_any(double x) { return (float)x; }
+#endif
+S2G_DI double widen(float x) {
+  const uint32_t b = bits_of(x);
+  if (((b >> 23) & 0xFF) - 1u >= 254u) return widen_any(x);
+  return double_of(((uint64_t)((b & 0x80000000u) | (((b & 0x7FFFFFFFu) >> 3) + (896u << 20))) << 32) | (b << 29));
+}
+S2G_DI float narrow(double x) {
+  const uint32_t hi = (uint32_t)(bits_of(x) >> 32), lo = (uint32_t)bits_of(x);
+  if (((hi >> 20) & 0x7FF) - 897u >= 254u) return narrow_any(x);
+  uint32_t f = (((hi & 0x7FFFFFFFu) - (896u << 20)) << 3) | (lo >> 29);
+  const uint32_t rem = lo & 0x1FFFFFFFu;
+  f += rem > 0x10000000u || (rem == 0x10000000u && (f & 1)) ? 1u : 0u;  // the carry runs into the exponent
+  return float_of((hi & 0x80000000u) | f);
+}
 }  // namespace
 }  // namespace s2g

@@ -107,21 +107,6 @@ __device__ __forceinline__ int job_of(const G &g, int block) {
 // maps) 13.08 ms instead of 12.70, and the memory of the FP64 copies.  The type
 // is a template parameter: as a run-time switch it slowed the FP64 launches by 1
 // to 8 %.
-__device__ __noinline__ double widen_any(float x) { return (double)x; }
-__device__ __noinline__ float narrow_any(double x) { return __double2float_rn(x); }
-__device__ __forceinline__ double widen(float x) {
-  const uint32_t b = __float_as_uint(x);
-  if (((b >> 23) & 0xFF) - 1u >= 254u) return widen_any(x);
-  return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7FFFFFFFu) >> 3) + (896u << 20))), (int)(b << 29));
-}
-__device__ __forceinline__ float narrow(double x) {
-  const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
-  if (((hi >> 20) & 0x7FF) - 897u >= 254u) return narrow_any(x);
-  uint32_t f = (((hi & 0x7FFFFFFFu) - (896u << 20)) << 3) | (lo >> 29);
-  const uint32_t rem = lo & 0x1FFFFFFFu;
-  f += rem > 0x10000000u || (rem == 0x10000000u && (f & 1)) ? 1u : 0u;  // the carry runs into the exponent
-  return __uint_as_float((hi & 0x80000000u) | f);
-}
 template <bool F32>
 __device__ __forceinline__ double ld_px(const void *p, int64_t i) {
   return F32 ? widen(((const float *)p)[i]) : ((const double *)p)[i];
