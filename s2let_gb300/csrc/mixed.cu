@@ -1149,10 +1149,11 @@ SlicedTable *sliced(const WignerTable &tb, int kind, bool eighth, cudaStream_t s
   const bool quad = mode == MX_QUAD;
   const int nm = quad ? 2 : tb.nm, tmlo = quad ? 0 : tb.mlo;
   const TableKey key = std::make_tuple(tb.bl, quad ? -1 : tb.an, tb.ss, kind);
+  if (eighth && !get_split_tables()) return nullptr;
   auto it = g_sliced.find(key);
   if (it != g_sliced.end() && (!eighth || it->second->panels8)) return it->second.get();
   if (eighth) {
-    if (!get_split_tables() || capturing(st)) return nullptr;
+    if (capturing(st)) return nullptr;
     const auto no = g_refused.find(key);
     if (no != g_refused.end() &&
         (no->second.given_back || std::chrono::steady_clock::now() - no->second.when < kAskAgain))

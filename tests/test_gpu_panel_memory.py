@@ -181,3 +181,18 @@ def test_longest_reduction_in_eight_slices(gpu, lib, L, ss, tensor):
     (f, back), n = _slicings(lib, lambda: (lambda f: (f, gpu.sht(0, f, L, 0, True, ss)))(gpu.sht(1, flm, L, 0, True, ss)))
     assert (n > 0) == tensor
     assert rel_err(back, flm) < 1e-12
+
+
+@pytest.mark.gpu
+def test_switched_off_after_they_were_built(gpu, lib):
+    """s2let_gpu_set_split_tables(0) means the FP64 tables from the next call on."""
+    p = make_parameters(130, 2.0, 6, 2, 0, 0)
+    f = np.random.default_rng(4).normal(size=gpu.sizes(p)["n_px"])
+    (w1, s1), n = _slicings(lib, lambda: gpu.px2wav(f, p, real=True))
+    assert n > 0
+    lib.s2let_gpu_set_split_tables(0)
+    (w0, s0), n = _slicings(lib, lambda: gpu.px2wav(f, p, real=True))
+    assert n == 0 and rel_err(w0, w1) < TOL
+    lib.s2let_gpu_set_split_tables(1)
+    (w2, s2), n = _slicings(lib, lambda: gpu.px2wav(f, p, real=True))
+    assert n > 0 and np.array_equal(w2, w1) and np.array_equal(s2, s1)
