@@ -416,8 +416,10 @@ const char *s2let_gpu_last_error_string(void);
 /* Arithmetic used by subsequent calls of this thread.
  *   0 = FP64 (default): FP64 inputs, outputs and rounding error throughout.
  *       On stored Wigner tables from band-limit 64 the contractions run on
- *       the tensor cores in eight bf16 digit slices (55-bit operands, products
- *       summed exactly but for terms below 2^-56 of the operands' scales), as
+ *       the tensor cores in eight bf16 digit slices (55-bit operands under one
+ *       power of two per table row and coefficient column, products summed
+ *       exactly but for terms below 2^-56 of these scales: FP64 accuracy relative
+ *       to the largest values, not value by value), as
  *       long as a third of the device memory stays free beside the sliced
  *       tables; else, and at smaller band-limits, on the FP64 pipe.  Ring and
  *       gamma DFTs run in 64-bit block fixed point.

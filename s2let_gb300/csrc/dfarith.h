@@ -48,16 +48,9 @@ __device__ __forceinline__ float4 dmk(float2 re, float2 im) { return make_float4
 __device__ __forceinline__ float4 dc_mul(float4 a, float4 b) {
   return dmk(df_dot2(dre(a), dre(b), df_neg(dim_(a)), dim_(b)), df_dot2(dre(a), dim_(b), dim_(a), dre(b)));
 }
-__device__ __forceinline__ float4 dc_mulc(float4 a, float4 b) {  // a * conj(b)
-  return dmk(df_dot2(dre(a), dre(b), dim_(a), dim_(b)), df_dot2(dim_(a), dre(b), df_neg(dre(a)), dim_(b)));
-}
 __device__ __forceinline__ float4 dc_add(float4 a, float4 b) {
   return dmk(df_add(dre(a), dre(b)), df_add(dim_(a), dim_(b)));
 }
-__device__ __forceinline__ float4 dc_sub(float4 a, float4 b) {
-  return dmk(df_add(dre(a), df_neg(dre(b))), df_add(dim_(a), df_neg(dim_(b))));
-}
-__device__ __forceinline__ float4 dc_conj(float4 a) { return make_float4(a.x, a.y, -a.z, -a.w); }
 // FP64 <-> double-float with a power-of-two block scale, by bit construction
 // (dfconv.h): no FP64 instructions but one add per value joined
 __device__ __forceinline__ float2 df_split(double v, int e) {

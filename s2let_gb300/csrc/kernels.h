@@ -37,6 +37,11 @@ struct RingJob {
 void ring_forward_many(const std::vector<RingJob> &jobs, int ss, bool real, cudaStream_t st);
 void ring_inverse_many(const std::vector<RingJob> &jobs, int ss, bool real, cudaStream_t st);
 
+// Kind of a per-l weight array: every entry real, every entry imaginary, or
+// general complex.  The directional weights are a real profile times 1 or i
+// (odd or even N), the axisymmetric and scaling weights are real.
+enum { WKIND_COMPLEX = 0, WKIND_REAL = 1, WKIND_IMAG = 2 };
+
 // Contraction over l producing ring spectra ("l -> t", t < tb->nt):
 //   out[b][t][m - omlo] = sum_l A_m[t][l] x_b(l, m) w(l)
 // A = D (use_q = false) or Q^T (use_q = true) of the |n| table at band-limit bl,
@@ -44,11 +49,6 @@ void ring_inverse_many(const std::vector<RingJob> &jobs, int ss, bool real, cuda
 // (band-limit xL >= bl); when x_half, x holds m >= 0 only and
 // x(l,-m) = (-1)^m conj(x(l,m)).  w(l) = wre/wim arrays (nullable => 1) times
 // wscale, conjugated when wconj.  Rows l < lmin contribute nothing.
-// Kind of a per-l weight array: every entry real, every entry imaginary, or
-// general complex.  The directional weights are a real profile times 1 or i
-// (odd or even N), the axisymmetric and scaling weights are real.
-enum { WKIND_COMPLEX = 0, WKIND_REAL = 1, WKIND_IMAG = 2 };
-
 struct L2T {
   const WignerTable *tb;
   int n;

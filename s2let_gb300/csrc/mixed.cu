@@ -21,7 +21,7 @@
 // Kernel k_contract_mx<NC, S>: persistent, one CTA per SM; NC real
 // coefficient columns (16, 32 or 64) per table pass.
 //   warp 0    producer: cp.async.bulk of digit blocks into a ring of 8 KB stages
-//             and of coefficient panels into a 2-deep ring (S slices x NC
+//             and of coefficient panels into a ring of 2 or 3 (S slices x NC
 //             columns x 64 K).
 //   converter warps (5; 2 at NC = 64): digit block -> 16 KB panel [128 rows][64
 //             bf16] in the 128-byte-swizzled K-major image that tcgen05 reads,
@@ -1444,16 +1444,15 @@ bool run_shapes(const Problem &p, const Prepared &pr, cudaStream_t st) {
   static const Shape kCand[7] = {{16, 1}, {16, 4}, {32, 1}, {32, 4}, {64, 1}, {64, 2}, {64, 4}};
   const int cols = 2 * p.nb * p.nparts;
   const int def = cols <= 16 ? 1 : (cols <= 32 ? 3 : 6);
-  // a candidate narrower than one part's two columns cannot hold a map
-  const int first = 2 * p.nparts > 16 ? (2 * p.nparts > 32 ? 4 : 2) : 0;
+  static_assert(2 * kMaxParts <= 16, "the narrowest candidate holds a map of every part");
   const auto run = [&](const Shape &sh) {
     if (sh.nc == 16) return run_mixed<16, S>(p, pr, st, sh.gpl);
     if (sh.nc == 32) return run_mixed<32, S>(p, pr, st, sh.gpl);
     return run_mixed<64, S>(p, pr, st, sh.gpl);
   };
-  const int c = tuned(TF_MIXED, tune_bucket(p.tb->bl), tune_bucket(cols), p.kind + (S == kSmax ? 4 : 0), 7 - first,
-                      def - first, st, [&](int i) { run(kCand[first + i]); });
-  return run(kCand[first + c]);
+  const int c = tuned(TF_MIXED, tune_bucket(p.tb->bl), tune_bucket(cols), p.kind + (S == kSmax ? 4 : 0), 7, def, st,
+                      [&](int i) { run(kCand[i]); });
+  return run(kCand[c]);
 }
 
 // false when the problem's optional table panels are not to be had
@@ -1526,15 +1525,11 @@ bool same_problem(const A &x, const A &y) {
 namespace {
 // The split-precision mode's forward contractions take 7 slices (8 below
 // band-limit 128, where double-float would be the alternative); the FP64 mode
-// and the adjoints of both modes 8.  Eight slices hold every value to 2^-56 of
-// its row's (column's) power of two; the dropped products (i + j = 8) and the
-// representation errors add about 2^-56 per term, summed exactly: classes 0-2
-// are exact up to reduction ranges of 1365 (longer ones stay on the FP64
-// kernels), the rounding of the others is below 2^-45-21 of the result.  An FP64
-// sum rounds each partial sum to 2^-53 of it.  Measured against a 64-bit
-// reference, errors equal the FP64 kernels' to 1 % at L = 128 to 1024 (7.6e-13 /
-// 7.5e-13 of f_wav at L = 1024), and px2wav + wav2px of 2 maps at L = 1024, N = 4
-// contracts in 15.8 ms against 64.9 on the FP64 pipe.
+// and the adjoints of both modes 8 (accuracy: mixed.h).  Reductions longer than
+// 1365, where classes 0-2 could leave the exact range, stay on the FP64 kernels.
+// Measured against a 64-bit reference, errors equal the FP64 kernels' to 1 % at L =
+// 128 to 1024 (7.6e-13 / 7.5e-13 of f_wav at L = 1024), and px2wav + wav2px of 2 maps
+// at L = 1024, N = 4 contracts in 13.0 ms against 64.9 on the FP64 pipe.
 constexpr int kMaxK8 = 1365;
 
 template <class A>

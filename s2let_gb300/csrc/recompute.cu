@@ -1,4 +1,5 @@
-// Contractions against recomputed (checkpointed) Wigner tables, FP64.
+// Contractions against recomputed (checkpointed) Wigner tables: FP64, and at split
+// precision the multiply-adds in double-float.
 //
 // A recomputed table keeps, per m, theta ring t and segment of kSeg degrees,
 // the pair (d^{lc}, d^{lc+1}) = (a, b) 2^E from the double-double recursion

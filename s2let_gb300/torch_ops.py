@@ -5,9 +5,10 @@ leading batch dimension: f is (batch, n_px), f_wav (batch, n_wav), f_scal
 (batch, n_scal) in the reference's MW / wavelet layouts
 (src/c/s2let_analysis.c:456-523, src/c/s2let_synthesis.c:472-539).  Real
 signals use float64 tensors, spin / complex signals complex128; float32 /
-complex64 tensors select the FP32-storage entry points (the same transforms on
-FP64 copies made on the device, the outputs rounded to single precision), and
-the outputs and gradients keep the input's precision.
+complex64 tensors select the FP32-storage entry points (the same transforms, the
+inputs widened to FP64 as they are read and the outputs rounded to single
+precision as they are written), and the outputs and gradients keep the input's
+precision.
 
 Backward passes run the hand-written adjoint kernels
 (s2let_gpu_analysis_adjoint_wav2px*_batch, s2let_gpu_synthesis_adjoint_px2wav*_batch),
