@@ -178,13 +178,12 @@ def measured_peaks():
 
 # DRAM traffic / algorithmic bytes per launch of the dominant kernel, from one
 # ncu capture each (DRAM bytes over the bytes the launch must move):
-# profiles/fp64_contraction_L512_N4_batch8.md (traffic grows with the table
-# size, so the ratio carries to the L=1024 launches) and
-# profiles/ring_gamma_fixed_point_L1024_N4_one_map.md (the fused ring + gamma DFT
-# launches that carry most of the ring-DFT bytes: 0.650 GB of DRAM traffic for
-# 0.738 GB of spectra and gamma slices, both directions of one map's two bl=1024
-# scales; the rest stays in L2)
-TRAFFIC_RATIO = {"fp64_contraction": 1.126, "ring_dft": 0.881}
+# k_contract<0, 8> at L=512, N=4, 8 maps (1.322 GB for 1.174 GB; traffic grows with
+# the table size, so the ratio carries to the L=1024 launches), and the fused ring
+# and gamma DFTs at L=512, N=4, 8 maps, two scales in one launch, whose spectra (268
+# MB) exceed L2 (0.688 and 0.713 GB, synthesis and analysis, for 0.738 GB of spectra
+# and gamma slices each)
+TRAFFIC_RATIO = {"fp64_contraction": 1.126, "ring_dft": 0.950}
 
 
 def profile_traffic(kernel, alg_bytes_per_launch):

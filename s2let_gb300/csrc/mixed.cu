@@ -42,8 +42,9 @@
 // bf16 panels in HBM; 32 maps, split precision, 64 columns: 31.1 against 33.5.
 // With a quarter of the MMAs the 16-column launches take 24 % less, without the
 // conversion's stores 10 %, without the combination 4 %: no single unit paces
-// them (DRAM 38 % busy, tensor pipe 17 %); what is left is the latency of 32
-// MMAs of N <= 128 per K-chunk behind one another.
+// them (one map at L = 512, bl = 512: DRAM 51 % busy, tensor pipe 23 %, issue 27-30
+// %); what is left is the latency of 32 MMAs of N <= 128 per K-chunk behind one
+// another.  At 64 columns, 32 maps: DRAM 39 %, tensor pipe 47 %, issue 36 %.
 // Every wait is bounded (about 2 s); on expiry the kernel raises an error flag,
 // drains its own copies and MMAs, frees TMEM and returns.
 #include <chrono>

@@ -1029,7 +1029,8 @@ bool same_form(const T2L &p, const T2L &q) {
 // Split precision: there from band-limit 513; up to 512 by the double-float kernel.
 // That one takes twice the time alone (32 maps of 64 <= L <= 320, one by one: 15.7
 // against 8.3 ms), but it shares the GPU with the other maps of a multi-map call,
-// which the tensor-core kernel's shared memory does not (20.9 against 21.8 ms).
+// which the tensor-core kernel's shared memory does not (20.9 against 21.8 ms).  The
+// rule looks at the band-limit only: calls of one map or one batch take it too.
 constexpr int kQuadDfMaxBl = 512;
 template <class A, class F>
 void quadrature(const A *p, int n, bool trans, F &&io, int64_t is, int iw, int i_mlo, int64_t os, int ow, int o_mlo,
