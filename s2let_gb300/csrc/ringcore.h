@@ -21,10 +21,10 @@
 // and chirp-shaped rings, P = 256 to 8192): at most 0.6 times its error; white
 // rings 5e-17 to 1.2e-16 against 3e-16 to 4e-16.  With one upward shift, between the
 // transforms, the same rings were up to 8 times FP64's error (K = 1023 white 1.7e-15
-// against 8e-16, K = 4095 3.3e-15, chirp-shaped 2e-14).  The shifts and the ORs cost
-// the ring kernels 3 to 4 % (8 maps at L = 1024, N = 4: 5.05 -> 5.26 ms analysis, 5.21
-// -> 5.34 synthesis; 64 at L = 128 0.772 -> 0.815, 0.793 -> 0.818); after every pass
-// 11 to 14 %.
+// against 8e-16, K = 4095 3.3e-15, chirp-shaped 2e-14).  The shifts, the ORs and the
+// rounding of the inverse butterfly cost the ring kernels 4 to 6 % (8 maps at L =
+// 1024, N = 4: 5.05 -> 5.30 ms analysis, 5.21 -> 5.41 synthesis; 64 at L = 128 0.772 ->
+// 0.817, 0.793 -> 0.823); shifts after every pass would cost 11 to 14 %.
 #pragma once
 
 #include "fxarith.h"
@@ -140,10 +140,20 @@ S2G_DI void dit4(longlong2 &a0, longlong2 &a1, longlong2 &a2, longlong2 &a3, int
   a1 = fx_sub(b1, b3);
   a3 = fx_add(b1, b3);
 }
-// inverse butterfly, natural to bit-reversed order, over 4
+// a / 4, rounded to nearest, ties to even
+S2G_DI longlong2 fx_quarter(longlong2 a) {
+  return make_longlong2((a.x + 1 + ((a.x >> 2) & 1)) >> 2, (a.y + 1 + ((a.y >> 2) & 1)) >> 2);
+}
+// inverse butterfly, natural to bit-reversed order, over 4.  a0 is rounded without
+// bias: y_0 is a sum along the a0 of every pass, so a downward shift gave the bin m = 0
+// of every ring an error of the same sign (mean over white rings 2e-16 to 1.4e-15 of
+// the level at P = 512 to 8192, against 1e-16 to 2e-16 in the worst bin of an FP64
+// transform; so 5e-17 at most), and the monopole of a map ten times FP64's error.
+// The forward butterfly's downward shift spreads over all bins (within the same 5e-17).
+// Costs 1 to 2 % of the ring kernels, 2 to 3 % in both butterflies.
 S2G_DI void dif4(longlong2 &a0, longlong2 &a1, longlong2 &a2, longlong2 &a3, int4 w1, int4 w2, int4 w3) {
   const longlong2 b0 = fx_add(a0, a2), b1 = fx_add(a1, a3), b2 = fx_sub(a0, a2), b3 = fx_mul_i(fx_sub(a1, a3));
-  a0 = fx_sar(fx_add(b0, b1), 2);
+  a0 = fx_quarter(fx_add(b0, b1));
   a1 = fx_mulc4(fx_sub(b0, b1), w1);
   a2 = fx_mulc4(fx_add(b2, b3), w2);
   a3 = fx_mulc4(fx_sub(b2, b3), w3);

@@ -35,3 +35,29 @@ def test_rings_of_few_orders(gpu, L, ss, ms):
     seen = level > 1e-200  # near the poles high orders underflow
     assert seen.sum() > 10
     assert (err[seen] / level[seen]).max() < 1e-15
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("table_mode", [1, 2])
+@pytest.mark.parametrize("L", [128, 512, 1024])
+def test_monopole_of_white_maps(gpu, L, table_mode):
+    """Rounding errors of one sign in every ring would add up in the monopole.  Bound
+    1e-14 of a coefficient's level: the worst degree of an FP64 transform of such
+    maps is 4e-15 off at L = 1024."""
+    rng = np.random.default_rng(L)
+    l = np.repeat(np.arange(L), 2 * np.arange(L) + 1)
+    m = np.arange(L * L) - l * l - l
+    flm = (rng.normal(size=L * L) + 1j * rng.normal(size=L * L)) / np.sqrt(2)
+    neg, mir = m < 0, l * l + l - m
+    flm[m == 0] = flm[m == 0].real * np.sqrt(2)
+    flm[neg] = (-1.0) ** m[neg] * np.conj(flm[mir[neg]])
+    flm[0] = 0.0
+    lib = gpu.lib
+    lib.s2let_gpu_release_plans()
+    try:
+        assert lib.s2let_gpu_set_table_mode(table_mode) == 0
+        back = gpu.sht(0, gpu.sht(1, flm, L, 0, True), L, 0, True)
+    finally:
+        lib.s2let_gpu_set_table_mode(0)
+        lib.s2let_gpu_release_plans()
+    assert abs(back[0]) < 1e-14

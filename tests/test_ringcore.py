@@ -94,8 +94,38 @@ double err(const std::vector<cd> &y, const vec<long double> &r) {
   }
   return (double)sqrtl(e / n);
 }
+// largest mean error of any bin over n white rings, over the rms level of a bin
+int mean_error(int K, int n) {
+  const RingTables t = ring_tables(K);
+  std::mt19937_64 g(K);
+  std::normal_distribution<double> nd;
+  vec<long double> fixed(K), fp64(K);
+  for (int r = 0; r < n; ++r) {
+    std::vector<cd> x(K);
+    vec<long double> xl(K);
+    for (int k = 0; k < K; ++k) {
+      x[k] = cd(nd(g), nd(g));
+      xl[k] = {x[k].real(), x[k].imag()};
+    }
+    const auto ref = bluestein_ref<long double>(xl, t.P);
+    const auto a = fixed_point(x, t), b = bluestein_ref<double>(x, t.P);
+    for (int k = 0; k < K; ++k) {
+      fixed[k] += std::complex<long double>(a[k].real(), a[k].imag()) - ref[k];
+      fp64[k] += std::complex<long double>(b[k].real(), b[k].imag()) - ref[k];
+    }
+  }
+  long double m[2] = {0, 0};
+  for (int k = 0; k < K; ++k) {
+    m[0] = std::max(m[0], std::abs(fixed[k]));
+    m[1] = std::max(m[1], std::abs(fp64[k]));
+  }
+  const long double scale = n * sqrtl(2.0L * K);
+  std::printf("mean %.3e %.3e\n", (double)(m[0] / scale), (double)(m[1] / scale));
+  return 0;
+}
 int main(int argc, char **argv) {
   const int K = atoi(argv[1]);
+  if (argc > 2) return mean_error(K, atoi(argv[2]));
   const RingTables t = ring_tables(K);
   std::mt19937_64 g(K);
   std::normal_distribution<double> nd;
@@ -170,3 +200,13 @@ def test_not_less_accurate_than_fp64(harness, K):
         # an FP64 transform may be exact on a ring (a spike at its first sample); half a
         # unit of the rounded outputs is always allowed
         assert float(fixed) <= max(float(fp64), 2.0 ** -53), line
+
+
+@pytest.mark.parametrize("K", [255, 511, 1023, 1024, 2047, 4095])
+def test_no_bias(harness, K):
+    """Errors of one sign in one bin of every ring add up over a map; an FP64
+    transform's mean error (of its constants, and of 100 rings) is the bound."""
+    out = subprocess.run([harness, str(K), "100"], capture_output=True, text=True)
+    assert out.returncode == 0, out.returncode
+    _, fixed, fp64 = out.stdout.split()
+    assert float(fixed) <= float(fp64), out.stdout
