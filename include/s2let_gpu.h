@@ -471,8 +471,8 @@ int s2let_gpu_get_df_max_maps(void);
  *       tables take a few MB and are shared by all plans): the kernels
  *       regenerate the Wigner d values from double-double checkpoints every 64
  *       degrees (≈ 1/50 of the memory) and apply the forward quadrature as a
- *       separate operator (on the tensor cores in eight digit slices, or in
- *       double-float at split precision up to band-limit 512).
+ *       separate operator (FP64; at split precision in double-float up to
+ *       band-limit 512, on the tensor cores in eight digit slices above).
  * Returns the status. */
 int s2let_gpu_set_table_mode(int mode);
 int s2let_gpu_get_table_mode(void);

@@ -43,7 +43,7 @@ bool contract_t2l_mixed(const T2L *a, int nparts, cudaStream_t st);
 
 // The quadrature operator W_eps(m) (trans: its transpose) of a recomputed table's
 // grid on the ring spectra of n <= kMaxParts problems, m in [mlo, mhi]: in eight
-// digit slices, with FP64 rounding error in both modes; false as above.
+// digit slices; false as above.
 struct QuadIO {
   const double2 *in;
   double2 *out;

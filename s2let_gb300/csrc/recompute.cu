@@ -1034,13 +1034,18 @@ bool same_form(const T2L &p, const T2L &q) {
          p.wscale == q.wscale && p.wconj == q.wconj && p.ys == q.ys && p.nb == q.nb;
 }
 
-// Quadrature of n problems, as many of one m range as a pass takes.  FP64 mode: on
-// the tensor cores (the FP64 kernel competes with the recursion for the FP64 pipe).
-// Split precision: there from band-limit 513; up to 512 by the double-float kernel.
-// That one takes twice the time alone (32 maps of 64 <= L <= 320, one by one: 15.7
-// against 8.3 ms), but it shares the GPU with the other maps of a multi-map call,
-// which the tensor-core kernel's shared memory does not (20.9 against 21.8 ms).  The
-// rule looks at the band-limit only: calls of one map or one batch take it too.
+// Quadrature of n problems, as many of one m range as a pass takes.
+// FP64 mode: the FP64 kernel.  Eight slices on the tensor cores are faster, but the
+// operator's rows are peaked (the largest entry, on the diagonal, stands far above the
+// rest), and slices err relative to it: forward transforms of white maps at L = 512 and
+// 700 came out 1.2 and 1.3 times as far off (at L = 128 1.07), while on the Wigner
+// tables, whose rows oscillate at one level, slices are the more accurate.
+// Split precision: on the tensor cores from band-limit 513; up to 512 by the
+// double-float kernel.  That one takes twice the time alone (32 maps of 64 <= L <= 320,
+// one by one: 15.7 against 8.3 ms), but it shares the GPU with the other maps of a
+// multi-map call, which the tensor-core kernel's shared memory does not (20.9 against
+// 21.8 ms).  The rule looks at the band-limit only: calls of one map or one batch take
+// it too.
 constexpr int kQuadDfMaxBl = 512;
 template <class A, class F>
 void quadrature(const A *p, int n, bool trans, F &&io, int64_t is, int iw, int i_mlo, int64_t os, int ow, int o_mlo,
@@ -1051,7 +1056,7 @@ void quadrature(const A *p, int n, bool trans, F &&io, int64_t is, int iw, int i
     int k = 0;
     for (; k < kMaxParts && i0 + k < n && p[i0 + k].mlo == p[i0].mlo && p[i0 + k].mhi == p[i0].mhi; ++k)
       io(i0 + k, &q[k].in, &q[k].out);
-    const bool tensor = t_precision == 0 || tb.bl > kQuadDfMaxBl;
+    const bool tensor = t_precision == 1 && tb.bl > kQuadDfMaxBl;
     if (!tensor || !quadrature_mixed(tb, trans, q, k, p[i0].mlo, p[i0].mhi, is, iw, i_mlo, os, ow, o_mlo, p[0].nb, st)) {
       WItems w{};
       w.n = k;
