@@ -14,8 +14,8 @@
 // 45 adds and shifts, against 256 FP32 instructions in double-float and 32
 // FP64 instructions at 1/64 rate.  Measured, px2wav + wav2px at L = 1024, N = 4
 // (real maps), rings and gamma DFTs: 2 maps in FP64 19.2 ms with FP64
-// butterflies, 3.2 ms so; 32 maps at split precision 60.6 ms in double-float,
-// 47 ms so.
+// butterflies, 3.3 ms so; 32 maps at split precision 60.6 ms in double-float,
+// 47.7 ms so.
 //
 // Table data comes as 62-bit fixed point (RingFFT, plan.h): chirp exp(i pi k^2
 // / K), the passes' twiddles level by level (the passes below the first read
