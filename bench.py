@@ -907,7 +907,7 @@ def run_recompute_workload(a, world, rank, local):
             "metric": "px2wav+wav2px maps/s at L=2048, N=4 (recomputed Wigner tables, split precision)",
             "per_kernel_ms_per_step": bd,
             "value": whole_job_rate(1, world, ms * 1e-3), "ms_per_step": ms,
-            "dtype": "double-float recomputed-table contractions, 64-bit fixed-point ring DFTs, FP64 quadrature",
+            "dtype": "double-float recomputed-table contractions and quadrature, 64-bit fixed-point ring DFTs",
             "fp64_path": {"value": whole_job_rate(1, world, ms64 * 1e-3), "ms_per_step": ms64,
                           "max_rel_err_round_trip": err64, "per_kernel_ms_per_step": bd64},
             "max_rel_err_f_wav_vs_fp64": float(((w - w64).abs().max() / w64.abs().max()).item()),

@@ -86,10 +86,17 @@ __device__ __forceinline__ void dot2_mac(float &s, float &c, float2 av, float xh
   c = __fmaf_rn(av.x, xl, c);
   c = __fmaf_rn(av.y, xh, c);
 }
-// complex sums (re.s, re.c, im.s, im.c) += v x
-__device__ __forceinline__ void dot2_cmac(float4 &s, float2 v, float4 x) {
-  dot2_mac(s.x, s.y, v, x.x, x.y);
-  dot2_mac(s.z, s.w, v, x.z, x.w);
+// a + b renormalised (fast two-sum of the result: |lo| <= ulp(hi) / 2), for
+// accumulators summing many terms, where the unnormalised lo would grow
+__device__ __forceinline__ float2 df_add_norm(float2 a, float2 b) {
+  const float2 s = df_add(a, b);
+  const float h = __fadd_rn(s.x, s.y);
+  return make_float2(h, __fsub_rn(s.y, __fsub_rn(h, s.x)));
+}
+// s += v x (double-float real times complex), the accumulator renormalised
+// after each add
+__device__ __forceinline__ void df_mac(float4 &s, float2 v, float4 x) {
+  s = dmk(df_add_norm(dre(s), df_mul(v, dre(x))), df_add_norm(dim_(s), df_mul(v, dim_(x))));
 }
 
 }  // namespace

@@ -408,7 +408,10 @@ __global__ void __launch_bounds__(kRcT) k_rc_t2l(const __grid_constant__ RcArgs 
 // lower rescaling threshold (2^kRenormDf) so that they stay in the float
 // range.  Coefficients (l -> t) and spectra (t -> l) enter as double-float
 // scaled by the largest power of two of their block (segment or tile, per
-// map).  The sums are Dot2 sums (dfarith.h).
+// map).  The sums are renormalised after every term: Dot2 sums (dfarith.h), 12
+// instructions a term instead of 15, gather their corrections in single precision and
+// came out 3 to 8 times as far off over 32 to 128 terms of one sign (df_mac 4e-15 to
+// 8e-15, emulated).
 // ---------------------------------------------------------------------------
 
 constexpr int kRenormDf = 60;
@@ -483,8 +486,8 @@ __global__ void __launch_bounds__(kRcT) k_rc_l2t_df(const __grid_constant__ RcAr
 #pragma unroll
         for (int b = 0; b < NBT; ++b) {
           sum[b] = make_float4(0.f, 0.f, 0.f, 0.f);
-          dot2_cmac(sum[b], dvp, sx[0][b]);
-          if (n > 1) dot2_cmac(sum[b], dv, sx[1][b]);
+          df_mac(sum[b], dvp, sx[0][b]);
+          if (n > 1) df_mac(sum[b], dv, sx[1][b]);
         }
       }
       for (int i = 1; i + 1 < n; ++i) {
@@ -507,7 +510,7 @@ __global__ void __launch_bounds__(kRcT) k_rc_l2t_df(const __grid_constant__ RcAr
         }
         const float2 dv = df_of(v);
 #pragma unroll
-        for (int b = 0; b < NBT; ++b) dot2_cmac(sum[b], dv, sx[i + 1][b]);
+        for (int b = 0; b < NBT; ++b) df_mac(sum[b], dv, sx[i + 1][b]);
       }
 #pragma unroll
       for (int b = 0; b < NBT; ++b) {
@@ -632,7 +635,7 @@ __global__ void __launch_bounds__(kRcT) k_rc_t2l_df(const __grid_constant__ RcAr
     for (int tl = tl_lo; tl < tl_hi; ++tl) {
       const float2 d = tile[tl * kTileLd + li];
 #pragma unroll
-      for (int j = 0; j < NH; ++j) dot2_cmac(sum[j], d, sg[tl * NBT + (SPLIT_T ? 0 : bh * NH) + j]);
+      for (int j = 0; j < NH; ++j) df_mac(sum[j], d, sg[tl * NBT + (SPLIT_T ? 0 : bh * NH) + j]);
     }
 #pragma unroll
     for (int j = 0; j < NH; ++j) {
@@ -759,8 +762,8 @@ __global__ void __launch_bounds__(256) k_apply_w(const double *__restrict__ Wp, 
 // The same operator in double-float (split-precision path).  Per K-slab of
 // AWD_K: W values as double-float pairs (unscaled: the operator's entries sit
 // well inside the float range), each real column's slab as double-float
-// scaled by its largest power of two; the slab's partial sums (Dot2) are flushed
-// into FP64 accumulators with that power of two.  12 FP32 instructions per
+// scaled by its largest power of two; the slab's partial sums are flushed
+// into FP64 accumulators with that power of two.  15 FP32 instructions per
 // multiply-add against one FP64 instruction at 1/64 of the rate.
 constexpr int AWD_K = 32;
 __global__ void __launch_bounds__(256) k_apply_w_df(const double *__restrict__ Wp, const double *__restrict__ Wm, int trans,
@@ -816,7 +819,7 @@ __global__ void __launch_bounds__(256) k_apply_w_df(const double *__restrict__ W
       sB[kk][cc] = df_split(*reinterpret_cast<const double *>(&sB[kk][cc]), sBe[cc]);
     }
     __syncthreads();
-    float2 sum[4][4];  // Dot2 sums (s, c)
+    float2 sum[4][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -831,7 +834,7 @@ __global__ void __launch_bounds__(256) k_apply_w_df(const double *__restrict__ W
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) dot2_mac(sum[i][j].x, sum[i][j].y, x[i], y[j].x, y[j].y);
+        for (int j = 0; j < 4; ++j) sum[i][j] = df_add_norm(sum[i][j], df_mul(x[i], y[j]));
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {

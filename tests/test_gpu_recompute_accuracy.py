@@ -49,3 +49,32 @@ def test_large_band_limits(gpu, L, spin, inv, fwd):
     e = errors(gpu, L, spin)
     assert e[0] <= inv
     assert e[1] <= fwd
+
+
+@pytest.mark.gpu
+def test_split_precision(gpu):
+    """The double-float sums: white maps, and a constant map, whose sums have one sign.
+    Bounds: the errors with sums renormalised after every term (geometric mean over the
+    band-limits, rings and recursion of the time included)."""
+    lib = gpu.lib
+    e = []
+    for L in (64, 70, 96, 100, 128, 150, 181, 200, 256, 300, 384, 512):
+        rng = np.random.default_rng(L)
+        flm = rng.normal(size=L * L) + 1j * rng.normal(size=L * L)
+        f00 = 0.7 * np.sqrt(4 * np.pi)
+        try:
+            lib.s2let_gpu_release_plans()
+            assert lib.s2let_gpu_set_table_mode(1) == 0
+            f = gpu.sht(1, flm, L, 0, False)
+            lib.s2let_gpu_release_plans()
+            assert lib.s2let_gpu_set_table_mode(2) == 0 and lib.s2let_gpu_set_precision(1) == 0
+            inv, fwd = gpu.sht(1, flm, L, 0, False), gpu.sht(0, f, L, 0, False)
+            const = gpu.sht(0, np.full(L * (2 * L - 1), 0.7), L, 0, True)
+        finally:
+            lib.s2let_gpu_set_precision(0)
+            lib.s2let_gpu_set_table_mode(0)
+            lib.s2let_gpu_release_plans()
+        const[0] -= f00
+        e.append([np.linalg.norm(inv - f) / np.linalg.norm(f), np.linalg.norm(fwd - flm) / np.linalg.norm(flm),
+                  np.linalg.norm(const) / f00])
+    assert (np.exp(np.log(e).mean(axis=0)) <= [2.37e-14, 1.94e-14, 1.66e-14]).all()
