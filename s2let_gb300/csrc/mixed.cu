@@ -1472,12 +1472,13 @@ bool run_problem(const Problem &p, cudaStream_t st) {
   {
     std::lock_guard<std::mutex> lk(g_mx_mu);
     pr.s = sliced(*p.tb, p.kind, p.eighth, st);
-    if (pr.s) pr.L = tile_list(*pr.s, p.n, p.mlo, p.mhi, pr.lmin, p.eighth, st);
-    if (!pr.L) return false;
-    pr.err = error_flag();
-    ++pr.s->users;
+    if (!pr.s) return false;
+    ++pr.s->users;  // before anything else is allocated
     user.s = pr.s;
     if (!p.eighth) pr.s->forward7 = true;
+    pr.L = tile_list(*pr.s, p.n, p.mlo, p.mhi, pr.lmin, p.eighth, st);
+    if (!pr.L) return false;
+    pr.err = error_flag();
     if (capturing(st)) pr.s->captured = true;
   }
   return p.eighth ? run_shapes<kSmax>(p, pr, st) : run_shapes<kS>(p, pr, st);
