@@ -196,3 +196,53 @@ def test_switched_off_after_they_were_built(gpu, lib):
     lib.s2let_gpu_set_split_tables(1)
     (w2, s2), n = _slicings(lib, lambda: gpu.px2wav(f, p, real=True))
     assert n > 0 and np.array_equal(w2, w1) and np.array_equal(s2, s1)
+
+
+@pytest.mark.gpu
+def test_given_back_beside_other_threads(gpu, lib):
+    """Calls refused for want of memory take panels back while three threads build and
+    use them; panels in use stay, the others' contractions go to the FP64 kernels."""
+    import threading
+
+    torch = pytest.importorskip("torch")
+    sizes = [64, 70, 80, 90, 100, 110, 120, 128, 130, 140]
+    maps, ref = {}, {}
+    for L in sizes:
+        p = make_parameters(L, 2.0, 4, 2, 0, 0)
+        maps[L] = (p, np.random.default_rng(L).normal(size=gpu.sizes(p)["n_px"]))
+        ref[L] = gpu.px2wav(maps[L][1], p, real=True)[0]
+    lib.s2let_gpu_release_plans()
+    bad, done = [], threading.Event()
+
+    def transform(order):
+        for L in order * 3:
+            p, f = maps[L]
+            w, _ = gpu.px2wav(f, p, real=True)
+            if lib.s2let_gpu_last_error() != 0 or rel_err(w, ref[L]) > TOL:
+                bad.append(L)
+
+    p = make_parameters(48, 2.0, 2, 3, 0, 0)
+    sz = gpu.sizes(p)
+    f, w, s = (torch.zeros(sz[k], dtype=torch.float64, device="cuda") for k in ("n_px", "n_wav", "n_scal"))
+    st = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+    def exhaust():
+        while not done.is_set():
+            rc = lib.s2let_gpu_analysis_px2wav_real_batch(C.c_void_p(w.data_ptr()), C.c_void_p(s.data_ptr()),
+                                                          C.c_void_p(f.data_ptr()), 20_000_000, C.byref(p), st)
+            if rc != 4:
+                bad.append(rc)
+            time.sleep(0.01)
+
+    lib.s2let_gpu_last_error()
+    threads = [threading.Thread(target=transform, args=(sizes[k:] + sizes[:k],)) for k in (0, 3, 6)]
+    other = threading.Thread(target=exhaust)
+    other.start()
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    done.set()
+    other.join()
+    assert not bad
+    assert lib.s2let_gpu_refused_tables() > 0
